@@ -338,7 +338,7 @@ int sv_batch_size(sv_batch* batch, int* n_members, uint64_t* device_bytes);
  * counterpart in the reference. It is for callers that must not allocate after start-up: a
  * host framework that owns every device allocation through its own pool and hands the solver
  * only pre-allocated buffers, or a real-time loop in which a cudaMalloc would synchronise the
- * device. Working memory is a fixed array inside this library (about 5.2 MB, held by every
+ * device. Working memory is a fixed array inside this library (about 4.6 MB, held by every
  * GPU that loads the library until the process exits), which limits the mesh to 65536 cells
  * (256 x 256); larger meshes return SV_E_LIMIT.
  *   inputs  (device, FP64, nx*ny each): z, h, u, v = U_[0]

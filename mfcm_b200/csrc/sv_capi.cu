@@ -362,7 +362,7 @@ struct Solver final : public sv_ctx {
     SV_CUDA(alloc(&fc, 1));
     long long maxp = vol_nblk;
     for (int v = 0; v < svk::kNumVariants; ++v) maxp = std::max(maxp, svk::variant_partials(v, m->nx, m->ny));
-    SV_CUDA(alloc(&part, size_t(svk::part_count(maxp, N))));
+    SV_CUDA(alloc(&part, size_t(svk::part_count(maxp))));
     SV_CUDA(alloc(&scalar, 4));
     Ctl c{};
     c.dt = p->initial_dt;
@@ -753,8 +753,6 @@ struct Solver final : public sv_ctx {
     F.ctl = ctl;
     F.part = part;
     F.nblk = nblk;
-    F.nstages = N;
-    for (int j = 0; j < 4; ++j) F.b[j] = j < N ? tab.b(j + 1) : 0.0;
     F.cn_target = prm.cn_target;
     F.max_dt = prm.max_dt;
     F.L = prm.step_duration;
@@ -1174,7 +1172,7 @@ struct Batch final : public sv_batch_base {
   int* d_done = nullptr;                    // [nact]
   svk::StepQueue* d_queue = nullptr;        // [nact] steps queued by the current advance
   int nact = 0, cap = 0;
-  long long total_tiles = 0;
+  long long total_tiles = 0, max_nblk = 0;  // partial slots of all members, of the largest one
   bool p2 = true, eddy = false, dirty = true;
   std::vector<int> active;                  // slot ids in launch order
   std::vector<unsigned long long> versions; // members' pversion at the last rebuild
@@ -1309,6 +1307,7 @@ struct Batch final : public sv_batch_base {
     std::vector<Ctl*> hc(std::max(nact, 1));
     p2 = true;
     eddy = false;
+    max_nblk = 0;
     for (int k = 0; k < nact; ++k) {
       Solver<T>* m = members[active[k]];
       // the tile prefix and the partials follow the batch kernel's decomposition
@@ -1318,6 +1317,7 @@ struct Batch final : public sv_batch_base {
         if (rs) return fail(rs, "member " + std::to_string(active[k]) + ": " + m->err);
       }
       ht[k + 1] = ht[k] + m->nblk;
+      max_nblk = std::max(max_nblk, m->nblk);
       int e2;
       p2 = p2 && std::frexp(m->mesh.dx, &e2) == 0.5 && std::frexp(m->mesh.dy, &e2) == 0.5;
       eddy = eddy || m->eddy_mode != SV_EDDY_OFF;
@@ -1351,7 +1351,7 @@ struct Batch final : public sv_batch_base {
                                                        eddy, stream);
       if (e != cudaSuccess) return cuda_fail(e, "batched stage kernel");
     }
-    cudaError_t e = svk::launch_finalize_batch(d_fin, nact, stream);
+    cudaError_t e = svk::launch_finalize_batch(d_fin, nact, max_nblk, stream);
     if (e != cudaSuccess) return cuda_fail(e, "batched finalize kernel");
     return SV_OK;
   }

@@ -8,14 +8,30 @@
 
 namespace svk {
 
-cudaError_t launch_finalize(const FinalizeParams& F, cudaStream_t s) {
-  finalize_kernel<1024><<<1, 1024, 0, s>>>(F);
-  return cudaGetLastError();
+// The finalize kernels with CTAS blocks per solver, as clusters when there are several.
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_clusters(void (*kern)(KArgs...), int solvers, int ctas, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(solvers * ctas));
+  cfg.blockDim = dim3(kFinalizeThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(ctas);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = ctas > 1 ? attr : nullptr;
+  cfg.numAttrs = ctas > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
 }
-cudaError_t launch_finalize_batch(const FinalizeParams* Fs, int ninst, cudaStream_t s) {
+cudaError_t launch_finalize(const FinalizeParams& F, cudaStream_t s) {
+  if (F.nblk > kFinalizeClusterSlots) return launch_clusters(finalize_kernel<kFinalizeCtas>, 1, kFinalizeCtas, s, F);
+  return launch_clusters(finalize_kernel<1>, 1, 1, s, F);
+}
+cudaError_t launch_finalize_batch(const FinalizeParams* Fs, int ninst, long long max_nblk, cudaStream_t s) {
   if (ninst <= 0) return cudaSuccess;
-  finalize_batch_kernel<1024><<<ninst, 1024, 0, s>>>(Fs);
-  return cudaGetLastError();
+  if (max_nblk > kFinalizeClusterSlots)
+    return launch_clusters(finalize_batch_kernel<kFinalizeCtas>, ninst, kFinalizeCtas, s, Fs);
+  return launch_clusters(finalize_batch_kernel<1>, ninst, 1, s, Fs);
 }
 cudaError_t launch_begin_queue(const FinalizeParams* Fs, int n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;

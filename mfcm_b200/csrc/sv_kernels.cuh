@@ -13,10 +13,14 @@
 //  debug kernels  the same per-face / per-cell functions over global arrays, one reference
 //                 kernel each, for per-function parity tests.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "sv_device.cuh"
 
 namespace svk {
 using namespace svd;
+
+constexpr unsigned kFull = 0xffffffffu;  // every lane of a warp
 
 // Device-resident controller state of one solver (FP64 times, TT = double).
 struct Ctl {
@@ -112,9 +116,23 @@ template <typename T> struct StageParams {
   T* pslp[6];
 };
 
-// partial layout: [0, nblk) cn max, [nblk, 2nblk) cn min, [2nblk, 3nblk) volume,
-// then rain[s] at (3 + 3s) nblk, outflow[s] at (4 + 3s) nblk, wall flow[s] at (5 + 3s) nblk.
-__host__ __device__ inline long long part_count(long long nblk, int nstages) { return (3 + 3LL * nstages) * nblk; }
+// partial layout: [0, nblk) cn max, [nblk, 2nblk) cn min, [2nblk, 3nblk) volume, then the
+// rain, outflow and wall-flow tallies at 3, 4 and 5 nblk. A block's (or warp's) tally slot
+// carries the weighted sum over the stages so far, sum_s b_s dt * tally_s, so the finalize
+// reads three tally arrays however many stages there are: at 4096 x 4096 and four stages 0.9 MB
+// instead of 2.3 MB.
+constexpr int kParts = 6;
+__host__ __device__ inline long long part_count(long long nblk) { return kParts * nblk; }
+// Adds one stage's tallies, weighted by b_s dt in the solver's value type, to slot `i`.
+template <typename T>
+__device__ __forceinline__ void store_tallies(const StageParams<T>& P, long long i, double rain, double removed,
+                                              double wall, bool first, double dt) {
+  const double w = double(T(P.b[P.stage] * dt));
+  double* p = P.part + 3 * P.nblk + i;
+  p[0] = first ? w * rain : p[0] + w * rain;
+  p[P.nblk] = first ? w * removed : p[P.nblk] + w * removed;
+  p[2 * P.nblk] = first ? w * wall : p[2 * P.nblk] + w * wall;
+}
 
 template <typename T> __device__ __forceinline__ T ld(const T* p, long long i) { return __ldg(p + i); }
 // Loads of the state, stage and accumulator buffers. A launch that writes and later reads them
@@ -608,11 +626,7 @@ __device__ __forceinline__ void stage_tile(const StageParams<T>& P, int bx, int 
     double rs = block_sum<NT>(rain, s.red);
     double os = block_sum<NT>(removed, s.red);
     double ws = block_sum<NT>(walls, s.red);
-    if (tid == 0) {
-      P.part[(3 + 3LL * P.stage) * P.nblk + blk] = rs;
-      P.part[(4 + 3LL * P.stage) * P.nblk + blk] = os;
-      P.part[(5 + 3LL * P.stage) * P.nblk + blk] = ws;
-    }
+    if (tid == 0) store_tallies(P, blk, rs, os, ws, first, dt_d);
   }
 }
 
@@ -688,7 +702,6 @@ __global__ void __launch_bounds__(TX * TY, MINB)
 // slopes that need it, and there is no block-level barrier. The arithmetic per face and
 // per cell is the same function as in the tiled kernel.
 // ---------------------------------------------------------------------------------------
-constexpr unsigned kFull = 0xffffffffu;
 template <typename T> __device__ __forceinline__ T up1(T v) { return __shfl_up_sync(kFull, v, 1); }
 template <typename T> __device__ __forceinline__ T dn1(T v) { return __shfl_down_sync(kFull, v, 1); }
 
@@ -998,11 +1011,7 @@ __device__ __forceinline__ void sweep_strip(const StageParams<T>& P, long long g
   }
   if (P.mode & M_TALLY) {
     double rs = warp_sum<T>(rain), os = warp_sum<T>(removed), ws = warp_sum<T>(walls);
-    if (lane == 0) {
-      P.part[(3 + 3LL * P.stage) * P.nblk + gw] = rs;
-      P.part[(4 + 3LL * P.stage) * P.nblk + gw] = os;
-      P.part[(5 + 3LL * P.stage) * P.nblk + gw] = ws;
-    }
+    if (lane == 0) store_tallies(P, gw, rs, os, ws, first, dt_d);
   }
 }
 
@@ -1205,11 +1214,7 @@ __device__ __forceinline__ void sweep_strip_interior(const StageParams<T>& P, lo
   }
   if (P.mode & M_TALLY) {
     double rs = warp_sum<T>(rain), os = warp_sum<T>(removed), ws = warp_sum<T>(walls);
-    if (lane == 0) {
-      P.part[(3 + 3LL * P.stage) * P.nblk + gw] = rs;
-      P.part[(4 + 3LL * P.stage) * P.nblk + gw] = os;
-      P.part[(5 + 3LL * P.stage) * P.nblk + gw] = ws;
-    }
+    if (lane == 0) store_tallies(P, gw, rs, os, ws, first, dt_d);
   }
 }
 
@@ -1453,12 +1458,8 @@ __device__ __forceinline__ void sweep_pair_interior(const StageParams<float>& P,
   if (P.mode & M_TALLY) {
     double rs = warp_sum<T>(rain), os = warp_sum<T>(removed), ws = warp_sum<T>(walls);
     if (lane == 0) {
-      P.part[(3 + 3LL * P.stage) * P.nblk + gw] = rs;
-      P.part[(4 + 3LL * P.stage) * P.nblk + gw] = os;
-      P.part[(5 + 3LL * P.stage) * P.nblk + gw] = ws;
-      P.part[(3 + 3LL * P.stage) * P.nblk + gw + 1] = 0.0;
-      P.part[(4 + 3LL * P.stage) * P.nblk + gw + 1] = 0.0;
-      P.part[(5 + 3LL * P.stage) * P.nblk + gw + 1] = 0.0;
+      store_tallies(P, gw, rs, os, ws, first, dt_d);
+      store_tallies(P, gw + 1, 0.0, 0.0, 0.0, first, dt_d);
     }
   }
 }
@@ -1606,8 +1607,6 @@ struct FinalizeParams {
   DevForcing* fc;    // batch members: the member's forcing slot read by its stage kernels
   const double* part;
   long long nblk;
-  int nstages;
-  double b[4];
   double cn_target, max_dt, L;
   double cell_area;
   int auto_mode;   // 1: accept/repeat, advance t_local, trim dt (TemporalScheme.hpp:119-146)
@@ -1633,46 +1632,85 @@ template <int NT> __device__ double fixed_sum(const double* p, long long n, doub
 __device__ __forceinline__ void finalize_control(const FinalizeParams& F, double mx, double mn, double vol,
                                                  double rain, double outf, double wall);
 
-template <int NT> __device__ __forceinline__ void finalize_body(const FinalizeParams& F, double* red) {
-  Ctl* ctl = F.ctl;
-  if (ctl->done) return;
-  // CFL max / min (NaN-propagating), order-independent
-  double mx = 0.0, mn = 1.0 / 0.0;
-  for (long long i = threadIdx.x; i < F.nblk; i += NT) {
-    mx = nmax(mx, F.part[i]);
-    mn = nmin(mn, F.part[F.nblk + i]);
+// The six reductions of a timestep's finalize over the partial slots.
+struct Reduced {
+  double mx, mn, vol, rain, outf, wall;
+  __device__ __forceinline__ void init() {
+    mx = vol = rain = outf = wall = 0.0;
+    mn = 1.0 / 0.0;
   }
-  red[threadIdx.x] = mx;
-  __syncthreads();
-  for (int st = NT / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) red[threadIdx.x] = nmax(red[threadIdx.x], red[threadIdx.x + st]);
-    __syncthreads();
+  __device__ __forceinline__ void add(const Reduced& o) {
+    mx = nmax(mx, o.mx);  // CFL max and min: NaN-propagating, order-independent
+    mn = nmin(mn, o.mn);
+    vol += o.vol;
+    rain += o.rain;
+    outf += o.outf;
+    wall += o.wall;
   }
-  mx = red[0];
-  __syncthreads();
-  red[threadIdx.x] = mn;
-  __syncthreads();
-  for (int st = NT / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) red[threadIdx.x] = nmin(red[threadIdx.x], red[threadIdx.x + st]);
-    __syncthreads();
+  __device__ __forceinline__ Reduced down(int o) const {
+    return {__shfl_down_sync(kFull, mx, o),   __shfl_down_sync(kFull, mn, o),   __shfl_down_sync(kFull, vol, o),
+            __shfl_down_sync(kFull, rain, o), __shfl_down_sync(kFull, outf, o), __shfl_down_sync(kFull, wall, o)};
   }
-  mn = red[0];
-  __syncthreads();
-  double vol = fixed_sum<NT>(F.part + 2 * F.nblk, F.nblk, red);
-  double rain = 0.0, outf = 0.0, wall = 0.0;
-  if (F.tally) {
-    for (int s = 0; s < F.nstages; ++s) {
-      double rs = fixed_sum<NT>(F.part + (3 + 3LL * s) * F.nblk, F.nblk, red);
-      double os = fixed_sum<NT>(F.part + (4 + 3LL * s) * F.nblk, F.nblk, red);
-      double ws = fixed_sum<NT>(F.part + (5 + 3LL * s) * F.nblk, F.nblk, red);
-      double w = F.is_float ? double(float(F.b[s] * ctl->dt)) : F.b[s] * ctl->dt;
-      rain += w * rs * F.cell_area;
-      outf += w * os * F.cell_area;
-      wall += w * ws * F.cell_area;
+  // slots t, t + n, t + 2n, ... of the partials, in that order
+  __device__ __forceinline__ void slots(const FinalizeParams& F, long long t, long long n) {
+    init();
+    const double* p = F.part;
+    const long long m = F.nblk;
+    for (long long i = t; i < m; i += n) {
+      Reduced x{p[i], p[m + i], p[2 * m + i], 0.0, 0.0, 0.0};
+      if (F.tally) {
+        x.rain = p[3 * m + i];
+        x.outf = p[4 * m + i];
+        x.wall = p[5 * m + i];
+      }
+      add(x);
     }
   }
+  __device__ __forceinline__ void over_warp() {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) add(down(o));
+  }
+};
+
+// The finalize of one solver by a cluster of CTAS blocks of 1024 threads (CTAS = 1: one block).
+// One pass over the partials, all six quantities at once: a fixed order for a given number of
+// blocks (strided slots per thread, shuffle tree per warp, warps, then blocks), one block
+// barrier and, with several blocks, one cluster barrier. What bounds it is latency: the six
+// separate trees of ten barriers each that this replaces took 27 us for a mesh of a few
+// strips, and one block reading 2.3 MB of partials 82 us at 4096 x 4096.
+constexpr int kFinalizeThreads = 1024;
+// slots above which a cluster of kFinalizeCtas blocks shares the reads: up to two slots per
+// thread one block is faster (no cluster launch, no cluster barrier)
+constexpr long long kFinalizeClusterSlots = 2 * kFinalizeThreads;
+constexpr int kFinalizeCtas = 8;
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+template <int CTAS> __device__ __forceinline__ void finalize_body(const FinalizeParams& F) {
+  __shared__ Reduced warp_sum_[kFinalizeThreads / 32];
+  __shared__ Reduced block_sum_[CTAS];
+  if (F.ctl->done) return;  // the same for every block of the cluster
+  const int rank = CTAS > 1 ? int(blockIdx.x % CTAS) : 0;
+  if constexpr (CTAS > 1) cluster_arrive();
+  Reduced r;
+  r.slots(F, (long long)rank * kFinalizeThreads + threadIdx.x, (long long)CTAS * kFinalizeThreads);
+  r.over_warp();
+  if ((threadIdx.x & 31) == 0) warp_sum_[threadIdx.x >> 5] = r;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    r = warp_sum_[threadIdx.x];
+    r.over_warp();
+  }
+  if constexpr (CTAS > 1) {
+    cluster_wait();  // every block of the cluster runs: block 0's shared memory may be written
+    if (threadIdx.x == 0) *cooperative_groups::this_cluster().map_shared_rank(&block_sum_[rank], 0) = r;
+    cluster_arrive();
+    cluster_wait();
+    if (rank != 0 || threadIdx.x != 0) return;
+    r = block_sum_[0];
+    for (int i = 1; i < CTAS; ++i) r.add(block_sum_[i]);
+  }
   if (threadIdx.x != 0) return;
-  finalize_control(F, mx, mn, vol, rain, outf, wall);
+  finalize_control(F, r.mx, r.mn, r.vol, r.rain * F.cell_area, r.outf * F.cell_area, r.wall * F.cell_area);
 }
 
 // The rest of a timestep's finalize, one thread, from its reductions (CFL max and min over
@@ -1757,18 +1795,17 @@ __device__ __forceinline__ void finalize_control(const FinalizeParams& F, double
   }
 }
 
-template <int NT> __global__ void __launch_bounds__(NT) finalize_kernel(const FinalizeParams F) {
-  __shared__ double red[NT];
-  finalize_body<NT>(F, red);
+template <int CTAS> __global__ void __launch_bounds__(kFinalizeThreads) finalize_kernel(const __grid_constant__ FinalizeParams F) {
+  finalize_body<CTAS>(F);
 }
 
-// Batched finalize: one CTA per instance of a batch.
-template <int NT> __global__ void __launch_bounds__(NT) finalize_batch_kernel(const FinalizeParams* __restrict__ Fs) {
-  __shared__ double red[NT];
+// Batched finalize: CTAS blocks per instance of a batch.
+template <int CTAS>
+__global__ void __launch_bounds__(kFinalizeThreads) finalize_batch_kernel(const FinalizeParams* __restrict__ Fs) {
   __shared__ FinalizeParams Fsh;
-  if (threadIdx.x == 0) Fsh = Fs[blockIdx.x];
+  if (threadIdx.x == 0) Fsh = Fs[blockIdx.x / CTAS];
   __syncthreads();
-  finalize_body<NT>(Fsh, red);
+  finalize_body<CTAS>(Fsh);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1829,68 +1866,20 @@ __global__ void persist_init_kernel(const FinalizeParams* Fs, PersistMember* mem
 }
 #endif
 
-// Fixed-order sum of p[0..n) by one warp, in exactly the order of fixed_sum<NT> (thread t of
-// NT adds p[t], p[t+NT], ..., then a binary tree): red holds NT doubles.
-template <int NT> __device__ double warp_fixed_sum(const double* p, long long n, double* red) {
-  const int lane = threadIdx.x & 31;
-  for (int t = lane; t < NT; t += 32) {
-    double a = 0.0;
-    for (long long i = t; i < n; i += NT) a += p[i];
-    red[t] = a;
-  }
-  __syncwarp();
-  for (int st = NT / 2; st > 0; st >>= 1) {
-    for (int t = lane; t < st; t += 32) red[t] += red[t + st];
-    __syncwarp();
-  }
-  const double r = red[0];
-  __syncwarp();
-  return r;
-}
-template <int NT, bool MAX> __device__ double warp_fixed_ext(const double* p, long long n, double* red) {
-  const int lane = threadIdx.x & 31;
-  for (int t = lane; t < NT; t += 32) {
-    double a = MAX ? 0.0 : 1.0 / 0.0;
-    for (long long i = t; i < n; i += NT) a = MAX ? nmax(a, p[i]) : nmin(a, p[i]);
-    red[t] = a;
-  }
-  __syncwarp();
-  for (int st = NT / 2; st > 0; st >>= 1) {
-    for (int t = lane; t < st; t += 32) red[t] = MAX ? nmax(red[t], red[t + st]) : nmin(red[t], red[t + st]);
-    __syncwarp();
-  }
-  const double r = red[0];
-  __syncwarp();
-  return r;
-}
-
-// finalize_body<1024> by one warp: the same reductions in the same order, then the controller
-__device__ __forceinline__ void finalize_warp(const FinalizeParams& F, double* red) {
-  constexpr int NT = 1024;
-  Ctl* ctl = F.ctl;
-  const double mx = warp_fixed_ext<NT, true>(F.part, F.nblk, red);
-  const double mn = warp_fixed_ext<NT, false>(F.part + F.nblk, F.nblk, red);
-  const double vol = warp_fixed_sum<NT>(F.part + 2 * F.nblk, F.nblk, red);
-  double rain = 0.0, outf = 0.0, wall = 0.0;
-  if (F.tally) {
-    for (int s = 0; s < F.nstages; ++s) {
-      double rs = warp_fixed_sum<NT>(F.part + (3 + 3LL * s) * F.nblk, F.nblk, red);
-      double os = warp_fixed_sum<NT>(F.part + (4 + 3LL * s) * F.nblk, F.nblk, red);
-      double ws = warp_fixed_sum<NT>(F.part + (5 + 3LL * s) * F.nblk, F.nblk, red);
-      double w = F.is_float ? double(float(F.b[s] * ctl->dt)) : F.b[s] * ctl->dt;
-      rain += w * rs * F.cell_area;
-      outf += w * os * F.cell_area;
-      wall += w * ws * F.cell_area;
-    }
-  }
-  if ((threadIdx.x & 31) == 0) finalize_control(F, mx, mn, vol, rain, outf, wall);
+// The finalize of one member by one warp: the same reductions over 32 strided chains (sums
+// agree with the block's to rounding; the CFL max and min, which set dt, are the same values).
+__device__ __forceinline__ void finalize_warp(const FinalizeParams& F) {
+  Reduced r;
+  r.slots(F, threadIdx.x & 31, 32);
+  r.over_warp();
+  if ((threadIdx.x & 31) == 0)
+    finalize_control(F, r.mx, r.mn, r.vol, r.rain * F.cell_area, r.outf * F.cell_area, r.wall * F.cell_area);
   __syncwarp();
 }
 
 template <typename T, bool P2, bool EDDY>
 __global__ void __launch_bounds__(32 * kPersistWarps, 4) persist_batch_kernel(const PersistParams<T> PP) {
   __shared__ __align__(16) StageParams<T> Psh[kPersistWarps];
-  __shared__ double red[kPersistWarps][1024];
   const int lane = threadIdx.x, wib = threadIdx.y;
   const int N = PP.nstages, nact = PP.nact;
   const long long gwarp = (long long)blockIdx.x * kPersistWarps + wib;
@@ -1999,7 +1988,7 @@ __global__ void __launch_bounds__(32 * kPersistWarps, 4) persist_batch_kernel(co
         sweep_strip<T, kPersistRows, P2, EDDY, true>(SP, item);
       __syncwarp();
     } else {
-      finalize_warp(PP.Fs[pick], red[wib]);
+      finalize_warp(PP.Fs[pick]);
     }
     __threadfence();  // release this item's writes before counting it
     int last = 0;

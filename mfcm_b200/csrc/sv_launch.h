@@ -81,7 +81,7 @@ template <typename T> cudaError_t launch_persist(const PersistParams<T>& PP, boo
 cudaError_t launch_persist_init(const FinalizeParams* Fs, PersistMember* mem, const long long* warp_start, int nact,
                                 cudaStream_t s);
 cudaError_t launch_finalize(const FinalizeParams& F, cudaStream_t s);
-cudaError_t launch_finalize_batch(const FinalizeParams* Fs, int ninst, cudaStream_t s);
+cudaError_t launch_finalize_batch(const FinalizeParams* Fs, int ninst, long long max_nblk, cudaStream_t s);
 cudaError_t launch_begin_queue(const FinalizeParams* Fs, int n, cudaStream_t s);
 cudaError_t launch_gather_done(Ctl* const* ctls, int n, int* done, cudaStream_t s);
 cudaError_t launch_sum(const double* p, long long n, double* out, cudaStream_t s);
