@@ -2,7 +2,8 @@
 .so travels with the source tree).
 
 sv_f64.cu is compiled with -fmad=false: the FP64 path must round every multiply and add
-separately, like the reference's CPU arithmetic. sv_f32.cu keeps contraction on.
+separately, like the reference's CPU arithmetic. sv_f32.cu writes its fused multiply-adds out
+(-fmad=false too), so that a cell's FP32 result does not depend on the kernel that computed it.
 """
 import os
 import subprocess
@@ -19,7 +20,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-I", INCLUDE] + ARCH
 UNITS = {
     "sv_f64.cu": ["-fmad=false"],
-    "sv_f32.cu": [],
+    "sv_f32.cu": ["-fmad=false"],
     "sv_capi.cu": [],
     "sv_noalloc.cu": [],
 }

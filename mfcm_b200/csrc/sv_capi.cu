@@ -195,94 +195,62 @@ struct Solver final : public sv_ctx {
     graph_dirty = true; ++pversion;
     return SV_OK;
   }
-  // interior / general strip lists of the column sweep, per strip height (16, 32, 64 rows):
-  // interior strips (whole window inside the mesh, no coded-out bed) run the interior kernel
+  // strip list of the column sweep per strip height: the strips' indices with their classes,
+  // general and edge strips first
   struct Strips {
-    int* d_i = nullptr;
-    int* d_b = nullptr;
-    int ni = 0, nb = 0;
-    // two-cells-per-lane variants (FP32): pairs of adjacent interior strips (first strip of
-    // each, nx even) and the interior strips left out of a pair
-    int* d_p = nullptr;
-    int* d_pi = nullptr;
-    int np = 0, npi = 0;
+    unsigned* d = nullptr;
     bool valid = false;
   };
-  Strips strips_[3];
-  unsigned char* d_sflags = nullptr;
-  static int strips_slot(int rows) { return rows == 16 ? 0 : (rows == 32 ? 1 : 2); }
+  std::map<int, Strips> strips_;
+  unsigned char* d_scls = nullptr;
+  size_t scls_size = 0;
+  int sweep_rows(int v) const { return svk::variant_sweep_rows(v, (long long)mesh.nx, (long long)mesh.ny); }
   void invalidate_strips() {
-    for (Strips& x : strips_) x.valid = false;
+    for (auto& x : strips_) x.second.valid = false;
     graph_dirty = true; ++pversion;
   }
-  // the lists for variant v (a column-sweep variant), built from the bed on the device
+  // the list for variant v (a column-sweep variant), classified from the bed on the device
   int ensure_strips(int v) {
-    const int rows = svk::variant_sweep_rows(v);
+    const int rows = sweep_rows(v);
     if (rows == 0) return SV_OK;
-    Strips& L = strips_[strips_slot(rows)];
+    Strips& L = strips_[rows];
     if (L.valid) return SV_OK;
     const long long n = svk::variant_partials(v, (long long)mesh.nx, (long long)mesh.ny);
-    if (!L.d_i) {
-      SV_CUDA(alloc(&L.d_i, size_t(n)));
-      SV_CUDA(alloc(&L.d_b, size_t(n)));
-      SV_CUDA(alloc(&L.d_p, size_t(n)));
-      SV_CUDA(alloc(&L.d_pi, size_t(n)));
+    if (n >= (1LL << 30)) return fail(SV_E_LIMIT, "mesh has too many sweep strips");
+    if (!L.d) SV_CUDA(alloc(&L.d, size_t(n)));
+    if (size_t(n) > scls_size) {
+      SV_CUDA(alloc(&d_scls, size_t(n)));
+      scls_size = size_t(n);
     }
-    if (!d_sflags)  // sized for the shortest strips, which are the most numerous
-      SV_CUDA(alloc(&d_sflags, size_t(svk::variant_partials(4, (long long)mesh.nx, (long long)mesh.ny))));
-    cudaError_t e = svk::launch_strip_flags<T>(z, int(mesh.nx), int(mesh.ny), rows, n, d_sflags, stream);
-    if (e != cudaSuccess) return cuda_fail(e, "strip flags");
-    std::vector<unsigned char> flags(static_cast<size_t>(n));
-    SV_CUDA(cudaMemcpyAsync(flags.data(), d_sflags, size_t(n), cudaMemcpyDeviceToHost, stream));
+    cudaError_t e = svk::launch_strip_classes<T>(z, int(mesh.nx), int(mesh.ny), mesh.dx, mesh.dy, rows, n, d_scls, stream);
+    if (e != cudaSuccess) return cuda_fail(e, "strip classes");
+    std::vector<unsigned char> cls(static_cast<size_t>(n));
+    SV_CUDA(cudaMemcpyAsync(cls.data(), d_scls, size_t(n), cudaMemcpyDeviceToHost, stream));
     SV_CUDA(cudaStreamSynchronize(stream));
-    std::vector<int> in, bd, pr, pin;
-    for (long long i = 0; i < n; ++i) (flags[size_t(i)] ? in : bd).push_back(int(i));
-    // pairs: strips (2t, 2t+1) of one row band, both interior; their vector loads need an even
-    // row length (every row then starts 8-byte aligned)
-    const long long tiles_x = (static_cast<long long>(mesh.nx) + svk::kSweepOut - 1) / svk::kSweepOut;
-    for (long long i = 0; i < n; ++i) {
-      if (!flags[size_t(i)]) continue;
-      const long long tx = i % tiles_x;
-      if (mesh.nx % 2 == 0 && tx % 2 == 0 && tx + 1 < tiles_x && flags[size_t(i + 1)]) {
-        pr.push_back(int(i));
-        ++i;  // the pair's second strip
-      } else {
-        pin.push_back(int(i));
-      }
-    }
-    auto up = [&](int* d, const std::vector<int>& h) -> cudaError_t {
-      if (h.empty()) return cudaSuccess;
-      return cudaMemcpyAsync(d, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice, stream);
-    };
-    SV_CUDA(up(L.d_i, in));
-    SV_CUDA(up(L.d_b, bd));
-    SV_CUDA(up(L.d_p, pr));
-    SV_CUDA(up(L.d_pi, pin));
+    std::vector<unsigned> list;
+    list.reserve(size_t(n));
+    for (unsigned c : {svk::kStripGeneral, svk::kStripEdge, svk::kStripInterior})
+      for (long long i = 0; i < n; ++i)
+        if (cls[size_t(i)] == c) list.push_back(unsigned(i) * 4u + c);
+    SV_CUDA(cudaMemcpyAsync(L.d, list.data(), size_t(n) * sizeof(unsigned), cudaMemcpyHostToDevice, stream));
     SV_CUDA(cudaStreamSynchronize(stream));
-    L.ni = int(in.size());
-    L.nb = int(bd.size());
-    L.np = int(pr.size());
-    L.npi = int(pin.size());
     L.valid = true;
     graph_dirty = true; ++pversion;
     return SV_OK;
   }
-  // the strip lists of variant v into P (none for other variants or lists not built yet)
+  // the strip list of variant v into P (none for other variants or lists not built yet)
   void set_strips(svk::StageParams<T>& P, int v) const {
-    const int rows = svk::variant_sweep_rows(v);
-    P.istrips = P.bstrips = nullptr;
-    P.ipairs = nullptr;
-    P.n_istrips = P.n_bstrips = P.n_ipairs = 0;
-    if (rows == 0) return;
-    const Strips& L = strips_[strips_slot(rows)];
-    if (!L.valid) return;
-    P.bstrips = L.d_b; P.n_bstrips = L.nb;
-    if (svk::variant_is_pair(v)) {
-      P.ipairs = L.d_p; P.n_ipairs = L.np;
-      P.istrips = L.d_pi; P.n_istrips = L.npi;
-    } else {
-      P.istrips = L.d_i; P.n_istrips = L.ni;
-    }
+    P.rows = sweep_rows(v);
+    P.strips = nullptr;
+    P.n_strips = 0;
+    auto it = strips_.find(P.rows);
+    if (P.rows == 0 || it == strips_.end() || !it->second.valid) return;
+    P.strips = it->second.d;
+    P.n_strips = int(svk::variant_partials(v, (long long)mesh.nx, (long long)mesh.ny));
+  }
+  // source terms, boundary fields or a tableau beyond the lean sweep (svk::sweep_rows)
+  bool extra() const {
+    return eddy_mode != SV_EDDY_OFF || (irate && icap) || (efx && efy) || (hb0 && hb1) || !diag;
   }
 
   ~Solver() override {
@@ -306,8 +274,9 @@ struct Solver final : public sv_ctx {
     *p = static_cast<U*>(q);
     return cudaSuccess;
   }
+  // a cell field, with the padding the sweeps' row copies may read (svk::kFieldPad)
   cudaError_t alloc_cells(T** p, bool zero = true) {
-    cudaError_t e = alloc(p, size_t(ncells));
+    cudaError_t e = alloc(p, size_t(ncells) + svk::kFieldPad / sizeof(T));
     if (e == cudaSuccess && zero) e = cudaMemsetAsync(*p, 0, size_t(ncells) * sizeof(T), stream);
     return e;
   }
@@ -687,6 +656,7 @@ struct Solver final : public sv_ctx {
     P.nx = int(mesh.nx); P.ny = int(mesh.ny);
     P.dx = mesh.dx; P.dy = mesh.dy; P.L = prm.step_duration;
     P.cell_area = mesh.dx * mesh.dy;
+    P.mc.set(mesh.dx, mesh.dy);
     for (int b = 0; b < 2; ++b)
       for (int f = 0; f < 3; ++f) P.S[b][f] = S[b][f];
     P.z = z;
@@ -763,14 +733,15 @@ struct Solver final : public sv_ctx {
     return F;
   }
 
-  bool batch_path(int v) const { return sizeof(T) == 4 && v == svk::batch_variant<T>(); }
+  bool batch_path(int v) const { return sizeof(T) == 4 && v == svk::kBatchVariant; }
   bool pow2_mesh() const {
     int e;
     return std::frexp(mesh.dx, &e) == 0.5 && std::frexp(mesh.dy, &e) == 0.5;
   }
   // Device copy of the stage parameters for the batch-of-one path (outside stream capture).
   int ensure_dev_params() {
-    if (!batch_path(variant)) return ensure_strips(variant);
+    int r = ensure_strips(variant);
+    if (r || !batch_path(variant)) return r;
     if (sp_version == pversion) return SV_OK;
     if (!d_sp) {
       SV_CUDA(alloc(&d_sp, size_t(N + 1)));
@@ -787,8 +758,8 @@ struct Solver final : public sv_ctx {
   }
   cudaError_t launch_stage_kernel(const svk::StageParams<T>& P, int st) {
     if (batch_path(variant))
-      return svk::launch_sweep_batch<T>(d_sp + st, d_ws, 1, nblk, pow2_mesh(), eddy_mode != SV_EDDY_OFF, stream);
-    return svk::launch_variant<T>(P, variant, stream);
+      return svk::launch_sweep_batch<T>(d_sp + st, d_ws, 1, nblk, pow2_mesh(), extra(), stream);
+    return svk::launch_variant<T>(P, variant, extra(), stream);
   }
 
   // Launch the N stages of one timestep and the finalize kernel (RungeKutta.cpp:147-167).
@@ -995,8 +966,7 @@ struct Solver final : public sv_ctx {
   int set_variant(int v) override {
     if (v < 0 || v >= svk::kNumVariants) return fail(SV_E_ARG, "unknown kernel variant");
     // with tile datums only the column sweep evaluates each face in one frame (face_frame)
-    if (datum && !svk::variant_is_sweep(v))
-      return fail(SV_E_ARG, "tile datums need a column-sweep variant (4-10, 12-15)");
+    if (datum && !svk::variant_is_sweep(v)) return fail(SV_E_ARG, "tile datums need a column-sweep variant");
     if (svk::variant_is_fp32_only(v) && sizeof(T) != 4) return fail(SV_E_ARG, "variants 12-15 are FP32 only");
     if (svk::variant_is_split(v)) {
       int r = ensure_split();
@@ -1049,7 +1019,7 @@ struct Solver final : public sv_ctx {
       if (datum && !svk::variant_is_sweep(v)) continue;
       if (svk::variant_is_fp32_only(v) && sizeof(T) != 4) continue;
       P.nblk = svk::variant_partials(v, (long long)mesh.nx, (long long)mesh.ny);
-      if (!batch_path(v)) {
+      {
         int rs = ensure_strips(v);
         if (rs) return rs;
       }
@@ -1061,8 +1031,8 @@ struct Solver final : public sv_ctx {
       set_strips(P, v);
       // the batch variant runs as the batched kernel (see launch_stage_kernel): time that one
       auto launch = [&]() -> cudaError_t {
-        if (!batch_path(v)) return svk::launch_variant<T>(P, v, stream);
-        return svk::launch_sweep_batch<T>(d_sp + N, d_ws + 2, 1, P.nblk, pow2_mesh(), eddy_mode != SV_EDDY_OFF, stream);
+        if (!batch_path(v)) return svk::launch_variant<T>(P, v, extra(), stream);
+        return svk::launch_sweep_batch<T>(d_sp + N, d_ws + 2, 1, P.nblk, pow2_mesh(), extra(), stream);
       };
       if (batch_path(v)) {
         if (!d_sp) {
@@ -1173,7 +1143,7 @@ struct Batch final : public sv_batch_base {
   svk::StepQueue* d_queue = nullptr;        // [nact] steps queued by the current advance
   int nact = 0, cap = 0;
   long long total_tiles = 0, max_nblk = 0;  // partial slots of all members, of the largest one
-  bool p2 = true, eddy = false, dirty = true;
+  bool p2 = true, extra = false, dirty = true;
   std::vector<int> active;                  // slot ids in launch order
   std::vector<unsigned long long> versions; // members' pversion at the last rebuild
   cudaGraphExec_t graph = nullptr;
@@ -1187,9 +1157,8 @@ struct Batch final : public sv_batch_base {
   svk::PersistMember* d_pmem = nullptr;        // [nact]
   int* d_pstatus = nullptr;                    // [0] status, then (8-byte aligned) the progress count
   unsigned long long* d_pprogress = nullptr;
-  // the members' kernel variant: the column sweep of 32 rows (variant 8) in persistent mode,
-  // whose strips are the persistent kernel's work items; else the batches' variant
-  int member_variant() const { return persistent ? 8 : svk::batch_variant<T>(); }
+  // the members' kernel variant: the column sweep, whose strips are the work items
+  int member_variant() const { return svk::kBatchVariant; }
 
   ~Batch() override {
     cudaSetDevice(device);
@@ -1306,21 +1275,19 @@ struct Batch final : public sv_batch_base {
     std::vector<long long> ht(nact + 1, 0);
     std::vector<Ctl*> hc(std::max(nact, 1));
     p2 = true;
-    eddy = false;
+    extra = false;
     max_nblk = 0;
     for (int k = 0; k < nact; ++k) {
       Solver<T>* m = members[active[k]];
       // the tile prefix and the partials follow the batch kernel's decomposition
       if (m->variant != member_variant()) m->set_variant(member_variant());
-      if (persistent) {  // the persistent kernel runs each member's interior strips in the interior sweep
-        int rs = m->ensure_strips(member_variant());
-        if (rs) return fail(rs, "member " + std::to_string(active[k]) + ": " + m->err);
-      }
+      int rs = m->ensure_strips(member_variant());
+      if (rs) return fail(rs, "member " + std::to_string(active[k]) + ": " + m->err);
       ht[k + 1] = ht[k] + m->nblk;
       max_nblk = std::max(max_nblk, m->nblk);
       int e2;
       p2 = p2 && std::frexp(m->mesh.dx, &e2) == 0.5 && std::frexp(m->mesh.dy, &e2) == 0.5;
-      eddy = eddy || m->eddy_mode != SV_EDDY_OFF;
+      extra = extra || m->extra();
       for (int st = 0; st < N; ++st) hp[size_t(st) * nact + k] = m->stage_params(st);
       hf[k] = m->finalize_params(true);
       hf[k].q = d_queue + k;
@@ -1344,11 +1311,8 @@ struct Batch final : public sv_batch_base {
 
   int enqueue_timestep() {
     for (int st = 0; st < N; ++st) {
-      cudaError_t e = svk::variant_is_sweep(svk::batch_variant<T>())
-                          ? svk::launch_sweep_batch<T>(d_params + size_t(st) * nact, d_tiles, nact, total_tiles, p2,
-                                                       eddy, stream)
-                          : svk::launch_stage_batch<T>(d_params + size_t(st) * nact, d_tiles, nact, total_tiles, p2,
-                                                       eddy, stream);
+      cudaError_t e = svk::launch_sweep_batch<T>(d_params + size_t(st) * nact, d_tiles, nact, total_tiles, p2, extra,
+                                                 stream);
       if (e != cudaSuccess) return cuda_fail(e, "batched stage kernel");
     }
     cudaError_t e = svk::launch_finalize_batch(d_fin, nact, max_nblk, stream);
@@ -1419,7 +1383,7 @@ struct Batch final : public sv_batch_base {
       PP.progress = d_pprogress;
       PP.spin_limit = spin_limit;
       PP.max_ns = (unsigned long long)(max_seconds * 1e9);
-      if (e == cudaSuccess) e = svk::launch_persist<T>(PP, p2, eddy, stream);
+      if (e == cudaSuccess) e = svk::launch_persist<T>(PP, p2, extra, stream);
       if (e != cudaSuccess) return cuda_fail(e, "persistent batch kernel");
       int st = 0;
       SV_CUDA(cudaMemcpyAsync(&st, d_pstatus, sizeof(int), cudaMemcpyDeviceToHost, stream));

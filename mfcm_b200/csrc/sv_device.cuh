@@ -445,11 +445,16 @@ __device__ __forceinline__ T head_target(T h0, T h1, const CC& c) {
 __device__ __forceinline__ double pow43_(double x) { return sv_math::pow43(x); }
 // FP32 path: x^(4/3) = 2^(4/3 log2 x) on the special-function unit (relative error about
 // 1e-6 over the range of 1/h here); 0 gives 0, infinity infinity, NaN NaN.
-__device__ __forceinline__ float pow43_(float x) { return __powf(x, 4.0f / 3.0f); }
+__device__ __forceinline__ float pow43_(float x) {
+  float l, r;  // subnormals as zero: 1/h is never one
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(l * (4.0f / 3.0f)));
+  return r;
+}
 // h / (h^2 + 1e-3) of the roughness term: IEEE division in FP64, the fast reciprocal form
 // in FP32
 __device__ __forceinline__ double manning_inv_h(double h) { return h / (h * h + 1e-3); }
-__device__ __forceinline__ float manning_inv_h(float h) { return __fdividef(h, h * h + 1e-3f); }
+__device__ __forceinline__ float manning_inv_h(float h) { return __fdividef(h, fmaf(h, h, 1e-3f)); }
 
 // Roughness term (ManningRoughnessSourceTerm.cpp): the increments fu, fv of du/dt, dv/dt;
 // false (no increment) on cells of 1e-6 m depth or less.

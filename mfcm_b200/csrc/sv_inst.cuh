@@ -25,6 +25,18 @@ static cudaError_t smem_optin(K kernel, int bytes, std::atomic<bool> (&done)[kMa
   return cudaSuccess;
 }
 
+// a launch with dynamic shared memory, opted in above 48 KB
+template <auto KERNEL, typename... Args>
+static cudaError_t launch_dynamic(dim3 grid, dim3 block, int smem, cudaStream_t s, const Args&... args) {
+  if (smem > 48 * 1024) {
+    static std::atomic<bool> attr_set[kMaxAttrDevices];
+    cudaError_t e = smem_optin(KERNEL, smem, attr_set);
+    if (e != cudaSuccess) return e;
+  }
+  KERNEL<<<grid, block, smem, s>>>(args...);
+  return cudaGetLastError();
+}
+
 // dx and dy both powers of two: the mesh divisions are exact multiplies
 inline bool pow2_mesh(double dx, double dy) {
   int e;
@@ -81,108 +93,52 @@ template <> cudaError_t launch_stage<SV_T>(const StageParams<SV_T>& P, int tile,
   }
 }
 
-// A sweep launch of a stage after the first: allowed to start while the one before it runs
-// (programmatic dependent launch; the sweeps of one stage touch disjoint outputs)
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, bool overlap,
-                                     Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = overlap ? attr : nullptr;
-  cfg.numAttrs = overlap ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
+// dynamic shared memory of the sweeps
+constexpr int kRingBytes = kSweepWarps * int(sizeof(SweepShared<SV_T>));
 
-template <typename T, int TY, int MINB, bool PAIR = false>
-static cudaError_t launch_sweep_t(const StageParams<T>& P, int variant, cudaStream_t s) {
-  constexpr int WPB = 4;
-  const long long ntiles = variant_partials(variant, P.nx, P.ny);
-  dim3 block(32, WPB);
-  const bool p2 = pow2_mesh(P.dx, P.dy);
-  bool overlap = false;  // the first launch of the stage waits for the previous stage
-  cudaError_t e = cudaSuccess;
-  // the general sweep over the edge and coded-out strips (every strip without lists) first:
-  // few warps, each slower than an interior one, so it runs beside the interior launches
-  const long long ngen = P.bstrips ? P.n_bstrips : ntiles;
-  if (ngen > 0) {
-    dim3 grid(unsigned((ngen + WPB - 1) / WPB));
-    void (*k)(const StageParams<T>) =
-        P.eddy ? (p2 ? sweep_kernel<T, TY, WPB, MINB, true, true> : sweep_kernel<T, TY, WPB, MINB, false, true>)
-               : (p2 ? sweep_kernel<T, TY, WPB, MINB, true, false> : sweep_kernel<T, TY, WPB, MINB, false, false>);
-    e = launch_overlapped(k, grid, block, s, overlap, P);
-    if (e != cudaSuccess) return e;
-    overlap = true;
-  }
-  // interior strip pairs (FP32, if listed) two cells per lane
-  if constexpr (PAIR && sizeof(T) == 4) {
-    if (P.ipairs && P.n_ipairs > 0) {
-      dim3 grid(unsigned((P.n_ipairs + WPB - 1) / WPB));
-      void (*k)(const StageParams<float>) =
-          P.eddy ? (p2 ? sweep_pair_kernel<TY, WPB, MINB, true, true> : sweep_pair_kernel<TY, WPB, MINB, false, true>)
-                 : (p2 ? sweep_pair_kernel<TY, WPB, MINB, true, false> : sweep_pair_kernel<TY, WPB, MINB, false, false>);
-      e = launch_overlapped(k, grid, block, s, overlap, P);
-      if (e != cudaSuccess) return e;
-      overlap = true;
+// The column sweep of a stage: the strips in P.strips, P.rows rows each. `cap`: resident blocks
+// per SM asked of the register allocator. FP32 multiplies by the reciprocal cell sizes whatever
+// they are, so it has no power-of-two form of its own.
+template <int MINB, bool EXTRA> static cudaError_t launch_sweep_c(const StageParams<SV_T>& P, cudaStream_t s) {
+  if (P.n_strips <= 0) return cudaSuccess;
+  const dim3 grid(unsigned((P.n_strips + kSweepWarps - 1) / kSweepWarps)), block(32, kSweepWarps);
+  if (sizeof(SV_T) == 8 && pow2_mesh(P.dx, P.dy))
+    return launch_dynamic<sweep_kernel<SV_T, MINB, sizeof(SV_T) == 8, EXTRA>>(grid, block, kRingBytes, s, P);
+  return launch_dynamic<sweep_kernel<SV_T, MINB, false, EXTRA>>(grid, block, kRingBytes, s, P);
+}
+static cudaError_t launch_sweep(const StageParams<SV_T>& P, int cap, bool extra, cudaStream_t s) {
+  if (extra) return launch_sweep_c<kExtraCap<SV_T>, true>(P, s);
+  if constexpr (sizeof(SV_T) == 8) {
+    switch (cap) {
+      case 3: return launch_sweep_c<3, false>(P, s);
+      case 4: return launch_sweep_c<4, false>(P, s);
+      case 5: return launch_sweep_c<5, false>(P, s);
+      default: return launch_sweep_c<6, false>(P, s);
+    }
+  } else {
+    switch (cap) {
+      case 3:
+      case 4: return launch_sweep_c<4, false>(P, s);
+      case 5: return launch_sweep_c<5, false>(P, s);
+      case 6: return launch_sweep_c<6, false>(P, s);
+      case 7: return launch_sweep_c<7, false>(P, s);
+      default: return launch_sweep_c<8, false>(P, s);
     }
   }
-  // interior strips (if listed) in the interior kernel
-  if (P.istrips && P.n_istrips > 0) {
-    dim3 grid(unsigned((P.n_istrips + WPB - 1) / WPB));
-    void (*k)(const StageParams<T>) =
-        P.eddy ? (p2 ? sweep_interior_kernel<T, TY, WPB, MINB, true, true>
-                     : sweep_interior_kernel<T, TY, WPB, MINB, false, true>)
-               : (p2 ? sweep_interior_kernel<T, TY, WPB, MINB, true, false>
-                     : sweep_interior_kernel<T, TY, WPB, MINB, false, false>);
-    e = launch_overlapped(k, grid, block, s, overlap, P);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaGetLastError();
 }
 
-// the FP32-only variants: two cells per lane with register caps for 3 and 4 blocks per SM
-// (12, 13), one cell per lane capped for 7 and 8 blocks per SM (14, 15); 32-row strips
-template <typename T> static cudaError_t v12_15(const StageParams<T>& P, int variant, cudaStream_t s) {
-  if constexpr (sizeof(T) == 4) {
-    switch (variant) {
-      case 12: return launch_sweep_t<T, 32, 3, true>(P, variant, s);
-      case 13: return launch_sweep_t<T, 32, 4, true>(P, variant, s);
-      case 14: return launch_sweep_t<T, 32, 7>(P, variant, s);
-      default: return launch_sweep_t<T, 32, 8>(P, variant, s);
-    }
-  }
-  return cudaErrorInvalidValue;
+template <> cudaError_t launch_variant<SV_T>(const StageParams<SV_T>& P, int variant, bool extra, cudaStream_t s) {
+  if (variant_is_split(variant)) return launch_split_t<SV_T>(P, s);
+  if (variant_is_sweep(variant)) return launch_sweep(P, variant_cap<SV_T>(variant), extra, s);
+  return launch_stage<SV_T>(P, variant, s);
 }
 
-template <> cudaError_t launch_variant<SV_T>(const StageParams<SV_T>& P, int variant, cudaStream_t s) {
-  switch (variant) {
-    case 4: return launch_sweep_t<SV_T, 16, 1>(P, variant, s);
-    case 5: return launch_sweep_t<SV_T, 32, 1>(P, variant, s);
-    case 6: return launch_sweep_t<SV_T, 64, 1>(P, variant, s);
-    case 7: return launch_sweep_t<SV_T, 32, 3>(P, variant, s);
-    case 8: return launch_sweep_t<SV_T, 32, 4>(P, variant, s);
-    case 9: return launch_sweep_t<SV_T, 32, 5>(P, variant, s);
-    case 10: return launch_sweep_t<SV_T, 32, 6>(P, variant, s);
-    case kSplitVariant: return launch_split_t<SV_T>(P, s);
-    case 12:
-    case 13:
-    case 14:
-    case 15:
-      if (sizeof(SV_T) != 4) return cudaErrorInvalidValue;  // FP32-only variants
-      return v12_15<SV_T>(P, variant, s);
-    default: return launch_stage<SV_T>(P, variant, s);
-  }
-}
-
-template <> cudaError_t launch_strip_flags<SV_T>(const SV_T* z, int nx, int ny, int ty, long long nstrips,
-                                                 unsigned char* flags, cudaStream_t s) {
+template <> cudaError_t launch_strip_classes<SV_T>(const SV_T* z, int nx, int ny, double dx, double dy, int rows,
+                                                   long long nstrips, unsigned char* cls, cudaStream_t s) {
   if (nstrips <= 0) return cudaSuccess;
-  strip_flags_kernel<SV_T><<<unsigned((nstrips + 7) / 8), 256, 0, s>>>(z, nx, ny, ty, nstrips, flags);
+  auto fits = [](double d) { return sizeof(SV_T) == 4 || (d >= 0x1p-30 && d <= 0x1p40); };
+  strip_class_kernel<SV_T><<<unsigned((nstrips + 7) / 8), 256, 0, s>>>(z, nx, ny, rows, nstrips, fits(dx) && fits(dy),
+                                                                       cls);
   return cudaGetLastError();
 }
 
@@ -214,61 +170,40 @@ template <> cudaError_t launch_to_f64<SV_T>(const SV_T* src, double* dst, long l
   return cudaGetLastError();
 }
 
-template <typename T, int TX, int TY, int MINB, bool P2, bool EDDY>
-static cudaError_t launch_stage_batch_p(const StageParams<T>* Ps, const long long* tile_start, int ninst,
-                                        long long total_tiles, cudaStream_t s) {
-  using SM = StageSmem<T, TX, TY>;
-  static std::atomic<bool> attr_set[kMaxAttrDevices];
-  cudaError_t e = smem_optin(stage_batch_kernel<T, TX, TY, MINB, P2, EDDY>, int(sizeof(SM)), attr_set);
-  if (e != cudaSuccess) return e;
-  if (total_tiles <= 0) return cudaSuccess;
-  stage_batch_kernel<T, TX, TY, MINB, P2, EDDY><<<unsigned(total_tiles), TX * TY, sizeof(SM), s>>>(Ps, tile_start,
-                                                                                                     ninst);
-  return cudaGetLastError();
-}
-
-template <> cudaError_t launch_stage_batch<SV_T>(const StageParams<SV_T>* Ps, const long long* tile_start, int ninst,
-                                                 long long total_tiles, bool p2, bool eddy, cudaStream_t s) {
-  if (eddy)
-    return p2 ? launch_stage_batch_p<SV_T, 32, 8, 3, true, true>(Ps, tile_start, ninst, total_tiles, s)
-              : launch_stage_batch_p<SV_T, 32, 8, 3, false, true>(Ps, tile_start, ninst, total_tiles, s);
-  return p2 ? launch_stage_batch_p<SV_T, 32, 8, 3, true, false>(Ps, tile_start, ninst, total_tiles, s)
-            : launch_stage_batch_p<SV_T, 32, 8, 3, false, false>(Ps, tile_start, ninst, total_tiles, s);
-}
-
 template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, const long long* warp_start, int ninst,
-                                                 long long total_warps, bool p2, bool eddy, cudaStream_t s) {
-  constexpr int WPB = 4, TY = 32, MINB = 4;  // variant 8
+                                                 long long total_warps, bool p2, bool extra, cudaStream_t s) {
   if (total_warps <= 0) return cudaSuccess;
-  dim3 block(32, WPB);
-  dim3 grid(unsigned((total_warps + WPB - 1) / WPB));
-  if (eddy) {
-    if (p2) sweep_batch_kernel<SV_T, TY, WPB, MINB, true, true><<<grid, block, 0, s>>>(Ps, warp_start, ninst);
-    else sweep_batch_kernel<SV_T, TY, WPB, MINB, false, true><<<grid, block, 0, s>>>(Ps, warp_start, ninst);
-  } else {
-    if (p2) sweep_batch_kernel<SV_T, TY, WPB, MINB, true, false><<<grid, block, 0, s>>>(Ps, warp_start, ninst);
-    else sweep_batch_kernel<SV_T, TY, WPB, MINB, false, false><<<grid, block, 0, s>>>(Ps, warp_start, ninst);
-  }
-  return cudaGetLastError();
+  const dim3 block(32, kSweepWarps), grid(unsigned((total_warps + kSweepWarps - 1) / kSweepWarps));
+  constexpr bool F64 = sizeof(SV_T) == 8;
+  constexpr int CAP = kBatchCap<SV_T>, XCAP = kExtraCap<SV_T>;
+  if (extra)
+    return p2 && F64 ? launch_dynamic<sweep_batch_kernel<SV_T, XCAP, F64, true>>(grid, block, kRingBytes, s, Ps, warp_start, ninst)
+                     : launch_dynamic<sweep_batch_kernel<SV_T, XCAP, false, true>>(grid, block, kRingBytes, s, Ps, warp_start, ninst);
+  return p2 && F64 ? launch_dynamic<sweep_batch_kernel<SV_T, CAP, F64, false>>(grid, block, kRingBytes, s, Ps, warp_start, ninst)
+                   : launch_dynamic<sweep_batch_kernel<SV_T, CAP, false, false>>(grid, block, kRingBytes, s, Ps, warp_start, ninst);
 }
 
 // Persistent batch kernel: one cooperative launch with as many 4-warp blocks as fit on the
 // device at once (every block resident, so warps that wait for another warp's work always
 // see it done).
-template <> cudaError_t launch_persist<SV_T>(const PersistParams<SV_T>& PP, bool p2, bool eddy, cudaStream_t s) {
+template <> cudaError_t launch_persist<SV_T>(const PersistParams<SV_T>& PP, bool p2, bool extra, cudaStream_t s) {
+  constexpr bool F64 = sizeof(SV_T) == 8;
+  constexpr int CAP = kBatchCap<SV_T>, XCAP = kExtraCap<SV_T>;
   void (*kern)(const PersistParams<SV_T>) =
-      eddy ? (p2 ? persist_batch_kernel<SV_T, true, true> : persist_batch_kernel<SV_T, false, true>)
-           : (p2 ? persist_batch_kernel<SV_T, true, false> : persist_batch_kernel<SV_T, false, false>);
+      extra ? (p2 ? persist_batch_kernel<SV_T, XCAP, F64, true> : persist_batch_kernel<SV_T, XCAP, false, true>)
+            : (p2 ? persist_batch_kernel<SV_T, CAP, F64, false> : persist_batch_kernel<SV_T, CAP, false, false>);
   int dev = 0, nsm = 0, per_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && kRingBytes > 48 * 1024)
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingBytes);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kPersistWarps, 0);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kPersistWarps, kRingBytes);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorCooperativeLaunchTooLarge;
   PersistParams<SV_T> arg = PP;
   void* args[] = {&arg};
   return cudaLaunchCooperativeKernel((const void*)kern, dim3(unsigned(per_sm * nsm)), dim3(32, kPersistWarps), args,
-                                     0, s);
+                                     kRingBytes, s);
 }
 
 template <typename T, int TX, int TY>

@@ -63,10 +63,24 @@ enum StageMode : int {
   M_DEBUGK = 32,  // debug: write k_s only (no RK combination)
 };
 
+// Constants of the mesh in the solver's value type, formed once on the host.
+template <typename T> struct MeshConst {
+  T dx, dy, rdx, rdy;    // cell sizes and their reciprocals
+  T dx2, dy2, kx, ky;    // 2 d and 1 / (2 d)
+  T hdx, hdy;            // d / 2
+  T ry;                  // dx / dy
+  void set(double x, double y) {
+    dx = T(x); dy = T(y); rdx = T(1.0 / x); rdy = T(1.0 / y);
+    dx2 = T(2.0 * x); dy2 = T(2.0 * y); kx = T(0.5) * rdx; ky = T(0.5) * rdy;
+    hdx = T(0.5) * dx; hdy = T(0.5) * dy; ry = T(x / y);
+  }
+};
+
 template <typename T> struct StageParams {
   int nx, ny;
   double dx, dy, L;
   double cell_area;
+  MeshConst<T> mc;
   T* S[2][3];            // state parity buffers: S[cur] = U_[0], S[cur^1] = acc / U_[N]
   const T* Yin[3];       // stage input (ignored on the first stage)
   T* Yout[3];            // Y_{s+1} (not on the last stage)
@@ -102,15 +116,10 @@ template <typename T> struct StageParams {
   // 2 energy loss, 3 eddy viscosity (each adds to du/dt and dv/dt, so the order sets the
   // rounding); used by the kernels compiled with eddy viscosity
   int term_order;
-  // column-sweep strips split by kind (see strip_flags_kernel): the interior strips run the
-  // interior kernel, the others the general one; null lists: every strip runs the general one
-  const int* istrips;
-  const int* bstrips;
-  int n_istrips, n_bstrips;
-  // two-cells-per-lane variants: pairs of adjacent interior strips (the first strip of each);
-  // istrips then lists the interior strips left out of a pair
-  const int* ipairs;
-  int n_ipairs;
+  // column sweep: strips of kSweepOut columns x `rows` rows, each listed as its index times 4
+  // plus its class (strip_class_kernel)
+  const unsigned* strips;
+  int n_strips, rows;
   // split schedule: the stage input's slopes dh/dx, du/dx, dv/dx, dh/dy, du/dy, dv/dy as
   // written by slopes_kernel (read by the stage kernel instead of computing them), or null
   T* pslp[6];
@@ -665,845 +674,11 @@ __global__ void __launch_bounds__(256) slopes_kernel(const StageParams<T> P) {
   }
 }
 
-// Batched stage: one launch covers every tile of every instance of a batch. tile_start has
-// ninst + 1 entries (prefix sums of the instances' tile counts); each CTA finds its instance,
-// copies that instance's parameters to shared memory and runs the same tile body. Instances
-// whose step is finished (their controller's done flag) return at once.
-template <typename T, int TX, int TY, int MINB, bool P2, bool EDDY>
-__global__ void __launch_bounds__(TX * TY, MINB)
-    stage_batch_kernel(const StageParams<T>* __restrict__ Ps, const long long* __restrict__ tile_start, int ninst) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  auto& s = *reinterpret_cast<StageSmem<T, TX, TY>*>(smem_raw);
-  __shared__ StageParams<T> Psh;
-  __shared__ int inst_sh;
-  const long long tile = blockIdx.x;
-  if (threadIdx.x == 0) {
-    int lo = 0, hi = ninst - 1;  // last instance with tile_start[i] <= tile
-    while (lo < hi) {
-      int mid = (lo + hi + 1) / 2;
-      if (tile_start[mid] <= tile) lo = mid;
-      else hi = mid - 1;
-    }
-    inst_sh = lo;
-    Psh = Ps[lo];
-  }
-  __syncthreads();
-  const long long local = tile - tile_start[inst_sh];
-  const int tiles_x = (Psh.nx + TX - 1) / TX;
-  stage_tile<T, TX, TY, P2, EDDY>(Psh, int(local % tiles_x), int(local / tiles_x), local, s);
-}
+}  // namespace svk
 
-// ---------------------------------------------------------------------------------------
-// Column-sweep stage kernel. One warp owns a strip of 32 columns (28 output columns plus a
-// 2-column halo on each side) and marches down TY output rows. Each lane holds its column's
-// last three rows of (h, u, v, z, dz/dx, dz/dy) and two rows of slopes in registers; x
-// neighbours come from warp shuffles, y neighbours from the rolling window. Every face
-// flux and every difference quotient is computed once and reused by both cells / both
-// slopes that need it, and there is no block-level barrier. The arithmetic per face and
-// per cell is the same function as in the tiled kernel.
-// ---------------------------------------------------------------------------------------
-template <typename T> __device__ __forceinline__ T up1(T v) { return __shfl_up_sync(kFull, v, 1); }
-template <typename T> __device__ __forceinline__ T dn1(T v) { return __shfl_down_sync(kFull, v, 1); }
+#include "sv_sweep.cuh"
 
-// The sweeps form slopes with svd::minmod3q (sv_device.cuh): Minmod3 from difference
-// quotients, its sign and NaN tests on the integer pipe.
-//
-// Two-sided Minmod3 of the FP32 interior sweeps: for finite quotients the reference's nested
-// pair minmods (Minmod3.hpp:66-80) reduce to sign * min(|2 qL|, |2 qR|, |qC / 2|) when the
-// three agree in sign and zero otherwise (up to the sign of a zero result). The NaN rules
-// only matter for a non-finite state, as for the dropped tangential terms.
-__device__ __forceinline__ float minmod3_finite(float qL, float qR, float qC) {
-  const float a = 2.0f * qL, b = 2.0f * qR, c = 0.5f * qC;
-  const int ia = __float_as_int(a), ib = __float_as_int(b), ic = __float_as_int(c);
-  const float m = fminf(fminf(fabsf(a), fabsf(b)), fabsf(c));
-  return ((ia ^ ib) | (ia ^ ic)) >= 0 ? __int_as_float(__float_as_int(m) | (ia & 0x80000000)) : 0.0f;
-}
-// the interior sweeps' two-sided slope: exact reference rules in FP64, the finite form in FP32
-template <typename T> __device__ __forceinline__ T slope2s(T qL, T qR, T qC) {
-  if constexpr (sizeof(T) == 4) return minmod3_finite(qL, qR, qC);
-  return minmod3q<T>(qL, true, qR, true, qC);
-}
-
-template <typename T> struct RowV { T h, u, v, z, zx, zy; };
-template <typename T> struct SlopeV { T hx, ux, vx, hy, uy, vy; };
-
-template <typename T>
-__device__ __forceinline__ CellV<T> mkcell(const RowV<T>& r, const SlopeV<T>& s) {
-  CellV<T> c;
-  c.h = r.h; c.u = r.u; c.v = r.v; c.z = r.z;
-  c.dhdx = s.hx; c.dudx = s.ux; c.dvdx = s.vx; c.dzdx = r.zx;
-  c.dhdy = s.hy; c.dudy = s.uy; c.dvdy = s.vy; c.dzdy = r.zy;
-  return c;
-}
-template <typename T> __device__ __forceinline__ CellV<T> shfl_cell_up(const CellV<T>& a) {
-  CellV<T> c;
-  c.h = up1(a.h); c.u = up1(a.u); c.v = up1(a.v); c.z = up1(a.z);
-  c.dhdx = up1(a.dhdx); c.dudx = up1(a.dudx); c.dvdx = up1(a.dvdx); c.dzdx = up1(a.dzdx);
-  c.dhdy = up1(a.dhdy); c.dudy = up1(a.dudy); c.dvdy = up1(a.dvdy); c.dzdy = up1(a.dzdy);
-  return c;
-}
-template <typename T> __device__ __forceinline__ double warp_sum(double v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(kFull, v, o);
-  return v;
-}
-__device__ __forceinline__ double warp_max(double v) {
-  for (int o = 16; o > 0; o >>= 1) v = nmax(v, __shfl_down_sync(kFull, v, o));
-  return v;
-}
-__device__ __forceinline__ double warp_min(double v) {
-  for (int o = 16; o > 0; o >>= 1) v = nmin(v, __shfl_down_sync(kFull, v, o));
-  return v;
-}
-
-constexpr int kSweepOut = 28;  // output columns per warp
-// Rows the column sweep prefetches into L1 ahead of use: the window fields of row k+1+0 and
-// the per-cell fields of output row k-2+3 at iteration k, one iteration ahead. A warp marches
-// its rows in order, so without these hints each row's loads wait a full memory latency with
-// only one row in flight. One iteration (about 4 us per row at 28 warps per SM) covers the
-// latency; prefetching further ahead kept more lines in flight than L1 holds (about 12 KB per
-// warp at 3 and 2 rows ahead), and the stages ran 1.5 % (FP32) and 4 % (FP64) slower.
-constexpr int kSweepPfWindow = 0, kSweepPfCell = 3;
-__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
-
-// Prefetch plan of the interior sweeps. A warp's row of one field is 32 consecutive values of
-// an interior strip (columns gx0 .. gx0+31, all inside the mesh): at most two 128-byte lines
-// in FP32 and three in FP64. The plan gives each lane kPfSlots (field, line) pairs of the
-// fields the stage reads -- the window fields (stage input, bed, bed slopes) first, then the
-// per-cell fields -- so that a row ahead costs kPfSlots prefetch instructions per warp instead
-// of one per field with its address arithmetic. Pairs beyond 32 * kPfSlots are not prefetched.
-constexpr int kPfSlots = 2;
-template <typename T> struct PfPlan {
-  const T* p[kPfSlots];  // the lane's line in row 0 of its field, or null
-  int d[kPfSlots];       // rows ahead of the loop row: the window's or the per-cell fields'
-  __device__ __forceinline__ void init(const StageParams<T>& P, const DevForcing& fc, const T* Yh, const T* Yu,
-                                       const T* Yv, bool first, int cur, int gx0, int lane) {
-    constexpr int kLines = sizeof(T) == 4 ? 2 : 3;
-    constexpr int kLineCols = 128 / int(sizeof(T));
-    int fi[kPfSlots];
-#pragma unroll
-    for (int s = 0; s < kPfSlots; ++s) {
-      fi[s] = (lane + 32 * s) / kLines;
-      p[s] = nullptr;
-      d[s] = fi[s] < 6 ? 1 + kSweepPfWindow : kSweepPfCell - 2;
-    }
-    int n = 0;
-    auto add = [&](const T* f) {
-#pragma unroll
-      for (int s = 0; s < kPfSlots; ++s)
-        if (fi[s] == n) p[s] = f;
-      ++n;
-    };
-    add(Yh); add(Yu); add(Yv); add(P.z); add(P.zx); add(P.zy);
-    if (!first) {
-      for (int f = 0; f < 3; ++f) { add(P.S[cur][f]); add(P.S[cur ^ 1][f]); }
-    }
-    if (P.manning) {
-      for (int f = 0; f < 4; ++f) {
-        const T* m = P.man_p[f];
-        bool dup = false;
-        for (int e = 0; e < f; ++e) dup = dup || (P.man_p[e] == m);
-        if (m && !dup) add(m);
-      }
-    }
-    if (P.irate) { add(P.irate); add(P.icap); }
-    if (P.efx) { add(P.efx); add(P.efy); }
-    if (fc.rain_kind == 3) add(P.pat);
-    if (fc.rain_kind == 2) { add(P.q0p); add(P.q1p); }
-    if (fc.head_kind == 2) { add(P.hb0p); add(P.hb1p); }
-#pragma unroll
-    for (int s = 0; s < kPfSlots; ++s)
-      if (p[s]) p[s] += gx0 + min(((lane + 32 * s) % kLines) * kLineCols, 31);
-  }
-  // the rows k + d of every slot, clamped into the mesh
-  __device__ __forceinline__ void rows(int k, int nx, int ny) const {
-#pragma unroll
-    for (int s = 0; s < kPfSlots; ++s)
-      if (p[s]) prefetch_l1(p[s] + (long long)min(max(k + d[s], 0), ny - 1) * nx);
-  }
-};
-
-// One warp's strip `gw` (row-major over strips of kSweepOut columns x TY rows) of one
-// solver's stage. Called by the single-solver kernel (P in parameter space) and by the
-// batched kernel (P in shared memory).
-template <typename T, int TY, bool P2, bool EDDY, bool COH = false>
-__device__ __forceinline__ void sweep_strip(const StageParams<T>& P, long long gw) {
-  using DX = DivX<T, P2>;
-  const Ctl* ctl = P.ctl;
-  const int nx = P.nx, ny = P.ny;
-  const int tiles_x = (nx + kSweepOut - 1) / kSweepOut;
-  const int lane = threadIdx.x;
-  const int tile_x = int(gw % tiles_x), tile_y = int(gw / tiles_x);
-  const int gx = tile_x * kSweepOut - 2 + lane;
-  const int gxc = min(max(gx, 0), nx - 1);
-  const bool out_lane = lane >= 2 && lane < 2 + kSweepOut && gx < nx;
-  const bool wface_lane = lane >= 2 && lane <= 2 + kSweepOut && gx <= nx;
-  const bool hasW = gx > 0, hasE = gx < nx - 1;
-  const int y0 = tile_y * TY;
-
-  const int cur = ctl->cur;
-  const double dt_d = ctl->dt;
-  const double tsub = ctl->t_local + P.c_s * dt_d;
-  const bool first = P.mode & M_FIRST, last = P.mode & M_LAST;
-  const T* Yh = first ? P.S[cur][0] : P.Yin[0];
-  const T* Yu = first ? P.S[cur][1] : P.Yin[1];
-  const T* Yv = first ? P.S[cur][2] : P.Yin[2];
-  const DX divx = MkDivX<DX>::make(P.dx), divy = MkDivX<DX>::make(P.dy);
-  const T hdx = T(0.5) * T(P.dx), hdy = T(0.5) * T(P.dy);
-  CellCtx<T, DX> c;
-  c.divx = divx; c.divy = divy;
-  c.divdt = mkdiv<T>(dt_d);
-  c.divL = mkdiv<T>(P.L);
-  c.dt = T(dt_d); c.dt_d = dt_d; c.tsub_d = tsub;
-  c.manning = P.manning; c.rain_mode = P.rain_mode; c.head_first = P.head_first;
-  const DevForcing fc = *P.fc;
-
-  // FP32 with tile datums: the window keeps each cell's raw bed offset; a face whose two
-  // cells lie in different datum tiles is evaluated in its lower cell's frame (face_frame),
-  // the same whichever strip computes it, so the flux out of one cell is the flux into the
-  // other and the volume is conserved across strip boundaries
-  auto load_row = [&](int gy) {
-    const int r = min(max(gy, 0), ny - 1);
-    const long long g = (long long)r * nx + gxc;
-    RowV<T> v;
-    v.h = ldst<COH>(Yh, g); v.u = ldst<COH>(Yu, g); v.v = ldst<COH>(Yv, g);
-    v.z = ld(P.z, g);
-    v.zx = ld(P.zx, g); v.zy = ld(P.zy, g);
-    return v;
-  };
-
-  RowV<T> Rm{}, R0{}, Rp{};   // rows k-2, k-1, k
-  SlopeV<T> Sm{}, S0{};       // slopes of rows k-2, k-1
-  T Smm_uy = T(0), Smm_vy = T(0);  // y slopes of u, v of row k-3 (eddy viscosity)
-  T fyA[3] = {}, fyB[3] = {};  // (U[k-1]-U[k-2])/dy, (U[k]-U[k-1])/dy
-  FaceF<T> FS{}, FN{};
-  double rain = 0.0, removed = 0.0, walls = 0.0, vol = 0.0;
-  T xcfl = T(0), xmin = T(1.0 / 0.0);
-
-  // L1 prefetch of rows ahead (addresses clamped into the mesh, like the loads)
-  auto prefetch_rows = [&](int k) {
-    {
-      const int r = min(max(k + 1 + kSweepPfWindow, 0), ny - 1);
-      const long long g = (long long)r * nx + gxc;
-      prefetch_l1(Yh + g); prefetch_l1(Yu + g); prefetch_l1(Yv + g);
-      prefetch_l1(P.z + g); prefetch_l1(P.zx + g); prefetch_l1(P.zy + g);
-    }
-    const int r = min(max(k - 2 + kSweepPfCell, 0), ny - 1);
-    const long long g = (long long)r * nx + gxc;
-    if (!first) {
-      for (int f = 0; f < 3; ++f) { prefetch_l1(P.S[cur][f] + g); prefetch_l1(P.S[cur ^ 1][f] + g); }
-    }
-    if (P.manning) {
-      for (int f = 0; f < 4; ++f)
-        if (P.man_p[f]) prefetch_l1(P.man_p[f] + g);
-    }
-    if (P.irate) { prefetch_l1(P.irate + g); prefetch_l1(P.icap + g); }
-    if (P.efx) { prefetch_l1(P.efx + g); prefetch_l1(P.efy + g); }
-    if (fc.rain_kind == 3) prefetch_l1(P.pat + g);
-    if (fc.rain_kind == 2) { prefetch_l1(P.q0p + g); prefetch_l1(P.q1p + g); }
-    if (fc.head_kind == 2) { prefetch_l1(P.hb0p + g); prefetch_l1(P.hb1p + g); }
-  };
-
-  for (int k = y0 - 2; k <= y0 + TY + 1; ++k) {
-    prefetch_rows(k);
-    // row k is loaded where it enters the window: the L1 prefetch issued three iterations
-    // earlier has brought it in, and not holding it a row ahead in registers leaves room
-    // for more resident warps
-    Rm = R0; R0 = Rp; Rp = load_row(k);
-    if constexpr (EDDY) { Smm_uy = Sm.uy; Smm_vy = Sm.vy; }
-    Sm = S0;
-    fyA[0] = fyB[0]; fyA[1] = fyB[1]; fyA[2] = fyB[2];
-    // forward y quotients between rows k-1 and k
-    if (k >= y0 - 1) {
-      fyB[0] = divy(Rp.h - R0.h);
-      fyB[1] = divy(Rp.u - R0.u);
-      fyB[2] = divy(Rp.v - R0.v);
-    }
-    // slopes of row k-1 (State.cpp:187-192): Y axis uses north (row k) as the left neighbour
-    if (k >= y0) {
-      const int r = k - 1;
-      const bool hasN = r < ny - 1, hasS = r > 0;
-      S0.hy = minmod3q<T>(-fyB[0], hasN, -fyA[0], hasS, divy(Rm.h - Rp.h));
-      S0.uy = minmod3q<T>(-fyB[1], hasN, -fyA[1], hasS, divy(Rm.u - Rp.u));
-      S0.vy = minmod3q<T>(-fyB[2], hasN, -fyA[2], hasS, divy(Rm.v - Rp.v));
-      {
-        T r_ = dn1(R0.h), l_ = up1(R0.h);
-        T fq = divx(r_ - R0.h);
-        S0.hx = minmod3q<T>(up1(fq), hasW, fq, hasE, divx(r_ - l_));
-      }
-      {
-        T r_ = dn1(R0.u), l_ = up1(R0.u);
-        T fq = divx(r_ - R0.u);
-        S0.ux = minmod3q<T>(up1(fq), hasW, fq, hasE, divx(r_ - l_));
-      }
-      {
-        T r_ = dn1(R0.v), l_ = up1(R0.v);
-        T fq = divx(r_ - R0.v);
-        S0.vx = minmod3q<T>(up1(fq), hasW, fq, hasE, divx(r_ - l_));
-      }
-    }
-    // horizontal face between rows k-2 and k-1 (face row fy = k-1), Fluxes.cpp:55-64
-    if (k >= y0 + 1 && out_lane) {
-      const int fy = k - 1;
-      if (fy <= ny) {
-        const int edge = fy == 0 ? -1 : (fy == ny ? 1 : 0);
-        const CellV<T> lo = mkcell(Rm, Sm), hi = mkcell(R0, S0);
-        if (P.zdat && edge == 0) {
-          CellV<T> lo2 = lo, hi2 = hi;
-          face_frame<T>(P, lo2, hi2, gx, fy - 1, gx, fy);
-          face_flux<T, 1>(lo2, hi2, edge, hdy, divy, FN);
-        } else {
-          face_flux<T, 1>(edge == -1 ? hi : lo, edge == 1 ? lo : hi, edge, hdy, divy, FN);
-        }
-      }
-    }
-    // output row k-2
-    if (k >= y0 + 2) {
-      const int r = k - 2;
-      const CellV<T> me = mkcell(Rm, Sm);
-      const CellV<T> lf = shfl_cell_up(me);
-      EddyIn<T> ed{};
-      if constexpr (EDDY) {
-        if (P.eddy) {  // second derivatives of row r: x by shuffles, y from rows r+1, r, r-1
-          ed.ux = Sm.ux; ed.uy = Sm.uy; ed.vx = Sm.vx; ed.vy = Sm.vy;
-          {
-            T r_ = dn1(Sm.ux), l_ = up1(Sm.ux);
-            T fq = divx(r_ - Sm.ux);
-            ed.uxx = minmod3q<T>(up1(fq), hasW, fq, hasE, divx(r_ - l_));
-          }
-          {
-            T r_ = dn1(Sm.vx), l_ = up1(Sm.vx);
-            T fq = divx(r_ - Sm.vx);
-            ed.vxx = minmod3q<T>(up1(fq), hasW, fq, hasE, divx(r_ - l_));
-          }
-          const bool hasN = r < ny - 1, hasS = r > 0;  // Y axis: north is the left neighbour
-          ed.uyy = minmod3q<T>(divy(Sm.uy - S0.uy), hasN, divy(Smm_uy - Sm.uy), hasS, divy(Smm_uy - S0.uy));
-          ed.vyy = minmod3q<T>(divy(Sm.vy - S0.vy), hasN, divy(Smm_vy - Sm.vy), hasS, divy(Smm_vy - S0.vy));
-        }
-      }
-      FaceF<T> FW{T(0), T(0), T(0), T(0)};
-      if (wface_lane && r < ny) {
-        const int edge = gx == 0 ? -1 : (gx == nx ? 1 : 0);
-        if (P.zdat && edge == 0) {
-          CellV<T> lf2 = lf, me2 = me;
-          face_frame<T>(P, lf2, me2, gx - 1, r, gx, r);
-          face_flux<T, 0>(lf2, me2, edge, hdx, divx, FW);
-        } else {
-          face_flux<T, 0>(edge == -1 ? me : lf, edge == 1 ? lf : me, edge, hdx, divx, FW);
-        }
-      }
-      const FaceF<T> FE{dn1(FW.h), dn1(FW.u), dn1(FW.v), dn1(FW.z)};
-      if (out_lane && r < ny) {
-        const long long g = (long long)r * nx + gx;
-        finish_cell<T, CellCtx<T, DX>, EDDY, true, COH>(P, fc, c, g, gx, r, me.h, me.u, me.v, me.dhdx, me.dhdy,
-                                                        me.dzdx, me.dzdy, FW, FE, FS, FN, first, last, cur, dt_d, rain,
-                                                        removed, walls, xcfl, xmin, vol, &ed);
-      }
-    }
-    FS = FN;
-  }
-  if (last && !(P.mode & M_DEBUGK)) {
-    double mx = warp_max(double(xcfl)), mn = warp_min(double(xmin)), vs = warp_sum<T>(vol);
-    if (lane == 0) {
-      P.part[gw] = mx;
-      P.part[P.nblk + gw] = mn;
-      P.part[2 * P.nblk + gw] = vs;
-    }
-  }
-  if (P.mode & M_TALLY) {
-    double rs = warp_sum<T>(rain), os = warp_sum<T>(removed), ws = warp_sum<T>(walls);
-    if (lane == 0) store_tallies(P, gw, rs, os, ws, first, dt_d);
-  }
-}
-
-// Whether strip `gw` of the column sweep with TY output rows is interior: its window (the
-// 32 columns x TY + 4 rows of cells it loads) lies inside the mesh with a cell to spare on
-// every side. Every slope it computes is then two-sided, none of its faces is a mesh-edge face
-// and none of its output cells lies on an edge strip.
-__host__ __device__ inline bool strip_inside(long long gw, int nx, int ny, int ty) {
-  const int tiles_x = (nx + kSweepOut - 1) / kSweepOut;
-  const int x0 = int(gw % tiles_x) * kSweepOut, y0 = int(gw / tiles_x) * ty;
-  return x0 >= 2 && x0 + 30 <= nx && y0 >= 2 && y0 + ty + 2 <= ny;
-}
-
-// Per strip: 1 for an interior strip whose window holds no coded-out (NaN) bed, so that no
-// edge or coded-out mask applies to any of its faces; else 0. One warp per strip.
-template <typename T>
-__global__ void strip_flags_kernel(const T* __restrict__ z, int nx, int ny, int ty, long long nstrips,
-                                   unsigned char* __restrict__ flag) {
-  const long long gw = (long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  if (gw >= nstrips) return;  // whole warp
-  const int lane = threadIdx.x & 31;
-  bool ok = strip_inside(gw, nx, ny, ty);
-  if (ok) {
-    const int tiles_x = (nx + kSweepOut - 1) / kSweepOut;
-    const int gx = int(gw % tiles_x) * kSweepOut - 2 + lane, y0 = int(gw / tiles_x) * ty;
-    for (int r = y0 - 2; r <= y0 + ty + 1; ++r) {
-      const T v = z[(long long)r * nx + gx];
-      if (v != v) ok = false;
-    }
-  }
-  ok = __all_sync(kFull, ok);
-  if (lane == 0) flag[gw] = ok ? 1 : 0;
-}
-
-// One interior strip (strip_flags_kernel) of one solver's stage: the column sweep of
-// sweep_strip with every neighbour present and no mask to apply. The face fluxes are formed
-// from reconstructed face sides (side_m / side_p, then face_combine): each lane reconstructs
-// its east side once and its east neighbour takes those four values by shuffles. In FP64 the
-// arithmetic is the general path's, operation for operation; in FP32 the tangential
-// finiteness tests are dropped (they only matter for slopes that are not finite, which an
-// interior window without coded-out beds produces only from a non-finite state).
-template <typename T, int TY, bool P2, bool EDDY, bool COH = false>
-__device__ __forceinline__ void sweep_strip_interior(const StageParams<T>& P, long long gw) {
-  using DX = DivX<T, P2>;
-  constexpr bool TCHK = sizeof(T) == 8;
-  const Ctl* ctl = P.ctl;
-  const int nx = P.nx, ny = P.ny;
-  const int tiles_x = (nx + kSweepOut - 1) / kSweepOut;
-  const int lane = threadIdx.x;
-  const int tile_x = int(gw % tiles_x), tile_y = int(gw / tiles_x);
-  const int gx = tile_x * kSweepOut - 2 + lane;  // inside the mesh for every lane
-  const bool out_lane = lane >= 2 && lane < 2 + kSweepOut;
-  const int y0 = tile_y * TY;
-
-  const int cur = ctl->cur;
-  const double dt_d = ctl->dt;
-  const double tsub = ctl->t_local + P.c_s * dt_d;
-  const bool first = P.mode & M_FIRST, last = P.mode & M_LAST;
-  const T* Yh = first ? P.S[cur][0] : P.Yin[0];
-  const T* Yu = first ? P.S[cur][1] : P.Yin[1];
-  const T* Yv = first ? P.S[cur][2] : P.Yin[2];
-  const DX divx = MkDivX<DX>::make(P.dx), divy = MkDivX<DX>::make(P.dy);
-  const T hdx = T(0.5) * T(P.dx), hdy = T(0.5) * T(P.dy);
-  CellCtx<T, DX> c;
-  c.divx = divx; c.divy = divy;
-  c.divdt = mkdiv<T>(dt_d);
-  c.divL = mkdiv<T>(P.L);
-  c.dt = T(dt_d); c.dt_d = dt_d; c.tsub_d = tsub;
-  c.manning = P.manning; c.rain_mode = P.rain_mode; c.head_first = P.head_first;
-  const DevForcing fc = *P.fc;
-  // FP32 with tile datums: a vertical face crosses datum tiles where its right cell starts a
-  // tile column, a horizontal face where its upper row starts a tile row; there the upper /
-  // right cell's bed moves into the other cell's frame (face_frame)
-  const bool xcross = P.zdat != nullptr && (gx % kDatumTX) == 0;
-
-  auto load_row = [&](int r) {
-    const long long g = (long long)r * nx + gx;
-    RowV<T> v;
-    v.h = ldst<COH>(Yh, g); v.u = ldst<COH>(Yu, g); v.v = ldst<COH>(Yv, g);
-    v.z = ld(P.z, g);
-    v.zx = ld(P.zx, g); v.zy = ld(P.zy, g);
-    return v;
-  };
-  PfPlan<T> pf;
-  pf.init(P, fc, Yh, Yu, Yv, first, cur, gx - lane, lane);
-
-  RowV<T> Rm{}, R0{}, Rp{};
-  SlopeV<T> Sm{}, S0{};
-  T Smm_uy = T(0), Smm_vy = T(0);
-  T fyA[3] = {}, fyB[3] = {};
-  FaceF<T> FS{}, FN{};
-  double rain = 0.0, removed = 0.0, walls = 0.0, vol = 0.0;
-  T xcfl = T(0), xmin = T(1.0 / 0.0);
-  T xstep = T(0);  // datum step of the west face in the current tile row (xcross lanes)
-
-  for (int k = y0 - 2; k <= y0 + TY + 1; ++k) {
-    pf.rows(k, nx, ny);
-    Rm = R0; R0 = Rp; Rp = load_row(k);
-    if constexpr (EDDY) { Smm_uy = Sm.uy; Smm_vy = Sm.vy; }
-    Sm = S0;
-    fyA[0] = fyB[0]; fyA[1] = fyB[1]; fyA[2] = fyB[2];
-    if (k >= y0 - 1) {
-      fyB[0] = divy(Rp.h - R0.h);
-      fyB[1] = divy(Rp.u - R0.u);
-      fyB[2] = divy(Rp.v - R0.v);
-    }
-    // slopes of row k-1 (State.cpp:187-192), two-sided; the Y axis uses north as the left side
-    if (k >= y0) {
-      S0.hy = slope2s<T>(-fyB[0], -fyA[0], divy(Rm.h - Rp.h));
-      S0.uy = slope2s<T>(-fyB[1], -fyA[1], divy(Rm.u - Rp.u));
-      S0.vy = slope2s<T>(-fyB[2], -fyA[2], divy(Rm.v - Rp.v));
-      {
-        T r_ = dn1(R0.h), l_ = up1(R0.h);
-        T fq = divx(r_ - R0.h);
-        S0.hx = slope2s<T>(up1(fq), fq, divx(r_ - l_));
-      }
-      {
-        T r_ = dn1(R0.u), l_ = up1(R0.u);
-        T fq = divx(r_ - R0.u);
-        S0.ux = slope2s<T>(up1(fq), fq, divx(r_ - l_));
-      }
-      {
-        T r_ = dn1(R0.v), l_ = up1(R0.v);
-        T fq = divx(r_ - R0.v);
-        S0.vx = slope2s<T>(up1(fq), fq, divx(r_ - l_));
-      }
-    }
-    // horizontal face between rows k-2 and k-1 (face row fy = k-1), Fluxes.cpp:55-64
-    if (k >= y0 + 1 && out_lane) {
-      const int fy = k - 1;
-      const CellV<T> lo = mkcell(Rm, Sm);
-      CellV<T> hi = mkcell(R0, S0);
-      if (P.zdat != nullptr && (fy % kDatumTY) == 0) {
-        const long long tb = datum_tile(gx, fy, P.dtiles_x);
-        hi.z = T(double(hi.z) + (P.zdat[tb] - P.zdat[tb - P.dtiles_x]));
-      }
-      face_combine<T, 1, TCHK>(side_m<T, 1, TCHK>(lo, hdy), side_p<T, 1, TCHK>(hi, hdy), divy, FN);
-    }
-    // output row k-2
-    if (k >= y0 + 2) {
-      const int r = k - 2;
-      const CellV<T> me = mkcell(Rm, Sm);
-      EddyIn<T> ed{};
-      if constexpr (EDDY) {
-        if (P.eddy) {  // second derivatives of row r: x by shuffles, y from rows r+1, r, r-1
-          ed.ux = Sm.ux; ed.uy = Sm.uy; ed.vx = Sm.vx; ed.vy = Sm.vy;
-          {
-            T r_ = dn1(Sm.ux), l_ = up1(Sm.ux);
-            T fq = divx(r_ - Sm.ux);
-            ed.uxx = slope2s<T>(up1(fq), fq, divx(r_ - l_));
-          }
-          {
-            T r_ = dn1(Sm.vx), l_ = up1(Sm.vx);
-            T fq = divx(r_ - Sm.vx);
-            ed.vxx = slope2s<T>(up1(fq), fq, divx(r_ - l_));
-          }
-          ed.uyy = slope2s<T>(divy(Sm.uy - S0.uy), divy(Smm_uy - Sm.uy), divy(Smm_uy - S0.uy));
-          ed.vyy = slope2s<T>(divy(Sm.vy - S0.vy), divy(Smm_vy - Sm.vy), divy(Smm_vy - S0.vy));
-        }
-      }
-      // west face: the left lane's east side against this lane's west side
-      const Side<T> mE = side_m<T, 0, TCHK>(me, hdx);
-      const Side<T> mW{up1(mE.zb), up1(mE.h), up1(mE.un), up1(mE.ut)};
-      CellV<T> meW = me;
-      if (xcross) {
-        // the datum step across the tile column edge, read once per tile row: datums are
-        // multiples of 2^-10 m, so the step is exact in FP32 (below 2^14 m) and me.z + step
-        // rounds as the FP64 sum does; an inexact step (NaN here) takes the FP64 sum
-        if (r == y0 || (r % kDatumTY) == 0) {
-          const long long tb = datum_tile(gx, r, P.dtiles_x);
-          const double st = P.zdat[tb] - P.zdat[tb - 1];
-          xstep = double(T(st)) == st ? T(st) : Lim<T>::nan();
-        }
-        if (xstep == xstep) {
-          meW.z = me.z + xstep;
-        } else {
-          const long long tb = datum_tile(gx, r, P.dtiles_x);
-          meW.z = T(double(me.z) + (P.zdat[tb] - P.zdat[tb - 1]));
-        }
-      }
-      FaceF<T> FW;
-      face_combine<T, 0, TCHK>(mW, side_p<T, 0, TCHK>(meW, hdx), divx, FW);
-      const FaceF<T> FE{dn1(FW.h), dn1(FW.u), dn1(FW.v), dn1(FW.z)};
-      if (out_lane) {
-        const long long g = (long long)r * nx + gx;
-        finish_cell<T, CellCtx<T, DX>, EDDY, false, COH>(P, fc, c, g, gx, r, me.h, me.u, me.v, me.dhdx, me.dhdy,
-                                                    me.dzdx, me.dzdy, FW, FE, FS, FN, first, last, cur, dt_d, rain,
-                                                    removed, walls, xcfl, xmin, vol, &ed);
-      }
-    }
-    FS = FN;
-  }
-  if (last && !(P.mode & M_DEBUGK)) {
-    double mx = warp_max(double(xcfl)), mn = warp_min(double(xmin)), vs = warp_sum<T>(vol);
-    if (lane == 0) {
-      P.part[gw] = mx;
-      P.part[P.nblk + gw] = mn;
-      P.part[2 * P.nblk + gw] = vs;
-    }
-  }
-  if (P.mode & M_TALLY) {
-    double rs = warp_sum<T>(rain), os = warp_sum<T>(removed), ws = warp_sum<T>(walls);
-    if (lane == 0) store_tallies(P, gw, rs, os, ws, first, dt_d);
-  }
-}
-
-// The column sweeps of one stage are split over disjoint strip lists (general, interior,
-// interior pairs) that read the same inputs and write disjoint cells and partial slots. Each
-// of them lets the launch queued after it start at once (programmatic dependent launch: the
-// launcher marks the next sweep of the same stage as allowed to overlap), so the small
-// general launch over the edge strips runs beside the interior ones instead of as a tail. A
-// launch not marked that way (the next stage, the finalize) still waits for all of them.
-__device__ __forceinline__ void allow_overlap() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-// The general column sweep over the strips in P.bstrips (every strip when the list is null).
-template <typename T, int TY, int WPB, int MINB, bool P2, bool EDDY>
-__global__ void __launch_bounds__(32 * WPB, MINB) sweep_kernel(const __grid_constant__ StageParams<T> P) {
-  allow_overlap();
-  if (P.ctl->done) return;
-  const long long i = (long long)blockIdx.x * WPB + threadIdx.y;
-  long long gw = i;
-  if (P.bstrips) {
-    if (i >= P.n_bstrips) return;  // whole warp: no block-level synchronisation below
-    gw = P.bstrips[i];
-  } else {
-    const int tiles_x = (P.nx + kSweepOut - 1) / kSweepOut;
-    if (i >= (long long)tiles_x * ((P.ny + TY - 1) / TY)) return;
-  }
-  sweep_strip<T, TY, P2, EDDY>(P, gw);
-}
-
-// The interior column sweep over the strips in P.istrips.
-template <typename T, int TY, int WPB, int MINB, bool P2, bool EDDY>
-__global__ void __launch_bounds__(32 * WPB, MINB) sweep_interior_kernel(const __grid_constant__ StageParams<T> P) {
-  allow_overlap();
-  if (P.ctl->done) return;
-  const long long i = (long long)blockIdx.x * WPB + threadIdx.y;
-  if (i >= P.n_istrips) return;  // whole warp
-  sweep_strip_interior<T, TY, P2, EDDY>(P, P.istrips[i]);
-}
-
-// ---------------------------------------------------------------------------------------
-// Interior column sweep with two cells per lane (FP32). One warp sweeps a pair of adjacent
-// interior strips, 2 x kSweepOut = 56 output columns: lane l holds columns gx0 + 2l and
-// gx0 + 2l + 1 (gx0 = the pair's first output column - 2) and loads both as one 8-byte
-// vector per field. Lanes 1-28 write output; lanes 0 and 29 hold the two-column halo; lanes
-// 30-31 hold nothing that is used (their loads are clamped into the mesh). Per pair of cells
-// the x neighbours take three shuffles per field (the left lane's second cell, the right
-// lane's first cell and the left lane's right difference quotient) and the vertical faces
-// eight (the left lane's east face side, the right lane's west face flux), half of what the
-// one-cell sweep needs; the face between a lane's two cells needs none. The arithmetic per
-// face and per cell is the interior sweep's.
-// ---------------------------------------------------------------------------------------
-template <int TY, bool P2, bool EDDY>
-__device__ __forceinline__ void sweep_pair_interior(const StageParams<float>& P, long long gw) {
-  using T = float;
-  using DX = DivX<T, P2>;
-  const Ctl* ctl = P.ctl;
-  const int nx = P.nx, ny = P.ny;
-  const int tiles_x = (nx + kSweepOut - 1) / kSweepOut;
-  const int lane = threadIdx.x;
-  const int tile_x = int(gw % tiles_x), tile_y = int(gw / tiles_x);  // the pair's first strip
-  const int ca = tile_x * kSweepOut - 2 + 2 * lane;                    // columns ca, ca + 1
-  const int lc = min(ca, nx - 2);  // load column: even (nx is even for pairs), inside the mesh
-  const bool out_lane = lane >= 1 && lane <= kSweepOut;
-  const int y0 = tile_y * TY;
-
-  const int cur = ctl->cur;
-  const double dt_d = ctl->dt;
-  const double tsub = ctl->t_local + P.c_s * dt_d;
-  const bool first = P.mode & M_FIRST, last = P.mode & M_LAST;
-  const T* Yh = first ? P.S[cur][0] : P.Yin[0];
-  const T* Yu = first ? P.S[cur][1] : P.Yin[1];
-  const T* Yv = first ? P.S[cur][2] : P.Yin[2];
-  const DX divx = MkDivX<DX>::make(P.dx), divy = MkDivX<DX>::make(P.dy);
-  const T hdx = T(0.5) * T(P.dx), hdy = T(0.5) * T(P.dy);
-  CellCtx<T, DX> c;
-  c.divx = divx; c.divy = divy;
-  c.divdt = mkdiv<T>(dt_d);
-  c.divL = mkdiv<T>(P.L);
-  c.dt = T(dt_d); c.dt_d = dt_d; c.tsub_d = tsub;
-  c.manning = P.manning; c.rain_mode = P.rain_mode; c.head_first = P.head_first;
-  const DevForcing fc = *P.fc;
-  // tile datums: the first cell of a lane can start a datum tile column (the second one, at an
-  // odd column, never does), so only the west face of the first cell crosses tiles in x
-  const bool xcross = P.zdat != nullptr && (ca % kDatumTX) == 0;
-
-  auto ld2 = [&](const T* p, long long g) { return __ldg(reinterpret_cast<const float2*>(p + g)); };
-  auto load_row = [&](int r, RowV<T>& A, RowV<T>& B) {
-    const long long g = (long long)r * nx + lc;
-    float2 t;
-    t = ld2(Yh, g); A.h = t.x; B.h = t.y;
-    t = ld2(Yu, g); A.u = t.x; B.u = t.y;
-    t = ld2(Yv, g); A.v = t.x; B.v = t.y;
-    t = ld2(P.z, g); A.z = t.x; B.z = t.y;
-    t = ld2(P.zx, g); A.zx = t.x; B.zx = t.y;
-    t = ld2(P.zy, g); A.zy = t.x; B.zy = t.y;
-  };
-  auto prefetch_rows = [&](int k) {
-    {
-      const int r = min(k + 1 + kSweepPfWindow, ny - 1);
-      const long long g = (long long)r * nx + lc;
-      prefetch_l1(Yh + g); prefetch_l1(Yu + g); prefetch_l1(Yv + g);
-      prefetch_l1(P.z + g); prefetch_l1(P.zx + g); prefetch_l1(P.zy + g);
-    }
-    const int r = min(k - 2 + kSweepPfCell, ny - 1);
-    const long long g = (long long)r * nx + lc;
-    if (!first) {
-      for (int f = 0; f < 3; ++f) { prefetch_l1(P.S[cur][f] + g); prefetch_l1(P.S[cur ^ 1][f] + g); }
-    }
-    if (P.manning) {
-      for (int f = 0; f < 4; ++f)
-        if (P.man_p[f]) prefetch_l1(P.man_p[f] + g);
-    }
-    if (P.irate) { prefetch_l1(P.irate + g); prefetch_l1(P.icap + g); }
-    if (P.efx) { prefetch_l1(P.efx + g); prefetch_l1(P.efy + g); }
-    if (fc.rain_kind == 3) prefetch_l1(P.pat + g);
-    if (fc.rain_kind == 2) { prefetch_l1(P.q0p + g); prefetch_l1(P.q1p + g); }
-    if (fc.head_kind == 2) { prefetch_l1(P.hb0p + g); prefetch_l1(P.hb1p + g); }
-  };
-  // x slopes of a lane's two cells (values A, B) from their neighbours in the adjacent lanes
-  auto xslopes = [&](T A, T B, T& sa, T& sb) {
-    const T Bl = up1(B);          // column ca - 1
-    const T Ar = dn1(A);          // column ca + 2
-    const T qab = divx(B - A);
-    const T qbr = divx(Ar - B);
-    const T qla = up1(qbr);       // (A - Bl) / dx, formed by the left lane
-    sa = minmod3_finite(qla, qab, divx(B - Bl));
-    sb = minmod3_finite(qab, qbr, divx(Ar - A));
-  };
-
-  RowV<T> Rm[2] = {}, R0[2] = {}, Rp[2] = {};
-  SlopeV<T> Sm[2] = {}, S0[2] = {};
-  T Smm_uy[2] = {}, Smm_vy[2] = {};
-  T fyA[2][3] = {}, fyB[2][3] = {};
-  FaceF<T> FS[2] = {}, FN[2] = {};
-  double rain = 0.0, removed = 0.0, walls = 0.0, vol = 0.0;
-  T xcfl = T(0), xmin = T(1.0 / 0.0);
-
-  for (int k = y0 - 2; k <= y0 + TY + 1; ++k) {
-    prefetch_rows(k);
-#pragma unroll
-    for (int j = 0; j < 2; ++j) { Rm[j] = R0[j]; R0[j] = Rp[j]; }
-    load_row(k, Rp[0], Rp[1]);
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      if constexpr (EDDY) { Smm_uy[j] = Sm[j].uy; Smm_vy[j] = Sm[j].vy; }
-      Sm[j] = S0[j];
-      fyA[j][0] = fyB[j][0]; fyA[j][1] = fyB[j][1]; fyA[j][2] = fyB[j][2];
-      if (k >= y0 - 1) {
-        fyB[j][0] = divy(Rp[j].h - R0[j].h);
-        fyB[j][1] = divy(Rp[j].u - R0[j].u);
-        fyB[j][2] = divy(Rp[j].v - R0[j].v);
-      }
-    }
-    // slopes of row k-1 (State.cpp:187-192), two-sided; the Y axis uses north as the left side
-    if (k >= y0) {
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        S0[j].hy = minmod3_finite(-fyB[j][0], -fyA[j][0], divy(Rm[j].h - Rp[j].h));
-        S0[j].uy = minmod3_finite(-fyB[j][1], -fyA[j][1], divy(Rm[j].u - Rp[j].u));
-        S0[j].vy = minmod3_finite(-fyB[j][2], -fyA[j][2], divy(Rm[j].v - Rp[j].v));
-      }
-      xslopes(R0[0].h, R0[1].h, S0[0].hx, S0[1].hx);
-      xslopes(R0[0].u, R0[1].u, S0[0].ux, S0[1].ux);
-      xslopes(R0[0].v, R0[1].v, S0[0].vx, S0[1].vx);
-    }
-    // horizontal faces between rows k-2 and k-1 (face row fy = k-1), Fluxes.cpp:55-64
-    if (k >= y0 + 1 && out_lane) {
-      const int fy = k - 1;
-      double dz = 0.0;
-      const bool ycross = P.zdat != nullptr && (fy % kDatumTY) == 0;
-      if (ycross) {  // both cells of the lane lie in one datum tile column
-        const long long tb = datum_tile(ca, fy, P.dtiles_x);
-        dz = P.zdat[tb] - P.zdat[tb - P.dtiles_x];
-      }
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const CellV<T> lo = mkcell(Rm[j], Sm[j]);
-        CellV<T> hi = mkcell(R0[j], S0[j]);
-        if (ycross) hi.z = T(double(hi.z) + dz);
-        face_combine<T, 1, false>(side_m<T, 1, false>(lo, hdy), side_p<T, 1, false>(hi, hdy), divy, FN[j]);
-      }
-    }
-    // output row k-2
-    if (k >= y0 + 2) {
-      const int r = k - 2;
-      const CellV<T> meA = mkcell(Rm[0], Sm[0]), meB = mkcell(Rm[1], Sm[1]);
-      EddyIn<T> ed[2] = {};
-      if constexpr (EDDY) {
-        if (P.eddy) {  // second derivatives of row r: x from the lanes' slopes, y from rows r+1, r, r-1
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            ed[j].ux = Sm[j].ux; ed[j].uy = Sm[j].uy; ed[j].vx = Sm[j].vx; ed[j].vy = Sm[j].vy;
-            ed[j].uyy = minmod3_finite(divy(Sm[j].uy - S0[j].uy), divy(Smm_uy[j] - Sm[j].uy),
-                                       divy(Smm_uy[j] - S0[j].uy));
-            ed[j].vyy = minmod3_finite(divy(Sm[j].vy - S0[j].vy), divy(Smm_vy[j] - Sm[j].vy),
-                                       divy(Smm_vy[j] - S0[j].vy));
-          }
-          xslopes(Sm[0].ux, Sm[1].ux, ed[0].uxx, ed[1].uxx);
-          xslopes(Sm[0].vx, Sm[1].vx, ed[0].vxx, ed[1].vxx);
-        }
-      }
-      // west face of the first cell: the left lane's second cell's east side against it
-      const Side<T> eB = side_m<T, 0, false>(meB, hdx);
-      const Side<T> wA{up1(eB.zb), up1(eB.h), up1(eB.un), up1(eB.ut)};
-      CellV<T> meAW = meA;
-      if (xcross) {
-        const long long tb = datum_tile(ca, r, P.dtiles_x);
-        meAW.z = T(double(meA.z) + (P.zdat[tb] - P.zdat[tb - 1]));
-      }
-      FaceF<T> FWa, Fab;
-      face_combine<T, 0, false>(wA, side_p<T, 0, false>(meAW, hdx), divx, FWa);
-      // the face between the lane's two cells
-      face_combine<T, 0, false>(side_m<T, 0, false>(meA, hdx), side_p<T, 0, false>(meB, hdx), divx, Fab);
-      // east face of the second cell: the right lane's west face
-      const FaceF<T> FEb{dn1(FWa.h), dn1(FWa.u), dn1(FWa.v), dn1(FWa.z)};
-      if (out_lane) {
-        const long long g = (long long)r * nx + ca;
-        finish_cell<T, CellCtx<T, DX>, EDDY, false>(P, fc, c, g, ca, r, meA.h, meA.u, meA.v, meA.dhdx, meA.dhdy,
-                                                    meA.dzdx, meA.dzdy, FWa, Fab, FS[0], FN[0], first, last, cur,
-                                                    dt_d, rain, removed, walls, xcfl, xmin, vol, &ed[0]);
-        finish_cell<T, CellCtx<T, DX>, EDDY, false>(P, fc, c, g + 1, ca + 1, r, meB.h, meB.u, meB.v, meB.dhdx,
-                                                    meB.dhdy, meB.dzdx, meB.dzdy, Fab, FEb, FS[1], FN[1], first, last,
-                                                    cur, dt_d, rain, removed, walls, xcfl, xmin, vol, &ed[1]);
-      }
-    }
-    FS[0] = FN[0];
-    FS[1] = FN[1];
-  }
-  // the pair's partials go to its first strip's slot; the second strip's slot gets the
-  // identities (max 0, min +inf, sums 0)
-  if (last && !(P.mode & M_DEBUGK)) {
-    double mx = warp_max(double(xcfl)), mn = warp_min(double(xmin)), vs = warp_sum<T>(vol);
-    if (lane == 0) {
-      P.part[gw] = mx;
-      P.part[P.nblk + gw] = mn;
-      P.part[2 * P.nblk + gw] = vs;
-      P.part[gw + 1] = 0.0;
-      P.part[P.nblk + gw + 1] = 1.0 / 0.0;
-      P.part[2 * P.nblk + gw + 1] = 0.0;
-    }
-  }
-  if (P.mode & M_TALLY) {
-    double rs = warp_sum<T>(rain), os = warp_sum<T>(removed), ws = warp_sum<T>(walls);
-    if (lane == 0) {
-      store_tallies(P, gw, rs, os, ws, first, dt_d);
-      store_tallies(P, gw + 1, 0.0, 0.0, 0.0, first, dt_d);
-    }
-  }
-}
-
-// The two-cells-per-lane interior sweep over the strip pairs in P.ipairs (each entry the
-// pair's first strip).
-template <int TY, int WPB, int MINB, bool P2, bool EDDY>
-__global__ void __launch_bounds__(32 * WPB, MINB) sweep_pair_kernel(const __grid_constant__ StageParams<float> P) {
-  allow_overlap();
-  if (P.ctl->done) return;
-  const long long i = (long long)blockIdx.x * WPB + threadIdx.y;
-  if (i >= P.n_ipairs) return;  // whole warp
-  sweep_pair_interior<TY, P2, EDDY>(P, P.ipairs[i]);
-}
-
-// Batched column sweep: the strips of every instance of a batch, warp_start[i] being the
-// first global warp of instance i. Each warp finds its instance, stages its parameters in
-// shared memory and sweeps its strip; instances whose step is finished return at once.
-template <typename T, int TY, int WPB, int MINB, bool P2, bool EDDY>
-__global__ void __launch_bounds__(32 * WPB, MINB)
-    sweep_batch_kernel(const StageParams<T>* __restrict__ Ps, const long long* __restrict__ warp_start, int ninst) {
-  __shared__ __align__(16) StageParams<T> Psh[WPB];
-  const long long gw = (long long)blockIdx.x * WPB + threadIdx.y;
-  if (gw >= warp_start[ninst]) return;  // whole warp
-  int inst = 0;
-  if (threadIdx.x == 0) {
-    int lo = 0, hi = ninst - 1;  // last instance with warp_start[i] <= gw
-    while (lo < hi) {
-      int mid = (lo + hi + 1) / 2;
-      if (warp_start[mid] <= gw) lo = mid;
-      else hi = mid - 1;
-    }
-    inst = lo;
-  }
-  inst = __shfl_sync(kFull, inst, 0);
-  static_assert(sizeof(StageParams<T>) % 4 == 0, "parameter block copied as 32-bit words");
-  const unsigned* src = reinterpret_cast<const unsigned*>(Ps + inst);
-  unsigned* dst = reinterpret_cast<unsigned*>(&Psh[threadIdx.y]);
-  for (int i = threadIdx.x; i < int(sizeof(StageParams<T>) / 4); i += 32) dst[i] = src[i];
-  __syncwarp();
-  const StageParams<T>& P = Psh[threadIdx.y];
-  if (P.ctl->done) return;
-  sweep_strip<T, TY, P2, EDDY>(P, gw - warp_start[inst]);
-}
+namespace svk {
 
 // Bed slopes once per bed upload (SaintVenantConstants, Constants.cpp:39-40).
 // The slopes are computed in T and stored as TO (FP32 with tile datums: FP64 slopes of the
@@ -1851,7 +1026,6 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 
 constexpr int kPersistWarps = 4;   // warps per block
-constexpr int kPersistRows = 32;   // column-sweep strip height (the batches' variant 8)
 
 #ifdef SV_DEFINE_COMMON_KERNELS
 // mark the members whose step queue starts with nothing to do (their controller is done)
@@ -1877,9 +1051,10 @@ __device__ __forceinline__ void finalize_warp(const FinalizeParams& F) {
   __syncwarp();
 }
 
-template <typename T, bool P2, bool EDDY>
-__global__ void __launch_bounds__(32 * kPersistWarps, 4) persist_batch_kernel(const PersistParams<T> PP) {
+template <typename T, int MINB, bool P2, bool EXTRA>
+__global__ void __launch_bounds__(32 * kPersistWarps, MINB) persist_batch_kernel(const PersistParams<T> PP) {
   __shared__ __align__(16) StageParams<T> Psh[kPersistWarps];
+  extern __shared__ __align__(16) unsigned char sweep_smem[];
   const int lane = threadIdx.x, wib = threadIdx.y;
   const int N = PP.nstages, nact = PP.nact;
   const long long gwarp = (long long)blockIdx.x * kPersistWarps + wib;
@@ -1977,15 +1152,8 @@ __global__ void __launch_bounds__(32 * kPersistWarps, 4) persist_batch_kernel(co
       unsigned* dst = reinterpret_cast<unsigned*>(&Psh[wib]);
       for (int i = lane; i < int(sizeof(StageParams<T>) / 4); i += 32) dst[i] = src[i];
       __syncwarp();
-      // the member's interior strips (listed first) run the interior sweep
       const StageParams<T>& SP = Psh[wib];
-      const long long item = (long long)(r % ns);
-      if (SP.istrips && item < SP.n_istrips)
-        sweep_strip_interior<T, kPersistRows, P2, EDDY, true>(SP, SP.istrips[item]);
-      else if (SP.bstrips)
-        sweep_strip<T, kPersistRows, P2, EDDY, true>(SP, SP.bstrips[item - SP.n_istrips]);
-      else
-        sweep_strip<T, kPersistRows, P2, EDDY, true>(SP, item);
+      sweep_strip<T, P2, EXTRA, true>(SP, SP.strips[r % ns], reinterpret_cast<SweepShared<T>*>(sweep_smem)[wib]);
       __syncwarp();
     } else {
       finalize_warp(PP.Fs[pick]);

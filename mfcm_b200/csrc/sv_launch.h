@@ -18,38 +18,56 @@ template <typename T> size_t stage_smem_bytes(int tile);
 template <typename T> cudaError_t launch_stage(const StageParams<T>& P, int tile, cudaStream_t s);
 
 // Stage-kernel variants, in two schedules:
-//  fused (one pass per RK stage): 0..3 the tiled shared-memory kernel with kTiles[v]; 4..10
-//   the column-sweep kernel with 16 / 32 / 64 / 32 / 32 / 32 / 32 output rows per warp, the
-//   last four with register caps for 3, 4, 5 and 6 resident 4-warp blocks per SM; 12, 13
-//   (FP32 only) the column sweep of 32-row strips whose interior strip pairs run two cells
-//   per lane (sweep_pair_kernel), with register caps for 3 and 4 blocks per SM; 14, 15 (FP32
-//   only) the one-cell sweep of 32-row strips capped for 7 and 8 blocks per SM;
+//  fused (one pass per RK stage): 0..3 the tiled shared-memory kernel with kTiles[v]; 4..10 and
+//   12..17 the column sweep with the strip heights and register caps (resident 4-warp blocks per
+//   SM) of kSweeps; variant 5 takes both from the mesh size;
 //  split (two passes per RK stage): 11 the slopes pass (slopes_kernel) then the tiled 32 x 8
 //   kernel at 3 CTAs/SM reading those slopes.
-constexpr int kNumVariants = 16;
+constexpr int kNumVariants = 18;
 constexpr int kSplitVariant = 11;
-constexpr int kSweepRows[7] = {16, 32, 64, 32, 32, 32, 32};
-inline bool variant_is_pair(int v) { return v == 12 || v == 13; }
-// variants compiled for FP32 solvers only (the two-cells-per-lane sweep, the tightest caps)
+constexpr int kAutoVariant = 5;
+struct SweepShape { int rows, cap; };
+constexpr SweepShape kSweeps[kNumVariants] = {{0, 0},  {0, 0},  {0, 0},  {0, 0},  {16, 4}, {32, 4},
+                                              {64, 4}, {32, 3}, {32, 4}, {32, 5}, {32, 6}, {0, 0},
+                                              {32, 3}, {32, 4}, {32, 7}, {32, 8}, {8, 4}, {4, 4}};
+// resident blocks per SM of the batch kernels, and of the sweeps with every source term
+template <typename T> constexpr int kBatchCap = sizeof(T) == 8 ? 4 : 6;
+template <typename T> constexpr int kExtraCap = sizeof(T) == 8 ? 3 : 4;
+// variants compiled for FP32 solvers only
 inline bool variant_is_fp32_only(int v) { return v >= 12 && v <= 15; }
-inline bool variant_is_sweep(int v) { return (v >= 4 && v <= 10) || (v >= 12 && v <= 15); }
+inline bool variant_is_sweep(int v) { return v >= 0 && v < kNumVariants && kSweeps[v].rows > 0; }
 inline bool variant_is_split(int v) { return v == kSplitVariant; }
-// column-sweep variants: output rows per strip (0 for the other variants)
-inline int variant_sweep_rows(int v) {
-  if (v >= 4 && v <= 10) return kSweepRows[v - 4];
-  return (v >= 12 && v <= 15) ? 32 : 0;
+// Strip height by mesh size: the tallest of 32, 16, 8 and 4 rows that still gives every SM its
+// 16 resident warps, else 4. A strip marches its rows one after another, so a mesh of few strips
+// waits for one warp's latency (2.0-3.3 us a row); a short strip repeats more of its neighbours'
+// rows. Per FP64 stage on B200, 32 / 16 / 8 / 4 rows: 117 / 64 / 38 / 27 us at 256 x 256,
+// 149 / 93 / 91 / 97 us at 1024 x 1024, 923 / 955 / 1059 / 1293 us at 4096 x 4096; FP32: 54 / 32 /
+// 22 / 17, 60 / 41 / 45 / 54, 445 / 485 / 581 / 793 us.
+constexpr long long kFillStrips = 148 * 16;
+inline int auto_rows(long long nx, long long ny) {
+  const long long tiles_x = (nx + kSweepOut - 1) / kSweepOut;
+  for (int rows = 32; rows > 4; rows /= 2)
+    if (tiles_x * ((ny + rows - 1) / rows) >= kFillStrips) return rows;
+  return 4;
 }
+// column-sweep variants: output rows per strip on a mesh (0 for the other variants)
+inline int variant_sweep_rows(int v, long long nx, long long ny) {
+  if (v == kAutoVariant) return auto_rows(nx, ny);
+  return variant_is_sweep(v) ? kSweeps[v].rows : 0;
+}
+template <typename T> inline int variant_cap(int v) { return kSweeps[v].cap; }
 // per-CTA (tiled) or per-warp (sweep) partial count
 inline long long variant_partials(int v, long long nx, long long ny) {
   if (v == kSplitVariant) v = 1;  // the split schedule's stage pass is the tiled 32 x 8 kernel
   if (v < 4) return ((nx + kTiles[v].tx - 1) / kTiles[v].tx) * ((ny + kTiles[v].ty - 1) / kTiles[v].ty);
-  const long long ty = variant_sweep_rows(v);
+  const long long ty = variant_sweep_rows(v, nx, ny);
   return ((nx + kSweepOut - 1) / kSweepOut) * ((ny + ty - 1) / ty);
 }
-template <typename T> cudaError_t launch_variant(const StageParams<T>& P, int variant, cudaStream_t s);
-// per-strip interior flags of the column sweep with `ty` output rows (strip_flags_kernel)
-template <typename T> cudaError_t launch_strip_flags(const T* z, int nx, int ny, int ty, long long nstrips,
-                                                     unsigned char* flags, cudaStream_t s);
+// extra: source terms, boundaries or a tableau that the lean sweep leaves out (sweep_rows)
+template <typename T> cudaError_t launch_variant(const StageParams<T>& P, int variant, bool extra, cudaStream_t s);
+// classes of the column sweep's strips of `rows` rows (strip_class_kernel)
+template <typename T> cudaError_t launch_strip_classes(const T* z, int nx, int ny, double dx, double dy, int rows,
+                                                       long long nstrips, unsigned char* cls, cudaStream_t s);
 template <typename T> cudaError_t launch_bed_slopes(const T* z, int nx, int ny, double dx, double dy, T* zx, T* zy,
                                                     cudaStream_t s);
 // FP64 <-> T conversion of a field on the device
@@ -67,17 +85,13 @@ template <typename T> cudaError_t launch_volume(const T* h, int nx, int ny, doub
                                                 cudaStream_t s);
 template <typename T> cudaError_t launch_debug(const StageParams<T>& P, const DebugParams<T>& D, T* nh, T* sf,
                                                cudaStream_t s);
-// batched launches: every tile of every instance (tiled 32 x 8 kernel, 3 CTAs/SM); p2 when
-// every instance's dx and dy are powers of two, eddy when any instance has eddy viscosity
-template <typename T> cudaError_t launch_stage_batch(const StageParams<T>* Ps, const long long* tile_start, int ninst,
-                                                     long long total_tiles, bool p2, bool eddy, cudaStream_t s);
-// batches of FP64 instances use the tiled variant 1; FP32 batches the column sweep of
-// variant 8 (launch_sweep_batch), the fastest single-solver kernels of each precision
-template <typename T> constexpr int batch_variant() { return sizeof(T) == 8 ? 1 : 8; }
+// batched launches: every strip of every instance; p2 when every instance's dx and dy are powers
+// of two, extra when any instance needs it
+constexpr int kBatchVariant = 8;
 template <typename T> cudaError_t launch_sweep_batch(const StageParams<T>* Ps, const long long* warp_start, int ninst,
-                                                     long long total_warps, bool p2, bool eddy, cudaStream_t s);
+                                                     long long total_warps, bool p2, bool extra, cudaStream_t s);
 // persistent batch kernel (persist_batch_kernel), cooperative launch filling the device
-template <typename T> cudaError_t launch_persist(const PersistParams<T>& PP, bool p2, bool eddy, cudaStream_t s);
+template <typename T> cudaError_t launch_persist(const PersistParams<T>& PP, bool p2, bool extra, cudaStream_t s);
 cudaError_t launch_persist_init(const FinalizeParams* Fs, PersistMember* mem, const long long* warp_start, int nact,
                                 cudaStream_t s);
 cudaError_t launch_finalize(const FinalizeParams& F, cudaStream_t s);

@@ -201,7 +201,7 @@ extern "C" int sv_timestep_noalloc(const sv_mesh_desc* mesh, const sv_params* pa
       P.Kout[fld] = nullptr;
       for (int j = 0; j < 4; ++j) P.Kin[j][fld] = nullptr;
     }
-    e = svk::launch_variant<double>(P, kVariant, s);
+    e = svk::launch_variant<double>(P, kVariant, false, s);
     if (e != cudaSuccess) return fail(SV_E_CUDA, cudaGetErrorString(e));
   }
   svk::FinalizeParams F{};

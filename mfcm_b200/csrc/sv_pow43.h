@@ -56,18 +56,31 @@ SV_HD double pow43(double x) {
   // h > 1e-6, i.e. x > 0; everything else is passed through unchanged
   // (NaN stays NaN, inf stays inf).
   if (!(x > 0.0) || !(x < 1.0e300)) return x;
-  int e;
 #if defined(__CUDA_ARCH__)
-  double m = frexp(x, &e);
+  // the split on the exponent bits (frexp and ldexp take every subnormal case into account,
+  // some sixty integer instructions; here only a subnormal x needs them)
+  int e, hi = __double2hiint(x);
+  double w;
+  if (hi < 0x00100000) {
+    const double m = frexp(x, &e);
+    hi = __double2hiint(m);
+    w = m;
+  } else {
+    e = (hi >> 20) - 1022;
+    w = x;
+  }
+  const int q = int(unsigned(e + 3072) / 3u) - 1024, r = e - 3 * q;
+  w = __hiloint2double((hi & 0x000fffff) | ((1022 + r) << 20), __double2loint(w));
 #else
+  int e;
   double m = std::frexp(x, &e);
-#endif
   // floor division of e by 3 (e may be negative)
   int q = (e >= 0) ? (e / 3) : -((-e + 2) / 3);
   int r = e - 3 * q;
   double w = m;
   if (r == 1) w = SVP_MUL(m, 2.0);
   else if (r == 2) w = SVP_MUL(m, 4.0);
+#endif
   double y = SVP_ADD(SVP_MUL(SVP_ADD(SVP_MUL(SVP_ADD(SVP_MUL(kRcbrtSeed3, w), kRcbrtSeed2), w),
                                      kRcbrtSeed1), w), kRcbrtSeed0);
   for (int it = 0; it < 3; ++it) {
@@ -78,7 +91,7 @@ SV_HD double pow43(double x) {
   double res = SVP_SUB(SVP_MUL(SVP_MUL(cb, cb), cb), w);
   cb = SVP_SUB(cb, SVP_MUL(res, SVP_MUL(SVP_MUL(y, y), kThird)));
 #if defined(__CUDA_ARCH__)
-  double c = ldexp(cb, q);
+  const double c = SVP_MUL(cb, __hiloint2double((1023 + q) << 20, 0));  // exact: 2^q is normal
 #else
   double c = std::ldexp(cb, q);
 #endif
