@@ -164,12 +164,6 @@ struct Solver final : public sv_ctx {
   T* eddy_mup = nullptr;
   int term_order_[3] = {SV_TERM_MANNING, SV_TERM_ELOSS, SV_TERM_EDDY};
   bool order_set = false;  // else roughness / energy loss per SV_FLAG_ELOSS_FIRST, then eddy viscosity
-  // FP32 with the batches' variant runs the batched column sweep as a batch of one, so a
-  // solver on its own and a batch member execute the same machine code and give the same
-  // bits (FP32 is contracted per kernel); that kernel reads its parameters from device memory
-  svk::StageParams<T>* d_sp = nullptr;  // [N] stage parameters + [1] for the autotuner
-  long long* d_ws = nullptr;            // warp starts: {0, nblk} and, for the autotuner, {0, n}
-  unsigned long long sp_version = ~0ull;
   // debug buffers (per-function parity path)
   T* dbg_slp[8] = {};
   T* dbg_face[5] = {};
@@ -204,7 +198,23 @@ struct Solver final : public sv_ctx {
   std::map<int, Strips> strips_;
   unsigned char* d_scls = nullptr;
   size_t scls_size = 0;
-  int sweep_rows(int v) const { return svk::variant_sweep_rows(v, (long long)mesh.nx, (long long)mesh.ny); }
+  int batch_rows = 0;  // a batch member's strip height, chosen by its batch (0: none)
+  int sweep_rows(int v) const {
+    return v == svk::kBatchVariant && batch_rows ? batch_rows
+                                                 : svk::variant_sweep_rows(v, (long long)mesh.nx, (long long)mesh.ny);
+  }
+  // partial slots of variant v
+  long long partials(int v) const {
+    const int rows = sweep_rows(v);
+    return rows ? svk::strip_count((long long)mesh.nx, (long long)mesh.ny, rows)
+                : svk::variant_partials(v, (long long)mesh.nx, (long long)mesh.ny);
+  }
+  void set_batch_rows(int rows) {
+    if (rows == batch_rows) return;
+    batch_rows = rows;
+    nblk = partials(variant);
+    graph_dirty = true; ++pversion;
+  }
   void invalidate_strips() {
     for (auto& x : strips_) x.second.valid = false;
     graph_dirty = true; ++pversion;
@@ -215,7 +225,7 @@ struct Solver final : public sv_ctx {
     if (rows == 0) return SV_OK;
     Strips& L = strips_[rows];
     if (L.valid) return SV_OK;
-    const long long n = svk::variant_partials(v, (long long)mesh.nx, (long long)mesh.ny);
+    const long long n = partials(v);
     if (n >= (1LL << 30)) return fail(SV_E_LIMIT, "mesh has too many sweep strips");
     if (!L.d) SV_CUDA(alloc(&L.d, size_t(n)));
     if (size_t(n) > scls_size) {
@@ -246,7 +256,7 @@ struct Solver final : public sv_ctx {
     auto it = strips_.find(P.rows);
     if (P.rows == 0 || it == strips_.end() || !it->second.valid) return;
     P.strips = it->second.d;
-    P.n_strips = int(svk::variant_partials(v, (long long)mesh.nx, (long long)mesh.ny));
+    P.n_strips = int(partials(v));
   }
   // source terms, boundary fields or a tableau beyond the lean sweep (svk::sweep_rows)
   bool extra() const {
@@ -683,39 +693,27 @@ struct Solver final : public sv_ctx {
     P.hc[1] = hcomp[1];
     P.manning = prm.manning; P.rain_mode = prm.rain_mode; P.head_first = prm.head_first;
     P.nstages = N;
+    P.mode = (diag ? svk::M_ACC : svk::M_STOREK) | ((prm.flags & SV_FLAG_NO_TALLIES) ? 0 : svk::M_TALLY);
+    for (int st = 0; st < N; ++st) {
+      P.c[st] = tab.c(st + 1);
+      P.b[st] = tab.b(st + 1);
+      if (st < N - 1)
+        for (int j = 0; j <= st; ++j) P.a[st][j] = tab.A(st + 2, j + 1);
+    }
+    for (int f = 0; f < 3; ++f) {
+      for (int b = 0; b < 2; ++b) P.Y[b][f] = Y[b][f];
+      for (int st = 0; st < 3; ++st) P.K[st][f] = K[st][f];
+    }
     P.ctl = ctl;
     P.part = part;
     P.nblk = nblk;
     return P;
   }
 
-  // Launch the N stages of one timestep and the finalize kernel (RungeKutta.cpp:147-167).
-  // Stage s of a timestep (RungeKutta.cpp:147-153): mode, RK coefficients and buffers.
-  svk::StageParams<T> stage_params(int st) const {
+  // every stage's parameters with the solver's kernel variant (RungeKutta.cpp:147-153)
+  svk::StageParams<T> stage_params() const {
     svk::StageParams<T> P = base_params();
     set_strips(P, variant);
-    const bool tally = !(prm.flags & SV_FLAG_NO_TALLIES);
-    P.stage = st;
-    P.c_s = tab.c(st + 1);
-    int mode = 0;
-    if (st == 0) mode |= svk::M_FIRST;
-    if (st == N - 1) mode |= svk::M_LAST;
-    if (diag) mode |= svk::M_ACC;
-    else if (st < N - 1) mode |= svk::M_STOREK;
-    if (tally) mode |= svk::M_TALLY;
-    P.mode = mode;
-    for (int j = 0; j < 4; ++j) { P.a_next[j] = 0.0; P.b[j] = 0.0; }
-    if (st < N - 1)
-      for (int j = 0; j <= st; ++j) P.a_next[j] = tab.A(st + 2, j + 1);
-    for (int j = 0; j < N; ++j) P.b[j] = tab.b(j + 1);
-    // stage inputs: U_[0] (s = 0), then Y[0], Y[1], Y[0] ...
-    const int in = (st - 1) & 1, out = st & 1;
-    for (int f = 0; f < 3; ++f) {
-      P.Yin[f] = st > 0 ? Y[in][f] : nullptr;
-      P.Yout[f] = st < N - 1 ? Y[out][f] : nullptr;
-      P.Kout[f] = (!diag && st < N - 1) ? K[st][f] : nullptr;
-      for (int j = 0; j < 4; ++j) P.Kin[j][f] = (!diag && j < N - 1) ? K[j][f] : nullptr;
-    }
     return P;
   }
   svk::FinalizeParams finalize_params(bool auto_mode) const {
@@ -733,50 +731,19 @@ struct Solver final : public sv_ctx {
     return F;
   }
 
-  bool batch_path(int v) const { return sizeof(T) == 4 && v == svk::kBatchVariant; }
-  bool pow2_mesh() const {
-    int e;
-    return std::frexp(mesh.dx, &e) == 0.5 && std::frexp(mesh.dy, &e) == 0.5;
-  }
-  // Device copy of the stage parameters for the batch-of-one path (outside stream capture).
-  int ensure_dev_params() {
-    int r = ensure_strips(variant);
-    if (r || !batch_path(variant)) return r;
-    if (sp_version == pversion) return SV_OK;
-    if (!d_sp) {
-      SV_CUDA(alloc(&d_sp, size_t(N + 1)));
-      SV_CUDA(alloc(&d_ws, size_t(4)));
-    }
-    std::vector<svk::StageParams<T>> hp(N);
-    for (int st = 0; st < N; ++st) hp[st] = stage_params(st);
-    long long ws[2] = {0, nblk};
-    SV_CUDA(cudaMemcpyAsync(d_sp, hp.data(), sizeof(svk::StageParams<T>) * N, cudaMemcpyHostToDevice, stream));
-    SV_CUDA(cudaMemcpyAsync(d_ws, ws, sizeof(ws), cudaMemcpyHostToDevice, stream));
-    SV_CUDA(cudaStreamSynchronize(stream));
-    sp_version = pversion;
-    return SV_OK;
-  }
-  cudaError_t launch_stage_kernel(const svk::StageParams<T>& P, int st) {
-    if (batch_path(variant))
-      return svk::launch_sweep_batch<T>(d_sp + st, d_ws, 1, nblk, pow2_mesh(), extra(), stream);
-    return svk::launch_variant<T>(P, variant, extra(), stream);
-  }
-
   // Launch the N stages of one timestep and the finalize kernel (RungeKutta.cpp:147-167).
   // ev: if non-null, 2*(N+1) events recorded around every kernel (stages, then finalize)
   int enqueue_timestep(bool auto_mode, cudaEvent_t* ev = nullptr) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     SV_CUDA(cudaStreamIsCapturing(stream, &cs));
     if (cs == cudaStreamCaptureStatusNone) {
-      int r = ensure_dev_params();
+      int r = ensure_strips(variant);
       if (r) return r;
-    } else if (batch_path(variant) && sp_version != pversion) {
-      return fail(SV_E_STATE, "stage parameters not on the device before capture");
     }
+    const svk::StageParams<T> P = stage_params();
     for (int st = 0; st < N; ++st) {
-      svk::StageParams<T> P = stage_params(st);
       if (ev) SV_CUDA(cudaEventRecord(ev[2 * st], stream));
-      cudaError_t e = launch_stage_kernel(P, st);
+      cudaError_t e = svk::launch_variant<T>(P, st, variant, extra(), stream);
       if (e != cudaSuccess) return cuda_fail(e, "stage kernel");
       if (ev) SV_CUDA(cudaEventRecord(ev[2 * st + 1], stream));
     }
@@ -807,9 +774,8 @@ struct Solver final : public sv_ctx {
     SV_CUDA(cudaMemcpyAsync(dbg_ctl, &c, sizeof(Ctl), cudaMemcpyHostToDevice, stream));
     svk::StageParams<T> P = base_params();
     P.ctl = dbg_ctl;
-    P.c_s = 0.0;
-    for (int f = 0; f < 3; ++f) P.Kout[f] = dbg_k[f];
     svk::DebugParams<T> D{};
+    for (int f = 0; f < 3; ++f) D.k[f] = dbg_k[f];
     D.nx = int(mesh.nx); D.ny = int(mesh.ny); D.dx = mesh.dx; D.dy = mesh.dy;
     D.h = S[cur][0]; D.u = S[cur][1]; D.v = S[cur][2]; D.z = z;
     D.dhdx = dbg_slp[0]; D.dudx = dbg_slp[1]; D.dvdx = dbg_slp[2]; D.dzdx = dbg_slp[3];
@@ -854,7 +820,7 @@ struct Solver final : public sv_ctx {
 
   int build_graph() {
     if (graph) { cudaGraphExecDestroy(graph); graph = nullptr; }
-    int r0 = ensure_dev_params();
+    int r0 = ensure_strips(variant);
     if (r0) return r0;
     cudaGraph_t g;
     SV_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
@@ -973,7 +939,7 @@ struct Solver final : public sv_ctx {
       if (r) return r;
     }
     variant = v;
-    nblk = svk::variant_partials(variant, (long long)mesh.nx, (long long)mesh.ny);
+    nblk = partials(variant);
     graph_dirty = true; ++pversion;
     return SV_OK;
   }
@@ -992,16 +958,7 @@ struct Solver final : public sv_ctx {
     SV_CUDA(cudaMemcpyAsync(dbg_ctl, &c, sizeof(Ctl), cudaMemcpyHostToDevice, stream));
     svk::StageParams<T> P = base_params();
     P.ctl = dbg_ctl;
-    P.stage = 0;
-    P.c_s = tab.c(1);
-    P.mode = svk::M_FIRST | (N == 1 ? svk::M_LAST : 0) | (diag ? svk::M_ACC : svk::M_STOREK);
-    for (int j = 0; j < 4; ++j) { P.a_next[j] = 0.0; P.b[j] = 0.0; }
-    if (N > 1) P.a_next[0] = tab.A(2, 1);
-    for (int j = 0; j < N; ++j) P.b[j] = tab.b(j + 1);
-    for (int f = 0; f < 3; ++f) {
-      P.Yout[f] = Y[0][f];
-      P.Kout[f] = (!diag && N > 1) ? K[0][f] : nullptr;
-    }
+    P.mode &= ~svk::M_TALLY;
     // the timing launches consume infiltration capacity: give them a copy
     T* cap_copy = nullptr;
     if (P.icap) {
@@ -1018,32 +975,16 @@ struct Solver final : public sv_ctx {
     for (int v = 0; v < svk::kNumVariants; ++v) {
       if (datum && !svk::variant_is_sweep(v)) continue;
       if (svk::variant_is_fp32_only(v) && sizeof(T) != 4) continue;
-      P.nblk = svk::variant_partials(v, (long long)mesh.nx, (long long)mesh.ny);
-      {
-        int rs = ensure_strips(v);
-        if (rs) return rs;
-      }
+      P.nblk = partials(v);
+      int rs = ensure_strips(v);
+      if (rs) return rs;
       if (svk::variant_is_split(v)) {
-        int rs = ensure_split();
+        rs = ensure_split();
         if (rs) return rs;
         for (int f = 0; f < 6; ++f) P.pslp[f] = pslp[f];
       }
       set_strips(P, v);
-      // the batch variant runs as the batched kernel (see launch_stage_kernel): time that one
-      auto launch = [&]() -> cudaError_t {
-        if (!batch_path(v)) return svk::launch_variant<T>(P, v, extra(), stream);
-        return svk::launch_sweep_batch<T>(d_sp + N, d_ws + 2, 1, P.nblk, pow2_mesh(), extra(), stream);
-      };
-      if (batch_path(v)) {
-        if (!d_sp) {
-          SV_CUDA(alloc(&d_sp, size_t(N + 1)));
-          SV_CUDA(alloc(&d_ws, size_t(4)));
-        }
-        long long ws[2] = {0, P.nblk};
-        SV_CUDA(cudaMemcpyAsync(d_sp + N, &P, sizeof(P), cudaMemcpyHostToDevice, stream));
-        SV_CUDA(cudaMemcpyAsync(d_ws + 2, ws, sizeof(ws), cudaMemcpyHostToDevice, stream));
-        SV_CUDA(cudaStreamSynchronize(stream));
-      }
+      auto launch = [&]() -> cudaError_t { return svk::launch_variant<T>(P, 0, v, extra(), stream); };
       cudaError_t e = launch();  // warm-up
       if (e != cudaSuccess) return cuda_fail(e, "autotune launch");
       SV_CUDA(cudaEventRecord(ev0, stream));
@@ -1135,15 +1076,16 @@ struct Batch final : public sv_batch_base {
   cudaStream_t stream = nullptr;
   std::vector<Solver<T>*> members;  // slot id -> member (nullptr when removed)
   // device arrays, rebuilt when membership changes
-  svk::StageParams<T>* d_params = nullptr;  // [N][nact]
+  svk::StageParams<T>* d_params = nullptr;  // [nact]
   svk::FinalizeParams* d_fin = nullptr;     // [nact]
   long long* d_tiles = nullptr;             // [nact + 1]
   Ctl** d_ctls = nullptr;                   // [nact]
   int* d_done = nullptr;                    // [nact]
   svk::StepQueue* d_queue = nullptr;        // [nact] steps queued by the current advance
   int nact = 0, cap = 0;
-  long long total_tiles = 0, max_nblk = 0;  // partial slots of all members, of the largest one
+  long long max_nblk = 0;  // partial slots of the largest member
   bool p2 = true, extra = false, dirty = true;
+  std::vector<svk::StageParams<T>> params;  // [nact], as on the device
   std::vector<int> active;                  // slot ids in launch order
   std::vector<unsigned long long> versions; // members' pversion at the last rebuild
   cudaGraphExec_t graph = nullptr;
@@ -1259,7 +1201,7 @@ struct Batch final : public sv_batch_base {
     if (nact > cap) {
       free_arrays();
       int c = std::max(nact, 8);
-      SV_CUDA(cudaMalloc(&d_params, sizeof(svk::StageParams<T>) * size_t(N) * c));
+      SV_CUDA(cudaMalloc(&d_params, sizeof(svk::StageParams<T>) * c));
       SV_CUDA(cudaMalloc(&d_fin, sizeof(svk::FinalizeParams) * c));
       SV_CUDA(cudaMalloc(&d_tiles, sizeof(long long) * (c + 1)));
       SV_CUDA(cudaMalloc(&d_ctls, sizeof(Ctl*) * c));
@@ -1270,17 +1212,25 @@ struct Batch final : public sv_batch_base {
       SV_CUDA(cudaMalloc(&d_pprogress, sizeof(unsigned long long)));
       cap = c;
     }
-    std::vector<svk::StageParams<T>> hp(size_t(N) * std::max(nact, 1));
+    params.assign(nact, svk::StageParams<T>{});
     std::vector<svk::FinalizeParams> hf(std::max(nact, 1));
     std::vector<long long> ht(nact + 1, 0);
     std::vector<Ctl*> hc(std::max(nact, 1));
     p2 = true;
     extra = false;
     max_nblk = 0;
+    // one strip height for all members, by the rule of a single mesh over all their strips
+    int rows = 32;
+    for (; rows > 4; rows /= 2) {
+      long long n = 0;
+      for (int id : active) n += svk::strip_count((long long)members[id]->mesh.nx, (long long)members[id]->mesh.ny, rows);
+      if (n >= svk::kFillStrips) break;
+    }
     for (int k = 0; k < nact; ++k) {
       Solver<T>* m = members[active[k]];
-      // the tile prefix and the partials follow the batch kernel's decomposition
+      // the strip prefix and the partials follow the batch kernel's decomposition
       if (m->variant != member_variant()) m->set_variant(member_variant());
+      m->set_batch_rows(rows);
       int rs = m->ensure_strips(member_variant());
       if (rs) return fail(rs, "member " + std::to_string(active[k]) + ": " + m->err);
       ht[k + 1] = ht[k] + m->nblk;
@@ -1288,18 +1238,17 @@ struct Batch final : public sv_batch_base {
       int e2;
       p2 = p2 && std::frexp(m->mesh.dx, &e2) == 0.5 && std::frexp(m->mesh.dy, &e2) == 0.5;
       extra = extra || m->extra();
-      for (int st = 0; st < N; ++st) hp[size_t(st) * nact + k] = m->stage_params(st);
+      params[k] = m->stage_params();
       hf[k] = m->finalize_params(true);
       hf[k].q = d_queue + k;
       hf[k].fc = m->fc;
       hc[k] = m->ctl;
     }
-    total_tiles = ht[nact];
     versions.assign(nact, 0);
     for (int k = 0; k < nact; ++k) versions[k] = members[active[k]]->pversion;
     if (nact > 0) {
-      SV_CUDA(cudaMemcpyAsync(d_params, hp.data(), sizeof(svk::StageParams<T>) * size_t(N) * nact,
-                              cudaMemcpyHostToDevice, stream));
+      SV_CUDA(cudaMemcpyAsync(d_params, params.data(), sizeof(svk::StageParams<T>) * nact, cudaMemcpyHostToDevice,
+                              stream));
       SV_CUDA(cudaMemcpyAsync(d_fin, hf.data(), sizeof(svk::FinalizeParams) * nact, cudaMemcpyHostToDevice, stream));
       SV_CUDA(cudaMemcpyAsync(d_tiles, ht.data(), sizeof(long long) * (nact + 1), cudaMemcpyHostToDevice, stream));
       SV_CUDA(cudaMemcpyAsync(d_ctls, hc.data(), sizeof(Ctl*) * nact, cudaMemcpyHostToDevice, stream));
@@ -1311,8 +1260,7 @@ struct Batch final : public sv_batch_base {
 
   int enqueue_timestep() {
     for (int st = 0; st < N; ++st) {
-      cudaError_t e = svk::launch_sweep_batch<T>(d_params + size_t(st) * nact, d_tiles, nact, total_tiles, p2, extra,
-                                                 stream);
+      cudaError_t e = svk::launch_sweep_batch<T>(params.data(), nact, st, p2, extra, stream);
       if (e != cudaSuccess) return cuda_fail(e, "batched stage kernel");
     }
     cudaError_t e = svk::launch_finalize_batch(d_fin, nact, max_nblk, stream);
@@ -1383,7 +1331,7 @@ struct Batch final : public sv_batch_base {
       PP.progress = d_pprogress;
       PP.spin_limit = spin_limit;
       PP.max_ns = (unsigned long long)(max_seconds * 1e9);
-      if (e == cudaSuccess) e = svk::launch_persist<T>(PP, p2, extra, stream);
+      if (e == cudaSuccess) e = svk::launch_persist<T>(PP, params.data(), p2, extra, stream);
       if (e != cudaSuccess) return cuda_fail(e, "persistent batch kernel");
       int st = 0;
       SV_CUDA(cudaMemcpyAsync(&st, d_pstatus, sizeof(int), cudaMemcpyDeviceToHost, stream));

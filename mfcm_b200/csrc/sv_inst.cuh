@@ -1,9 +1,10 @@
 // sv_inst.cuh -- launcher definitions, included once per value type by sv_f64.cu / sv_f32.cu
 // with SV_T defined to the value type.
 #pragma once
+#include <algorithm>
 #include <atomic>
 #include <cmath>
-#include <utility>
+#include <memory>
 
 #include "sv_launch.h"
 
@@ -44,35 +45,35 @@ inline bool pow2_mesh(double dx, double dy) {
 }
 
 template <typename T, int TX, int TY, int MINB, bool P2, bool EDDY, bool PRE = false>
-static cudaError_t launch_stage_p(const StageParams<T>& P, cudaStream_t s) {
+static cudaError_t launch_stage_p(const StageParams<T>& P, int st, cudaStream_t s) {
   using SM = StageSmem<T, TX, TY>;
   static std::atomic<bool> attr_set[kMaxAttrDevices];
   cudaError_t e = smem_optin(stage_kernel<T, TX, TY, MINB, P2, EDDY, PRE>, int(sizeof(SM)), attr_set);
   if (e != cudaSuccess) return e;
   dim3 grid((P.nx + TX - 1) / TX, (P.ny + TY - 1) / TY);
-  stage_kernel<T, TX, TY, MINB, P2, EDDY, PRE><<<grid, TX * TY, sizeof(SM), s>>>(P);
+  stage_kernel<T, TX, TY, MINB, P2, EDDY, PRE><<<grid, TX * TY, sizeof(SM), s>>>(P, st);
   return cudaGetLastError();
 }
 
 // split schedule: the slopes pass, then the tiled 32 x 8 stage kernel reading its slopes
-template <typename T> static cudaError_t launch_split_t(const StageParams<T>& P, cudaStream_t s) {
+template <typename T> static cudaError_t launch_split_t(const StageParams<T>& P, int st, cudaStream_t s) {
   const bool p2 = pow2_mesh(P.dx, P.dy);
   const long long n = (long long)P.nx * P.ny;
   const unsigned blocks = unsigned((n + 255) / 256);
-  if (p2) slopes_kernel<T, true><<<blocks, 256, 0, s>>>(P);
-  else slopes_kernel<T, false><<<blocks, 256, 0, s>>>(P);
+  if (p2) slopes_kernel<T, true><<<blocks, 256, 0, s>>>(P, st);
+  else slopes_kernel<T, false><<<blocks, 256, 0, s>>>(P, st);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (P.eddy)
-    return p2 ? launch_stage_p<T, 32, 8, 3, true, true, true>(P, s) : launch_stage_p<T, 32, 8, 3, false, true, true>(P, s);
-  return p2 ? launch_stage_p<T, 32, 8, 3, true, false, true>(P, s) : launch_stage_p<T, 32, 8, 3, false, false, true>(P, s);
+    return p2 ? launch_stage_p<T, 32, 8, 3, true, true, true>(P, st, s) : launch_stage_p<T, 32, 8, 3, false, true, true>(P, st, s);
+  return p2 ? launch_stage_p<T, 32, 8, 3, true, false, true>(P, st, s) : launch_stage_p<T, 32, 8, 3, false, false, true>(P, st, s);
 }
 // kernels compiled with the eddy-viscosity term run only for solvers that have it
-template <typename T, int TX, int TY, int MINB> static cudaError_t launch_stage_t(const StageParams<T>& P, cudaStream_t s) {
+template <typename T, int TX, int TY, int MINB> static cudaError_t launch_stage_t(const StageParams<T>& P, int st, cudaStream_t s) {
   const bool p2 = pow2_mesh(P.dx, P.dy);
   if (P.eddy)
-    return p2 ? launch_stage_p<T, TX, TY, MINB, true, true>(P, s) : launch_stage_p<T, TX, TY, MINB, false, true>(P, s);
-  return p2 ? launch_stage_p<T, TX, TY, MINB, true, false>(P, s) : launch_stage_p<T, TX, TY, MINB, false, false>(P, s);
+    return p2 ? launch_stage_p<T, TX, TY, MINB, true, true>(P, st, s) : launch_stage_p<T, TX, TY, MINB, false, true>(P, st, s);
+  return p2 ? launch_stage_p<T, TX, TY, MINB, true, false>(P, st, s) : launch_stage_p<T, TX, TY, MINB, false, false>(P, st, s);
 }
 
 template <> size_t stage_smem_bytes<SV_T>(int tile) {
@@ -84,12 +85,12 @@ template <> size_t stage_smem_bytes<SV_T>(int tile) {
   }
 }
 
-template <> cudaError_t launch_stage<SV_T>(const StageParams<SV_T>& P, int tile, cudaStream_t s) {
+template <> cudaError_t launch_stage<SV_T>(const StageParams<SV_T>& P, int st, int tile, cudaStream_t s) {
   switch (tile) {
-    case 0: return launch_stage_t<SV_T, 32, 8, 1>(P, s);
-    case 1: return launch_stage_t<SV_T, 32, 8, 3>(P, s);
-    case 2: return launch_stage_t<SV_T, 32, 4, 4>(P, s);
-    default: return launch_stage_t<SV_T, 64, 4, 3>(P, s);
+    case 0: return launch_stage_t<SV_T, 32, 8, 1>(P, st, s);
+    case 1: return launch_stage_t<SV_T, 32, 8, 3>(P, st, s);
+    case 2: return launch_stage_t<SV_T, 32, 4, 4>(P, st, s);
+    default: return launch_stage_t<SV_T, 64, 4, 3>(P, st, s);
   }
 }
 
@@ -99,38 +100,38 @@ constexpr int kRingBytes = kSweepWarps * int(sizeof(SweepShared<SV_T>));
 // The column sweep of a stage: the strips in P.strips, P.rows rows each. `cap`: resident blocks
 // per SM asked of the register allocator. FP32 multiplies by the reciprocal cell sizes whatever
 // they are, so it has no power-of-two form of its own.
-template <int MINB, bool EXTRA> static cudaError_t launch_sweep_c(const StageParams<SV_T>& P, cudaStream_t s) {
+template <int MINB, bool EXTRA> static cudaError_t launch_sweep_c(const StageParams<SV_T>& P, int st, cudaStream_t s) {
   if (P.n_strips <= 0) return cudaSuccess;
   const dim3 grid(unsigned((P.n_strips + kSweepWarps - 1) / kSweepWarps)), block(32, kSweepWarps);
   if (sizeof(SV_T) == 8 && pow2_mesh(P.dx, P.dy))
-    return launch_dynamic<sweep_kernel<SV_T, MINB, sizeof(SV_T) == 8, EXTRA>>(grid, block, kRingBytes, s, P);
-  return launch_dynamic<sweep_kernel<SV_T, MINB, false, EXTRA>>(grid, block, kRingBytes, s, P);
+    return launch_dynamic<sweep_kernel<SV_T, MINB, sizeof(SV_T) == 8, EXTRA>>(grid, block, kRingBytes, s, P, st);
+  return launch_dynamic<sweep_kernel<SV_T, MINB, false, EXTRA>>(grid, block, kRingBytes, s, P, st);
 }
-static cudaError_t launch_sweep(const StageParams<SV_T>& P, int cap, bool extra, cudaStream_t s) {
-  if (extra) return launch_sweep_c<kExtraCap<SV_T>, true>(P, s);
+static cudaError_t launch_sweep(const StageParams<SV_T>& P, int st, int cap, bool extra, cudaStream_t s) {
+  if (extra) return launch_sweep_c<kExtraCap<SV_T>, true>(P, st, s);
   if constexpr (sizeof(SV_T) == 8) {
     switch (cap) {
-      case 3: return launch_sweep_c<3, false>(P, s);
-      case 4: return launch_sweep_c<4, false>(P, s);
-      case 5: return launch_sweep_c<5, false>(P, s);
-      default: return launch_sweep_c<6, false>(P, s);
+      case 3: return launch_sweep_c<3, false>(P, st, s);
+      case 4: return launch_sweep_c<4, false>(P, st, s);
+      case 5: return launch_sweep_c<5, false>(P, st, s);
+      default: return launch_sweep_c<6, false>(P, st, s);
     }
   } else {
     switch (cap) {
       case 3:
-      case 4: return launch_sweep_c<4, false>(P, s);
-      case 5: return launch_sweep_c<5, false>(P, s);
-      case 6: return launch_sweep_c<6, false>(P, s);
-      case 7: return launch_sweep_c<7, false>(P, s);
-      default: return launch_sweep_c<8, false>(P, s);
+      case 4: return launch_sweep_c<4, false>(P, st, s);
+      case 5: return launch_sweep_c<5, false>(P, st, s);
+      case 6: return launch_sweep_c<6, false>(P, st, s);
+      case 7: return launch_sweep_c<7, false>(P, st, s);
+      default: return launch_sweep_c<8, false>(P, st, s);
     }
   }
 }
 
-template <> cudaError_t launch_variant<SV_T>(const StageParams<SV_T>& P, int variant, bool extra, cudaStream_t s) {
-  if (variant_is_split(variant)) return launch_split_t<SV_T>(P, s);
-  if (variant_is_sweep(variant)) return launch_sweep(P, variant_cap<SV_T>(variant), extra, s);
-  return launch_stage<SV_T>(P, variant, s);
+template <> cudaError_t launch_variant<SV_T>(const StageParams<SV_T>& P, int st, int variant, bool extra, cudaStream_t s) {
+  if (variant_is_split(variant)) return launch_split_t<SV_T>(P, st, s);
+  if (variant_is_sweep(variant)) return launch_sweep(P, st, variant_cap<SV_T>(variant), extra, s);
+  return launch_stage<SV_T>(P, st, variant, s);
 }
 
 template <> cudaError_t launch_strip_classes<SV_T>(const SV_T* z, int nx, int ny, double dx, double dy, int rows,
@@ -170,40 +171,63 @@ template <> cudaError_t launch_to_f64<SV_T>(const SV_T* src, double* dst, long l
   return cudaGetLastError();
 }
 
-template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, const long long* warp_start, int ninst,
-                                                 long long total_warps, bool p2, bool extra, cudaStream_t s) {
-  if (total_warps <= 0) return cudaSuccess;
-  const dim3 block(32, kSweepWarps), grid(unsigned((total_warps + kSweepWarps - 1) / kSweepWarps));
+template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, int n, int st, bool p2, bool extra,
+                                                 cudaStream_t s) {
   constexpr bool F64 = sizeof(SV_T) == 8;
   constexpr int CAP = kBatchCap<SV_T>, XCAP = kExtraCap<SV_T>;
-  if (extra)
-    return p2 && F64 ? launch_dynamic<sweep_batch_kernel<SV_T, XCAP, F64, true>>(grid, block, kRingBytes, s, Ps, warp_start, ninst)
-                     : launch_dynamic<sweep_batch_kernel<SV_T, XCAP, false, true>>(grid, block, kRingBytes, s, Ps, warp_start, ninst);
-  return p2 && F64 ? launch_dynamic<sweep_batch_kernel<SV_T, CAP, F64, false>>(grid, block, kRingBytes, s, Ps, warp_start, ninst)
-                   : launch_dynamic<sweep_batch_kernel<SV_T, CAP, false, false>>(grid, block, kRingBytes, s, Ps, warp_start, ninst);
+  for (int k0 = 0; k0 < n; k0 += kBatchMembers) {
+    BatchParams<SV_T> B;
+    B.n = std::min(n - k0, kBatchMembers);
+    B.first_block[0] = 0;
+    for (int k = 0; k < B.n; ++k) {
+      B.m[k] = Ps[k0 + k];
+      B.first_block[k + 1] = B.first_block[k] + (B.m[k].n_strips + kSweepWarps - 1) / kSweepWarps;
+    }
+    const dim3 block(32, kSweepWarps), grid(unsigned(B.first_block[B.n]));
+    if (grid.x == 0) continue;
+    cudaError_t e;
+    if (extra)
+      e = p2 && F64 ? launch_dynamic<sweep_batch_kernel<SV_T, XCAP, F64, true>>(grid, block, kRingBytes, s, B, st)
+                    : launch_dynamic<sweep_batch_kernel<SV_T, XCAP, false, true>>(grid, block, kRingBytes, s, B, st);
+    else
+      e = p2 && F64 ? launch_dynamic<sweep_batch_kernel<SV_T, CAP, F64, false>>(grid, block, kRingBytes, s, B, st)
+                    : launch_dynamic<sweep_batch_kernel<SV_T, CAP, false, false>>(grid, block, kRingBytes, s, B, st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 // Persistent batch kernel: one cooperative launch with as many 4-warp blocks as fit on the
 // device at once (every block resident, so warps that wait for another warp's work always
 // see it done).
-template <> cudaError_t launch_persist<SV_T>(const PersistParams<SV_T>& PP, bool p2, bool extra, cudaStream_t s) {
+template <int BANK>
+static cudaError_t launch_persist_t(const PersistParams<SV_T>& PP, const StageParams<SV_T>* Ps, bool p2, bool extra,
+                                    cudaStream_t s) {
   constexpr bool F64 = sizeof(SV_T) == 8;
   constexpr int CAP = kBatchCap<SV_T>, XCAP = kExtraCap<SV_T>;
-  void (*kern)(const PersistParams<SV_T>) =
-      extra ? (p2 ? persist_batch_kernel<SV_T, XCAP, F64, true> : persist_batch_kernel<SV_T, XCAP, false, true>)
-            : (p2 ? persist_batch_kernel<SV_T, CAP, F64, false> : persist_batch_kernel<SV_T, CAP, false, false>);
+  void (*kern)(const PersistParams<SV_T>, const MemberBank<SV_T, BANK>) =
+      extra ? (p2 ? persist_batch_kernel<SV_T, XCAP, F64, true, BANK> : persist_batch_kernel<SV_T, XCAP, false, true, BANK>)
+            : (p2 ? persist_batch_kernel<SV_T, CAP, F64, false, BANK> : persist_batch_kernel<SV_T, CAP, false, false, BANK>);
   int dev = 0, nsm = 0, per_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess && kRingBytes > 48 * 1024)
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingBytes);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kPersistWarps, kRingBytes);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kPersistWarps, kRingBytes);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorCooperativeLaunchTooLarge;
   PersistParams<SV_T> arg = PP;
-  void* args[] = {&arg};
+  auto bank = std::make_unique<MemberBank<SV_T, BANK>>();
+  if (BANK > 1) std::copy(Ps, Ps + PP.nact, bank->m);
+  void* args[] = {&arg, bank.get()};
   return cudaLaunchCooperativeKernel((const void*)kern, dim3(unsigned(per_sm * nsm)), dim3(32, kPersistWarps), args,
                                      kRingBytes, s);
+}
+template <> cudaError_t launch_persist<SV_T>(const PersistParams<SV_T>& PP, const StageParams<SV_T>* Ps, bool p2,
+                                             bool extra, cudaStream_t s) {
+  if (PP.nact <= kBatchMembers) return launch_persist_t<kBatchMembers>(PP, Ps, p2, extra, s);
+  return launch_persist_t<1>(PP, Ps, p2, extra, s);
 }
 
 template <typename T, int TX, int TY>

@@ -55,12 +55,9 @@ struct DevForcing {
 };
 
 enum StageMode : int {
-  M_FIRST = 1,    // stage 0: input is U_[0]
-  M_LAST = 2,     // last stage: writes U_[N] and the CFL / volume partials
   M_ACC = 4,      // diagonal tableau: running accumulator instead of stored k's
   M_STOREK = 8,   // store k_s for later stages (non-diagonal tableaux)
   M_TALLY = 16,   // rain / outflow partials
-  M_DEBUGK = 32,  // debug: write k_s only (no RK combination)
 };
 
 // Constants of the mesh in the solver's value type, formed once on the host.
@@ -76,16 +73,16 @@ template <typename T> struct MeshConst {
   }
 };
 
+// One solver's parameters for every stage of a timestep; the stage's index (0-based) goes beside
+// them. Stage 0 reads U_[0] and the last one writes U_[N] and the CFL and volume partials.
 template <typename T> struct StageParams {
   int nx, ny;
   double dx, dy, L;
   double cell_area;
   MeshConst<T> mc;
   T* S[2][3];            // state parity buffers: S[cur] = U_[0], S[cur^1] = acc / U_[N]
-  const T* Yin[3];       // stage input (ignored on the first stage)
-  T* Yout[3];            // Y_{s+1} (not on the last stage)
-  T* Kout[3];            // k_s (M_STOREK / M_DEBUGK)
-  const T* Kin[4][3];    // stored k_j, j < s (M_STOREK)
+  T* Y[2][3];            // stage s reads Y[(s - 1) & 1] (s > 0) and writes Y[s & 1]
+  T* K[3][3];            // stored k_s, all but the last stage's (M_STOREK)
   const T* z;
   const T* zx; const T* zy;   // bed slopes dz/dx, dz/dy (Constants.cpp:39-40), precomputed
   const double* zdat;         // FP32-with-datum mode: per datum tile FP64 datum (z = datum + z_off)
@@ -100,9 +97,9 @@ template <typename T> struct StageParams {
   T* hc[2];              // FP32: per-cell compensation of the depth update (state parity), or nullptr
   int manning, rain_mode, head_first;
   int eloss_first;       // energy loss applied before roughness (configuration order)
-  int stage, nstages, mode;
-  double c_s;            // c of this stage: t_sub = t_local + c_s * dt
-  double a_next[4];      // a(s+2, j+1), j = 0..s: coefficients of Y_{s+1}
+  int nstages, mode;
+  double c[4];           // stage s is evaluated at t_local + c[s] * dt
+  double a[4][4];        // a[s][j] = a(s+2, j+1), j = 0..s: coefficients of Y_{s+1}
   double b[4];           // b_1..b_N
   Ctl* ctl;
   double* part;          // per-CTA partials (see part_* offsets)
@@ -123,6 +120,12 @@ template <typename T> struct StageParams {
   // split schedule: the stage input's slopes dh/dx, du/dx, dv/dx, dh/dy, du/dy, dv/dy as
   // written by slopes_kernel (read by the stage kernel instead of computing them), or null
   T* pslp[6];
+
+  // field f of stage `st`'s input, of its output
+  __device__ __forceinline__ const T* in(int st, int cur, int f) const {
+    return st == 0 ? S[cur][f] : Y[(st - 1) & 1][f];
+  }
+  __device__ __forceinline__ T* out(int st, int f) const { return Y[st & 1][f]; }
 };
 
 // partial layout: [0, nblk) cn max, [nblk, 2nblk) cn min, [2nblk, 3nblk) volume, then the
@@ -134,9 +137,10 @@ constexpr int kParts = 6;
 __host__ __device__ inline long long part_count(long long nblk) { return kParts * nblk; }
 // Adds one stage's tallies, weighted by b_s dt in the solver's value type, to slot `i`.
 template <typename T>
-__device__ __forceinline__ void store_tallies(const StageParams<T>& P, long long i, double rain, double removed,
-                                              double wall, bool first, double dt) {
-  const double w = double(T(P.b[P.stage] * dt));
+__device__ __forceinline__ void store_tallies(const StageParams<T>& P, int st, long long i, double rain,
+                                              double removed, double wall, double dt) {
+  const bool first = st == 0;
+  const double w = double(T(P.b[st] * dt));
   double* p = P.part + 3 * P.nblk + i;
   p[0] = first ? w * rain : p[0] + w * rain;
   p[P.nblk] = first ? w * removed : p[P.nblk] + w * removed;
@@ -367,12 +371,11 @@ __device__ __forceinline__ void cell_dudt(const StageParams<T>& P, const DevForc
 // One cell of one stage after its four face fluxes are known: dU/dt, then the Runge-Kutta
 // combination (RungeKutta.hpp:377-388) and, on the last stage, the CFL quantity and volume.
 template <typename T, typename CC, bool EDDY = false, bool EDGE = true, bool COH = false>
-__device__ __forceinline__ void finish_cell(const StageParams<T>& P, const DevForcing& fc, const CC& c,
+__device__ __forceinline__ void finish_cell(const StageParams<T>& P, int st, const DevForcing& fc, const CC& c,
                                             long long g, int gx, int gy, T h, T u, T v, T dhdx, T dhdy, T dzdx,
                                             T dzdy, const FaceF<T>& fw, const FaceF<T>& fe, const FaceF<T>& fs,
-                                            const FaceF<T>& fn, bool first, bool last, int cur, double dt_d,
-                                            double& rain, double& removed, double& walls, T& xcfl,
-                                            T& xcfl_min, double& vol, const EddyIn<T>* ed = nullptr) {
+                                            const FaceF<T>& fn, int cur, double dt_d, double& rain,
+                                            double& removed, double& walls, T& xcfl, T& xcfl_min, double& vol, const EddyIn<T>* ed = nullptr) {
   T kh, ku, kv;
   double r_, o_, w_;
   cell_dudt<T, CC, EDDY, EDGE>(P, fc, c, g, gx, gy, h, u, v, dhdx, dhdy, dzdx, dzdy, fw, fe, fs, fn, kh, ku, kv, r_,
@@ -380,11 +383,10 @@ __device__ __forceinline__ void finish_cell(const StageParams<T>& P, const DevFo
   rain += r_;
   removed += o_;
   walls += w_;
-  if (P.mode & (M_STOREK | M_DEBUGK)) {
-    P.Kout[0][g] = kh; P.Kout[1][g] = ku; P.Kout[2][g] = kv;
+  const bool first = st == 0, last = st == P.nstages - 1;
+  if ((P.mode & M_STOREK) && !last) {
+    P.K[st][0][g] = kh; P.K[st][1][g] = ku; P.K[st][2][g] = kv;
   }
-  if (P.mode & M_DEBUGK) return;
-  const int st = P.stage;
   T* A[3] = {P.S[cur ^ 1][0], P.S[cur ^ 1][1], P.S[cur ^ 1][2]};
   const T* U0[3] = {P.S[cur][0], P.S[cur][1], P.S[cur][2]};
   T k[3] = {kh, ku, kv};
@@ -407,14 +409,14 @@ __device__ __forceinline__ void finish_cell(const StageParams<T>& P, const DevFo
       accv[f] = first ? (incr ? T(0) : u0v[f]) : ldst<COH>(A[f], g);
     }
     if (!last) {
-      const T cA = T(P.a_next[st] * dt_d);
+      const T cA = T(P.a[st][st] * dt_d);
 #pragma unroll
       for (int f = 0; f < 3; ++f) {
         T y = u0v[f] + k[f] * cA;
         // FP32 leaves this out: a non-finite accumulator reaches U_N at the last stage anyway
         if constexpr (sizeof(T) == 8)
           if (!first && finite_(u0v[f]) && !finite_(accv[f])) y = Lim<T>::nan();
-        P.Yout[f][g] = y;
+        P.out(st, f)[g] = y;
       }
     }
     if (!incr) {
@@ -447,15 +449,15 @@ __device__ __forceinline__ void finish_cell(const StageParams<T>& P, const DevFo
     T u0v[3];
 #pragma unroll
     for (int f = 0; f < 3; ++f) u0v[f] = first ? (f == 0 ? h : (f == 1 ? u : v)) : ldst<COH>(U0[f], g);
-    const double* coef = last ? P.b : P.a_next;
+    const double* coef = last ? P.b : P.a[st];
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
       T y = u0v[f];
-      for (int j = 0; j < st; ++j) y = y + ldst<COH>(P.Kin[j][f], g) * T(coef[j] * dt_d);
+      for (int j = 0; j < st; ++j) y = y + ldst<COH>(P.K[j][f], g) * T(coef[j] * dt_d);
       y = y + k[f] * T(coef[st] * dt_d);
       out[f] = y;
       if (last) A[f][g] = y;
-      else P.Yout[f][g] = y;
+      else P.out(st, f)[g] = y;
     }
   }
   if (last) {
@@ -483,7 +485,7 @@ struct StageSmem {
 
 // One TX x TY tile of one stage: bx, by = tile coordinates, blk = partial-sum slot.
 template <typename T, int TX, int TY, bool P2, bool EDDY, bool PRE = false>
-__device__ __forceinline__ void stage_tile(const StageParams<T>& P, int bx, int by, long long blk,
+__device__ __forceinline__ void stage_tile(const StageParams<T>& P, int st, int bx, int by, long long blk,
                                            StageSmem<T, TX, TY>& s) {
   using DX = DivX<T, P2>;
   using SM = StageSmem<T, TX, TY>;
@@ -493,15 +495,12 @@ __device__ __forceinline__ void stage_tile(const StageParams<T>& P, int bx, int 
   if (ctl->done) return;
   const int cur = ctl->cur;
   const double dt_d = ctl->dt;
-  const double tsub = ctl->t_local + P.c_s * dt_d;
+  const double tsub = ctl->t_local + P.c[st] * dt_d;
 
   const int tid = threadIdx.x;
   const int x0 = bx * TX, y0 = by * TY;
   const int nx = P.nx, ny = P.ny;
-  const bool first = P.mode & M_FIRST;
-  const T* Yh = first ? P.S[cur][0] : P.Yin[0];
-  const T* Yu = first ? P.S[cur][1] : P.Yin[1];
-  const T* Yv = first ? P.S[cur][2] : P.Yin[2];
+  const T *Yh = P.in(st, cur, 0), *Yu = P.in(st, cur, 1), *Yv = P.in(st, cur, 2);
 
   // phase 1: tile + 2-cell halo of h, u, v, z (clamped at the mesh edge; the clamped
   // copies are never used because edge faces and edge slopes use the cell itself)
@@ -590,7 +589,7 @@ __device__ __forceinline__ void stage_tile(const StageParams<T>& P, int bx, int 
   const bool valid = gx < nx && gy < ny;
   double rain = 0.0, removed = 0.0, walls = 0.0, vol = 0.0;
   T xcfl = T(0), xcfl_min = T(1.0 / 0.0);
-  const bool last = P.mode & M_LAST;
+  const bool last = st == P.nstages - 1;
   if (valid) {
     const long long g = (long long)gy * nx + gx;
     CellCtx<T, DX> c;
@@ -617,11 +616,11 @@ __device__ __forceinline__ void stage_tile(const StageParams<T>& P, int bx, int 
         ed.vyy = minmod3<T>(s.slp[6][sy + 1][sx], hasN, ed.vy, hasS, s.slp[6][sy - 1][sx], divy);
       }
     }
-    finish_cell<T, CellCtx<T, DX>, EDDY>(P, fc, c, g, gx, gy, h, u, v, s.slp[0][sy][sx], s.slp[4][sy][sx],
-                                         s.slp[3][sy][sx], s.slp[7][sy][sx], fw, fe, fs, fn, first, last, cur, dt_d,
+    finish_cell<T, CellCtx<T, DX>, EDDY>(P, st, fc, c, g, gx, gy, h, u, v, s.slp[0][sy][sx], s.slp[4][sy][sx],
+                                         s.slp[3][sy][sx], s.slp[7][sy][sx], fw, fe, fs, fn, cur, dt_d,
                                          rain, removed, walls, xcfl, xcfl_min, vol, &ed);
   }
-  if (last && !(P.mode & M_DEBUGK)) {
+  if (last) {
     double mx = block_max<NT>(double(xcfl), s.red);
     double mn = block_min<NT>(double(xcfl_min), s.red);
     double vs = block_sum<NT>(vol, s.red);
@@ -635,22 +634,22 @@ __device__ __forceinline__ void stage_tile(const StageParams<T>& P, int bx, int 
     double rs = block_sum<NT>(rain, s.red);
     double os = block_sum<NT>(removed, s.red);
     double ws = block_sum<NT>(walls, s.red);
-    if (tid == 0) store_tallies(P, blk, rs, os, ws, first, dt_d);
+    if (tid == 0) store_tallies(P, st, blk, rs, os, ws, dt_d);
   }
 }
 
 template <typename T, int TX, int TY, int MINB, bool P2, bool EDDY, bool PRE = false>
-__global__ void __launch_bounds__(TX * TY, MINB) stage_kernel(const StageParams<T> P) {
+__global__ void __launch_bounds__(TX * TY, MINB) stage_kernel(const __grid_constant__ StageParams<T> P, int st) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& s = *reinterpret_cast<StageSmem<T, TX, TY>*>(smem_raw);
-  stage_tile<T, TX, TY, P2, EDDY, PRE>(P, blockIdx.x, blockIdx.y, (long long)blockIdx.y * gridDim.x + blockIdx.x, s);
+  stage_tile<T, TX, TY, P2, EDDY, PRE>(P, st, blockIdx.x, blockIdx.y, (long long)blockIdx.y * gridDim.x + blockIdx.x, s);
 }
 
 // Split schedule, first pass: the Minmod3 slopes of the stage input (State.cpp:176-193), one
 // thread per cell, into P.pslp; the stage kernel that follows reads them instead of forming
 // them from its tile.
 template <typename T, bool P2>
-__global__ void __launch_bounds__(256) slopes_kernel(const StageParams<T> P) {
+__global__ void __launch_bounds__(256) slopes_kernel(const __grid_constant__ StageParams<T> P, int st) {
   using DX = DivX<T, P2>;
   const Ctl* ctl = P.ctl;
   if (ctl->done) return;
@@ -658,13 +657,12 @@ __global__ void __launch_bounds__(256) slopes_kernel(const StageParams<T> P) {
   const int nx = P.nx, ny = P.ny;
   if (i >= (long long)nx * ny) return;
   const int cur = ctl->cur;
-  const bool first = P.mode & M_FIRST;
   const int gx = int(i % nx), gy = int(i / nx);
   const bool hasW = gx > 0, hasE = gx < nx - 1, hasN = gy < ny - 1, hasS = gy > 0;
   const DX divx = MkDivX<DX>::make(P.dx), divy = MkDivX<DX>::make(P.dy);
 #pragma unroll
   for (int f = 0; f < 3; ++f) {
-    const T* a = first ? P.S[cur][f] : P.Yin[f];
+    const T* a = P.in(st, cur, f);
     const T c = ld(a, i);
     const T l = hasW ? ld(a, i - 1) : c, r = hasE ? ld(a, i + 1) : c;
     P.pslp[f][i] = minmod3<T>(l, hasW, c, hasE, r, divx);
@@ -1009,7 +1007,7 @@ struct PersistMember {
 };
 
 template <typename T> struct PersistParams {
-  const StageParams<T>* Ps;   // stage s of member k at Ps[s * nact + k]
+  const StageParams<T>* Ps;   // [nact]
   const FinalizeParams* Fs;   // [nact]
   PersistMember* mem;         // [nact]
   int nact, nstages;
@@ -1051,11 +1049,17 @@ __device__ __forceinline__ void finalize_warp(const FinalizeParams& F) {
   __syncwarp();
 }
 
-template <typename T, int MINB, bool P2, bool EXTRA>
-__global__ void __launch_bounds__(32 * kPersistWarps, MINB) persist_batch_kernel(const PersistParams<T> PP) {
-  __shared__ __align__(16) StageParams<T> Psh[kPersistWarps];
+// The members' parameters as kernel parameters, for batches of up to kBatchMembers members
+// (constant operands of the sweep, see sweep_batch_kernel); BANK = 1: a larger batch, whose
+// warps copy an item's parameters to shared memory.
+template <typename T, int BANK> struct MemberBank { StageParams<T> m[BANK]; };
+
+template <typename T, int MINB, bool P2, bool EXTRA, int BANK>
+__global__ void __launch_bounds__(32 * kPersistWarps, MINB)
+    persist_batch_kernel(const __grid_constant__ PersistParams<T> PP, const __grid_constant__ MemberBank<T, BANK> bank) {
+  __shared__ __align__(16) StageParams<T> Psh[BANK > 1 ? 1 : kPersistWarps];
   extern __shared__ __align__(16) unsigned char sweep_smem[];
-  const int lane = threadIdx.x, wib = threadIdx.y;
+  const int lane = threadIdx.x, wib = uniform(threadIdx.y);
   const int N = PP.nstages, nact = PP.nact;
   const long long gwarp = (long long)blockIdx.x * kPersistWarps + wib;
   const int k0 = nact > 0 ? int(gwarp % nact) : 0;
@@ -1146,14 +1150,21 @@ __global__ void __launch_bounds__(32 * kPersistWarps, MINB) persist_batch_kernel
     if (dropped) continue;
     __threadfence();  // acquire: the previous phases' writes of every warp
     if (s < N) {
-      // stage s, strip item r % ns: the member's parameters to shared memory, then the sweep
-      static_assert(sizeof(StageParams<T>) % 4 == 0, "parameter block copied as 32-bit words");
-      const unsigned* src = reinterpret_cast<const unsigned*>(PP.Ps + size_t(s) * nact + pick);
-      unsigned* dst = reinterpret_cast<unsigned*>(&Psh[wib]);
-      for (int i = lane; i < int(sizeof(StageParams<T>) / 4); i += 32) dst[i] = src[i];
-      __syncwarp();
-      const StageParams<T>& SP = Psh[wib];
-      sweep_strip<T, P2, EXTRA, true>(SP, SP.strips[r % ns], reinterpret_cast<SweepShared<T>*>(sweep_smem)[wib]);
+      // stage s, strip item r % ns
+      auto& sm = reinterpret_cast<SweepShared<T>*>(sweep_smem)[wib];
+      const int pk = uniform(pick), st = uniform(s);
+      if constexpr (BANK > 1) {
+        const StageParams<T>& SP = bank.m[pk];
+        sweep_strip<T, P2, EXTRA, true>(SP, st, SP.strips[r % ns], sm);
+      } else {
+        static_assert(sizeof(StageParams<T>) % 4 == 0, "parameter block copied as 32-bit words");
+        const unsigned* src = reinterpret_cast<const unsigned*>(PP.Ps + pk);
+        unsigned* dst = reinterpret_cast<unsigned*>(&Psh[wib]);
+        for (int i = lane; i < int(sizeof(StageParams<T>) / 4); i += 32) dst[i] = src[i];
+        __syncwarp();
+        const StageParams<T>& SP = Psh[wib];
+        sweep_strip<T, P2, EXTRA, true>(SP, st, SP.strips[r % ns], sm);
+      }
       __syncwarp();
     } else {
       finalize_warp(PP.Fs[pick]);
@@ -1259,6 +1270,7 @@ template <typename T> struct DebugParams {
   const T *h, *u, *v, *z;
   T *dhdx, *dudx, *dvdx, *dzdx, *dhdy, *dudy, *dvdy, *dzdy;
   T *fh, *fu, *fv, *fz, *fb;
+  T* k[3];
 };
 
 // SpatialDerivativeOperationKernel over global arrays (State.cpp:187-192, Constants.cpp:39-40)
@@ -1326,7 +1338,7 @@ __global__ void debug_cell_kernel(const StageParams<T> P, const DebugParams<T> D
   CellCtx<T> c;
   c.divx = mkdiv<T>(P.dx); c.divy = mkdiv<T>(P.dy);
   c.divdt = mkdiv<T>(dt_d); c.divL = mkdiv<T>(P.L);
-  c.dt = T(dt_d); c.dt_d = dt_d; c.tsub_d = ctl->t_local + P.c_s * dt_d;
+  c.dt = T(dt_d); c.dt_d = dt_d; c.tsub_d = ctl->t_local;
   c.manning = P.manning; c.rain_mode = P.rain_mode; c.head_first = P.head_first;
   long long w = (long long)gy * (P.nx + 1) + gx, e = w + 1;
   long long sf_ = (long long)(P.nx + 1) * P.ny + (long long)gy * P.nx + gx, nf_ = sf_ + P.nx;
@@ -1347,7 +1359,7 @@ __global__ void debug_cell_kernel(const StageParams<T> P, const DebugParams<T> D
   }
   cell_dudt<T, CellCtx<T>, true>(P, fc, c, g, gx, gy, D.h[g], D.u[g], D.v[g], D.dhdx[g], D.dhdy[g], D.dzdx[g],
                                  D.dzdy[g], fw, fe, fs, fn, kh, ku, kv, rain, removed, wall, nh + g, sf + g, &ed);
-  P.Kout[0][g] = kh; P.Kout[1][g] = ku; P.Kout[2][g] = kv;
+  D.k[0][g] = kh; D.k[1][g] = ku; D.k[2][g] = kv;
 }
 
 }  // namespace svk

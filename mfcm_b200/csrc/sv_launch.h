@@ -15,7 +15,7 @@ constexpr TileShape kTiles[] = {{32, 8, 1}, {32, 8, 3}, {32, 4, 4}, {64, 4, 3}};
 constexpr int kNumTiles = 4;
 
 template <typename T> size_t stage_smem_bytes(int tile);
-template <typename T> cudaError_t launch_stage(const StageParams<T>& P, int tile, cudaStream_t s);
+template <typename T> cudaError_t launch_stage(const StageParams<T>& P, int st, int tile, cudaStream_t s);
 
 // Stage-kernel variants, in two schedules:
 //  fused (one pass per RK stage): 0..3 the tiled shared-memory kernel with kTiles[v]; 4..10 and
@@ -37,6 +37,10 @@ template <typename T> constexpr int kExtraCap = sizeof(T) == 8 ? 3 : 4;
 inline bool variant_is_fp32_only(int v) { return v >= 12 && v <= 15; }
 inline bool variant_is_sweep(int v) { return v >= 0 && v < kNumVariants && kSweeps[v].rows > 0; }
 inline bool variant_is_split(int v) { return v == kSplitVariant; }
+// strips of `rows` rows of a mesh
+inline long long strip_count(long long nx, long long ny, int rows) {
+  return ((nx + kSweepOut - 1) / kSweepOut) * ((ny + rows - 1) / rows);
+}
 // Strip height by mesh size: the tallest of 32, 16, 8 and 4 rows that still gives every SM its
 // 16 resident warps, else 4. A strip marches its rows one after another, so a mesh of few strips
 // waits for one warp's latency (2.0-3.3 us a row); a short strip repeats more of its neighbours'
@@ -45,9 +49,8 @@ inline bool variant_is_split(int v) { return v == kSplitVariant; }
 // 22 / 17, 60 / 41 / 45 / 54, 445 / 485 / 581 / 793 us.
 constexpr long long kFillStrips = 148 * 16;
 inline int auto_rows(long long nx, long long ny) {
-  const long long tiles_x = (nx + kSweepOut - 1) / kSweepOut;
   for (int rows = 32; rows > 4; rows /= 2)
-    if (tiles_x * ((ny + rows - 1) / rows) >= kFillStrips) return rows;
+    if (strip_count(nx, ny, rows) >= kFillStrips) return rows;
   return 4;
 }
 // column-sweep variants: output rows per strip on a mesh (0 for the other variants)
@@ -60,11 +63,10 @@ template <typename T> inline int variant_cap(int v) { return kSweeps[v].cap; }
 inline long long variant_partials(int v, long long nx, long long ny) {
   if (v == kSplitVariant) v = 1;  // the split schedule's stage pass is the tiled 32 x 8 kernel
   if (v < 4) return ((nx + kTiles[v].tx - 1) / kTiles[v].tx) * ((ny + kTiles[v].ty - 1) / kTiles[v].ty);
-  const long long ty = variant_sweep_rows(v, nx, ny);
-  return ((nx + kSweepOut - 1) / kSweepOut) * ((ny + ty - 1) / ty);
+  return strip_count(nx, ny, variant_sweep_rows(v, nx, ny));
 }
-// extra: source terms, boundaries or a tableau that the lean sweep leaves out (sweep_rows)
-template <typename T> cudaError_t launch_variant(const StageParams<T>& P, int variant, bool extra, cudaStream_t s);
+// stage `st` of a timestep. extra: source terms, boundaries or a tableau that the lean sweep leaves out (sweep_rows)
+template <typename T> cudaError_t launch_variant(const StageParams<T>& P, int st, int variant, bool extra, cudaStream_t s);
 // classes of the column sweep's strips of `rows` rows (strip_class_kernel)
 template <typename T> cudaError_t launch_strip_classes(const T* z, int nx, int ny, double dx, double dy, int rows,
                                                        long long nstrips, unsigned char* cls, cudaStream_t s);
@@ -85,13 +87,15 @@ template <typename T> cudaError_t launch_volume(const T* h, int nx, int ny, doub
                                                 cudaStream_t s);
 template <typename T> cudaError_t launch_debug(const StageParams<T>& P, const DebugParams<T>& D, T* nh, T* sf,
                                                cudaStream_t s);
-// batched launches: every strip of every instance; p2 when every instance's dx and dy are powers
-// of two, extra when any instance needs it
+// stage `st` of every one of n solvers (host array Ps) in one launch per kBatchMembers of them;
+// p2 when every solver's dx and dy are powers of two, extra when any solver needs it
 constexpr int kBatchVariant = 8;
-template <typename T> cudaError_t launch_sweep_batch(const StageParams<T>* Ps, const long long* warp_start, int ninst,
-                                                     long long total_warps, bool p2, bool extra, cudaStream_t s);
-// persistent batch kernel (persist_batch_kernel), cooperative launch filling the device
-template <typename T> cudaError_t launch_persist(const PersistParams<T>& PP, bool p2, bool extra, cudaStream_t s);
+template <typename T> cudaError_t launch_sweep_batch(const StageParams<T>* Ps, int n, int st, bool p2, bool extra,
+                                                     cudaStream_t s);
+// persistent batch kernel (persist_batch_kernel), cooperative launch filling the device; Ps: the
+// members' parameters on the host (PP.Ps: the same on the device)
+template <typename T> cudaError_t launch_persist(const PersistParams<T>& PP, const StageParams<T>* Ps, bool p2,
+                                                 bool extra, cudaStream_t s);
 cudaError_t launch_persist_init(const FinalizeParams* Fs, PersistMember* mem, const long long* warp_start, int nact,
                                 cudaStream_t s);
 cudaError_t launch_finalize(const FinalizeParams& F, cudaStream_t s);

@@ -189,19 +189,16 @@ extern "C" int sv_timestep_noalloc(const sv_mesh_desc* mesh, const sv_params* pa
   P.part = part;
   P.nblk = nblk;
   const bool tally = !(params->flags & SV_FLAG_NO_TALLIES);
+  P.mode = svk::M_ACC | (tally ? svk::M_TALLY : 0);
+  for (int st = 0; st < 4; ++st) {
+    P.c[st] = k.c[st];
+    P.b[st] = k.b[st];
+    for (int j = 0; j < 4; ++j) P.a[st][j] = k.a_next[st][j];
+  }
+  for (int b = 0; b < 2; ++b)
+    for (int fld = 0; fld < 3; ++fld) P.Y[b][fld] = Y + (size_t(b) * 3 + fld) * size_t(kMaxCells);
   for (int st = 0; st < k.N; ++st) {
-    P.stage = st;
-    P.c_s = k.c[st];
-    P.mode = svk::M_ACC | (st == 0 ? svk::M_FIRST : 0) | (st == k.N - 1 ? svk::M_LAST : 0) | (tally ? svk::M_TALLY : 0);
-    for (int j = 0; j < 4; ++j) { P.a_next[j] = k.a_next[st][j]; P.b[j] = k.b[j]; }
-    const int in = (st - 1) & 1, out = st & 1;
-    for (int fld = 0; fld < 3; ++fld) {
-      P.Yin[fld] = st > 0 ? Y + (size_t(in) * 3 + fld) * size_t(kMaxCells) : nullptr;
-      P.Yout[fld] = st < k.N - 1 ? Y + (size_t(out) * 3 + fld) * size_t(kMaxCells) : nullptr;
-      P.Kout[fld] = nullptr;
-      for (int j = 0; j < 4; ++j) P.Kin[j][fld] = nullptr;
-    }
-    e = svk::launch_variant<double>(P, kVariant, false, s);
+    e = svk::launch_variant<double>(P, st, kVariant, false, s);
     if (e != cudaSuccess) return fail(SV_E_CUDA, cudaGetErrorString(e));
   }
   svk::FinalizeParams F{};

@@ -137,7 +137,7 @@ static_assert(sizeof(SweepShared<float>) % 16 == 0 && sizeof(SweepShared<double>
 // of a strip whose state leaves the range of sweep_rows. Out of line: one copy per kernel.
 // ---------------------------------------------------------------------------------------
 template <typename T, bool EDDY, bool COH>
-__device__ __noinline__ void sweep_rows_general(const StageParams<T>& P, int tile_x, int y0, int y1, SweepAcc<T>& acc) {
+__device__ __noinline__ void sweep_rows_general(const StageParams<T>& P, int st, int tile_x, int y0, int y1, SweepAcc<T>& acc) {
   using DX = Div<T>;
   const Ctl* ctl = P.ctl;
   const int nx = P.nx, ny = P.ny;
@@ -150,11 +150,8 @@ __device__ __noinline__ void sweep_rows_general(const StageParams<T>& P, int til
 
   const int cur = ctl->cur;
   const double dt_d = ctl->dt;
-  const double tsub = ctl->t_local + P.c_s * dt_d;
-  const bool first = P.mode & M_FIRST, last = P.mode & M_LAST;
-  const T* Yh = first ? P.S[cur][0] : P.Yin[0];
-  const T* Yu = first ? P.S[cur][1] : P.Yin[1];
-  const T* Yv = first ? P.S[cur][2] : P.Yin[2];
+  const double tsub = ctl->t_local + P.c[st] * dt_d;
+  const T *Yh = P.in(st, cur, 0), *Yu = P.in(st, cur, 1), *Yv = P.in(st, cur, 2);
   const DX divx = MkDivX<DX>::make(P.dx), divy = MkDivX<DX>::make(P.dy);
   const T hdx = T(0.5) * T(P.dx), hdy = T(0.5) * T(P.dy);
   CellCtx<T, DX> c;
@@ -273,8 +270,8 @@ __device__ __noinline__ void sweep_rows_general(const StageParams<T>& P, int til
       const FaceF<T> FE{dn1(FW.h), dn1(FW.u), dn1(FW.v), dn1(FW.z)};
       if (out_lane && r < ny) {
         const long long g = (long long)r * nx + gx;
-        finish_cell<T, CellCtx<T, DX>, EDDY, true, COH>(P, fc, c, g, gx, r, me.h, me.u, me.v, me.dhdx, me.dhdy,
-                                                        me.dzdx, me.dzdy, FW, FE, FS, FN, first, last, cur, dt_d,
+        finish_cell<T, CellCtx<T, DX>, EDDY, true, COH>(P, st, fc, c, g, gx, r, me.h, me.u, me.v, me.dhdx, me.dhdy,
+                                                        me.dzdx, me.dzdy, FW, FE, FS, FN, cur, dt_d,
                                                         acc.rain, acc.removed, acc.walls, acc.xmax, acc.xmin, acc.vol,
                                                         &ed);
       }
@@ -440,7 +437,7 @@ template <typename T> __device__ __forceinline__ void sweep_totals(SweepShared<T
 // EXTRA: any source term, boundary kind and tableau (the rates of faces and slopes go through
 // finish_cell); without it Manning friction, rain, edge heads and a running accumulator.
 template <typename T, bool P2, bool EXTRA, bool EDGE, bool COH>
-__device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int tile_x, int y0, int y1, SweepShared<T>& sm,
+__device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int tile_x, int y0, int y1, SweepShared<T>& sm,
                                           SweepAcc<T>& acc) {
   constexpr bool F32 = sizeof(T) == 4;
   constexpr bool SCALED = F32 || P2;  // slopes and fluxes undivided, one scaling per cell
@@ -455,10 +452,8 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int tile_x, i
 
   const int cur = uniform(ctl->cur);
   const double dt_d = ctl->dt;
-  const bool first = P.mode & M_FIRST, last = P.mode & M_LAST;
-  const T* Yh = first ? P.S[cur][0] : P.Yin[0];
-  const T* Yu = first ? P.S[cur][1] : P.Yin[1];
-  const T* Yv = first ? P.S[cur][2] : P.Yin[2];
+  const bool first = st == 0, last = st == P.nstages - 1;
+  const T *Yh = P.in(st, cur, 0), *Yu = P.in(st, cur, 1), *Yv = P.in(st, cur, 2);
 
   // mesh constants (operands in the parameter bank: no registers)
   const auto& mc = P.mc;
@@ -478,11 +473,11 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int tile_x, i
   const bool rain_any = uniform(P.fc->rq0 != 0.0 || P.fc->rq1 != 0.0);
   __syncwarp();  // a strip swept before this one is done with them and with its rows
   if (lane == 0) {
-    const double tsub = ctl->t_local + P.c_s * dt_d, w = (tsub + 0.5 * dt_d) / P.L;
+    const double tsub = ctl->t_local + P.c[st] * dt_d, w = (tsub + 0.5 * dt_d) / P.L;
     vs.dt_d = dt_d; vs.tsub_d = tsub; vs.L = P.L; vs.rL = 1.0 / P.L;
     vs.dt = T(dt_d);
     vs.rdt = F32 ? T(1.0 / dt_d) : T(0);
-    vs.cA = T(P.a_next[P.stage] * dt_d); vs.cB = T(P.b[P.stage] * dt_d);
+    vs.cA = T(P.a[st][st] * dt_d); vs.cB = T(P.b[st] * dt_d);
     const double q0 = P.fc->rq0, q1 = P.fc->rq1;
     vs.rq0 = T(q0); vs.rq1 = T(q1);
     // FP32 rain: the mean of the step's linear rain over the stage's timestep, as a weight of its
@@ -497,7 +492,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int tile_x, i
   if constexpr (EXTRA) {
     fc = *P.fc;
     c.divL = mkdiv<T>(P.L);
-    c.dt = T(dt_d); c.dt_d = dt_d; c.tsub_d = ctl->t_local + P.c_s * dt_d;
+    c.dt = T(dt_d); c.dt_d = dt_d; c.tsub_d = ctl->t_local + P.c[st] * dt_d;
     c.rain_mode = P.rain_mode;
     c.divx = mkdiv<T>(P.dx); c.divy = mkdiv<T>(P.dy);
     c.divdt = mkdiv<T>(dt_d);
@@ -755,9 +750,9 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int tile_x, i
         if constexpr (EXTRA) {
           const T f = T(0.5);
           finish_cell<T, CellCtx<T>, true, EDGE, COH>(
-              P, fc, c, g, gx, r, h, u, v, Sm.hx, Sm.hy, Rm.zx, Rm.zy, {f * W.h, f * W.n, f * W.t, f * W.z},
+              P, st, fc, c, g, gx, r, h, u, v, Sm.hx, Sm.hy, Rm.zx, Rm.zy, {f * W.h, f * W.n, f * W.t, f * W.z},
               {f * E.h, f * E.n, f * E.t, f * E.z}, {f * GS.h, f * GS.t, f * GS.n, f * GS.z},
-              {f * GN.h, f * GN.t, f * GN.n, f * GN.z}, first, last, cur, dt_d, acc.rain, acc.removed, acc.walls,
+              {f * GN.h, f * GN.t, f * GN.n, f * GN.z}, cur, dt_d, acc.rain, acc.removed, acc.walls,
               acc.xmax, acc.xmin, acc.vol, &ed);
         } else {
           // flux divergence, depth slope, bed step (TemporalDerivativeKernel.cpp:53-98)
@@ -875,7 +870,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int tile_x, i
             if constexpr (F32) {  // the accumulator holds the increment
               const T d = mad_(kk[f], cB, a0);
               if (!last) {
-                P.Yout[f][g] = mad_(kk[f], cA, u0);
+                P.out(st, f)[g] = mad_(kk[f], cA, u0);
                 A[g] = d;
               } else if (f == 0) {  // U_N.h = U0.h + d with the carried compensation (Neumaier)
                 const int o = o_hc;
@@ -890,7 +885,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int tile_x, i
               }
             } else {
               const T a = first ? u0 : a0;
-              if (!last) P.Yout[f][g] = mad_(kk[f], cA, u0);
+              if (!last) P.out(st, f)[g] = mad_(kk[f], cA, u0);
               out[f] = mad_(kk[f], cB, a);
               A[g] = out[f];
             }
@@ -917,7 +912,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int tile_x, i
 // strip's index (row-major over strips of kSweepOut columns x P.rows rows) times 4 plus its
 // class.
 template <typename T, bool P2, bool EXTRA, bool COH>
-__device__ __forceinline__ void sweep_strip(const StageParams<T>& P, unsigned entry, SweepShared<T>& sm) {
+__device__ __forceinline__ void sweep_strip(const StageParams<T>& P, int st, unsigned entry, SweepShared<T>& sm) {
   const unsigned e = unsigned(uniform(int(entry)));
   const long long gw = e >> 2;
   const unsigned cls = e & 3u;
@@ -926,15 +921,15 @@ __device__ __forceinline__ void sweep_strip(const StageParams<T>& P, unsigned en
   const int tile_x = int(gw) - tile_y * tiles_x, y0 = tile_y * P.rows, y1 = min(y0 + P.rows, P.ny);
   SweepAcc<T> acc;
   int y = y0;
-  if (cls == kStripInterior) y = sweep_rows<T, P2, EXTRA, false, COH>(P, tile_x, y0, y1, sm, acc);
-  else if (cls == kStripEdge) y = sweep_rows<T, P2, EXTRA, true, COH>(P, tile_x, y0, y1, sm, acc);
+  if (cls == kStripInterior) y = sweep_rows<T, P2, EXTRA, false, COH>(P, st, tile_x, y0, y1, sm, acc);
+  else if (cls == kStripEdge) y = sweep_rows<T, P2, EXTRA, true, COH>(P, st, tile_x, y0, y1, sm, acc);
   if (y < y1) {
     SweepAcc<T> rest = acc;
-    sweep_rows_general<T, EXTRA, COH>(P, tile_x, y, y1, rest);
+    sweep_rows_general<T, EXTRA, COH>(P, st, tile_x, y, y1, rest);
     acc = rest;
   }
   const int lane = threadIdx.x;
-  if (P.mode & M_LAST) {
+  if (st == P.nstages - 1) {
     const double mx = warp_max(double(acc.xmax)), mn = warp_min(double(acc.xmin)), vs = warp_sum(acc.vol);
     if (lane == 0) {
       P.part[gw] = mx;
@@ -944,7 +939,7 @@ __device__ __forceinline__ void sweep_strip(const StageParams<T>& P, unsigned en
   }
   if (P.mode & M_TALLY) {
     const double rs = warp_sum(acc.rain), os = warp_sum(acc.removed), ws = warp_sum(acc.walls);
-    if (lane == 0) store_tallies(P, gw, rs, os, ws, P.mode & M_FIRST, P.ctl->dt);
+    if (lane == 0) store_tallies(P, st, gw, rs, os, ws, P.ctl->dt);
   }
 }
 
@@ -953,44 +948,39 @@ constexpr int kSweepWarps = 4;  // warps (strips) per block
 // The strips listed in P.strips (general and edge strips first: they are the longer ones, so
 // they do not end up as the launch's tail).
 template <typename T, int MINB, bool P2, bool EXTRA>
-__global__ void __launch_bounds__(32 * kSweepWarps, MINB) sweep_kernel(const __grid_constant__ StageParams<T> P) {
-  if (P.ctl->done) return;
-  const long long i = (long long)blockIdx.x * kSweepWarps + threadIdx.y;
-  if (i >= P.n_strips) return;  // whole warp: no block-level synchronisation below
+__global__ void __launch_bounds__(32 * kSweepWarps, MINB)
+    sweep_kernel(const __grid_constant__ StageParams<T> P, const int st) {
   extern __shared__ __align__(16) unsigned char sweep_smem[];
-  sweep_strip<T, P2, EXTRA, false>(P, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[uniform(threadIdx.y)]);
+  if (P.ctl->done) return;
+  const int w = uniform(threadIdx.y), i = int(blockIdx.x) * kSweepWarps + w;
+  if (i >= P.n_strips) return;  // whole warp: no block-level synchronisation below
+  sweep_strip<T, P2, EXTRA, false>(P, st, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[w]);
 }
 
-// Batched column sweep: the strips of every instance of a batch, warp_start[i] being the
-// first global warp of instance i. Each warp finds its instance, stages its parameters in
-// shared memory and sweeps its strip; instances whose step is finished return at once.
+// Batched column sweep: the strips of up to kBatchMembers solvers in one launch. Their parameters
+// are kernel parameters, so a block reads them as constants, as the single-solver kernel does
+// (staged in shared memory instead they took registers from the sweep, which then spilled). A
+// block sweeps strips of one solver: first_block[k] is member k's first block.
+constexpr int kBatchMembers = 32;
+template <typename T> struct BatchParams {
+  int n;
+  int first_block[kBatchMembers + 1];
+  StageParams<T> m[kBatchMembers];
+};
+static_assert(sizeof(BatchParams<double>) <= 32764 && sizeof(BatchParams<float>) <= 32764, "kernel parameters");
+
 template <typename T, int MINB, bool P2, bool EXTRA>
 __global__ void __launch_bounds__(32 * kSweepWarps, MINB)
-    sweep_batch_kernel(const StageParams<T>* __restrict__ Ps, const long long* __restrict__ warp_start, int ninst) {
-  __shared__ __align__(16) StageParams<T> Psh[kSweepWarps];
-  const long long gw = (long long)blockIdx.x * kSweepWarps + threadIdx.y;
-  if (gw >= warp_start[ninst]) return;  // whole warp
-  int inst = 0;
-  if (threadIdx.x == 0) {
-    int lo = 0, hi = ninst - 1;  // last instance with warp_start[i] <= gw
-    while (lo < hi) {
-      int mid = (lo + hi + 1) / 2;
-      if (warp_start[mid] <= gw) lo = mid;
-      else hi = mid - 1;
-    }
-    inst = lo;
-  }
-  inst = __shfl_sync(kFull, inst, 0);
-  if (Ps[inst].ctl->done) return;
-  static_assert(sizeof(StageParams<T>) % 4 == 0, "parameter block copied as 32-bit words");
-  const unsigned* src = reinterpret_cast<const unsigned*>(Ps + inst);
-  unsigned* dst = reinterpret_cast<unsigned*>(&Psh[threadIdx.y]);
-  for (int i = threadIdx.x; i < int(sizeof(StageParams<T>) / 4); i += 32) dst[i] = src[i];
-  __syncwarp();
-  const StageParams<T>& P = Psh[threadIdx.y];
+    sweep_batch_kernel(const __grid_constant__ BatchParams<T> B, const int st) {
   extern __shared__ __align__(16) unsigned char sweep_smem[];
-  sweep_strip<T, P2, EXTRA, false>(P, P.strips[gw - warp_start[inst]],
-                                   reinterpret_cast<SweepShared<T>*>(sweep_smem)[uniform(threadIdx.y)]);
+  int k = 0;
+  for (int step = kBatchMembers / 2; step > 0; step /= 2)  // the last member that starts at or before this block
+    if (k + step < B.n && B.first_block[k + step] <= int(blockIdx.x)) k += step;
+  const StageParams<T>& P = B.m[k];
+  if (P.ctl->done) return;
+  const int w = uniform(threadIdx.y), i = (int(blockIdx.x) - B.first_block[k]) * kSweepWarps + w;
+  if (i >= P.n_strips) return;
+  sweep_strip<T, P2, EXTRA, false>(P, st, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[w]);
 }
 
 }  // namespace svk
