@@ -6,13 +6,17 @@
 // rolling window. Every face flux and every difference quotient is computed once and reused by
 // both cells / both slopes that need it, and there is no block-level barrier.
 //
-// A strip is one of three classes (strip_class_kernel):
-//   kStripInterior  its whole window lies inside the mesh: no edge test anywhere
-//   kStripEdge      the window meets the mesh edge: one-sided slopes, wall faces and
-//                   edge boundaries as selects on the same code
-//   kStripGeneral   the window holds a coded-out (NaN) bed, or a bed outside the range below
-// The first two run sweep_rows, the third sweep_rows_general, which follows the reference's
-// functions literally.
+// A strip is of one of three classes (strip_class_kernel):
+//   kStripInterior  its whole window lies inside the mesh: sweep_rows without edge tests
+//   kStripEdge      the window meets the mesh edge: sweep_rows with warp-uniform branches for
+//                   one-sided slopes, wall faces and edge boundaries
+//   kStripGeneral   the window holds a coded-out (NaN) bed or one outside the range below:
+//                   sweep_rows_general, which follows the reference's functions literally
+// The edge form costs an interior strip 15 % (FP32: 474 against 403 us a stage at 4096 x 4096;
+// FP64: 1028 against 923). The persistent batch kernel runs every strip in the edge form all the
+// same: its warps mix strips of all members at all times, and the two codes evicted each other
+// from the instruction cache (3.3 cycles of no_instruction stall per issue; 149 ms against 122
+// for 16 catchments).
 //
 // sweep_rows computes the same values as sweep_rows_general with far fewer instructions. In
 // FP64 the results are bit-identical (up to the sign of zeros) as long as every h, u, v of the
@@ -89,7 +93,7 @@ constexpr int kSweepOut = 28;  // output columns per warp
 // of 16 bytes cover it; the chunks of all fields are numbered and dealt to the lanes, kWSlots
 // chunks per lane for the window and kCSlots for the per-cell fields, five (FP32) or nine (FP64)
 // copy instructions per row instead of fourteen loads with their address arithmetic. Fields have
-// at least kFieldPad bytes behind them (chunks reach past the last cell); in rows whose length is
+// at least kFieldPad bytes behind them (a row of chunks reaches past the last cell); in rows whose length is
 // not a multiple of the chunk the first column's place in its chunk changes from row to row.
 template <typename T> struct RowRing {
   static constexpr int kChunk = 16 / int(sizeof(T));               // values per chunk
@@ -102,7 +106,8 @@ template <typename T> struct RowRing {
   static constexpr int kBytes = kStages * kStage;                  // per warp
   static constexpr int kFieldBytes = kCpr * 16;
 };
-constexpr int kFieldPad = 16;
+constexpr int kFieldPad = 288;
+static_assert(kFieldPad >= RowRing<float>::kFieldBytes && kFieldPad >= RowRing<double>::kFieldBytes, "row of chunks");
 __device__ __forceinline__ void copy16(unsigned dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -294,7 +299,7 @@ __device__ __forceinline__ bool in_range(double x) {
 __device__ __forceinline__ bool in_range(float x) { return x == x; }
 
 // Whether the whole window (32 columns x the output rows and two more on each side) of strip
-// `gw` of strips of `rows` output rows lies inside the mesh.
+// `gw` of strips of `rows` output rows lies inside the mesh, with a column to spare.
 __host__ __device__ inline bool strip_inside(long long gw, int nx, int ny, int rows) {
   const int tiles_x = (nx + kSweepOut - 1) / kSweepOut;
   const int x0 = int(gw % tiles_x) * kSweepOut, y0 = int(gw / tiles_x) * rows;
@@ -448,7 +453,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
   const int gx = gx0 + lane;
   const int gxc = EDGE ? min(max(gx, 0), nx - 1) : gx;
   const bool out_lane = lane >= 2 && lane < 2 + kSweepOut && (!EDGE || gx < nx);
-  const bool hasW = gx > 0, hasE = gx < nx - 1;  // EDGE
+  const bool xedge = EDGE && (gx0 < 0 || gx0 + 31 >= nx - 1);  // the strip holds the mesh's first or last column
 
   const int cur = uniform(ctl->cur);
   const double dt_d = ctl->dt;
@@ -498,7 +503,6 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
     c.divdt = mkdiv<T>(dt_d);
     c.manning = P.manning; c.head_first = P.head_first;
   }
-  const T ry = mc.ry;
 
   // FP32 with tile datums: a vertical face crosses datum tiles where its right cell starts a
   // tile column, a horizontal face where its upper row starts a tile row; there the upper /
@@ -541,38 +545,20 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
   const int ncopies = ncell * RR::kCpr;  // chunks of the per-cell fields
   __syncwarp();
   const unsigned ring0 = unsigned(__cvta_generic_to_shared(sm.ring));
-  const long long last_chunk = ((long long)nx * ny - 1) & ~(long long)(RR::kChunk - 1);
-  // copies of window row w and per-cell row q into the ring's stage `k & 1`
+  // copies of window row w (the mesh's nearest one) and per-cell row q into the ring's stage `k & 1`
   auto fetch = [&](int k, int w, int q) {
     const unsigned dst = ring0 + (k & 1) * RR::kStage + lane * 16;
     if (w <= y1 + 1) {
-      const long long off =
-          ((long long)(EDGE ? min(max(w, 0), ny - 1) : w) * nx + c0) & ~(long long)(RR::kChunk - 1);
+      const long long off = ((long long)(EDGE ? min(max(w, 0), ny - 1) : w) * nx + c0) & ~(long long)(RR::kChunk - 1);
 #pragma unroll
-      for (int s = 0; s < RR::kWSlots; ++s) {
-        if (lane + 32 * s >= 6 * RR::kCpr) continue;
-        const T* src = vs.src[s][lane];
-        if constexpr (EDGE) {  // rows of the last columns: stay inside the field
-          const int j = ((lane + 32 * s) % RR::kCpr) * RR::kChunk;
-          copy16(dst + s * 512, src + (min(off + j, last_chunk) - j));
-        } else {
-          copy16(dst + s * 512, src + off);
-        }
-      }
+      for (int s = 0; s < RR::kWSlots; ++s)
+        if (lane + 32 * s < 6 * RR::kCpr) copy16(dst + s * 512, vs.src[s][lane] + off);
     }
     if (!EXTRA && q >= y0 && q < y1) {
       const long long off = ((long long)q * nx + c0) & ~(long long)(RR::kChunk - 1);
 #pragma unroll
-      for (int s = 0; s < RR::kCSlots; ++s) {
-        if (lane + 32 * s >= ncopies) continue;
-        const T* src = vs.src[RR::kWSlots + s][lane];
-        if constexpr (EDGE) {
-          const int j = ((lane + 32 * s) % RR::kCpr) * RR::kChunk;
-          copy16(dst + (RR::kWSlots + s) * 512, src + (min(off + j, last_chunk) - j));
-        } else {
-          copy16(dst + (RR::kWSlots + s) * 512, src + off);
-        }
-      }
+      for (int s = 0; s < RR::kCSlots; ++s)
+        if (lane + 32 * s < ncopies) copy16(dst + (RR::kWSlots + s) * 512, vs.src[RR::kWSlots + s][lane] + off);
     }
     copies_commit();
   };
@@ -622,15 +608,14 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
     // half slopes of row k-1 (State.cpp:187-192). Along y they are formed towards row + 1, the
     // negative of the reference's (its Y axis takes north as the left side).
     if (k >= y0) {
-      const bool hasN = !EDGE || k - 1 < ny - 1, hasS = !EDGE || k - 1 > 0;
+      const int row = k - 1;
+      const bool yedge = EDGE && (row <= 0 || row >= ny - 1);
       auto yslope = [&](T a, T b, T lo, T hi, T& j, T& s) {
-        T cc = F32 ? a + b : qy(hi - lo);
-        if constexpr (EDGE) {  // one-sided: the present quotient
-          if (!hasN) { b = a; cc = a + a; }
-          if (!hasS) { a = b; cc = hasN ? b + b : T(0); }
-          if (!hasN && !hasS) a = b = T(0);
+        T hs = half_slope(a, b, F32 ? a + b : qy(hi - lo));
+        if (yedge) {  // one-sided: the slope is the present quotient
+          if (row >= ny - 1) hs = T(0.5) * a;
+          if (row <= 0) hs = ny > 1 ? T(0.5) * b : T(0);
         }
-        const T hs = half_slope(a, b, cc);
         if constexpr (SCALED) {
           j = hs;
           if constexpr (EXTRA) s = T(-2) * hs * mc.rdy;
@@ -644,17 +629,15 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
       yslope(fyA[2], fyB[2], Rm.v, Rp.v, J0.vy, S0.vy);
       auto xslope = [&](T x, T& j, T& s) {
         const T e = dn1(x);
-        T b = qx(e - x);
-        T a = up1(b);
+        const T b = qx(e - x), a = up1(b);
         T cc;
         if constexpr (F32) cc = a + b;
         else cc = qx(e - up1(x));
-        if constexpr (EDGE) {
-          if (!hasE) { b = a; cc = a + a; }
-          if (!hasW) { a = b; cc = hasE ? b + b : T(0); }
-          if (!hasE && !hasW) a = b = T(0);
+        T hs = half_slope(a, b, cc);
+        if (xedge) {
+          if (gx >= nx - 1) hs = T(0.5) * a;
+          if (gx <= 0) hs = nx > 1 ? T(0.5) * b : T(0);
         }
-        const T hs = half_slope(a, b, cc);
         if constexpr (SCALED) {
           j = hs;
           if constexpr (EXTRA) s = T(2) * hs * mc.rdx;
@@ -680,7 +663,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
       }
       Side<T> m{zside(mc.hdy, Rm.zy, Rm.z), Rm.h - Jm.hy, Rm.v - Jm.vy, Rm.u - Jm.uy};
       Side<T> p{zside(-mc.hdy, R0.zy, zhi), R0.h + J0.hy, R0.v + J0.vy, R0.u + J0.uy};
-      if constexpr (EDGE) {  // walls at the mesh edge, FluxKernel.cpp:111-157
+      if (EDGE && (fy <= 0 || fy >= ny)) {  // walls at the mesh edge, FluxKernel.cpp:111-157
         if (fy == 0) m = {R0.z + R0.h * T(2), T(0), T(0), R0.u - J0.uy};
         if (fy == ny) p = {Rm.z + Rm.h * T(2), T(0), T(0), Rm.u + Jm.uy};
       }
@@ -712,7 +695,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
       Side<T> p{zside(-mc.hdx, Rm.zx, zw), Rm.h - Jm.hx, Rm.u - Jm.ux, Rm.v - Jm.vx};
       const T eut = Rm.v + Jm.vx;
       Side<T> m{up1(zside(mc.hdx, Rm.zx, Rm.z)), up1(Rm.h + Jm.hx), up1(Rm.u + Jm.ux), up1(eut)};
-      if constexpr (EDGE) {
+      if (xedge) {
         const T wall = Rm.z + Rm.h * T(2);
         const T wl = up1(wall), utl = up1(p.ut);
         if (gx == 0) m = {wall, T(0), T(0), eut};
@@ -724,7 +707,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
       if constexpr (EXTRA) {
         if (P.eddy) {  // second derivatives of row r: x by shuffles, y from rows r+1, r, r-1
           ed.ux = Sm.ux; ed.uy = Sm.uy; ed.vx = Sm.vx; ed.vy = Sm.vy;
-          const bool w = !EDGE || hasW, e = !EDGE || hasE;
+          const bool w = !EDGE || gx > 0, e = !EDGE || gx < nx - 1;
           {
             T r_ = dn1(Sm.ux), l_ = up1(Sm.ux);
             T fq = c.divx(r_ - Sm.ux);
@@ -757,8 +740,20 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
         } else {
           // flux divergence, depth slope, bed step (TemporalDerivativeKernel.cpp:53-98)
           T dh, du, dv;
-          if constexpr (SCALED) {
+          if constexpr (F32) {
+            // each difference is scaled before the next is added: beside a wall the momentum and
+            // bed-step fluxes of one face are large and cancel, and the order decides what is left
+            // of their rounding
+            dh = mad_(GS.h - GN.h, mc.ky, (W.h - E.h) * mc.kx);
+            du = mad_(GS.t - GN.t, mc.ky, (W.n - E.n) * mc.kx);
+            dv = mad_(GS.n - GN.n, mc.ky, (W.t - E.t) * mc.kx);
+            du = mad_(-mc.gx, Jm.hx, du);
+            dv = mad_(mc.gy, Jm.hy, dv);
+            du = mad_(W.z - E.z, mc.kx, du);
+            dv = mad_(GS.z - GN.z, mc.ky, dv);
+          } else if constexpr (SCALED) {
             const T g4 = T(4) * T(kG);
+            const T ry = mc.ry;
             dh = sfma_(GS.h - GN.h, ry, W.h - E.h) * mc.kx;
             du = sfma_(GS.t - GN.t, ry, W.n - E.n);
             dv = sfma_(GS.n - GN.n, ry, W.t - E.t);
@@ -791,7 +786,8 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
                                P.man_p[3] ? ld(P.man_p[3], g) : P.man_s[3]);
             friction(h, u, v, n, vs.dt, vs.rdt, du, dv);
           }
-          if constexpr (EDGE) {
+          const bool medge = EDGE && (xedge || r == 0 || r == ny - 1);
+          if (medge) {
             double w = 0.0;
             if (gx == 0) w += double(dvx(W.h));
             if (gx == nx - 1) w -= double(dvx(E.h));
@@ -830,7 +826,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
             if (applied) { dh = dh + rate; acc.rain += double(rate); }
           };
           auto do_head = [&]() {
-            if constexpr (EDGE) {
+            if (medge) {
               const DevForcing& f = *P.fc;
               const bool sel = ((f.head_edges & 1u) && gx == 0) || ((f.head_edges & 2u) && gx == nx - 1) ||
                                ((f.head_edges & 4u) && r == 0) || ((f.head_edges & 8u) && r == ny - 1);
@@ -910,8 +906,8 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
 
 // One strip of one solver's stage: its class's sweep, then its partial sums. `entry` is the
 // strip's index (row-major over strips of kSweepOut columns x P.rows rows) times 4 plus its
-// class.
-template <typename T, bool P2, bool EXTRA, bool COH>
+// class. SPLIT: interior strips run the form without edge tests.
+template <typename T, bool P2, bool EXTRA, bool SPLIT, bool COH>
 __device__ __forceinline__ void sweep_strip(const StageParams<T>& P, int st, unsigned entry, SweepShared<T>& sm) {
   const unsigned e = unsigned(uniform(int(entry)));
   const long long gw = e >> 2;
@@ -921,8 +917,8 @@ __device__ __forceinline__ void sweep_strip(const StageParams<T>& P, int st, uns
   const int tile_x = int(gw) - tile_y * tiles_x, y0 = tile_y * P.rows, y1 = min(y0 + P.rows, P.ny);
   SweepAcc<T> acc;
   int y = y0;
-  if (cls == kStripInterior) y = sweep_rows<T, P2, EXTRA, false, COH>(P, st, tile_x, y0, y1, sm, acc);
-  else if (cls == kStripEdge) y = sweep_rows<T, P2, EXTRA, true, COH>(P, st, tile_x, y0, y1, sm, acc);
+  if (SPLIT && cls == kStripInterior) y = sweep_rows<T, P2, EXTRA, false, COH>(P, st, tile_x, y0, y1, sm, acc);
+  else if (cls != kStripGeneral) y = sweep_rows<T, P2, EXTRA, true, COH>(P, st, tile_x, y0, y1, sm, acc);
   if (y < y1) {
     SweepAcc<T> rest = acc;
     sweep_rows_general<T, EXTRA, COH>(P, st, tile_x, y, y1, rest);
@@ -945,8 +941,8 @@ __device__ __forceinline__ void sweep_strip(const StageParams<T>& P, int st, uns
 
 constexpr int kSweepWarps = 4;  // warps (strips) per block
 
-// The strips listed in P.strips (general and edge strips first: they are the longer ones, so
-// they do not end up as the launch's tail).
+// The strips listed in P.strips (general and edge strips first: they take longer, so they do
+// not end up as the launch's tail).
 template <typename T, int MINB, bool P2, bool EXTRA>
 __global__ void __launch_bounds__(32 * kSweepWarps, MINB)
     sweep_kernel(const __grid_constant__ StageParams<T> P, const int st) {
@@ -954,7 +950,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, MINB)
   if (P.ctl->done) return;
   const int w = uniform(threadIdx.y), i = int(blockIdx.x) * kSweepWarps + w;
   if (i >= P.n_strips) return;  // whole warp: no block-level synchronisation below
-  sweep_strip<T, P2, EXTRA, false>(P, st, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[w]);
+  sweep_strip<T, P2, EXTRA, !EXTRA, false>(P, st, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[w]);
 }
 
 // Batched column sweep: the strips of up to kBatchMembers solvers in one launch. Their parameters
@@ -980,7 +976,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, MINB)
   if (P.ctl->done) return;
   const int w = uniform(threadIdx.y), i = (int(blockIdx.x) - B.first_block[k]) * kSweepWarps + w;
   if (i >= P.n_strips) return;
-  sweep_strip<T, P2, EXTRA, false>(P, st, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[w]);
+  sweep_strip<T, P2, EXTRA, !EXTRA, false>(P, st, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[w]);
 }
 
 }  // namespace svk
