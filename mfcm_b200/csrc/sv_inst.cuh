@@ -110,27 +110,20 @@ template <int MINB, bool EXTRA> static cudaError_t launch_sweep_c(const StagePar
 static cudaError_t launch_sweep(const StageParams<SV_T>& P, int st, int cap, bool extra, cudaStream_t s) {
   if (extra) return launch_sweep_c<kExtraCap<SV_T>, true>(P, st, s);
   if constexpr (sizeof(SV_T) == 8) {
-    switch (cap) {
-      case 3: return launch_sweep_c<3, false>(P, st, s);
-      case 4: return launch_sweep_c<4, false>(P, st, s);
-      case 5: return launch_sweep_c<5, false>(P, st, s);
-      default: return launch_sweep_c<6, false>(P, st, s);
-    }
+    return cap == 3 ? launch_sweep_c<3, false>(P, st, s) : launch_sweep_c<4, false>(P, st, s);
   } else {
     switch (cap) {
-      case 3:
       case 4: return launch_sweep_c<4, false>(P, st, s);
       case 5: return launch_sweep_c<5, false>(P, st, s);
       case 6: return launch_sweep_c<6, false>(P, st, s);
-      case 7: return launch_sweep_c<7, false>(P, st, s);
-      default: return launch_sweep_c<8, false>(P, st, s);
+      default: return launch_sweep_c<7, false>(P, st, s);
     }
   }
 }
 
 template <> cudaError_t launch_variant<SV_T>(const StageParams<SV_T>& P, int st, int variant, bool extra, cudaStream_t s) {
   if (variant_is_split(variant)) return launch_split_t<SV_T>(P, st, s);
-  if (variant_is_sweep(variant)) return launch_sweep(P, st, variant_cap<SV_T>(variant), extra, s);
+  if (variant_is_sweep(variant)) return launch_sweep(P, st, variant_cap<SV_T>(variant, P.n_strips), extra, s);
   return launch_stage<SV_T>(P, st, variant, s);
 }
 

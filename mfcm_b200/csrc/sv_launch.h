@@ -58,7 +58,18 @@ inline int variant_sweep_rows(int v, long long nx, long long ny) {
   if (v == kAutoVariant) return auto_rows(nx, ny);
   return variant_is_sweep(v) ? kSweeps[v].rows : 0;
 }
-template <typename T> inline int variant_cap(int v) { return kSweeps[v].cap; }
+// register caps compiled: FP64 3 and 4 blocks per SM, FP32 4 to 7 (tighter ones spill: FP64 stages at 4096 x 4096
+// 1.3 ms at 5 blocks against 0.92 at 4, FP32 455 us at 8 against 408 at 6)
+template <typename T> inline int clamp_cap(int cap) {
+  const int lo = sizeof(T) == 8 ? 3 : 4, hi = sizeof(T) == 8 ? 4 : 7;
+  return cap < lo ? lo : (cap > hi ? hi : cap);
+}
+// FP32, variant 5: 4 blocks per SM while all strips are resident at once (each warp then runs
+// fastest), else 6: 43 against 70 us a stage at 1024 x 1024, 445 against 408 at 4096 x 4096
+template <typename T> inline int variant_cap(int v, long long strips) {
+  if (v == kAutoVariant && sizeof(T) == 4) return strips <= kFillStrips + kFillStrips / 4 ? 4 : 6;
+  return clamp_cap<T>(kSweeps[v].cap);
+}
 // per-CTA (tiled) or per-warp (sweep) partial count
 inline long long variant_partials(int v, long long nx, long long ny) {
   if (v == kSplitVariant) v = 1;  // the split schedule's stage pass is the tiled 32 x 8 kernel

@@ -131,6 +131,7 @@ template <typename T> struct alignas(16) SweepShared {  // rings of 16-byte copi
   T xmax[32], xmin[32];
   double dt_d, tsub_d, L, rL;
   T dt, rdt, cA, cB, rq0, rq1, rain_w, rain_q;
+  T ck[4];                                      // general tableaux: the coefficients of k_0 .. k_st
 };
 static_assert(sizeof(SweepShared<float>) % 16 == 0 && sizeof(SweepShared<double>) % 16 == 0 &&
                   offsetof(SweepShared<float>, ring) == 0 && offsetof(SweepShared<double>, ring) == 0,
@@ -350,6 +351,10 @@ __device__ __forceinline__ float pick_max(float a, float b) { return fmaxf(a, b)
 __device__ __forceinline__ double pick_max(double a, double b) { return a > b ? a : b; }
 __device__ __forceinline__ float clip0(float x) { return fmaxf(x, 0.0f); }
 __device__ __forceinline__ double clip0(double x) { return __double2hiint(x) < 0 ? 0.0 : x; }
+// the divider of a launch constant and its reciprocal
+template <typename T> __device__ __forceinline__ Div<T> div_by(T d, T rd);
+template <> __device__ __forceinline__ DivD div_by<double>(double d, double rd) { return DivD{d, rd}; }
+template <> __device__ __forceinline__ DivF div_by<float>(float, float rd) { return DivF{rd}; }
 // a * b + c, rounded once
 __device__ __forceinline__ float sfma_(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double sfma_(double a, double b, double c) { return fma(a, b, c); }
@@ -439,8 +444,8 @@ template <typename T> __device__ __forceinline__ void sweep_totals(SweepShared<T
 
 // Output rows y0 .. y1-1 (inside the mesh) of the strip of column `tile_x`. Returns y1, or the
 // first row not computed because the state left the range this function is exact for.
-// EXTRA: any source term, boundary kind and tableau (the rates of faces and slopes go through
-// finish_cell); without it Manning friction, rain, edge heads and a running accumulator.
+// EXTRA: any source term, boundary kind and tableau; without it Manning friction, rain, edge
+// heads and a running accumulator.
 template <typename T, bool P2, bool EXTRA, bool EDGE, bool COH>
 __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int tile_x, int y0, int y1, SweepShared<T>& sm,
                                           SweepAcc<T>& acc) {
@@ -481,8 +486,10 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
     const double tsub = ctl->t_local + P.c[st] * dt_d, w = (tsub + 0.5 * dt_d) / P.L;
     vs.dt_d = dt_d; vs.tsub_d = tsub; vs.L = P.L; vs.rL = 1.0 / P.L;
     vs.dt = T(dt_d);
-    vs.rdt = F32 ? T(1.0 / dt_d) : T(0);
+    vs.rdt = T(1.0 / dt_d);
     vs.cA = T(P.a[st][st] * dt_d); vs.cB = T(P.b[st] * dt_d);
+    if constexpr (EXTRA)
+      for (int j = 0; j <= st; ++j) vs.ck[j] = T((last ? P.b[j] : P.a[st][j]) * dt_d);
     const double q0 = P.fc->rq0, q1 = P.fc->rq1;
     vs.rq0 = T(q0); vs.rq1 = T(q1);
     // FP32 rain: the mean of the step's linear rain over the stage's timestep, as a weight of its
@@ -492,18 +499,6 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
   vs.vol[lane] = 0.0;
   vs.xmax[lane] = T(0);
   vs.xmin[lane] = T(1.0 / 0.0);
-  CellCtx<T> c;  // EXTRA (the rates go through finish_cell)
-  DevForcing fc;
-  if constexpr (EXTRA) {
-    fc = *P.fc;
-    c.divL = mkdiv<T>(P.L);
-    c.dt = T(dt_d); c.dt_d = dt_d; c.tsub_d = ctl->t_local + P.c[st] * dt_d;
-    c.rain_mode = P.rain_mode;
-    c.divx = mkdiv<T>(P.dx); c.divy = mkdiv<T>(P.dy);
-    c.divdt = mkdiv<T>(dt_d);
-    c.manning = P.manning; c.head_first = P.head_first;
-  }
-
   // FP32 with tile datums: a vertical face crosses datum tiles where its right cell starts a
   // tile column, a horizontal face where its upper row starts a tile row; there the upper /
   // right cell's bed moves into the other cell's frame (face_frame)
@@ -512,7 +507,8 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
   // the row ring: this lane's chunks
   using RR = RowRing<T>;
   const int c0 = EDGE ? max(gx0, 0) : gx0;  // first column of the rows copied
-  int o_ns = -1, o_nd = -1, o_r0 = -1, o_r1 = -1, o_hc = -1;  // per-cell fields: place in the ring's row, or -1
+  // per-cell fields: place in the ring's row, or -1
+  int o_ns = -1, o_nd = -1, o_r0 = -1, o_r1 = -1, o_hc = -1, o_ex = -1, o_ey = -1, o_ir = -1, o_ic = -1;
   int ncell = 0;                                              // per-cell fields in the ring
   {
     auto deal = [&](const T* f, int n, int slot0, int slots) {  // field number n of a class
@@ -523,23 +519,30 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
     };
     deal(Yh, 0, 0, RR::kWSlots); deal(Yu, 1, 0, RR::kWSlots); deal(Yv, 2, 0, RR::kWSlots);
     deal(P.z, 3, 0, RR::kWSlots); deal(P.zx, 4, 0, RR::kWSlots); deal(P.zy, 5, 0, RR::kWSlots);
-    if constexpr (!EXTRA) {
-      auto add = [&](const T* f) {
-        if (ncell >= RR::kCellFields) return -1;
-        deal(f, ncell, RR::kWSlots, RR::kCSlots);
-        return ncell++ * RR::kFieldBytes;
-      };
-      if (!first) {
-        for (int f = 0; f < 3; ++f) add(P.S[cur][f]);
+    auto add = [&](const T* f) {
+      if (ncell >= RR::kCellFields) return -1;
+      deal(f, ncell, RR::kWSlots, RR::kCSlots);
+      return ncell++ * RR::kFieldBytes;
+    };
+    if (!first) {  // U_[0], then the running sum or, of a general tableau, the stored k's
+      for (int f = 0; f < 3; ++f) add(P.S[cur][f]);
+      if (!EXTRA || (P.mode & M_ACC)) {
         for (int f = 0; f < 3; ++f) add(P.S[cur ^ 1][f]);
+      } else {
+        for (int j = 0; j < st; ++j)
+          for (int f = 0; f < 3; ++f) add(P.K[j][f]);
       }
-      if (P.manning) {
-        if (P.man_p[0]) o_ns = add(P.man_p[0]);
-        if (P.man_p[1] && P.man_p[1] != P.man_p[0]) o_nd = add(P.man_p[1]);
-      }
-      if (rk == 3) o_r0 = add(P.pat);
-      if (rk == 2) { o_r0 = add(P.q0p); o_r1 = add(P.q1p); }
-      if (F32 && last && P.hc[0]) o_hc = add(P.hc[cur]);
+    }
+    if (P.manning) {
+      if (P.man_p[0]) o_ns = add(P.man_p[0]);
+      if (P.man_p[1] && P.man_p[1] != P.man_p[0]) o_nd = add(P.man_p[1]);
+    }
+    if (rk == 3) o_r0 = add(P.pat);
+    if (rk == 2) { o_r0 = add(P.q0p); o_r1 = add(P.q1p); }
+    if (F32 && last && P.hc[0] && (!EXTRA || (P.mode & M_ACC))) o_hc = add(P.hc[cur]);
+    if constexpr (EXTRA) {
+      if (P.efx) { o_ex = add(P.efx); o_ey = add(P.efy); }
+      if (P.irate) { o_ir = add(P.irate); o_ic = add(P.icap); }
     }
   }
   const int ncopies = ncell * RR::kCpr;  // chunks of the per-cell fields
@@ -554,7 +557,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
       for (int s = 0; s < RR::kWSlots; ++s)
         if (lane + 32 * s < 6 * RR::kCpr) copy16(dst + s * 512, vs.src[s][lane] + off);
     }
-    if (!EXTRA && q >= y0 && q < y1) {
+    if (q >= y0 && q < y1) {
       const long long off = ((long long)q * nx + c0) & ~(long long)(RR::kChunk - 1);
 #pragma unroll
       for (int s = 0; s < RR::kCSlots; ++s)
@@ -707,20 +710,26 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
       if constexpr (EXTRA) {
         if (P.eddy) {  // second derivatives of row r: x by shuffles, y from rows r+1, r, r-1
           ed.ux = Sm.ux; ed.uy = Sm.uy; ed.vx = Sm.vx; ed.vy = Sm.vy;
-          const bool w = !EDGE || gx > 0, e = !EDGE || gx < nx - 1;
-          {
-            T r_ = dn1(Sm.ux), l_ = up1(Sm.ux);
-            T fq = c.divx(r_ - Sm.ux);
-            ed.uxx = minmod3q<T>(up1(fq), w, fq, e, c.divx(r_ - l_));
-          }
-          {
-            T r_ = dn1(Sm.vx), l_ = up1(Sm.vx);
-            T fq = c.divx(r_ - Sm.vx);
-            ed.vxx = minmod3q<T>(up1(fq), w, fq, e, c.divx(r_ - l_));
-          }
-          const bool hasN = !EDGE || r < ny - 1, hasS = !EDGE || r > 0;
-          ed.uyy = minmod3q<T>(c.divy(Sm.uy - S0.uy), hasN, c.divy(Smm_uy - Sm.uy), hasS, c.divy(Smm_uy - S0.uy));
-          ed.vyy = minmod3q<T>(c.divy(Sm.vy - S0.vy), hasN, c.divy(Smm_vy - Sm.vy), hasS, c.divy(Smm_vy - S0.vy));
+          auto along_x = [&](T x) {
+            const T e = dn1(x), b = over_dx(e - x), a = up1(b);
+            T hs = half_slope(a, b, over_dx(e - up1(x)));
+            if (xedge) {
+              if (gx >= nx - 1) hs = T(0.5) * a;
+              if (gx <= 0) hs = nx > 1 ? T(0.5) * b : T(0);
+            }
+            return T(2) * hs;
+          };
+          auto along_y = [&](T south, T x, T north) {  // the reference's Y axis: north on the left
+            const T a = over_dy(x - north), b = over_dy(south - x);
+            T hs = half_slope(a, b, over_dy(south - north));
+            if (EDGE && r >= ny - 1) hs = T(0.5) * b;
+            if (EDGE && r <= 0) hs = ny > 1 ? T(0.5) * a : T(0);
+            return T(2) * hs;
+          };
+          ed.uxx = along_x(Sm.ux);
+          ed.vxx = along_x(Sm.vx);
+          ed.uyy = along_y(Smm_uy, Sm.uy, S0.uy);
+          ed.vyy = along_y(Smm_vy, Sm.vy, S0.vy);
         }
       }
       if (out_lane) {
@@ -730,14 +739,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
         const unsigned char* cell = stage + RR::kWSlots * 512 +
                                     (gxc - c0 + ((int(unsigned(r) * unsigned(nx)) + c0) & (RR::kChunk - 1))) * int(sizeof(T));
         auto field = [&](int o, const T* p) { return o >= 0 ? *reinterpret_cast<const T*>(cell + o) : ld(p, g); };
-        if constexpr (EXTRA) {
-          const T f = T(0.5);
-          finish_cell<T, CellCtx<T>, true, EDGE, COH>(
-              P, st, fc, c, g, gx, r, h, u, v, Sm.hx, Sm.hy, Rm.zx, Rm.zy, {f * W.h, f * W.n, f * W.t, f * W.z},
-              {f * E.h, f * E.n, f * E.t, f * E.z}, {f * GS.h, f * GS.t, f * GS.n, f * GS.z},
-              {f * GN.h, f * GN.t, f * GN.n, f * GN.z}, cur, dt_d, acc.rain, acc.removed, acc.walls,
-              acc.xmax, acc.xmin, acc.vol, &ed);
-        } else {
+        {
           // flux divergence, depth slope, bed step (TemporalDerivativeKernel.cpp:53-98)
           T dh, du, dv;
           if constexpr (F32) {
@@ -777,7 +779,8 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
             du = mad_(T(-kG), (sfabs(zx) > lx && zx != T(0)) ? flip_sign(lx, zx) : zx, du);
             dv = mad_(T(-kG), (sfabs(zy) > ly && zy != T(0)) ? flip_sign(ly, zy) : zy, dv);
           }
-          if (P.manning && h > T(1e-6)) {
+          auto roughness = [&]() {
+            if (!(P.manning && h > T(1e-6))) return;
             const T ns = P.man_p[0] ? field(o_ns, P.man_p[0]) : P.man_s[0];
             const T nd = P.man_p[1] ? (P.man_p[1] == P.man_p[0] ? ns : field(o_nd, P.man_p[1])) : P.man_s[1];
             T n = ns;
@@ -785,6 +788,32 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
               n = manning_n<T>(h, ns, nd, P.man_p[2] ? ld(P.man_p[2], g) : P.man_s[2],
                                P.man_p[3] ? ld(P.man_p[3], g) : P.man_s[3]);
             friction(h, u, v, n, vs.dt, vs.rdt, du, dv);
+          };
+          if constexpr (!EXTRA) {
+            roughness();
+          } else {  // the momentum terms in configuration order, then infiltration
+            CellCtx<T> c;
+            c.dt = vs.dt;
+            c.divdt = div_by<T>(vs.dt, vs.rdt);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+              const int term = (P.term_order >> (2 * i)) & 3;
+              if (term == 1) roughness();
+              if (term == 2 && P.efx)
+                energy_loss_apply<T>(h, u, v, field(o_ex, P.efx), field(o_ey, P.efy), c, du, dv);
+              if (term == 3 && P.eddy) {
+                const T mu = P.eddy == 2 ? smagorinsky_mu<T>(P.eddy_c, P.eddy_s, T(P.cell_area), ed)
+                                         : (P.eddy_mup ? ld(P.eddy_mup, g) : P.eddy_mu);
+                T fu = T(0), fv = T(0);
+                if (eddy_term<T>(h, u, v, mu, ed, c, fu, fv)) { du = du + fu; dv = dv + fv; }
+              }
+            }
+            if (P.irate) {  // infiltration (InfiltrationSourceTerm.cpp:43-62), capacity consumed in place
+              const T cap = o_ic >= 0 ? *reinterpret_cast<const T*>(cell + o_ic) : P.icap[g];
+              const T d = infiltration_depth<T>(h, field(o_ir, P.irate), cap, c);
+              dh = dh - c.divdt(d);
+              P.icap[g] = cap - d;
+            }
           }
           const bool medge = EDGE && (xedge || r == 0 || r == ny - 1);
           if (medge) {
@@ -826,30 +855,37 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
             if (applied) { dh = dh + rate; acc.rain += double(rate); }
           };
           auto do_head = [&]() {
-            if (medge) {
-              const DevForcing& f = *P.fc;
+            if (!EXTRA && !medge) return;
+            const DevForcing& f = *P.fc;
+            const int hk = f.head_kind;
+            T h0, h1;
+            if (medge && (hk == 1 || hk == 3)) {
               const bool sel = ((f.head_edges & 1u) && gx == 0) || ((f.head_edges & 2u) && gx == nx - 1) ||
                                ((f.head_edges & 4u) && r == 0) || ((f.head_edges & 8u) && r == ny - 1);
-              if (!(sel && (f.head_kind == 1 || f.head_kind == 3))) return;
-              T h0 = T(f.hh0), h1 = T(f.hh1);
-              if (f.head_kind == 3) {  // water levels: less the bed, in FP64 with tile datums
-                if (P.zdat) {
-                  const double zb = P.zdat[datum_tile(gx, r, P.dtiles_x)] + double(Rm.z);
-                  h0 = T(double(h0) - zb); h1 = T(double(h1) - zb);
-                } else {
-                  h0 = h0 - Rm.z; h1 = h1 - Rm.z;
-                }
-              }
-              if (!(h0 == h0 && h1 == h1)) return;  // NaN = not selected
-              CellCtx<T> hcx;
-              hcx.divL = mkdiv<T>(P.L);
-              hcx.dt = vs.dt; hcx.tsub_d = vs.tsub_d;
-              const T before = dh;
-              const T d = head_target<T>(h0, h1, hcx) - h;
-              if constexpr (F32) dh = d * vs.rdt;
-              else dh = div_slow(d, vs.dt);
-              acc.removed += double(before) - double(dh);
+              if (!sel) return;
+              h0 = T(f.hh0); h1 = T(f.hh1);
+            } else if (EXTRA && (hk == 2 || hk == 4)) {
+              h0 = ld(P.hb0p, g); h1 = ld(P.hb1p, g);
+            } else {
+              return;
             }
+            if (hk >= 3) {  // water levels: less the bed, in FP64 with tile datums
+              if (P.zdat) {
+                const double zb = P.zdat[datum_tile(gx, r, P.dtiles_x)] + double(Rm.z);
+                h0 = T(double(h0) - zb); h1 = T(double(h1) - zb);
+              } else {
+                h0 = h0 - Rm.z; h1 = h1 - Rm.z;
+              }
+            }
+            if (!(h0 == h0 && h1 == h1)) return;  // NaN = not selected
+            CellCtx<T> c;
+            c.divL = mkdiv<T>(P.L);
+            c.dt = vs.dt; c.tsub_d = vs.tsub_d;
+            const T before = dh;
+            const T d = head_target<T>(h0, h1, c) - h;
+            if constexpr (F32) dh = d * vs.rdt;
+            else dh = div_slow(d, vs.dt);
+            acc.removed += double(before) - double(dh);
           };
           if (P.head_first) { do_head(); do_rain(); }
           else { do_rain(); do_head(); }
@@ -857,6 +893,26 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
           const T kk[3] = {dh, du, dv}, U[3] = {h, u, v};
           const T cA = vs.cA, cB = vs.cB;
           T out[3];
+          if (EXTRA && !(P.mode & M_ACC)) {  // general tableau: U0 + k_0 c_0 + k_1 c_1 + ..., stored k's
+#pragma unroll
+            for (int f = 0; f < 3; ++f) {
+              T y = first ? U[f] : *reinterpret_cast<const T*>(cell + f * RR::kFieldBytes);
+              for (int j = 0; j < st; ++j) {
+                const int o = 3 + 3 * j + f;
+                const T kj = o < RR::kCellFields ? *reinterpret_cast<const T*>(cell + o * RR::kFieldBytes)
+                                                 : ldst<COH>(P.K[j][f], g);
+                y = mad_(kj, T(vs.ck[j]), y);
+              }
+              y = mad_(kk[f], T(vs.ck[st]), y);
+              out[f] = y;
+              if (last) {
+                P.S[cur ^ 1][f][g] = y;
+              } else {
+                P.K[st][f][g] = kk[f];
+                P.out(st, f)[g] = y;
+              }
+            }
+          } else
 #pragma unroll
           for (int f = 0; f < 3; ++f) {
             const T* ua = reinterpret_cast<const T*>(cell + f * RR::kFieldBytes);
