@@ -203,9 +203,16 @@ struct Solver final : public sv_ctx {
     return v == svk::kBatchVariant && batch_rows ? batch_rows
                                                  : svk::variant_sweep_rows(v, (long long)mesh.nx, (long long)mesh.ny);
   }
+  // the kernel that variant v launches: variant 5 is the row-tile kernel on small meshes without
+  // further terms
+  int kernel_of(int v) const {
+    return v == svk::kAutoVariant && !extra() && svk::prefers_tile_rows<T>((long long)mesh.nx, (long long)mesh.ny)
+               ? svk::kTileRowsVariant
+               : v;
+  }
   // partial slots of variant v
   long long partials(int v) const {
-    const int rows = sweep_rows(v);
+    const int rows = kernel_of(v) == svk::kTileRowsVariant ? svk::kTileRows : sweep_rows(v);
     return rows ? svk::strip_count((long long)mesh.nx, (long long)mesh.ny, rows)
                 : svk::variant_partials(v, (long long)mesh.nx, (long long)mesh.ny);
   }
@@ -221,8 +228,9 @@ struct Solver final : public sv_ctx {
   }
   // the list for variant v (a column-sweep variant), classified from the bed on the device
   int ensure_strips(int v) {
+    if (v == variant) nblk = partials(v);  // variant 5's kernel follows the terms in use
     const int rows = sweep_rows(v);
-    if (rows == 0) return SV_OK;
+    if (rows == 0 || kernel_of(v) == svk::kTileRowsVariant) return SV_OK;
     Strips& L = strips_[rows];
     if (L.valid) return SV_OK;
     const long long n = partials(v);
@@ -256,7 +264,7 @@ struct Solver final : public sv_ctx {
     auto it = strips_.find(P.rows);
     if (P.rows == 0 || it == strips_.end() || !it->second.valid) return;
     P.strips = it->second.d;
-    P.n_strips = int(partials(v));
+    P.n_strips = int(svk::strip_count((long long)mesh.nx, (long long)mesh.ny, P.rows));
   }
   // source terms, boundary fields or a tableau beyond the lean sweep (svk::sweep_rows)
   bool extra() const {
@@ -667,6 +675,7 @@ struct Solver final : public sv_ctx {
     P.dx = mesh.dx; P.dy = mesh.dy; P.L = prm.step_duration;
     P.cell_area = mesh.dx * mesh.dy;
     P.mc.set(mesh.dx, mesh.dy);
+    P.exact = svk::exact_mesh(mesh.dx, mesh.dy, sizeof(T) == 8);
     for (int b = 0; b < 2; ++b)
       for (int f = 0; f < 3; ++f) P.S[b][f] = S[b][f];
     P.z = z;
@@ -743,7 +752,7 @@ struct Solver final : public sv_ctx {
     const svk::StageParams<T> P = stage_params();
     for (int st = 0; st < N; ++st) {
       if (ev) SV_CUDA(cudaEventRecord(ev[2 * st], stream));
-      cudaError_t e = svk::launch_variant<T>(P, st, variant, extra(), stream);
+      cudaError_t e = svk::launch_variant<T>(P, st, kernel_of(variant), extra(), stream);
       if (e != cudaSuccess) return cuda_fail(e, "stage kernel");
       if (ev) SV_CUDA(cudaEventRecord(ev[2 * st + 1], stream));
     }
@@ -984,7 +993,7 @@ struct Solver final : public sv_ctx {
         for (int f = 0; f < 6; ++f) P.pslp[f] = pslp[f];
       }
       set_strips(P, v);
-      auto launch = [&]() -> cudaError_t { return svk::launch_variant<T>(P, 0, v, extra(), stream); };
+      auto launch = [&]() -> cudaError_t { return svk::launch_variant<T>(P, 0, kernel_of(v), extra(), stream); };
       cudaError_t e = launch();  // warm-up
       if (e != cudaSuccess) return cuda_fail(e, "autotune launch");
       SV_CUDA(cudaEventRecord(ev0, stream));

@@ -122,6 +122,13 @@ static cudaError_t launch_sweep(const StageParams<SV_T>& P, int st, int cap, boo
 }
 
 template <> cudaError_t launch_variant<SV_T>(const StageParams<SV_T>& P, int st, int variant, bool extra, cudaStream_t s) {
+  if (variant == kTileRowsVariant) {
+    if (P.nblk <= 0) return cudaSuccess;
+    const dim3 grid{unsigned(P.nblk)}, block(32, kTileWarps);
+    if (sizeof(SV_T) == 8 && pow2_mesh(P.dx, P.dy)) tile_rows_kernel<SV_T, sizeof(SV_T) == 8><<<grid, block, 0, s>>>(P, st);
+    else tile_rows_kernel<SV_T, false><<<grid, block, 0, s>>>(P, st);
+    return cudaGetLastError();
+  }
   if (variant_is_split(variant)) return launch_split_t<SV_T>(P, st, s);
   if (variant_is_sweep(variant)) return launch_sweep(P, st, variant_cap<SV_T>(variant, P.n_strips), extra, s);
   return launch_stage<SV_T>(P, st, variant, s);
@@ -130,9 +137,8 @@ template <> cudaError_t launch_variant<SV_T>(const StageParams<SV_T>& P, int st,
 template <> cudaError_t launch_strip_classes<SV_T>(const SV_T* z, int nx, int ny, double dx, double dy, int rows,
                                                    long long nstrips, unsigned char* cls, cudaStream_t s) {
   if (nstrips <= 0) return cudaSuccess;
-  auto fits = [](double d) { return sizeof(SV_T) == 4 || (d >= 0x1p-30 && d <= 0x1p40); };
-  strip_class_kernel<SV_T><<<unsigned((nstrips + 7) / 8), 256, 0, s>>>(z, nx, ny, rows, nstrips, fits(dx) && fits(dy),
-                                                                       cls);
+  strip_class_kernel<SV_T><<<unsigned((nstrips + 7) / 8), 256, 0, s>>>(z, nx, ny, rows, nstrips,
+                                                                       exact_mesh(dx, dy, sizeof(SV_T) == 8), cls);
   return cudaGetLastError();
 }
 

@@ -119,6 +119,7 @@ template <typename T> struct StageParams {
   // plus its class (strip_class_kernel)
   const unsigned* strips;
   int n_strips, rows;
+  int exact;  // the cell sizes allow sweep_rows (exact_mesh)
   // split schedule: the stage input's slopes dh/dx, du/dx, dv/dx, dh/dy, du/dy, dv/dy as
   // written by slopes_kernel (read by the stage kernel instead of computing them), or null
   T* pslp[6];

@@ -30,6 +30,13 @@ struct SweepShape { int rows, cap; };
 constexpr SweepShape kSweeps[kNumVariants] = {{0, 0},  {0, 0},  {0, 0},  {0, 0},  {16, 4}, {32, 4},
                                               {64, 4}, {32, 3}, {32, 4}, {32, 5}, {32, 6}, {0, 0},
                                               {32, 3}, {32, 4}, {32, 7}, {32, 8}, {8, 4}, {4, 4}};
+// the row-tile kernel (tile_rows_kernel): what variant 5 runs on small meshes
+constexpr int kTileRowsVariant = kNumVariants;
+// cell sizes within which the sweeps' FP64 quotients stay in the range of the exact division
+inline bool exact_mesh(double dx, double dy, bool fp64) {
+  auto fits = [](double d) { return d >= 0x1p-30 && d <= 0x1p40; };
+  return !fp64 || (fits(dx) && fits(dy));
+}
 // resident blocks per SM of the batch kernels, and of the sweeps with every source term
 template <typename T> constexpr int kBatchCap = sizeof(T) == 8 ? 4 : 6;
 template <typename T> constexpr int kExtraCap = sizeof(T) == 8 ? 3 : 4;
@@ -52,6 +59,13 @@ inline int auto_rows(long long nx, long long ny) {
   for (int rows = 32; rows > 4; rows /= 2)
     if (strip_count(nx, ny, rows) >= kFillStrips) return rows;
   return 4;
+}
+// Whether variant 5 runs the row-tile kernel on a mesh: while its blocks (12 warps; one resident per
+// SM in FP64, two in FP32) take about two rounds. Per stage on B200, row tiles against 4-row
+// strips: FP64 13 / 27 us at 100 x 100, 23 / 28 at 256 x 256, 38 / 31 at 400 x 400; FP32 11 / 17 at
+// 64 x 64, 15 / 18 at 256 x 256, 20 / 20 at 400 x 400.
+template <typename T> inline bool prefers_tile_rows(long long nx, long long ny) {
+  return strip_count(nx, ny, kTileRows) <= (sizeof(T) == 8 ? 330 : 660);
 }
 // column-sweep variants: output rows per strip on a mesh (0 for the other variants)
 inline int variant_sweep_rows(int v, long long nx, long long ny) {

@@ -27,10 +27,10 @@ void set_global_error(const std::string& msg);
 namespace {
 
 constexpr long long kMaxCells = 65536;  // 256 x 256
-// partial-sum slots of the 32 x 8 tiled stage kernel: at most 8192 CTAs for any mesh of at
-// most kMaxCells cells (reached by a 1-cell-wide strip), times svk::kParts
+// partial-sum slots of the row-tile kernel (28 x 8 cells a block): at most 8192 blocks for any mesh
+// of at most kMaxCells cells (reached by a 1-cell-wide strip), times svk::kParts
 constexpr long long kMaxBlocks = 8192;
-constexpr int kVariant = 1;  // tiled stage kernel, 32 x 8 cells per CTA
+constexpr int kVariant = svk::kTileRowsVariant;
 constexpr size_t kFieldBytes = size_t(kMaxCells) * sizeof(double);
 constexpr size_t kYOffset = 0;                           // Y[2][3]: stage inputs
 constexpr size_t kZxOffset = kYOffset + 6 * kFieldBytes;  // bed slopes dz/dx, dz/dy
@@ -137,7 +137,7 @@ extern "C" int sv_timestep_noalloc(const sv_mesh_desc* mesh, const sv_params* pa
     return fail(SV_E_ARG, "only uniform rain (or none) is available without allocation");
   if (forcing->head_kind != SV_HEAD_NONE && forcing->head_kind != SV_HEAD_EDGES)
     return fail(SV_E_ARG, "only edge-strip head boundaries (or none) are available without allocation");
-  const long long nblk = svk::variant_partials(kVariant, (long long)mesh->nx, (long long)mesh->ny);
+  const long long nblk = svk::strip_count((long long)mesh->nx, (long long)mesh->ny, svk::kTileRows);
   if (nblk > kMaxBlocks) return fail(SV_E_LIMIT, "mesh needs more partial-sum slots than the working array holds");
   const size_t field_bytes = size_t(mesh->nx * mesh->ny) * sizeof(double);
   const double* outs[3] = {h_out, u_out, v_out};
@@ -177,6 +177,8 @@ extern "C" int sv_timestep_noalloc(const sv_mesh_desc* mesh, const sv_params* pa
   P.nx = int(mesh->nx); P.ny = int(mesh->ny);
   P.dx = dx; P.dy = dy; P.L = params->step_duration;
   P.cell_area = dx * dy;
+  P.mc.set(dx, dy);
+  P.exact = svk::exact_mesh(dx, dy, true);
   // U_[0] is read from the inputs (cur = 0); the accumulator and U_[N] go to the outputs
   P.S[0][0] = const_cast<double*>(h); P.S[0][1] = const_cast<double*>(u); P.S[0][2] = const_cast<double*>(v);
   P.S[1][0] = h_out; P.S[1][1] = u_out; P.S[1][2] = v_out;

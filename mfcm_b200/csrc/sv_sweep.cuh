@@ -120,6 +120,25 @@ template <typename T> struct SweepAcc {
   T xmax = T(0), xmin = T(1.0 / 0.0);
 };
 
+// Constants of a stage at the solver's present timestep.
+template <typename T> struct StepConst {
+  double dt_d, tsub_d, L, rL;
+  T dt, rdt, cA, cB, rq0, rq1, rain_w, rain_q;
+  T ck[4];  // general tableaux: the coefficients of k_0 .. k_st
+  __device__ __forceinline__ void set(const StageParams<T>& P, int st) volatile {
+    const double d = P.ctl->dt, tsub = P.ctl->t_local + P.c[st] * d, w = (tsub + 0.5 * d) / P.L;
+    dt_d = d; tsub_d = tsub; L = P.L; rL = 1.0 / P.L;
+    dt = T(d); rdt = T(1.0 / d);
+    cA = T(P.a[st][st] * d); cB = T(P.b[st] * d);
+    for (int j = 0; j <= st; ++j) ck[j] = T((st == P.nstages - 1 ? P.b[j] : P.a[st][j]) * d);
+    const double q0 = P.fc->rq0, q1 = P.fc->rq1;
+    rq0 = T(q0); rq1 = T(q1);
+    // FP32 rain: the mean of the step's linear rain over the stage's timestep, as a weight of its
+    // two ends formed in FP64
+    rain_w = T(w); rain_q = T(q0 + (q1 - q0) * w);
+  }
+};
+
 // What a sweeping warp keeps in shared memory besides its row ring: addresses and constants that
 // every row uses once or twice. In registers they would cost the sweep a third of its resident
 // warps (FP32: 50 registers of 128) or be spilled.
@@ -129,9 +148,7 @@ template <typename T> struct alignas(16) SweepShared {  // rings of 16-byte copi
   const T* src[RR::kWSlots + RR::kCSlots][32];  // each lane's chunks: address in row 0
   double vol[32];                               // last stage: per-lane volume and CFL extremes
   T xmax[32], xmin[32];
-  double dt_d, tsub_d, L, rL;
-  T dt, rdt, cA, cB, rq0, rq1, rain_w, rain_q;
-  T ck[4];                                      // general tableaux: the coefficients of k_0 .. k_st
+  StepConst<T> step;
 };
 static_assert(sizeof(SweepShared<float>) % 16 == 0 && sizeof(SweepShared<double>) % 16 == 0 &&
                   offsetof(SweepShared<float>, ring) == 0 && offsetof(SweepShared<double>, ring) == 0,
@@ -372,6 +389,28 @@ __device__ __forceinline__ double flip_sign(double x, double s) {
   return __hiloint2double(__double2hiint(x) ^ (__double2hiint(s) & 0x80000000), __double2loint(x));
 }
 
+// Quotients by the mesh spacing. FP32, or dx and dy powers of two: differences are kept undivided
+// (diff_x, diff_y) and scaled where they are used; else exact divisions (div_exact).
+template <typename T, bool P2> struct MeshOps {
+  static constexpr bool SCALED = sizeof(T) == 4 || P2;
+  const MeshConst<T>& mc;
+  __device__ __forceinline__ T diff_x(T x) const { if constexpr (SCALED) return x; else return div_exact(x, mc.dx, mc.rdx); }
+  __device__ __forceinline__ T diff_y(T x) const { if constexpr (SCALED) return x; else return div_exact(x, mc.dy, mc.rdy); }
+  __device__ __forceinline__ T over_2dx(T x) const {
+    if constexpr (SCALED) return x * mc.kx; else return div_exact(x, mc.dx2, mc.kx);
+  }
+  __device__ __forceinline__ T over_2dy(T x) const {
+    if constexpr (SCALED) return x * mc.ky; else return div_exact(x, mc.dy2, mc.ky);
+  }
+  __device__ __forceinline__ T over_dx(T x) const { if constexpr (SCALED) return x * mc.rdx; else return diff_x(x); }
+  __device__ __forceinline__ T over_dy(T x) const { if constexpr (SCALED) return x * mc.rdy; else return diff_y(x); }
+  // bed at a face side: z + 0.5 d * slope, the product rounded by itself unless it is exact
+  __device__ __forceinline__ static T zside(T hd, T s, T z) { if constexpr (SCALED) return sfma_(hd, s, z); else return z + hd * s; }
+  // half jump across half a cell (0.5 d * slope) from half a slope
+  __device__ __forceinline__ T jump_x(T hs) const { if constexpr (SCALED) return hs; else return mc.dx * hs; }
+  __device__ __forceinline__ T jump_y(T hs) const { if constexpr (SCALED) return hs; else return mc.dy * hs; }
+};
+
 // Doubled fluxes of a face: depth, normal and tangential momentum, bed step.
 template <typename T> struct FaceG { T h, n, t, z; };
 
@@ -434,6 +473,235 @@ __device__ __forceinline__ void friction(float h, float u, float v, float n, flo
   dv = mad_(-rate, v, dv);
 }
 
+// One cell of a stage after its four face fluxes are known (W, E: faces along x; GS, GN: along y;
+// doubled): its rates, then the Runge-Kutta combination (RungeKutta.hpp:377-388) and, on the last
+// stage, the CFL quantity and depth passed to totals(). jhx, jhy: half jumps of h (y: towards
+// row + 1); shx, shy: its slopes where they are not kept undivided. medge: the cell may lie on the
+// mesh edge. cells: the cell's values of U_[0], the running sum and the per-cell fields.
+template <typename T, bool P2, bool EXTRA, bool COH, typename Cells, typename Totals>
+__device__ __forceinline__ void lean_cell(const StageParams<T>& P, int st, int cur, const volatile StepConst<T>& k, int rk,
+                                          bool rain_any, long long g, int gx, int r, const RowV<T>& R, T jhx, T jhy,
+                                          T shx, T shy, const FaceG<T>& W, const FaceG<T>& E, const FaceG<T>& GS,
+                                          const FaceG<T>& GN, bool medge, const EddyIn<T>& ed, const Cells& cells,
+                                          SweepAcc<T>& acc, const Totals& totals) {
+  constexpr bool F32 = sizeof(T) == 4;
+  constexpr bool SCALED = F32 || P2;
+  const int nx = P.nx, ny = P.ny;
+  const bool first = st == 0, last = st == P.nstages - 1;
+  const auto& mc = P.mc;
+  const MeshOps<T, P2> mo{mc};
+  const T h = R.h, u = R.u, v = R.v;
+  // flux divergence, depth slope, bed step (TemporalDerivativeKernel.cpp:53-98)
+  T dh, du, dv;
+  if constexpr (F32) {
+    // each difference is scaled before the next is added: beside a wall the momentum and
+    // bed-step fluxes of one face are large and cancel, and the order decides what is left
+    // of their rounding
+    dh = mad_(GS.h - GN.h, mc.ky, (W.h - E.h) * mc.kx);
+    du = mad_(GS.t - GN.t, mc.ky, (W.n - E.n) * mc.kx);
+    dv = mad_(GS.n - GN.n, mc.ky, (W.t - E.t) * mc.kx);
+    du = mad_(-mc.gx, jhx, du);
+    dv = mad_(mc.gy, jhy, dv);
+    du = mad_(W.z - E.z, mc.kx, du);
+    dv = mad_(GS.z - GN.z, mc.ky, dv);
+  } else if constexpr (SCALED) {
+    const T g4 = T(4) * T(kG);
+    const T ry = mc.ry;
+    dh = sfma_(GS.h - GN.h, ry, W.h - E.h) * mc.kx;
+    du = sfma_(GS.t - GN.t, ry, W.n - E.n);
+    dv = sfma_(GS.n - GN.n, ry, W.t - E.t);
+    du = mad_(-g4, jhx, du);
+    dv = sfma_(g4 * jhy, ry, dv);
+    du = (du + (W.z - E.z)) * mc.kx;
+    dv = sfma_(GS.z - GN.z, ry, dv) * mc.kx;
+  } else {
+    dh = mo.over_2dx(W.h - E.h) + mo.over_2dy(GS.h - GN.h);
+    du = mo.over_2dx(W.n - E.n) + mo.over_2dy(GS.t - GN.t);
+    dv = mo.over_2dx(W.t - E.t) + mo.over_2dy(GS.n - GN.n);
+    du = du + shx * T(-kG);
+    dv = dv + shy * T(-kG);
+    du = du + mo.over_2dx(W.z - E.z);
+    dv = dv + mo.over_2dy(GS.z - GN.z);
+  }
+  // limited bed slope
+  {
+    const T lx = mo.over_dx(h), ly = mo.over_dy(h);
+    const T zx = R.zx, zy = R.zy;
+    du = mad_(T(-kG), (sfabs(zx) > lx && zx != T(0)) ? flip_sign(lx, zx) : zx, du);
+    dv = mad_(T(-kG), (sfabs(zy) > ly && zy != T(0)) ? flip_sign(ly, zy) : zy, dv);
+  }
+  auto roughness = [&]() {
+    if (!(P.manning && h > T(1e-6))) return;
+    const T ns = P.man_p[0] ? cells.ns(g) : P.man_s[0];
+    const T nd = P.man_p[1] ? (P.man_p[1] == P.man_p[0] ? ns : cells.nd(g)) : P.man_s[1];
+    T n = ns;
+    if (ns != nd)
+      n = manning_n<T>(h, ns, nd, P.man_p[2] ? ld(P.man_p[2], g) : P.man_s[2],
+                       P.man_p[3] ? ld(P.man_p[3], g) : P.man_s[3]);
+    friction(h, u, v, n, k.dt, k.rdt, du, dv);
+  };
+  if constexpr (!EXTRA) {
+    roughness();
+  } else {  // the momentum terms in configuration order, then infiltration
+    CellCtx<T> c;
+    c.dt = k.dt;
+    c.divdt = div_by<T>(k.dt, k.rdt);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int term = (P.term_order >> (2 * i)) & 3;
+      if (term == 1) roughness();
+      if (term == 2 && P.efx)
+        energy_loss_apply<T>(h, u, v, cells.ex(g), cells.ey(g), c, du, dv);
+      if (term == 3 && P.eddy) {
+        const T mu = P.eddy == 2 ? smagorinsky_mu<T>(P.eddy_c, P.eddy_s, T(P.cell_area), ed)
+                                 : (P.eddy_mup ? ld(P.eddy_mup, g) : P.eddy_mu);
+        T fu = T(0), fv = T(0);
+        if (eddy_term<T>(h, u, v, mu, ed, c, fu, fv)) { du = du + fu; dv = dv + fv; }
+      }
+    }
+    if (P.irate) {  // infiltration (InfiltrationSourceTerm.cpp:43-62), capacity consumed in place
+      const T cap = cells.ic(g);
+      const T d = infiltration_depth<T>(h, cells.ir(g), cap, c);
+      dh = dh - c.divdt(d);
+      P.icap[g] = cap - d;
+    }
+  }
+  if (medge) {
+    double w = 0.0;
+    if (gx == 0) w += double(mo.over_2dx(W.h));
+    if (gx == nx - 1) w -= double(mo.over_2dx(E.h));
+    if (r == 0) w += double(mo.over_2dy(GS.h));
+    if (r == ny - 1) w -= double(mo.over_2dy(GN.h));
+    acc.walls += w;
+  }
+  auto do_rain = [&]() {
+    if (rk == 0) return;
+    T rate;
+    bool applied;
+    const T dt = k.dt;
+    if constexpr (F32) {
+      if (rk == 2) {
+        const T q0 = cells.r0(P.q0p, g), q1 = cells.r1(P.q1p, g);
+        applied = q0 != T(0) || q1 != T(0);
+        rate = mad_(q1 - q0, k.rain_w, q0);
+      } else {
+        const T pp = rk == 3 ? cells.r0(P.pat, g) : T(1);
+        applied = rain_any && pp != T(0);
+        rate = pp * k.rain_q;
+      }
+      const T dhr = rate * dt;
+      if (P.rain_mode == 0 ? (h - dhr <= T(0)) : (h + dhr <= T(0))) rate = -h * k.rdt;
+    } else {
+      T q0 = k.rq0, q1 = k.rq1;
+      if (rk == 2) { q0 = cells.r0(P.q0p, g); q1 = cells.r1(P.q1p, g); }
+      else if (rk == 3) { const T pp = cells.r0(P.pat, g); q0 = pp * q0; q1 = pp * q1; }
+      applied = q0 != T(0) || q1 != T(0);
+      const T dq = DivD{k.L, k.rL}(q1 - q0);
+      const T qn = q0 + T(k.tsub_d) * dq;
+      rate = T(0.5) * (qn + (qn + dt * dq));
+      const T dhr = rate * dt;
+      if (P.rain_mode == 0 ? (h - dhr <= T(0)) : (h + dhr <= T(0))) rate = -div_slow(h, dt);
+    }
+    if (applied) { dh = dh + rate; acc.rain += double(rate); }
+  };
+  auto do_head = [&]() {
+    if (!EXTRA && !medge) return;
+    const DevForcing& f = *P.fc;
+    const int hk = f.head_kind;
+    T h0, h1;
+    if (medge && (hk == 1 || hk == 3)) {
+      const bool sel = ((f.head_edges & 1u) && gx == 0) || ((f.head_edges & 2u) && gx == nx - 1) ||
+                       ((f.head_edges & 4u) && r == 0) || ((f.head_edges & 8u) && r == ny - 1);
+      if (!sel) return;
+      h0 = T(f.hh0); h1 = T(f.hh1);
+    } else if (EXTRA && (hk == 2 || hk == 4)) {
+      h0 = ld(P.hb0p, g); h1 = ld(P.hb1p, g);
+    } else {
+      return;
+    }
+    if (hk >= 3) {  // water levels: less the bed, in FP64 with tile datums
+      if (P.zdat) {
+        const double zb = P.zdat[datum_tile(gx, r, P.dtiles_x)] + double(R.z);
+        h0 = T(double(h0) - zb); h1 = T(double(h1) - zb);
+      } else {
+        h0 = h0 - R.z; h1 = h1 - R.z;
+      }
+    }
+    if (!(h0 == h0 && h1 == h1)) return;  // NaN = not selected
+    CellCtx<T> c;
+    c.divL = mkdiv<T>(P.L);
+    c.dt = k.dt; c.tsub_d = k.tsub_d;
+    const T before = dh;
+    const T d = head_target<T>(h0, h1, c) - h;
+    if constexpr (F32) dh = d * k.rdt;
+    else dh = div_slow(d, k.dt);
+    acc.removed += double(before) - double(dh);
+  };
+  if (P.head_first) { do_head(); do_rain(); }
+  else { do_rain(); do_head(); }
+  // Runge-Kutta combination (RungeKutta.hpp:377-388), running accumulator; see finish_cell
+  const T kk[3] = {dh, du, dv}, U[3] = {h, u, v};
+  const T cA = k.cA, cB = k.cB;
+  T out[3];
+  bool running_sum = true;
+  if constexpr (EXTRA) {
+  if (!(P.mode & M_ACC)) {  // general tableau: U0 + k_0 c_0 + k_1 c_1 + ..., stored k's
+    running_sum = false;
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      T y = first ? U[f] : cells.u0(f);
+      for (int j = 0; j < st; ++j) {
+        const T kj = cells.k(j, f, g);
+        y = mad_(kj, T(k.ck[j]), y);
+      }
+      y = mad_(kk[f], T(k.ck[st]), y);
+      out[f] = y;
+      if (last) {
+        P.S[cur ^ 1][f][g] = y;
+      } else {
+        P.K[st][f][g] = kk[f];
+        P.out(st, f)[g] = y;
+      }
+    }
+  }
+  }
+  if (running_sum)
+#pragma unroll
+  for (int f = 0; f < 3; ++f) {
+        const T u0 = first ? U[f] : cells.u0(f);
+    const T a0 = first ? T(0) : cells.a0(f);
+    T* A = P.S[cur ^ 1][f];
+    if constexpr (F32) {  // the accumulator holds the increment
+      const T d = mad_(kk[f], cB, a0);
+      if (!last) {
+        P.out(st, f)[g] = mad_(kk[f], cA, u0);
+        A[g] = d;
+      } else if (f == 0) {  // U_N.h = U0.h + d with the carried compensation (Neumaier)
+        const T y = d + cells.hc(g);
+        const T t = u0 + y;
+        P.hc[cur ^ 1][g] = (sfabs(u0) >= sfabs(y)) ? (u0 - t) + y : (y - t) + u0;
+        out[0] = t;
+        A[g] = t;
+      } else {
+        out[f] = u0 + d;
+        A[g] = out[f];
+      }
+    } else {
+      const T a = first ? u0 : a0;
+      if (!last) P.out(st, f)[g] = mad_(kk[f], cA, u0);
+      out[f] = mad_(kk[f], cB, a);
+      A[g] = out[f];
+    }
+  }
+  if (last) {  // CFL quantity and volume of U_[N] (State.cpp:204-228)
+    const T cc = ssqrt(T(kG) * sfmax(out[0], T(0)));
+    T xx;
+    if constexpr (SCALED) xx = mad_(sfabs(out[1]) + cc, mc.rdx, (sfabs(out[2]) + cc) * mc.rdy);
+    else xx = DivD{mc.dx, mc.rdx}(sfabs(out[1]) + cc) + DivD{mc.dy, mc.rdy}(sfabs(out[2]) + cc);
+    totals(xx, out[0]);
+  }
+}
+
 // the last stage's sums of a strip's rows from shared memory
 template <typename T> __device__ __forceinline__ void sweep_totals(SweepShared<T>& sm, SweepAcc<T>& acc) {
   const int lane = threadIdx.x;
@@ -441,6 +709,31 @@ template <typename T> __device__ __forceinline__ void sweep_totals(SweepShared<T
   acc.xmax = nmax(acc.xmax, sm.xmax[lane]);
   acc.xmin = nmin(acc.xmin, sm.xmin[lane]);
 }
+
+// A cell's values from its row in the ring; o_*: place of a field in the row, or -1 (read directly).
+template <typename T, bool COH> struct RingCells {
+  const StageParams<T>& P;
+  int cur;
+  const unsigned char* cell;
+  int o_ns, o_nd, o_r0, o_r1, o_hc, o_ex, o_ey, o_ir, o_ic;
+  __device__ __forceinline__ T at(int o) const { return *reinterpret_cast<const T*>(cell + o); }
+  __device__ __forceinline__ T field(int o, const T* p, long long g) const { return o >= 0 ? at(o) : ld(p, g); }
+  __device__ __forceinline__ T u0(int f) const { return at(f * RowRing<T>::kFieldBytes); }
+  __device__ __forceinline__ T a0(int f) const { return at((3 + f) * RowRing<T>::kFieldBytes); }
+  __device__ __forceinline__ T k(int j, int f, long long g) const {
+    const int n = 3 + 3 * j + f;
+    return n < RowRing<T>::kCellFields ? at(n * RowRing<T>::kFieldBytes) : ldst<COH>(P.K[j][f], g);
+  }
+  __device__ __forceinline__ T ns(long long g) const { return field(o_ns, P.man_p[0], g); }
+  __device__ __forceinline__ T nd(long long g) const { return field(o_nd, P.man_p[1], g); }
+  __device__ __forceinline__ T r0(const T* p, long long g) const { return field(o_r0, p, g); }
+  __device__ __forceinline__ T r1(const T* p, long long g) const { return field(o_r1, p, g); }
+  __device__ __forceinline__ T hc(long long g) const { return o_hc >= 0 ? at(o_hc) : ldst<COH>(P.hc[cur], g); }
+  __device__ __forceinline__ T ex(long long g) const { return field(o_ex, P.efx, g); }
+  __device__ __forceinline__ T ey(long long g) const { return field(o_ey, P.efy, g); }
+  __device__ __forceinline__ T ir(long long g) const { return field(o_ir, P.irate, g); }
+  __device__ __forceinline__ T ic(long long g) const { return o_ic >= 0 ? at(o_ic) : P.icap[g]; }
+};
 
 // Output rows y0 .. y1-1 (inside the mesh) of the strip of column `tile_x`. Returns y1, or the
 // first row not computed because the state left the range this function is exact for.
@@ -461,41 +754,18 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
   const bool xedge = EDGE && (gx0 < 0 || gx0 + 31 >= nx - 1);  // the strip holds the mesh's first or last column
 
   const int cur = uniform(ctl->cur);
-  const double dt_d = ctl->dt;
   const bool first = st == 0, last = st == P.nstages - 1;
   const T *Yh = P.in(st, cur, 0), *Yu = P.in(st, cur, 1), *Yv = P.in(st, cur, 2);
 
-  // mesh constants (operands in the parameter bank: no registers)
+  const MeshOps<T, P2> mo{P.mc};
   const auto& mc = P.mc;
-  const auto qx = [&](T x) { if constexpr (SCALED) return x; else return div_exact(x, mc.dx, mc.rdx); };
-  const auto qy = [&](T x) { if constexpr (SCALED) return x; else return div_exact(x, mc.dy, mc.rdy); };
-  // x / (2 d) (scaled mode: the quotient itself, used off the common path)
-  const auto dvx = [&](T x) { if constexpr (SCALED) return x * mc.kx; else return div_exact(x, mc.dx2, mc.kx); };
-  const auto dvy = [&](T x) { if constexpr (SCALED) return x * mc.ky; else return div_exact(x, mc.dy2, mc.ky); };
-  const auto over_dx = [&](T x) { if constexpr (SCALED) return x * mc.rdx; else return qx(x); };
-  const auto over_dy = [&](T x) { if constexpr (SCALED) return x * mc.rdy; else return qy(x); };
-  // bed at a face side: z + 0.5 d * slope, the product rounded by itself unless it is exact
-  const auto zside = [](T hd, T s, T z) { if constexpr (SCALED) return sfma_(hd, s, z); else return z + hd * s; };
 
-  // step constants and result addresses, in shared memory
+  // step constants, in shared memory
   volatile SweepShared<T>& vs = sm;
   const int rk = uniform(P.fc->rain_kind);
   const bool rain_any = uniform(P.fc->rq0 != 0.0 || P.fc->rq1 != 0.0);
   __syncwarp();  // a strip swept before this one is done with them and with its rows
-  if (lane == 0) {
-    const double tsub = ctl->t_local + P.c[st] * dt_d, w = (tsub + 0.5 * dt_d) / P.L;
-    vs.dt_d = dt_d; vs.tsub_d = tsub; vs.L = P.L; vs.rL = 1.0 / P.L;
-    vs.dt = T(dt_d);
-    vs.rdt = T(1.0 / dt_d);
-    vs.cA = T(P.a[st][st] * dt_d); vs.cB = T(P.b[st] * dt_d);
-    if constexpr (EXTRA)
-      for (int j = 0; j <= st; ++j) vs.ck[j] = T((last ? P.b[j] : P.a[st][j]) * dt_d);
-    const double q0 = P.fc->rq0, q1 = P.fc->rq1;
-    vs.rq0 = T(q0); vs.rq1 = T(q1);
-    // FP32 rain: the mean of the step's linear rain over the stage's timestep, as a weight of its
-    // two ends formed in FP64
-    vs.rain_w = T(w); vs.rain_q = T(q0 + (q1 - q0) * w);
-  }
+  if (lane == 0) vs.step.set(P, st);
   vs.vol[lane] = 0.0;
   vs.xmax[lane] = T(0);
   vs.xmin[lane] = T(1.0 / 0.0);
@@ -603,7 +873,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
     }
     if constexpr (!SCALED) {
       fyA[0] = fyB[0]; fyA[1] = fyB[1]; fyA[2] = fyB[2];
-      fyB[0] = qy(Rp.h - R0.h); fyB[1] = qy(Rp.u - R0.u); fyB[2] = qy(Rp.v - R0.v);
+      fyB[0] = mo.diff_y(Rp.h - R0.h); fyB[1] = mo.diff_y(Rp.u - R0.u); fyB[2] = mo.diff_y(Rp.v - R0.v);
     } else {
       fyA[0] = R0.h - Rm.h; fyA[1] = R0.u - Rm.u; fyA[2] = R0.v - Rm.v;
       fyB[0] = Rp.h - R0.h; fyB[1] = Rp.u - R0.u; fyB[2] = Rp.v - R0.v;
@@ -614,7 +884,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
       const int row = k - 1;
       const bool yedge = EDGE && (row <= 0 || row >= ny - 1);
       auto yslope = [&](T a, T b, T lo, T hi, T& j, T& s) {
-        T hs = half_slope(a, b, F32 ? a + b : qy(hi - lo));
+        T hs = half_slope(a, b, F32 ? a + b : mo.diff_y(hi - lo));
         if (yedge) {  // one-sided: the slope is the present quotient
           if (row >= ny - 1) hs = T(0.5) * a;
           if (row <= 0) hs = ny > 1 ? T(0.5) * b : T(0);
@@ -632,10 +902,10 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
       yslope(fyA[2], fyB[2], Rm.v, Rp.v, J0.vy, S0.vy);
       auto xslope = [&](T x, T& j, T& s) {
         const T e = dn1(x);
-        const T b = qx(e - x), a = up1(b);
+        const T b = mo.diff_x(e - x), a = up1(b);
         T cc;
         if constexpr (F32) cc = a + b;
-        else cc = qx(e - up1(x));
+        else cc = mo.diff_x(e - up1(x));
         T hs = half_slope(a, b, cc);
         if (xedge) {
           if (gx >= nx - 1) hs = T(0.5) * a;
@@ -664,13 +934,13 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
           zhi = T(double(zhi) + (P.zdat[tb] - P.zdat[tb - P.dtiles_x]));
         }
       }
-      Side<T> m{zside(mc.hdy, Rm.zy, Rm.z), Rm.h - Jm.hy, Rm.v - Jm.vy, Rm.u - Jm.uy};
-      Side<T> p{zside(-mc.hdy, R0.zy, zhi), R0.h + J0.hy, R0.v + J0.vy, R0.u + J0.uy};
+      Side<T> m{mo.zside(mc.hdy, Rm.zy, Rm.z), Rm.h - Jm.hy, Rm.v - Jm.vy, Rm.u - Jm.uy};
+      Side<T> p{mo.zside(-mc.hdy, R0.zy, zhi), R0.h + J0.hy, R0.v + J0.vy, R0.u + J0.uy};
       if (EDGE && (fy <= 0 || fy >= ny)) {  // walls at the mesh edge, FluxKernel.cpp:111-157
         if (fy == 0) m = {R0.z + R0.h * T(2), T(0), T(0), R0.u - J0.uy};
         if (fy == ny) p = {Rm.z + Rm.h * T(2), T(0), T(0), Rm.u + Jm.uy};
       }
-      GN = face_pair(m, p, dvy);
+      GN = face_pair(m, p, [&](T x) { return mo.over_2dy(x); });
     }
     // output row k-2
     if (k >= y0 + 2) {
@@ -695,24 +965,24 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
           }
         }
       }
-      Side<T> p{zside(-mc.hdx, Rm.zx, zw), Rm.h - Jm.hx, Rm.u - Jm.ux, Rm.v - Jm.vx};
+      Side<T> p{mo.zside(-mc.hdx, Rm.zx, zw), Rm.h - Jm.hx, Rm.u - Jm.ux, Rm.v - Jm.vx};
       const T eut = Rm.v + Jm.vx;
-      Side<T> m{up1(zside(mc.hdx, Rm.zx, Rm.z)), up1(Rm.h + Jm.hx), up1(Rm.u + Jm.ux), up1(eut)};
+      Side<T> m{up1(mo.zside(mc.hdx, Rm.zx, Rm.z)), up1(Rm.h + Jm.hx), up1(Rm.u + Jm.ux), up1(eut)};
       if (xedge) {
         const T wall = Rm.z + Rm.h * T(2);
         const T wl = up1(wall), utl = up1(p.ut);
         if (gx == 0) m = {wall, T(0), T(0), eut};
         if (gx == nx) p = {wl, T(0), T(0), utl};
       }
-      const FaceG<T> W = face_pair(m, p, dvx);
+      const FaceG<T> W = face_pair(m, p, [&](T x) { return mo.over_2dx(x); });
       const FaceG<T> E{dn1(W.h), dn1(W.n), dn1(W.t), dn1(W.z)};
       EddyIn<T> ed{};
       if constexpr (EXTRA) {
         if (P.eddy) {  // second derivatives of row r: x by shuffles, y from rows r+1, r, r-1
           ed.ux = Sm.ux; ed.uy = Sm.uy; ed.vx = Sm.vx; ed.vy = Sm.vy;
           auto along_x = [&](T x) {
-            const T e = dn1(x), b = over_dx(e - x), a = up1(b);
-            T hs = half_slope(a, b, over_dx(e - up1(x)));
+            const T e = dn1(x), b = mo.over_dx(e - x), a = up1(b);
+            T hs = half_slope(a, b, mo.over_dx(e - up1(x)));
             if (xedge) {
               if (gx >= nx - 1) hs = T(0.5) * a;
               if (gx <= 0) hs = nx > 1 ? T(0.5) * b : T(0);
@@ -720,8 +990,8 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
             return T(2) * hs;
           };
           auto along_y = [&](T south, T x, T north) {  // the reference's Y axis: north on the left
-            const T a = over_dy(x - north), b = over_dy(south - x);
-            T hs = half_slope(a, b, over_dy(south - north));
+            const T a = mo.over_dy(x - north), b = mo.over_dy(south - x);
+            T hs = half_slope(a, b, mo.over_dy(south - north));
             if (EDGE && r >= ny - 1) hs = T(0.5) * b;
             if (EDGE && r <= 0) hs = ny > 1 ? T(0.5) * a : T(0);
             return T(2) * hs;
@@ -734,230 +1004,41 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
       }
       if (out_lane) {
         const long long g = (long long)r * nx + gx;
-        const T h = Rm.h, u = Rm.u, v = Rm.v;
         // the per-cell fields of this row in the ring
-        const unsigned char* cell = stage + RR::kWSlots * 512 +
-                                    (gxc - c0 + ((int(unsigned(r) * unsigned(nx)) + c0) & (RR::kChunk - 1))) * int(sizeof(T));
-        auto field = [&](int o, const T* p) { return o >= 0 ? *reinterpret_cast<const T*>(cell + o) : ld(p, g); };
-        {
-          // flux divergence, depth slope, bed step (TemporalDerivativeKernel.cpp:53-98)
-          T dh, du, dv;
-          if constexpr (F32) {
-            // each difference is scaled before the next is added: beside a wall the momentum and
-            // bed-step fluxes of one face are large and cancel, and the order decides what is left
-            // of their rounding
-            dh = mad_(GS.h - GN.h, mc.ky, (W.h - E.h) * mc.kx);
-            du = mad_(GS.t - GN.t, mc.ky, (W.n - E.n) * mc.kx);
-            dv = mad_(GS.n - GN.n, mc.ky, (W.t - E.t) * mc.kx);
-            du = mad_(-mc.gx, Jm.hx, du);
-            dv = mad_(mc.gy, Jm.hy, dv);
-            du = mad_(W.z - E.z, mc.kx, du);
-            dv = mad_(GS.z - GN.z, mc.ky, dv);
-          } else if constexpr (SCALED) {
-            const T g4 = T(4) * T(kG);
-            const T ry = mc.ry;
-            dh = sfma_(GS.h - GN.h, ry, W.h - E.h) * mc.kx;
-            du = sfma_(GS.t - GN.t, ry, W.n - E.n);
-            dv = sfma_(GS.n - GN.n, ry, W.t - E.t);
-            du = mad_(-g4, Jm.hx, du);
-            dv = sfma_(g4 * Jm.hy, ry, dv);
-            du = (du + (W.z - E.z)) * mc.kx;
-            dv = sfma_(GS.z - GN.z, ry, dv) * mc.kx;
-          } else {
-            dh = dvx(W.h - E.h) + dvy(GS.h - GN.h);
-            du = dvx(W.n - E.n) + dvy(GS.t - GN.t);
-            dv = dvx(W.t - E.t) + dvy(GS.n - GN.n);
-            du = du + Sm.hx * T(-kG);
-            dv = dv + Sm.hy * T(-kG);
-            du = du + dvx(W.z - E.z);
-            dv = dv + dvy(GS.z - GN.z);
-          }
-          // limited bed slope
-          {
-            const T lx = over_dx(h), ly = over_dy(h);
-            const T zx = Rm.zx, zy = Rm.zy;
-            du = mad_(T(-kG), (sfabs(zx) > lx && zx != T(0)) ? flip_sign(lx, zx) : zx, du);
-            dv = mad_(T(-kG), (sfabs(zy) > ly && zy != T(0)) ? flip_sign(ly, zy) : zy, dv);
-          }
-          auto roughness = [&]() {
-            if (!(P.manning && h > T(1e-6))) return;
-            const T ns = P.man_p[0] ? field(o_ns, P.man_p[0]) : P.man_s[0];
-            const T nd = P.man_p[1] ? (P.man_p[1] == P.man_p[0] ? ns : field(o_nd, P.man_p[1])) : P.man_s[1];
-            T n = ns;
-            if (ns != nd)
-              n = manning_n<T>(h, ns, nd, P.man_p[2] ? ld(P.man_p[2], g) : P.man_s[2],
-                               P.man_p[3] ? ld(P.man_p[3], g) : P.man_s[3]);
-            friction(h, u, v, n, vs.dt, vs.rdt, du, dv);
-          };
-          if constexpr (!EXTRA) {
-            roughness();
-          } else {  // the momentum terms in configuration order, then infiltration
-            CellCtx<T> c;
-            c.dt = vs.dt;
-            c.divdt = div_by<T>(vs.dt, vs.rdt);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-              const int term = (P.term_order >> (2 * i)) & 3;
-              if (term == 1) roughness();
-              if (term == 2 && P.efx)
-                energy_loss_apply<T>(h, u, v, field(o_ex, P.efx), field(o_ey, P.efy), c, du, dv);
-              if (term == 3 && P.eddy) {
-                const T mu = P.eddy == 2 ? smagorinsky_mu<T>(P.eddy_c, P.eddy_s, T(P.cell_area), ed)
-                                         : (P.eddy_mup ? ld(P.eddy_mup, g) : P.eddy_mu);
-                T fu = T(0), fv = T(0);
-                if (eddy_term<T>(h, u, v, mu, ed, c, fu, fv)) { du = du + fu; dv = dv + fv; }
-              }
-            }
-            if (P.irate) {  // infiltration (InfiltrationSourceTerm.cpp:43-62), capacity consumed in place
-              const T cap = o_ic >= 0 ? *reinterpret_cast<const T*>(cell + o_ic) : P.icap[g];
-              const T d = infiltration_depth<T>(h, field(o_ir, P.irate), cap, c);
-              dh = dh - c.divdt(d);
-              P.icap[g] = cap - d;
-            }
-          }
-          const bool medge = EDGE && (xedge || r == 0 || r == ny - 1);
-          if (medge) {
-            double w = 0.0;
-            if (gx == 0) w += double(dvx(W.h));
-            if (gx == nx - 1) w -= double(dvx(E.h));
-            if (r == 0) w += double(dvy(GS.h));
-            if (r == ny - 1) w -= double(dvy(GN.h));
-            acc.walls += w;
-          }
-          auto do_rain = [&]() {
-            if (rk == 0) return;
-            T rate;
-            bool applied;
-            const T dt = vs.dt;
-            if constexpr (F32) {
-              if (rk == 2) {
-                const T q0 = field(o_r0, P.q0p), q1 = field(o_r1, P.q1p);
-                applied = q0 != T(0) || q1 != T(0);
-                rate = mad_(q1 - q0, vs.rain_w, q0);
-              } else {
-                const T pp = rk == 3 ? field(o_r0, P.pat) : T(1);
-                applied = rain_any && pp != T(0);
-                rate = pp * vs.rain_q;
-              }
-              const T dhr = rate * dt;
-              if (P.rain_mode == 0 ? (h - dhr <= T(0)) : (h + dhr <= T(0))) rate = -h * vs.rdt;
-            } else {
-              T q0 = vs.rq0, q1 = vs.rq1;
-              if (rk == 2) { q0 = field(o_r0, P.q0p); q1 = field(o_r1, P.q1p); }
-              else if (rk == 3) { const T pp = field(o_r0, P.pat); q0 = pp * q0; q1 = pp * q1; }
-              applied = q0 != T(0) || q1 != T(0);
-              const T dq = DivD{vs.L, vs.rL}(q1 - q0);
-              const T qn = q0 + T(vs.tsub_d) * dq;
-              rate = T(0.5) * (qn + (qn + dt * dq));
-              const T dhr = rate * dt;
-              if (P.rain_mode == 0 ? (h - dhr <= T(0)) : (h + dhr <= T(0))) rate = -div_slow(h, dt);
-            }
-            if (applied) { dh = dh + rate; acc.rain += double(rate); }
-          };
-          auto do_head = [&]() {
-            if (!EXTRA && !medge) return;
-            const DevForcing& f = *P.fc;
-            const int hk = f.head_kind;
-            T h0, h1;
-            if (medge && (hk == 1 || hk == 3)) {
-              const bool sel = ((f.head_edges & 1u) && gx == 0) || ((f.head_edges & 2u) && gx == nx - 1) ||
-                               ((f.head_edges & 4u) && r == 0) || ((f.head_edges & 8u) && r == ny - 1);
-              if (!sel) return;
-              h0 = T(f.hh0); h1 = T(f.hh1);
-            } else if (EXTRA && (hk == 2 || hk == 4)) {
-              h0 = ld(P.hb0p, g); h1 = ld(P.hb1p, g);
-            } else {
-              return;
-            }
-            if (hk >= 3) {  // water levels: less the bed, in FP64 with tile datums
-              if (P.zdat) {
-                const double zb = P.zdat[datum_tile(gx, r, P.dtiles_x)] + double(Rm.z);
-                h0 = T(double(h0) - zb); h1 = T(double(h1) - zb);
-              } else {
-                h0 = h0 - Rm.z; h1 = h1 - Rm.z;
-              }
-            }
-            if (!(h0 == h0 && h1 == h1)) return;  // NaN = not selected
-            CellCtx<T> c;
-            c.divL = mkdiv<T>(P.L);
-            c.dt = vs.dt; c.tsub_d = vs.tsub_d;
-            const T before = dh;
-            const T d = head_target<T>(h0, h1, c) - h;
-            if constexpr (F32) dh = d * vs.rdt;
-            else dh = div_slow(d, vs.dt);
-            acc.removed += double(before) - double(dh);
-          };
-          if (P.head_first) { do_head(); do_rain(); }
-          else { do_rain(); do_head(); }
-          // Runge-Kutta combination (RungeKutta.hpp:377-388), running accumulator; see finish_cell
-          const T kk[3] = {dh, du, dv}, U[3] = {h, u, v};
-          const T cA = vs.cA, cB = vs.cB;
-          T out[3];
-          if (EXTRA && !(P.mode & M_ACC)) {  // general tableau: U0 + k_0 c_0 + k_1 c_1 + ..., stored k's
-#pragma unroll
-            for (int f = 0; f < 3; ++f) {
-              T y = first ? U[f] : *reinterpret_cast<const T*>(cell + f * RR::kFieldBytes);
-              for (int j = 0; j < st; ++j) {
-                const int o = 3 + 3 * j + f;
-                const T kj = o < RR::kCellFields ? *reinterpret_cast<const T*>(cell + o * RR::kFieldBytes)
-                                                 : ldst<COH>(P.K[j][f], g);
-                y = mad_(kj, T(vs.ck[j]), y);
-              }
-              y = mad_(kk[f], T(vs.ck[st]), y);
-              out[f] = y;
-              if (last) {
-                P.S[cur ^ 1][f][g] = y;
-              } else {
-                P.K[st][f][g] = kk[f];
-                P.out(st, f)[g] = y;
-              }
-            }
-          } else
-#pragma unroll
-          for (int f = 0; f < 3; ++f) {
-            const T* ua = reinterpret_cast<const T*>(cell + f * RR::kFieldBytes);
-            const T u0 = first ? U[f] : ua[0];
-            const T a0 = first ? T(0) : ua[3 * RR::kFieldBytes / int(sizeof(T))];
-            T* A = P.S[cur ^ 1][f];
-            if constexpr (F32) {  // the accumulator holds the increment
-              const T d = mad_(kk[f], cB, a0);
-              if (!last) {
-                P.out(st, f)[g] = mad_(kk[f], cA, u0);
-                A[g] = d;
-              } else if (f == 0) {  // U_N.h = U0.h + d with the carried compensation (Neumaier)
-                const int o = o_hc;
-                const T y = d + (o >= 0 ? *reinterpret_cast<const T*>(cell + o) : ldst<COH>(P.hc[cur], g));
-                const T t = u0 + y;
-                P.hc[cur ^ 1][g] = (sfabs(u0) >= sfabs(y)) ? (u0 - t) + y : (y - t) + u0;
-                out[0] = t;
-                A[g] = t;
-              } else {
-                out[f] = u0 + d;
-                A[g] = out[f];
-              }
-            } else {
-              const T a = first ? u0 : a0;
-              if (!last) P.out(st, f)[g] = mad_(kk[f], cA, u0);
-              out[f] = mad_(kk[f], cB, a);
-              A[g] = out[f];
-            }
-          }
-          if (last) {  // CFL quantity and volume of U_[N] (State.cpp:204-228)
-            const T cc = ssqrt(T(kG) * sfmax(out[0], T(0)));
-            T xx;
-            if constexpr (SCALED) xx = mad_(sfabs(out[1]) + cc, mc.rdx, (sfabs(out[2]) + cc) * mc.rdy);
-            else xx = DivD{mc.dx, mc.rdx}(sfabs(out[1]) + cc) + DivD{mc.dy, mc.rdy}(sfabs(out[2]) + cc);
-            vs.xmax[lane] = nmax(T(vs.xmax[lane]), xx);
-            vs.xmin[lane] = nmin(T(vs.xmin[lane]), xx);
-            vs.vol[lane] = vs.vol[lane] + double(out[0]) * P.cell_area;
-          }
-        }
+        RingCells<T, COH> cells{P, cur, stage + RR::kWSlots * 512 +
+                                    (gxc - c0 + ((int(unsigned(r) * unsigned(nx)) + c0) & (RR::kChunk - 1))) * int(sizeof(T)),
+                                o_ns, o_nd, o_r0, o_r1, o_hc, o_ex, o_ey, o_ir, o_ic};
+        lean_cell<T, P2, EXTRA, COH>(P, st, cur, sm.step, rk, rain_any, g, gx, r, Rm, Jm.hx, Jm.hy, Sm.hx, Sm.hy, W, E, GS, GN,
+                                     EDGE && (xedge || r == 0 || r == ny - 1), ed, cells, acc,
+                                     [&](T xx, T hN) {
+                                       vs.xmax[lane] = nmax(T(vs.xmax[lane]), xx);
+                                       vs.xmin[lane] = nmin(T(vs.xmin[lane]), xx);
+                                       vs.vol[lane] = vs.vol[lane] + double(hN) * P.cell_area;
+                                     });
       }
     }
     GS = GN;
   }
   sweep_totals(sm, acc);
   return y1;
+}
+
+// A warp's strip sums into the strip's partial slot.
+template <typename T>
+__device__ __forceinline__ void store_strip_sums(const StageParams<T>& P, int st, long long gw, const SweepAcc<T>& acc) {
+  const int lane = threadIdx.x;
+  if (st == P.nstages - 1) {
+    const double mx = warp_max(double(acc.xmax)), mn = warp_min(double(acc.xmin)), vs = warp_sum(acc.vol);
+    if (lane == 0) {
+      P.part[gw] = mx;
+      P.part[P.nblk + gw] = mn;
+      P.part[2 * P.nblk + gw] = vs;
+    }
+  }
+  if (P.mode & M_TALLY) {
+    const double rs = warp_sum(acc.rain), os = warp_sum(acc.removed), ws = warp_sum(acc.walls);
+    if (lane == 0) store_tallies(P, st, gw, rs, os, ws, P.ctl->dt);
+  }
 }
 
 // One strip of one solver's stage: its class's sweep, then its partial sums. `entry` is the
@@ -980,18 +1061,196 @@ __device__ __forceinline__ void sweep_strip(const StageParams<T>& P, int st, uns
     sweep_rows_general<T, EXTRA, COH>(P, st, tile_x, y, y1, rest);
     acc = rest;
   }
-  const int lane = threadIdx.x;
-  if (st == P.nstages - 1) {
-    const double mx = warp_max(double(acc.xmax)), mn = warp_min(double(acc.xmin)), vs = warp_sum(acc.vol);
-    if (lane == 0) {
-      P.part[gw] = mx;
-      P.part[P.nblk + gw] = mn;
-      P.part[2 * P.nblk + gw] = vs;
+  store_strip_sums(P, st, gw, acc);
+}
+
+// ---------------------------------------------------------------------------------------
+// Row-tile kernel: a strip's rows side by side instead of one after another. One block per strip
+// of kTileRows output rows, one warp per row of its window: each warp forms its row's slopes and
+// sides, then the face below it, then its cells; neighbours in y come from shared memory. The
+// lean sweep's arithmetic, so the same bits. For meshes of few strips, where a marching warp's
+// latency is the whole stage's time. A block whose window holds a value out of sweep_rows' range
+// hands its rows to sweep_rows_general.
+// ---------------------------------------------------------------------------------------
+constexpr int kTileRows = 8, kTileWarps = kTileRows + 4;
+
+// a cell's values loaded ahead into registers (fields the tile kernel does not expect: directly)
+template <typename T> struct LoadedCells {
+  const StageParams<T>& P;
+  int cur;
+  T u[3], a[3], n, r;
+  __device__ __forceinline__ T u0(int f) const { return u[f]; }
+  __device__ __forceinline__ T a0(int f) const { return a[f]; }
+  __device__ __forceinline__ T ns(long long) const { return n; }
+  __device__ __forceinline__ T nd(long long g) const { return ld(P.man_p[1], g); }
+  __device__ __forceinline__ T r0(const T*, long long) const { return r; }
+  __device__ __forceinline__ T r1(const T* p, long long g) const { return ld(p, g); }
+  __device__ __forceinline__ T hc(long long g) const { return ld(P.hc[cur], g); }
+};
+
+template <typename T, bool P2>
+__global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 8 ? 1 : 2)
+    tile_rows_kernel(const __grid_constant__ StageParams<T> P, const int st) {
+  constexpr bool F32 = sizeof(T) == 4;
+  constexpr bool SCALED = F32 || P2;
+  __shared__ StepConst<T> step;
+  __shared__ T val[3][kTileWarps][32];    // h, u, v
+  __shared__ T upper[5][kTileWarps][32];  // a row's upper side: bed, h, normal, tangential; its lower tangential
+  __shared__ T face[4][kTileWarps][32];   // the face below a row
+  __shared__ double sums[6][kTileRows];
+  if (P.ctl->done) return;
+  const int lane = threadIdx.x, w = uniform(threadIdx.y);
+  const int nx = P.nx, ny = P.ny;
+  const int tiles_x = (nx + kSweepOut - 1) / kSweepOut;
+  const int gw = blockIdx.x, tile_y = gw / tiles_x, tile_x = gw - tile_y * tiles_x;
+  const int y0 = tile_y * kTileRows, y1 = min(y0 + kTileRows, ny);
+  const int row = y0 - 2 + w;
+  const int gx = tile_x * kSweepOut - 2 + lane, gxc = min(max(gx, 0), nx - 1);
+  const bool out_row = w >= 2 && row < y1;
+  const bool out = out_row && lane >= 2 && lane < 2 + kSweepOut && gx < nx;
+  const int cur = uniform(P.ctl->cur);
+  const bool first = st == 0, last = st == P.nstages - 1;
+  const MeshOps<T, P2> mo{P.mc};
+  const auto& mc = P.mc;
+  const int rk = uniform(P.fc->rain_kind);
+  const bool rain_any = uniform(P.fc->rq0 != 0.0 || P.fc->rq1 != 0.0);
+
+  // every load of the row at once
+  const long long gc = (long long)min(max(row, 0), ny - 1) * nx + gxc;
+  RowV<T> R;
+  R.h = ld(P.in(st, cur, 0), gc); R.u = ld(P.in(st, cur, 1), gc); R.v = ld(P.in(st, cur, 2), gc);
+  R.z = ld(P.z, gc); R.zx = ld(P.zx, gc); R.zy = ld(P.zy, gc);
+  LoadedCells<T> cells{P, cur};
+  if (out_row) {
+    if (!first)
+#pragma unroll
+      for (int f = 0; f < 3; ++f) { cells.u[f] = ld(P.S[cur][f], gc); cells.a[f] = ld(P.S[cur ^ 1][f], gc); }
+    if (P.manning && P.man_p[0]) cells.n = ld(P.man_p[0], gc);
+    if (rk == 3) cells.r = ld(P.pat, gc);
+    if (rk == 2) cells.r = ld(P.q0p, gc);
+  }
+  if (w == 0 && lane == 0) const_cast<volatile StepConst<T>&>(step).set(P, st);
+  val[0][w][lane] = R.h; val[1][w][lane] = R.u; val[2][w][lane] = R.v;
+  const bool bad = !(in_range(R.z) && (F32 || (in_range(R.h) && in_range(R.u) && in_range(R.v)))) || !P.exact;
+  SweepAcc<T> acc;
+  if (__syncthreads_or(bad)) {
+    if (w > 0) return;
+    sweep_rows_general<T, false, false>(P, st, tile_x, y0, y1, acc);
+    store_strip_sums(P, st, gw, acc);
+    return;
+  }
+
+  // half slopes of the row (State.cpp:187-192), y towards row + 1
+  SlopeV<T> J{}, S{};
+  if (w > 0 && w < kTileWarps - 1) {
+    auto yslope = [&](int f, T x, T& j, T& s) {
+      const T lo = val[f][w - 1][lane], hi = val[f][w + 1][lane];
+      const T a = mo.diff_y(x - lo), b = mo.diff_y(hi - x);
+      T hs = half_slope(a, b, F32 ? a + b : mo.diff_y(hi - lo));
+      if (row >= ny - 1) hs = T(0.5) * a;
+      if (row <= 0) hs = ny > 1 ? T(0.5) * b : T(0);
+      j = mo.jump_y(hs);
+      s = T(-2) * hs;
+    };
+    yslope(0, R.h, J.hy, S.hy);
+    yslope(1, R.u, J.uy, S.uy);
+    yslope(2, R.v, J.vy, S.vy);
+    auto xslope = [&](T x, T& j, T& s) {
+      const T e = dn1(x), b = mo.diff_x(e - x), a = up1(b);
+      T cc;
+      if constexpr (F32) cc = a + b;
+      else cc = mo.diff_x(e - up1(x));
+      T hs = half_slope(a, b, cc);
+      if (gx >= nx - 1) hs = T(0.5) * a;
+      if (gx <= 0) hs = nx > 1 ? T(0.5) * b : T(0);
+      j = mo.jump_x(hs);
+      s = T(2) * hs;
+    };
+    xslope(R.h, J.hx, S.hx);
+    xslope(R.u, J.ux, S.ux);
+    xslope(R.v, J.vx, S.vx);
+    upper[0][w][lane] = mo.zside(mc.hdy, R.zy, R.z);
+    upper[1][w][lane] = R.h - J.hy;
+    upper[2][w][lane] = R.v - J.vy;
+    upper[3][w][lane] = R.u - J.uy;
+    upper[4][w][lane] = R.u + J.uy;
+  }
+  __syncthreads();
+  // the face below the row (fy = row), Fluxes.cpp:55-64
+  FaceG<T> GS{};
+  if (w >= 2 && w < kTileWarps - 1) {
+    T zhi = R.z;
+    if constexpr (F32) {
+      if (P.zdat != nullptr && (row % kDatumTY) == 0 && row > 0 && row < ny) {
+        const long long tb = datum_tile(gxc, row, P.dtiles_x);
+        zhi = T(double(zhi) + (P.zdat[tb] - P.zdat[tb - P.dtiles_x]));
+      }
+    }
+    Side<T> m{upper[0][w - 1][lane], upper[1][w - 1][lane], upper[2][w - 1][lane], upper[3][w - 1][lane]};
+    Side<T> p{mo.zside(-mc.hdy, R.zy, zhi), R.h + J.hy, R.v + J.vy, R.u + J.uy};
+    // walls at the mesh edge, FluxKernel.cpp:111-157 (rows past it hold the edge row's values)
+    if (row == 0) m = {R.z + R.h * T(2), T(0), T(0), R.u - J.uy};
+    if (row == ny) p = {R.z + R.h * T(2), T(0), T(0), upper[4][w - 1][lane]};
+    GS = face_pair(m, p, [&](T x) { return mo.over_2dy(x); });
+    face[0][w][lane] = GS.h; face[1][w][lane] = GS.n; face[2][w][lane] = GS.t; face[3][w][lane] = GS.z;
+  }
+  FaceG<T> W{};
+  if (out_row) {  // west faces: the left lane's east side against this lane's west side
+    T zw = R.z;
+    if constexpr (F32) {
+      if (P.zdat != nullptr && (gx % kDatumTX) == 0 && gx > 0 && gx < nx) {
+        const long long tb = datum_tile(gx, row, P.dtiles_x);
+        const double d = P.zdat[tb] - P.zdat[tb - 1];
+        zw = double(T(d)) == d ? R.z + T(d) : T(double(R.z) + d);
+      }
+    }
+    Side<T> p{mo.zside(-mc.hdx, R.zx, zw), R.h - J.hx, R.u - J.ux, R.v - J.vx};
+    const T eut = R.v + J.vx, wall = R.z + R.h * T(2);
+    Side<T> m{up1(mo.zside(mc.hdx, R.zx, R.z)), up1(R.h + J.hx), up1(R.u + J.ux), up1(eut)};
+    const T wl = up1(wall), utl = up1(p.ut);
+    if (gx == 0) m = {wall, T(0), T(0), eut};
+    if (gx == nx) p = {wl, T(0), T(0), utl};
+    W = face_pair(m, p, [&](T x) { return mo.over_2dx(x); });
+  }
+  __syncthreads();
+  if (out_row) {
+    const FaceG<T> E{dn1(W.h), dn1(W.n), dn1(W.t), dn1(W.z)};
+    const FaceG<T> GN{face[0][w + 1][lane], face[1][w + 1][lane], face[2][w + 1][lane], face[3][w + 1][lane]};
+    if (out)
+      lean_cell<T, P2, false, false>(P, st, cur, step, rk, rain_any, gc, gx, row, R, J.hx, J.hy, S.hx, S.hy, W, E, GS, GN,
+                                     gx == 0 || gx == nx - 1 || row == 0 || row == ny - 1, EddyIn<T>{}, cells, acc, [&](T xx, T hN) {
+                                       acc.xmax = nmax(acc.xmax, xx);
+                                       acc.xmin = nmin(acc.xmin, xx);
+                                       acc.vol += double(hN) * P.cell_area;
+                                     });
+  }
+  if (!last && !(P.mode & M_TALLY)) return;
+  // the strip's sums: rows by shuffles, then the first warp's lane 0 over the rows in order
+  if (out_row) {
+    const int i = w - 2;
+    if (last) {
+      const double mx = warp_max(double(acc.xmax)), mn = warp_min(double(acc.xmin)), vs = warp_sum(acc.vol);
+      if (lane == 0) { sums[0][i] = mx; sums[1][i] = mn; sums[2][i] = vs; }
+    }
+    if (P.mode & M_TALLY) {
+      const double rs = warp_sum(acc.rain), os = warp_sum(acc.removed), ws = warp_sum(acc.walls);
+      if (lane == 0) { sums[3][i] = rs; sums[4][i] = os; sums[5][i] = ws; }
     }
   }
+  __syncthreads();
+  if (w != 0 || lane != 0) return;
+  const int n = y1 - y0;
+  if (last) {
+    double mx = sums[0][0], mn = sums[1][0], vs = sums[2][0];
+    for (int i = 1; i < n; ++i) { mx = nmax(mx, sums[0][i]); mn = nmin(mn, sums[1][i]); vs += sums[2][i]; }
+    P.part[gw] = mx;
+    P.part[P.nblk + gw] = mn;
+    P.part[2 * P.nblk + gw] = vs;
+  }
   if (P.mode & M_TALLY) {
-    const double rs = warp_sum(acc.rain), os = warp_sum(acc.removed), ws = warp_sum(acc.walls);
-    if (lane == 0) store_tallies(P, st, gw, rs, os, ws, P.ctl->dt);
+    double rs = 0.0, os = 0.0, ws = 0.0;
+    for (int i = 0; i < n; ++i) { rs += sums[3][i]; os += sums[4][i]; ws += sums[5][i]; }
+    store_tallies(P, st, gw, rs, os, ws, step.dt_d);
   }
 }
 
