@@ -98,13 +98,12 @@ template <> cudaError_t launch_stage<SV_T>(const StageParams<SV_T>& P, int st, i
 constexpr int kRingBytes = kSweepWarps * int(sizeof(SweepShared<SV_T>));
 
 // The column sweep of a stage: the strips in P.strips, P.rows rows each. `cap`: resident blocks
-// per SM asked of the register allocator. FP32 multiplies by the reciprocal cell sizes whatever
-// they are, so it has no power-of-two form of its own.
+// per SM asked of the register allocator.
 template <int MINB, bool EXTRA> static cudaError_t launch_sweep_c(const StageParams<SV_T>& P, int st, cudaStream_t s) {
   if (P.n_strips <= 0) return cudaSuccess;
   const dim3 grid(unsigned((P.n_strips + kSweepWarps - 1) / kSweepWarps)), block(32, kSweepWarps);
-  if (sizeof(SV_T) == 8 && pow2_mesh(P.dx, P.dy))
-    return launch_dynamic<sweep_kernel<SV_T, MINB, sizeof(SV_T) == 8, EXTRA>>(grid, block, kRingBytes, s, P, st);
+  if (pow2_mesh(P.dx, P.dy))
+    return launch_dynamic<sweep_kernel<SV_T, MINB, true, EXTRA>>(grid, block, kRingBytes, s, P, st);
   return launch_dynamic<sweep_kernel<SV_T, MINB, false, EXTRA>>(grid, block, kRingBytes, s, P, st);
 }
 static cudaError_t launch_sweep(const StageParams<SV_T>& P, int st, int cap, bool extra, cudaStream_t s) {
@@ -125,7 +124,7 @@ template <> cudaError_t launch_variant<SV_T>(const StageParams<SV_T>& P, int st,
   if (variant == kTileRowsVariant) {
     if (P.nblk <= 0) return cudaSuccess;
     const dim3 grid{unsigned(P.nblk)}, block(32, kTileWarps);
-    if (sizeof(SV_T) == 8 && pow2_mesh(P.dx, P.dy)) tile_rows_kernel<SV_T, sizeof(SV_T) == 8><<<grid, block, 0, s>>>(P, st);
+    if (pow2_mesh(P.dx, P.dy)) tile_rows_kernel<SV_T, true><<<grid, block, 0, s>>>(P, st);
     else tile_rows_kernel<SV_T, false><<<grid, block, 0, s>>>(P, st);
     return cudaGetLastError();
   }
@@ -172,7 +171,6 @@ template <> cudaError_t launch_to_f64<SV_T>(const SV_T* src, double* dst, long l
 
 template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, int n, int st, bool p2, bool extra,
                                                  cudaStream_t s) {
-  constexpr bool F64 = sizeof(SV_T) == 8;
   constexpr int CAP = kBatchCap<SV_T>, XCAP = kExtraCap<SV_T>;
   for (int k0 = 0; k0 < n; k0 += kBatchMembers) {
     BatchParams<SV_T> B;
@@ -186,10 +184,10 @@ template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, in
     if (grid.x == 0) continue;
     cudaError_t e;
     if (extra)
-      e = p2 && F64 ? launch_dynamic<sweep_batch_kernel<SV_T, XCAP, F64, true>>(grid, block, kRingBytes, s, B, st)
+      e = p2 ? launch_dynamic<sweep_batch_kernel<SV_T, XCAP, true, true>>(grid, block, kRingBytes, s, B, st)
                     : launch_dynamic<sweep_batch_kernel<SV_T, XCAP, false, true>>(grid, block, kRingBytes, s, B, st);
     else
-      e = p2 && F64 ? launch_dynamic<sweep_batch_kernel<SV_T, CAP, F64, false>>(grid, block, kRingBytes, s, B, st)
+      e = p2 ? launch_dynamic<sweep_batch_kernel<SV_T, CAP, true, false>>(grid, block, kRingBytes, s, B, st)
                     : launch_dynamic<sweep_batch_kernel<SV_T, CAP, false, false>>(grid, block, kRingBytes, s, B, st);
     if (e != cudaSuccess) return e;
   }
@@ -202,11 +200,10 @@ template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, in
 template <int BANK>
 static cudaError_t launch_persist_t(const PersistParams<SV_T>& PP, const StageParams<SV_T>* Ps, bool p2, bool extra,
                                     cudaStream_t s) {
-  constexpr bool F64 = sizeof(SV_T) == 8;
   constexpr int CAP = kBatchCap<SV_T>, XCAP = kExtraCap<SV_T>;
   void (*kern)(const PersistParams<SV_T>, const MemberBank<SV_T, BANK>) =
-      extra ? (p2 ? persist_batch_kernel<SV_T, XCAP, F64, true, BANK> : persist_batch_kernel<SV_T, XCAP, false, true, BANK>)
-            : (p2 ? persist_batch_kernel<SV_T, CAP, F64, false, BANK> : persist_batch_kernel<SV_T, CAP, false, false, BANK>);
+      extra ? (p2 ? persist_batch_kernel<SV_T, XCAP, true, true, BANK> : persist_batch_kernel<SV_T, XCAP, false, true, BANK>)
+            : (p2 ? persist_batch_kernel<SV_T, CAP, true, false, BANK> : persist_batch_kernel<SV_T, CAP, false, false, BANK>);
   int dev = 0, nsm = 0, per_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess && kRingBytes > 48 * 1024)

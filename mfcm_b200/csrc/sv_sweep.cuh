@@ -389,10 +389,14 @@ __device__ __forceinline__ double flip_sign(double x, double s) {
   return __hiloint2double(__double2hiint(x) ^ (__double2hiint(s) & 0x80000000), __double2loint(x));
 }
 
-// Quotients by the mesh spacing. FP32, or dx and dy powers of two: differences are kept undivided
-// (diff_x, diff_y) and scaled where they are used; else exact divisions (div_exact).
+// Quotients by the mesh spacing. With dx and dy powers of two, differences are kept undivided
+// (diff_x, diff_y) and scaled where they are used; else they are divided (FP64: exactly; FP32: by
+// the rounded reciprocal). FP32 could stay undivided with any spacing, and would be a little
+// faster, but a velocity reconstructed across a full one-sided slope is then an exact zero where
+// the quotients leave a rounding error, and a face whose velocity is an exact zero has no
+// upwinding at all: results would move by 1e-4 of the velocity at a dam break's first timesteps.
 template <typename T, bool P2> struct MeshOps {
-  static constexpr bool SCALED = sizeof(T) == 4 || P2;
+  static constexpr bool SCALED = P2;
   const MeshConst<T>& mc;
   __device__ __forceinline__ T diff_x(T x) const { if constexpr (SCALED) return x; else return div_exact(x, mc.dx, mc.rdx); }
   __device__ __forceinline__ T diff_y(T x) const { if constexpr (SCALED) return x; else return div_exact(x, mc.dy, mc.rdy); }
@@ -405,17 +409,22 @@ template <typename T, bool P2> struct MeshOps {
   __device__ __forceinline__ T over_dx(T x) const { if constexpr (SCALED) return x * mc.rdx; else return diff_x(x); }
   __device__ __forceinline__ T over_dy(T x) const { if constexpr (SCALED) return x * mc.rdy; else return diff_y(x); }
   // bed at a face side: z + 0.5 d * slope, the product rounded by itself unless it is exact
-  __device__ __forceinline__ static T zside(T hd, T s, T z) { if constexpr (SCALED) return sfma_(hd, s, z); else return z + hd * s; }
-  // half jump across half a cell (0.5 d * slope) from half a slope
-  __device__ __forceinline__ T jump_x(T hs) const { if constexpr (SCALED) return hs; else return mc.dx * hs; }
-  __device__ __forceinline__ T jump_y(T hs) const { if constexpr (SCALED) return hs; else return mc.dy * hs; }
+  __device__ __forceinline__ static T zside(T hd, T s, T z) { if constexpr (SCALED || sizeof(T) == 4) return sfma_(hd, s, z); else return z + hd * s; }
+  // what is kept of half a slope for the faces: the half jump 0.5 d * slope, but in FP32 with
+  // quotients half the slope itself (side_x and side_y then add d times it, fused)
+  __device__ __forceinline__ T jump_x(T hs) const { if constexpr (SCALED || sizeof(T) == 4) return hs; else return mc.dx * hs; }
+  __device__ __forceinline__ T jump_y(T hs) const { if constexpr (SCALED || sizeof(T) == 4) return hs; else return mc.dy * hs; }
+  // a cell's value plus a half jump
+  __device__ __forceinline__ T side_x(T v, T j) const { if constexpr (!SCALED && sizeof(T) == 4) return sfma_(mc.dx, j, v); else return v + j; }
+  __device__ __forceinline__ T side_y(T v, T j) const { if constexpr (!SCALED && sizeof(T) == 4) return sfma_(mc.dy, j, v); else return v + j; }
 };
 
 // Doubled fluxes of a face: depth, normal and tangential momentum, bed step.
 template <typename T> struct FaceG { T h, n, t, z; };
 
 // The doubled fluxes of a face from its two sides (FluxKernel.cpp:189-291); dv(x) is x / (2 d).
-template <typename T, typename DV>
+// STRICT: products rounded by themselves (the same thing in FP64).
+template <typename T, bool STRICT, typename DV>
 __device__ __forceinline__ FaceG<T> face_pair(const Side<T>& m, const Side<T>& p, const DV& dv) {
   const T g = T(kG);
   const bool rise = p.zb > m.zb;
@@ -443,9 +452,15 @@ __device__ __forceinline__ FaceG<T> face_pair(const Side<T>& m, const Side<T>& p
   const T a = pick_max(a_p, a_m);
   const T nm = mad_(um, T(0.5) * um, gm);
   const T np = mad_(up, T(0.5) * up, am ? -gp : gp);
-  G.h = mad_(-a, hp - hm, mad_(hp, up, hm * um));
-  G.n = mad_(-a, up - um, np + nm);
-  G.t = mad_(-a, tp - tm, mad_(tp, up, tm * um));
+  if constexpr (STRICT) {
+    G.h = (hp * up + hm * um) - a * (hp - hm);
+    G.n = (np + nm) - a * (up - um);
+    G.t = (tp * up + tm * um) - a * (tp - tm);
+  } else {
+    G.h = mad_(-a, hp - hm, mad_(hp, up, hm * um));
+    G.n = mad_(-a, up - um, np + nm);
+    G.t = mad_(-a, tp - tm, mad_(tp, up, tm * um));
+  }
   if (dry) G.n = dry_n;
   return G;
 }
@@ -458,6 +473,7 @@ template <typename T> __device__ __forceinline__ T manning_n(T h, T ns, T nd, T 
   const T ss = t * t * (T(3) - T(2) * t);
   return ns + (nd - ns) * ss;
 }
+template <bool>
 __device__ __forceinline__ void friction(double h, double u, double v, double n, double dt, double, double& du,
                                          double& dv) {
   const double sf = n * n * ssqrt(u * u + v * v) * pow43_(manning_inv_h(h));
@@ -467,7 +483,17 @@ __device__ __forceinline__ void friction(double h, double u, double v, double n,
   du = du + fu;
   dv = dv + fv;
 }
-__device__ __forceinline__ void friction(float h, float u, float v, float n, float, float rdt, float& du, float& dv) {
+template <bool STRICT>
+__device__ __forceinline__ void friction(float h, float u, float v, float n, float dt, float rdt, float& du, float& dv) {
+  if constexpr (STRICT) {
+    const float sf = n * n * ssqrt(mad_(u, u, v * v)) * pow43_(manning_inv_h(h));
+    float fu = -float(kG) * sf * u, fv = -float(kG) * sf * v;
+    if (fabsf(fu * dt) > fabsf(u)) fu = -u * rdt;
+    if (fabsf(fv * dt) > fabsf(v)) fv = -v * rdt;
+    du = du + fu;
+    dv = dv + fv;
+    return;
+  }
   const float rate = fminf(float(kG) * (n * n * ssqrt(mad_(u, u, v * v)) * pow43_(manning_inv_h(h))), rdt);
   du = mad_(-rate, u, du);
   dv = mad_(-rate, v, dv);
@@ -485,7 +511,7 @@ __device__ __forceinline__ void lean_cell(const StageParams<T>& P, int st, int c
                                           const FaceG<T>& GN, bool medge, const EddyIn<T>& ed, const Cells& cells,
                                           SweepAcc<T>& acc, const Totals& totals) {
   constexpr bool F32 = sizeof(T) == 4;
-  constexpr bool SCALED = F32 || P2;
+  constexpr bool SCALED = P2;
   const int nx = P.nx, ny = P.ny;
   const bool first = st == 0, last = st == P.nstages - 1;
   const auto& mc = P.mc;
@@ -500,8 +526,13 @@ __device__ __forceinline__ void lean_cell(const StageParams<T>& P, int st, int c
     dh = mad_(GS.h - GN.h, mc.ky, (W.h - E.h) * mc.kx);
     du = mad_(GS.t - GN.t, mc.ky, (W.n - E.n) * mc.kx);
     dv = mad_(GS.n - GN.n, mc.ky, (W.t - E.t) * mc.kx);
-    du = mad_(-mc.gx, jhx, du);
-    dv = mad_(mc.gy, jhy, dv);
+    if constexpr (SCALED) {
+      du = mad_(-mc.gx, jhx, du);
+      dv = mad_(mc.gy, jhy, dv);
+    } else {
+      du = mad_(T(-kG), shx, du);
+      dv = mad_(T(-kG), shy, dv);
+    }
     du = mad_(W.z - E.z, mc.kx, du);
     dv = mad_(GS.z - GN.z, mc.ky, dv);
   } else if constexpr (SCALED) {
@@ -538,7 +569,7 @@ __device__ __forceinline__ void lean_cell(const StageParams<T>& P, int st, int c
     if (ns != nd)
       n = manning_n<T>(h, ns, nd, P.man_p[2] ? ld(P.man_p[2], g) : P.man_s[2],
                        P.man_p[3] ? ld(P.man_p[3], g) : P.man_s[3]);
-    friction(h, u, v, n, k.dt, k.rdt, du, dv);
+    friction<!P2>(h, u, v, n, k.dt, k.rdt, du, dv);
   };
   if constexpr (!EXTRA) {
     roughness();
@@ -696,7 +727,7 @@ __device__ __forceinline__ void lean_cell(const StageParams<T>& P, int st, int c
   if (last) {  // CFL quantity and volume of U_[N] (State.cpp:204-228)
     const T cc = ssqrt(T(kG) * sfmax(out[0], T(0)));
     T xx;
-    if constexpr (SCALED) xx = mad_(sfabs(out[1]) + cc, mc.rdx, (sfabs(out[2]) + cc) * mc.rdy);
+    if constexpr (SCALED || F32) xx = mad_(sfabs(out[1]) + cc, mc.rdx, (sfabs(out[2]) + cc) * mc.rdy);
     else xx = DivD{mc.dx, mc.rdx}(sfabs(out[1]) + cc) + DivD{mc.dy, mc.rdy}(sfabs(out[2]) + cc);
     totals(xx, out[0]);
   }
@@ -743,7 +774,7 @@ template <typename T, bool P2, bool EXTRA, bool EDGE, bool COH>
 __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int tile_x, int y0, int y1, SweepShared<T>& sm,
                                           SweepAcc<T>& acc) {
   constexpr bool F32 = sizeof(T) == 4;
-  constexpr bool SCALED = F32 || P2;  // slopes and fluxes undivided, one scaling per cell
+  constexpr bool SCALED = P2;  // slopes and fluxes undivided, one scaling per cell
   const Ctl* ctl = P.ctl;
   const int nx = P.nx, ny = P.ny;
   const int lane = threadIdx.x;
@@ -884,18 +915,14 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
       const int row = k - 1;
       const bool yedge = EDGE && (row <= 0 || row >= ny - 1);
       auto yslope = [&](T a, T b, T lo, T hi, T& j, T& s) {
-        T hs = half_slope(a, b, F32 ? a + b : mo.diff_y(hi - lo));
+        T hs = half_slope(a, b, F32 && SCALED ? a + b : mo.diff_y(hi - lo));
         if (yedge) {  // one-sided: the slope is the present quotient
           if (row >= ny - 1) hs = T(0.5) * a;
           if (row <= 0) hs = ny > 1 ? T(0.5) * b : T(0);
         }
-        if constexpr (SCALED) {
-          j = hs;
-          if constexpr (EXTRA) s = T(-2) * hs * mc.rdy;
-        } else {
-          j = mc.dy * hs;
-          s = T(-2) * hs;
-        }
+        j = mo.jump_y(hs);
+        if constexpr (!SCALED) s = T(-2) * hs;
+        else if constexpr (EXTRA) s = T(-2) * hs * mc.rdy;
       };
       yslope(fyA[0], fyB[0], Rm.h, Rp.h, J0.hy, S0.hy);
       yslope(fyA[1], fyB[1], Rm.u, Rp.u, J0.uy, S0.uy);
@@ -904,20 +931,16 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
         const T e = dn1(x);
         const T b = mo.diff_x(e - x), a = up1(b);
         T cc;
-        if constexpr (F32) cc = a + b;
+        if constexpr (F32 && SCALED) cc = a + b;
         else cc = mo.diff_x(e - up1(x));
         T hs = half_slope(a, b, cc);
         if (xedge) {
           if (gx >= nx - 1) hs = T(0.5) * a;
           if (gx <= 0) hs = nx > 1 ? T(0.5) * b : T(0);
         }
-        if constexpr (SCALED) {
-          j = hs;
-          if constexpr (EXTRA) s = T(2) * hs * mc.rdx;
-        } else {
-          j = mc.dx * hs;
-          s = T(2) * hs;
-        }
+        j = mo.jump_x(hs);
+        if constexpr (!SCALED) s = T(2) * hs;
+        else if constexpr (EXTRA) s = T(2) * hs * mc.rdx;
       };
       xslope(R0.h, J0.hx, S0.hx);
       xslope(R0.u, J0.ux, S0.ux);
@@ -934,13 +957,13 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
           zhi = T(double(zhi) + (P.zdat[tb] - P.zdat[tb - P.dtiles_x]));
         }
       }
-      Side<T> m{mo.zside(mc.hdy, Rm.zy, Rm.z), Rm.h - Jm.hy, Rm.v - Jm.vy, Rm.u - Jm.uy};
-      Side<T> p{mo.zside(-mc.hdy, R0.zy, zhi), R0.h + J0.hy, R0.v + J0.vy, R0.u + J0.uy};
+      Side<T> m{mo.zside(mc.hdy, Rm.zy, Rm.z), mo.side_y(Rm.h, -Jm.hy), mo.side_y(Rm.v, -Jm.vy), mo.side_y(Rm.u, -Jm.uy)};
+      Side<T> p{mo.zside(-mc.hdy, R0.zy, zhi), mo.side_y(R0.h, J0.hy), mo.side_y(R0.v, J0.vy), mo.side_y(R0.u, J0.uy)};
       if (EDGE && (fy <= 0 || fy >= ny)) {  // walls at the mesh edge, FluxKernel.cpp:111-157
-        if (fy == 0) m = {R0.z + R0.h * T(2), T(0), T(0), R0.u - J0.uy};
-        if (fy == ny) p = {Rm.z + Rm.h * T(2), T(0), T(0), Rm.u + Jm.uy};
+        if (fy == 0) m = {R0.z + R0.h * T(2), T(0), T(0), mo.side_y(R0.u, -J0.uy)};
+        if (fy == ny) p = {Rm.z + Rm.h * T(2), T(0), T(0), mo.side_y(Rm.u, Jm.uy)};
       }
-      GN = face_pair(m, p, [&](T x) { return mo.over_2dy(x); });
+      GN = face_pair<T, !P2>(m, p, [&](T x) { return mo.over_2dy(x); });
     }
     // output row k-2
     if (k >= y0 + 2) {
@@ -965,16 +988,16 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
           }
         }
       }
-      Side<T> p{mo.zside(-mc.hdx, Rm.zx, zw), Rm.h - Jm.hx, Rm.u - Jm.ux, Rm.v - Jm.vx};
-      const T eut = Rm.v + Jm.vx;
-      Side<T> m{up1(mo.zside(mc.hdx, Rm.zx, Rm.z)), up1(Rm.h + Jm.hx), up1(Rm.u + Jm.ux), up1(eut)};
+      Side<T> p{mo.zside(-mc.hdx, Rm.zx, zw), mo.side_x(Rm.h, -Jm.hx), mo.side_x(Rm.u, -Jm.ux), mo.side_x(Rm.v, -Jm.vx)};
+      const T eut = mo.side_x(Rm.v, Jm.vx);
+      Side<T> m{up1(mo.zside(mc.hdx, Rm.zx, Rm.z)), up1(mo.side_x(Rm.h, Jm.hx)), up1(mo.side_x(Rm.u, Jm.ux)), up1(eut)};
       if (xedge) {
         const T wall = Rm.z + Rm.h * T(2);
         const T wl = up1(wall), utl = up1(p.ut);
         if (gx == 0) m = {wall, T(0), T(0), eut};
         if (gx == nx) p = {wl, T(0), T(0), utl};
       }
-      const FaceG<T> W = face_pair(m, p, [&](T x) { return mo.over_2dx(x); });
+      const FaceG<T> W = face_pair<T, !P2>(m, p, [&](T x) { return mo.over_2dx(x); });
       const FaceG<T> E{dn1(W.h), dn1(W.n), dn1(W.t), dn1(W.z)};
       EddyIn<T> ed{};
       if constexpr (EXTRA) {
@@ -1092,7 +1115,7 @@ template <typename T, bool P2>
 __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 8 ? 1 : 2)
     tile_rows_kernel(const __grid_constant__ StageParams<T> P, const int st) {
   constexpr bool F32 = sizeof(T) == 4;
-  constexpr bool SCALED = F32 || P2;
+  constexpr bool SCALED = P2;
   __shared__ StepConst<T> step;
   __shared__ T val[3][kTileWarps][32];    // h, u, v
   __shared__ T upper[5][kTileWarps][32];  // a row's upper side: bed, h, normal, tangential; its lower tangential
@@ -1146,7 +1169,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 8 ? 1 : 2)
     auto yslope = [&](int f, T x, T& j, T& s) {
       const T lo = val[f][w - 1][lane], hi = val[f][w + 1][lane];
       const T a = mo.diff_y(x - lo), b = mo.diff_y(hi - x);
-      T hs = half_slope(a, b, F32 ? a + b : mo.diff_y(hi - lo));
+      T hs = half_slope(a, b, F32 && SCALED ? a + b : mo.diff_y(hi - lo));
       if (row >= ny - 1) hs = T(0.5) * a;
       if (row <= 0) hs = ny > 1 ? T(0.5) * b : T(0);
       j = mo.jump_y(hs);
@@ -1158,7 +1181,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 8 ? 1 : 2)
     auto xslope = [&](T x, T& j, T& s) {
       const T e = dn1(x), b = mo.diff_x(e - x), a = up1(b);
       T cc;
-      if constexpr (F32) cc = a + b;
+      if constexpr (F32 && SCALED) cc = a + b;
       else cc = mo.diff_x(e - up1(x));
       T hs = half_slope(a, b, cc);
       if (gx >= nx - 1) hs = T(0.5) * a;
@@ -1170,10 +1193,10 @@ __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 8 ? 1 : 2)
     xslope(R.u, J.ux, S.ux);
     xslope(R.v, J.vx, S.vx);
     upper[0][w][lane] = mo.zside(mc.hdy, R.zy, R.z);
-    upper[1][w][lane] = R.h - J.hy;
-    upper[2][w][lane] = R.v - J.vy;
-    upper[3][w][lane] = R.u - J.uy;
-    upper[4][w][lane] = R.u + J.uy;
+    upper[1][w][lane] = mo.side_y(R.h, -J.hy);
+    upper[2][w][lane] = mo.side_y(R.v, -J.vy);
+    upper[3][w][lane] = mo.side_y(R.u, -J.uy);
+    upper[4][w][lane] = mo.side_y(R.u, J.uy);
   }
   __syncthreads();
   // the face below the row (fy = row), Fluxes.cpp:55-64
@@ -1187,11 +1210,11 @@ __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 8 ? 1 : 2)
       }
     }
     Side<T> m{upper[0][w - 1][lane], upper[1][w - 1][lane], upper[2][w - 1][lane], upper[3][w - 1][lane]};
-    Side<T> p{mo.zside(-mc.hdy, R.zy, zhi), R.h + J.hy, R.v + J.vy, R.u + J.uy};
+    Side<T> p{mo.zside(-mc.hdy, R.zy, zhi), mo.side_y(R.h, J.hy), mo.side_y(R.v, J.vy), mo.side_y(R.u, J.uy)};
     // walls at the mesh edge, FluxKernel.cpp:111-157 (rows past it hold the edge row's values)
-    if (row == 0) m = {R.z + R.h * T(2), T(0), T(0), R.u - J.uy};
+    if (row == 0) m = {R.z + R.h * T(2), T(0), T(0), mo.side_y(R.u, -J.uy)};
     if (row == ny) p = {R.z + R.h * T(2), T(0), T(0), upper[4][w - 1][lane]};
-    GS = face_pair(m, p, [&](T x) { return mo.over_2dy(x); });
+    GS = face_pair<T, !P2>(m, p, [&](T x) { return mo.over_2dy(x); });
     face[0][w][lane] = GS.h; face[1][w][lane] = GS.n; face[2][w][lane] = GS.t; face[3][w][lane] = GS.z;
   }
   FaceG<T> W{};
@@ -1204,13 +1227,13 @@ __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 8 ? 1 : 2)
         zw = double(T(d)) == d ? R.z + T(d) : T(double(R.z) + d);
       }
     }
-    Side<T> p{mo.zside(-mc.hdx, R.zx, zw), R.h - J.hx, R.u - J.ux, R.v - J.vx};
-    const T eut = R.v + J.vx, wall = R.z + R.h * T(2);
-    Side<T> m{up1(mo.zside(mc.hdx, R.zx, R.z)), up1(R.h + J.hx), up1(R.u + J.ux), up1(eut)};
+    Side<T> p{mo.zside(-mc.hdx, R.zx, zw), mo.side_x(R.h, -J.hx), mo.side_x(R.u, -J.ux), mo.side_x(R.v, -J.vx)};
+    const T eut = mo.side_x(R.v, J.vx), wall = R.z + R.h * T(2);
+    Side<T> m{up1(mo.zside(mc.hdx, R.zx, R.z)), up1(mo.side_x(R.h, J.hx)), up1(mo.side_x(R.u, J.ux)), up1(eut)};
     const T wl = up1(wall), utl = up1(p.ut);
     if (gx == 0) m = {wall, T(0), T(0), eut};
     if (gx == nx) p = {wl, T(0), T(0), utl};
-    W = face_pair(m, p, [&](T x) { return mo.over_2dx(x); });
+    W = face_pair<T, !P2>(m, p, [&](T x) { return mo.over_2dx(x); });
   }
   __syncthreads();
   if (out_row) {
