@@ -1,8 +1,8 @@
 """Build the CUDA library mfcm_b200/lib/libsv_b200.so for sm_100a (in-tree, so the built
 .so travels with the source tree).
 
-sv_f64.cu is compiled with -fmad=false: the FP64 path must round every multiply and add
-separately, like the reference's CPU arithmetic. sv_f32.cu writes its fused multiply-adds out
+sv_f64.cu and sv_noalloc.cu (which forms FP64 bed slopes) are compiled with -fmad=false: the FP64
+path must round every multiply and add separately, like the reference's CPU arithmetic. sv_f32.cu writes its fused multiply-adds out
 (-fmad=false too), so that a cell's FP32 result does not depend on the kernel that computed it.
 """
 import os
@@ -22,7 +22,7 @@ UNITS = {
     "sv_f64.cu": ["-fmad=false"],
     "sv_f32.cu": ["-fmad=false"],
     "sv_capi.cu": [],
-    "sv_noalloc.cu": [],
+    "sv_noalloc.cu": ["-fmad=false"],
 }
 
 

@@ -984,6 +984,7 @@ struct Solver final : public sv_ctx {
     for (int v = 0; v < svk::kNumVariants; ++v) {
       if (datum && !svk::variant_is_sweep(v)) continue;
       if (svk::variant_is_fp32_only(v) && sizeof(T) != 4) continue;
+      if (svk::variant_repeats<T>(v)) continue;
       P.nblk = partials(v);
       int rs = ensure_strips(v);
       if (rs) return rs;

@@ -8,19 +8,22 @@
 
 namespace svk {
 
-// The finalize kernels with CTAS blocks per solver, as clusters when there are several.
+// The finalize kernels in the chain of a timestep's launches, with `ctas` blocks per solver (a
+// cluster when there are several).
 template <typename... KArgs, typename... Args>
 static cudaError_t launch_clusters(void (*kern)(KArgs...), int solvers, int ctas, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(solvers * ctas));
   cfg.blockDim = dim3(kFinalizeThreads);
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = unsigned(ctas);
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = ctas > 1 ? attr : nullptr;
-  cfg.numAttrs = ctas > 1 ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = unsigned(ctas);
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ctas > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 cudaError_t launch_finalize(const FinalizeParams& F, cudaStream_t s) {

@@ -26,16 +26,25 @@ static cudaError_t smem_optin(K kernel, int bytes, std::atomic<bool> (&done)[kMa
   return cudaSuccess;
 }
 
-// a launch with dynamic shared memory, opted in above 48 KB
+// a launch in a chain (chain_wait), with dynamic shared memory opted in above 48 KB
 template <auto KERNEL, typename... Args>
-static cudaError_t launch_dynamic(dim3 grid, dim3 block, int smem, cudaStream_t s, const Args&... args) {
+static cudaError_t launch_chained(dim3 grid, dim3 block, int smem, cudaStream_t s, const Args&... args) {
   if (smem > 48 * 1024) {
     static std::atomic<bool> attr_set[kMaxAttrDevices];
     cudaError_t e = smem_optin(KERNEL, smem, attr_set);
     if (e != cudaSuccess) return e;
   }
-  KERNEL<<<grid, block, smem, s>>>(args...);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, KERNEL, args...);
 }
 
 // dx and dy both powers of two: the mesh divisions are exact multiplies
@@ -103,8 +112,8 @@ template <int MINB, bool EXTRA> static cudaError_t launch_sweep_c(const StagePar
   if (P.n_strips <= 0) return cudaSuccess;
   const dim3 grid(unsigned((P.n_strips + kSweepWarps - 1) / kSweepWarps)), block(32, kSweepWarps);
   if (pow2_mesh(P.dx, P.dy))
-    return launch_dynamic<sweep_kernel<SV_T, MINB, true, EXTRA>>(grid, block, kRingBytes, s, P, st);
-  return launch_dynamic<sweep_kernel<SV_T, MINB, false, EXTRA>>(grid, block, kRingBytes, s, P, st);
+    return launch_chained<sweep_kernel<SV_T, MINB, true, EXTRA>>(grid, block, kRingBytes, s, P, st);
+  return launch_chained<sweep_kernel<SV_T, MINB, false, EXTRA>>(grid, block, kRingBytes, s, P, st);
 }
 static cudaError_t launch_sweep(const StageParams<SV_T>& P, int st, int cap, bool extra, cudaStream_t s) {
   if (extra) return launch_sweep_c<kExtraCap<SV_T>, true>(P, st, s);
@@ -124,9 +133,8 @@ template <> cudaError_t launch_variant<SV_T>(const StageParams<SV_T>& P, int st,
   if (variant == kTileRowsVariant) {
     if (P.nblk <= 0) return cudaSuccess;
     const dim3 grid{unsigned(P.nblk)}, block(32, kTileWarps);
-    if (pow2_mesh(P.dx, P.dy)) tile_rows_kernel<SV_T, true><<<grid, block, 0, s>>>(P, st);
-    else tile_rows_kernel<SV_T, false><<<grid, block, 0, s>>>(P, st);
-    return cudaGetLastError();
+    if (pow2_mesh(P.dx, P.dy)) return launch_chained<tile_rows_kernel<SV_T, true>>(grid, block, 0, s, P, st);
+    return launch_chained<tile_rows_kernel<SV_T, false>>(grid, block, 0, s, P, st);
   }
   if (variant_is_split(variant)) return launch_split_t<SV_T>(P, st, s);
   if (variant_is_sweep(variant)) return launch_sweep(P, st, variant_cap<SV_T>(variant, P.n_strips), extra, s);
@@ -184,11 +192,11 @@ template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, in
     if (grid.x == 0) continue;
     cudaError_t e;
     if (extra)
-      e = p2 ? launch_dynamic<sweep_batch_kernel<SV_T, XCAP, true, true>>(grid, block, kRingBytes, s, B, st)
-                    : launch_dynamic<sweep_batch_kernel<SV_T, XCAP, false, true>>(grid, block, kRingBytes, s, B, st);
+      e = p2 ? launch_chained<sweep_batch_kernel<SV_T, XCAP, true, true>>(grid, block, kRingBytes, s, B, st)
+                    : launch_chained<sweep_batch_kernel<SV_T, XCAP, false, true>>(grid, block, kRingBytes, s, B, st);
     else
-      e = p2 ? launch_dynamic<sweep_batch_kernel<SV_T, CAP, true, false>>(grid, block, kRingBytes, s, B, st)
-                    : launch_dynamic<sweep_batch_kernel<SV_T, CAP, false, false>>(grid, block, kRingBytes, s, B, st);
+      e = p2 ? launch_chained<sweep_batch_kernel<SV_T, CAP, true, false>>(grid, block, kRingBytes, s, B, st)
+                    : launch_chained<sweep_batch_kernel<SV_T, CAP, false, false>>(grid, block, kRingBytes, s, B, st);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

@@ -90,6 +90,15 @@ inline long long variant_partials(int v, long long nx, long long ny) {
   if (v < 4) return ((nx + kTiles[v].tx - 1) / kTiles[v].tx) * ((ny + kTiles[v].ty - 1) / kTiles[v].ty);
   return strip_count(nx, ny, variant_sweep_rows(v, nx, ny));
 }
+// a column-sweep variant with the shape of a lower one (the autotuner skips it)
+template <typename T> inline bool variant_repeats(int v) {
+  if (!variant_is_sweep(v) || v == kAutoVariant) return false;
+  for (int u = 0; u < v; ++u)
+    if (u != kAutoVariant && variant_is_sweep(u) && kSweeps[u].rows == kSweeps[v].rows &&
+        clamp_cap<T>(kSweeps[u].cap) == clamp_cap<T>(kSweeps[v].cap))
+      return true;
+  return false;
+}
 // stage `st` of a timestep. extra: source terms, boundaries or a tableau that the lean sweep leaves out (sweep_rows)
 template <typename T> cudaError_t launch_variant(const StageParams<T>& P, int st, int variant, bool extra, cudaStream_t s);
 // classes of the column sweep's strips of `rows` rows (strip_class_kernel)

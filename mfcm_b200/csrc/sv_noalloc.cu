@@ -90,21 +90,18 @@ bool overlap(const void* a, const void* b, size_t n) {
   return x < y + n && y < x + n;
 }
 
-// Controller and forcing slots are rewritten on every call (the array keeps the previous
-// call's contents); the stage buffers and partial sums are fully written before being read.
-__global__ void noalloc_init_kernel(svk::Ctl* ctl, svk::DevForcing* fc, double t_local, double dt,
-                                    svk::DevForcing f) {
-  svk::Ctl c{};
-  c.t_local = t_local;
-  c.dt = dt;
-  *ctl = c;
-  *fc = f;
-}
-
-__global__ void noalloc_result_kernel(const svk::Ctl* ctl, double* result) {
-  result[0] = ctl->cn;
-  result[1] = ctl->new_dt;
-  result[2] = double(ctl->repeat);
+// Starts a call: the bed slopes, and the controller and forcing slots (the array keeps the previous
+// call's contents; the stage buffers and partial sums are fully written before being read).
+__global__ void noalloc_begin_kernel(const double* z, int nx, int ny, double dx, double dy, double* zx, double* zy,
+                                     svk::Ctl* ctl, svk::DevForcing* fc, double t_local, double dt, svk::DevForcing f) {
+  svk::bed_slope_cell<double>(z, nx, ny, dx, dy, zx, zy);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    svk::Ctl c{};
+    c.t_local = t_local;
+    c.dt = dt;
+    *ctl = c;
+    *fc = f;
+  }
 }
 
 int fail(int code, const char* msg) {
@@ -169,8 +166,10 @@ extern "C" int sv_timestep_noalloc(const sv_mesh_desc* mesh, const sv_params* pa
   f.head_edges = forcing->head_edges;
   f.rq0 = forcing->rain_q0; f.rq1 = forcing->rain_q1;
   f.hh0 = forcing->head_h0; f.hh1 = forcing->head_h1;
-  noalloc_init_kernel<<<1, 1, 0, s>>>(ctl, fc, t_local, dt, f);
-  e = svk::launch_bed_slopes<double>(z, int(mesh->nx), int(mesh->ny), dx, dy, zx, zy, s);
+  const long long ncells = (long long)(mesh->nx * mesh->ny);
+  noalloc_begin_kernel<<<unsigned((ncells + 255) / 256), 256, 0, s>>>(z, int(mesh->nx), int(mesh->ny), dx, dy, zx, zy,
+                                                                     ctl, fc, t_local, dt, f);
+  e = cudaGetLastError();
   if (e != cudaSuccess) return fail(SV_E_CUDA, cudaGetErrorString(e));
 
   svk::StageParams<double> P{};
@@ -214,10 +213,8 @@ extern "C" int sv_timestep_noalloc(const sv_mesh_desc* mesh, const sv_params* pa
   F.auto_mode = 0;
   F.tally = tally ? 1 : 0;
   F.is_float = 0;
+  F.result = result;
   e = svk::launch_finalize(F, s);
-  if (e != cudaSuccess) return fail(SV_E_CUDA, cudaGetErrorString(e));
-  noalloc_result_kernel<<<1, 1, 0, s>>>(ctl, result);
-  e = cudaGetLastError();
   if (e != cudaSuccess) return fail(SV_E_CUDA, cudaGetErrorString(e));
   return SV_OK;
 }

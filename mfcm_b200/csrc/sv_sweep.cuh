@@ -1121,6 +1121,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 8 ? 1 : 2)
   __shared__ T upper[5][kTileWarps][32];  // a row's upper side: bed, h, normal, tangential; its lower tangential
   __shared__ T face[4][kTileWarps][32];   // the face below a row
   __shared__ double sums[6][kTileRows];
+  chain_wait();
   if (P.ctl->done) return;
   const int lane = threadIdx.x, w = uniform(threadIdx.y);
   const int nx = P.nx, ny = P.ny;
@@ -1285,6 +1286,7 @@ template <typename T, int MINB, bool P2, bool EXTRA>
 __global__ void __launch_bounds__(32 * kSweepWarps, MINB)
     sweep_kernel(const __grid_constant__ StageParams<T> P, const int st) {
   extern __shared__ __align__(16) unsigned char sweep_smem[];
+  chain_wait();
   if (P.ctl->done) return;
   const int w = uniform(threadIdx.y), i = int(blockIdx.x) * kSweepWarps + w;
   if (i >= P.n_strips) return;  // whole warp: no block-level synchronisation below
@@ -1311,6 +1313,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, MINB)
   for (int step = kBatchMembers / 2; step > 0; step /= 2)  // the last member that starts at or before this block
     if (k + step < B.n && B.first_block[k + step] <= int(blockIdx.x)) k += step;
   const StageParams<T>& P = B.m[k];
+  chain_wait();
   if (P.ctl->done) return;
   const int w = uniform(threadIdx.y), i = (int(blockIdx.x) - B.first_block[k]) * kSweepWarps + w;
   if (i >= P.n_strips) return;
