@@ -5,11 +5,11 @@
 //   S[2][h,u,v]  two state buffers; S[cur] holds U_[0], S[cur^1] is the RK accumulator and
 //                receives U_[N]; accepting a timestep flips `cur` (no copy)
 //   Y[2][h,u,v]  ping-pong stage inputs Y_1..Y_{N-1}
-//   z            bed elevation (its slopes are recomputed in-kernel from the tile)
+//   z, zx, zy    bed elevation and its slopes (computed when the bed is set)
 //   K[s][h,u,v]  stored stage derivatives, only for non-diagonal tableaux
 //   optional per-cell Manning n / depths, rain q0/q1 or pattern, head targets
 //   ctl, forcing  small device structs (controller state, per-step boundary values)
-//   part         per-CTA FP64 partials of the CFL max/min, volume and tallies
+//   part         per-strip or per-CTA FP64 partials of the CFL max/min, volume and tallies
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -347,7 +347,9 @@ struct Solver final : public sv_ctx {
     SV_CUDA(alloc(&ctl, 1));
     SV_CUDA(alloc(&dbg_ctl, 1));
     SV_CUDA(alloc(&fc, 1));
-    long long maxp = vol_nblk;
+    // the shortest strips (4 rows: variant 5 or a batch member on a small mesh) make the most slots
+    // of a sweep; kTileRows rows and more make fewer
+    long long maxp = std::max(vol_nblk, svk::strip_count((long long)m->nx, (long long)m->ny, 4));
     for (int v = 0; v < svk::kNumVariants; ++v) maxp = std::max(maxp, svk::variant_partials(v, m->nx, m->ny));
     SV_CUDA(alloc(&part, size_t(svk::part_count(maxp))));
     SV_CUDA(alloc(&scalar, 4));
@@ -676,6 +678,7 @@ struct Solver final : public sv_ctx {
     P.cell_area = mesh.dx * mesh.dy;
     P.mc.set(mesh.dx, mesh.dy);
     P.exact = svk::exact_mesh(mesh.dx, mesh.dy, sizeof(T) == 8);
+    P.p2 = svk::pow2_mesh(mesh.dx, mesh.dy);
     for (int b = 0; b < 2; ++b)
       for (int f = 0; f < 3; ++f) P.S[b][f] = S[b][f];
     P.z = z;
@@ -1094,7 +1097,8 @@ struct Batch final : public sv_batch_base {
   svk::StepQueue* d_queue = nullptr;        // [nact] steps queued by the current advance
   int nact = 0, cap = 0;
   long long max_nblk = 0;  // partial slots of the largest member
-  bool p2 = true, extra = false, dirty = true;
+  int p2 = svk::kP2None;  // of the members' cell sizes
+  bool extra = false, dirty = true;
   std::vector<svk::StageParams<T>> params;  // [nact], as on the device
   std::vector<int> active;                  // slot ids in launch order
   std::vector<unsigned long long> versions; // members' pversion at the last rebuild
@@ -1226,7 +1230,7 @@ struct Batch final : public sv_batch_base {
     std::vector<svk::FinalizeParams> hf(std::max(nact, 1));
     std::vector<long long> ht(nact + 1, 0);
     std::vector<Ctl*> hc(std::max(nact, 1));
-    p2 = true;
+    int n_p2 = 0;
     extra = false;
     max_nblk = 0;
     // One strip height for all members: the tallest that gives the GPU two rounds of warps. Twice
@@ -1248,8 +1252,7 @@ struct Batch final : public sv_batch_base {
       if (rs) return fail(rs, "member " + std::to_string(active[k]) + ": " + m->err);
       ht[k + 1] = ht[k] + m->nblk;
       max_nblk = std::max(max_nblk, m->nblk);
-      int e2;
-      p2 = p2 && std::frexp(m->mesh.dx, &e2) == 0.5 && std::frexp(m->mesh.dy, &e2) == 0.5;
+      n_p2 += svk::pow2_mesh(m->mesh.dx, m->mesh.dy);
       extra = extra || m->extra();
       params[k] = m->stage_params();
       hf[k] = m->finalize_params(true);
@@ -1257,6 +1260,7 @@ struct Batch final : public sv_batch_base {
       hf[k].fc = m->fc;
       hc[k] = m->ctl;
     }
+    p2 = n_p2 == nact ? svk::kP2All : (n_p2 > 0 && sizeof(T) == 4 ? svk::kP2Some : svk::kP2None);
     versions.assign(nact, 0);
     for (int k = 0; k < nact; ++k) versions[k] = members[active[k]]->pversion;
     if (nact > 0) {

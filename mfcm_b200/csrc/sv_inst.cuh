@@ -47,12 +47,6 @@ static cudaError_t launch_chained(dim3 grid, dim3 block, int smem, cudaStream_t 
   return cudaLaunchKernelEx(&cfg, KERNEL, args...);
 }
 
-// dx and dy both powers of two: the mesh divisions are exact multiplies
-inline bool pow2_mesh(double dx, double dy) {
-  int e;
-  return std::frexp(dx, &e) == 0.5 && std::frexp(dy, &e) == 0.5;
-}
-
 template <typename T, int TX, int TY, int MINB, bool P2, bool EDDY, bool PRE = false>
 static cudaError_t launch_stage_p(const StageParams<T>& P, int st, cudaStream_t s) {
   using SM = StageSmem<T, TX, TY>;
@@ -177,9 +171,19 @@ template <> cudaError_t launch_to_f64<SV_T>(const SV_T* src, double* dst, long l
   return cudaGetLastError();
 }
 
-template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, int n, int st, bool p2, bool extra,
+// kernels of a batch by the members' cell sizes (kP2Some: FP32 only)
+template <bool EXTRA> static cudaError_t launch_batch_chunk(const BatchParams<SV_T>& B, int st, int p2, cudaStream_t s) {
+  constexpr int CAP = EXTRA ? kExtraCap<SV_T> : kBatchCap<SV_T>;
+  const dim3 block(32, kSweepWarps), grid(unsigned(B.first_block[B.n]));
+  if (grid.x == 0) return cudaSuccess;
+  if (p2 == kP2All) return launch_chained<sweep_batch_kernel<SV_T, CAP, kP2All, EXTRA>>(grid, block, kRingBytes, s, B, st);
+  if constexpr (sizeof(SV_T) == 4)
+    if (p2 == kP2Some)
+      return launch_chained<sweep_batch_kernel<SV_T, CAP, kP2Some, EXTRA>>(grid, block, kRingBytes, s, B, st);
+  return launch_chained<sweep_batch_kernel<SV_T, CAP, kP2None, EXTRA>>(grid, block, kRingBytes, s, B, st);
+}
+template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, int n, int st, int p2, bool extra,
                                                  cudaStream_t s) {
-  constexpr int CAP = kBatchCap<SV_T>, XCAP = kExtraCap<SV_T>;
   for (int k0 = 0; k0 < n; k0 += kBatchMembers) {
     BatchParams<SV_T> B;
     B.n = std::min(n - k0, kBatchMembers);
@@ -188,15 +192,7 @@ template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, in
       B.m[k] = Ps[k0 + k];
       B.first_block[k + 1] = B.first_block[k] + (B.m[k].n_strips + kSweepWarps - 1) / kSweepWarps;
     }
-    const dim3 block(32, kSweepWarps), grid(unsigned(B.first_block[B.n]));
-    if (grid.x == 0) continue;
-    cudaError_t e;
-    if (extra)
-      e = p2 ? launch_chained<sweep_batch_kernel<SV_T, XCAP, true, true>>(grid, block, kRingBytes, s, B, st)
-                    : launch_chained<sweep_batch_kernel<SV_T, XCAP, false, true>>(grid, block, kRingBytes, s, B, st);
-    else
-      e = p2 ? launch_chained<sweep_batch_kernel<SV_T, CAP, true, false>>(grid, block, kRingBytes, s, B, st)
-                    : launch_chained<sweep_batch_kernel<SV_T, CAP, false, false>>(grid, block, kRingBytes, s, B, st);
+    const cudaError_t e = extra ? launch_batch_chunk<true>(B, st, p2, s) : launch_batch_chunk<false>(B, st, p2, s);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -206,12 +202,17 @@ template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, in
 // device at once (every block resident, so warps that wait for another warp's work always
 // see it done).
 template <int BANK>
-static cudaError_t launch_persist_t(const PersistParams<SV_T>& PP, const StageParams<SV_T>* Ps, bool p2, bool extra,
+static cudaError_t launch_persist_t(const PersistParams<SV_T>& PP, const StageParams<SV_T>* Ps, int p2, bool extra,
                                     cudaStream_t s) {
   constexpr int CAP = kBatchCap<SV_T>, XCAP = kExtraCap<SV_T>;
   void (*kern)(const PersistParams<SV_T>, const MemberBank<SV_T, BANK>) =
-      extra ? (p2 ? persist_batch_kernel<SV_T, XCAP, true, true, BANK> : persist_batch_kernel<SV_T, XCAP, false, true, BANK>)
-            : (p2 ? persist_batch_kernel<SV_T, CAP, true, false, BANK> : persist_batch_kernel<SV_T, CAP, false, false, BANK>);
+      extra ? persist_batch_kernel<SV_T, XCAP, kP2None, true, BANK> : persist_batch_kernel<SV_T, CAP, kP2None, false, BANK>;
+  if (p2 == kP2All)
+    kern = extra ? persist_batch_kernel<SV_T, XCAP, kP2All, true, BANK> : persist_batch_kernel<SV_T, CAP, kP2All, false, BANK>;
+  if constexpr (sizeof(SV_T) == 4)
+    if (p2 == kP2Some)
+      kern = extra ? persist_batch_kernel<SV_T, XCAP, kP2Some, true, BANK>
+                   : persist_batch_kernel<SV_T, CAP, kP2Some, false, BANK>;
   int dev = 0, nsm = 0, per_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess && kRingBytes > 48 * 1024)
@@ -228,7 +229,7 @@ static cudaError_t launch_persist_t(const PersistParams<SV_T>& PP, const StagePa
   return cudaLaunchCooperativeKernel((const void*)kern, dim3(unsigned(per_sm * nsm)), dim3(32, kPersistWarps), args,
                                      kRingBytes, s);
 }
-template <> cudaError_t launch_persist<SV_T>(const PersistParams<SV_T>& PP, const StageParams<SV_T>* Ps, bool p2,
+template <> cudaError_t launch_persist<SV_T>(const PersistParams<SV_T>& PP, const StageParams<SV_T>* Ps, int p2,
                                              bool extra, cudaStream_t s) {
   if (PP.nact <= kBatchMembers) return launch_persist_t<kBatchMembers>(PP, Ps, p2, extra, s);
   return launch_persist_t<1>(PP, Ps, p2, extra, s);

@@ -1,15 +1,18 @@
 // sv_kernels.cuh -- kernels of the Saint-Venant RK time step on sm_100a.
 //
+//  column sweeps  (sv_sweep.cuh) one launch per RK stage, the form that every caller gets unless
+//                 it asks for another variant: warps march strips of 28 columns; slopes and fluxes
+//                 stay in registers.
 //  stage_kernel   one launch per RK stage. A CTA owns a TX x TY tile of cells, stages the
 //                 tile plus a 2-cell halo of (h, u, v, z) in shared memory, computes the
 //                 Minmod3 slopes of every cell of the tile plus a 1-cell ring, the fluxes of
 //                 every face of the tile, then per cell dU/dt (flux divergence, depth-slope,
 //                 limited bed slope, zflux), Manning friction, rainfall and outflow, and the
-//                 Runge-Kutta combination. Faces and slopes never leave the SM. The last
-//                 stage also reduces the CFL quantity and the FP64 volume per CTA.
-//  finalize_kernel  one CTA: fixed-order reduction of the per-CTA partials, the control
-//                 number, and the dt controller (accept / repeat / new dt / end-of-step
-//                 trimming) in FP64, so a whole step runs without a host round trip.
+//                 Runge-Kutta combination. Faces and slopes never leave the SM.
+//                 The last stage of either also reduces the CFL quantity and the FP64 volume.
+//  finalize_kernel  fixed-order reduction of the partials, the control number, and the dt
+//                 controller (accept / repeat / new dt / end-of-step trimming) in FP64, so a
+//                 whole step runs without a host round trip.
 //  debug kernels  the same per-face / per-cell functions over global arrays, one reference
 //                 kernel each, for per-function parity tests.
 #pragma once
@@ -130,6 +133,7 @@ template <typename T> struct StageParams {
   const unsigned* strips;
   int n_strips, rows;
   int exact;  // the cell sizes allow sweep_rows (exact_mesh)
+  int p2;     // dx and dy are powers of two (pow2_mesh)
   // split schedule: the stage input's slopes dh/dx, du/dx, dv/dx, dh/dy, du/dy, dv/dy as
   // written by slopes_kernel (read by the stage kernel instead of computing them), or null
   T* pslp[6];
@@ -255,7 +259,7 @@ template <> struct MkDivX<DivF> { __device__ static DivF make(double d) { return
 // fluxes; returns the rain rate added, the depth rate removed by the head assignment and the
 // depth rate that entered through mesh-edge faces (the reference's walls pass flow through
 // their one-sided branches; taken before any boundary assignment).
-template <typename T, typename CC, bool EDDY = false, bool EDGE = true>
+template <typename T, typename CC, bool EDDY = false>
 __device__ __forceinline__ void cell_dudt(const StageParams<T>& P, const DevForcing& fc, const CC& c,
                                           long long g, int gx,
                                           int gy, T h, T u, T v, T dhdx, T dhdy, T dzdx, T dzdy,
@@ -328,23 +332,19 @@ __device__ __forceinline__ void cell_dudt(const StageParams<T>& P, const DevForc
   rain = 0.0;
   removed = 0.0;
   wall = 0.0;
-  if constexpr (EDGE) {  // cells away from the mesh edge have no wall faces
-    if (gx == 0) wall += double(c.divx(fw.h));
-    if (gx == P.nx - 1) wall -= double(c.divx(fe.h));
-    if (gy == 0) wall += double(c.divy(fs.h));
-    if (gy == P.ny - 1) wall -= double(c.divy(fn.h));
-  }
+  if (gx == 0) wall += double(c.divx(fw.h));
+  if (gx == P.nx - 1) wall -= double(c.divx(fe.h));
+  if (gy == 0) wall += double(c.divy(fs.h));
+  if (gy == P.ny - 1) wall -= double(c.divy(fn.h));
   // head boundary target values for this cell (NaN = not selected); a stage boundary
   // (StageBoundarySourceTerm.cpp:48-52) gives water levels, from which the bed is subtracted
   bool head_sel = false;
   T h0 = T(0), h1 = T(0);
   const int hk = fc.head_kind;
   if (hk == 1 || hk == 3) {
-    if constexpr (EDGE) {  // edge strips: never a cell away from the mesh edge
-      head_sel = ((fc.head_edges & 1u) && gx == 0) || ((fc.head_edges & 2u) && gx == P.nx - 1) ||
-                 ((fc.head_edges & 4u) && gy == 0) || ((fc.head_edges & 8u) && gy == P.ny - 1);
-      h0 = T(fc.hh0); h1 = T(fc.hh1);
-    }
+    head_sel = ((fc.head_edges & 1u) && gx == 0) || ((fc.head_edges & 2u) && gx == P.nx - 1) ||
+               ((fc.head_edges & 4u) && gy == 0) || ((fc.head_edges & 8u) && gy == P.ny - 1);
+    h0 = T(fc.hh0); h1 = T(fc.hh1);
   } else if (hk == 2 || hk == 4) {
     h0 = ld(P.hb0p, g); h1 = ld(P.hb1p, g);
     head_sel = true;
@@ -383,7 +383,7 @@ __device__ __forceinline__ void cell_dudt(const StageParams<T>& P, const DevForc
 
 // One cell of one stage after its four face fluxes are known: dU/dt, then the Runge-Kutta
 // combination (RungeKutta.hpp:377-388) and, on the last stage, the CFL quantity and volume.
-template <typename T, typename CC, bool EDDY = false, bool EDGE = true, bool COH = false>
+template <typename T, typename CC, bool EDDY = false, bool COH = false>
 __device__ __forceinline__ void finish_cell(const StageParams<T>& P, int st, const DevForcing& fc, const CC& c,
                                             long long g, int gx, int gy, T h, T u, T v, T dhdx, T dhdy, T dzdx,
                                             T dzdy, const FaceF<T>& fw, const FaceF<T>& fe, const FaceF<T>& fs,
@@ -391,7 +391,7 @@ __device__ __forceinline__ void finish_cell(const StageParams<T>& P, int st, con
                                             double& removed, double& walls, T& xcfl, T& xcfl_min, double& vol, const EddyIn<T>* ed = nullptr) {
   T kh, ku, kv;
   double r_, o_, w_;
-  cell_dudt<T, CC, EDDY, EDGE>(P, fc, c, g, gx, gy, h, u, v, dhdx, dhdy, dzdx, dzdy, fw, fe, fs, fn, kh, ku, kv, r_,
+  cell_dudt<T, CC, EDDY>(P, fc, c, g, gx, gy, h, u, v, dhdx, dhdy, dzdx, dzdy, fw, fe, fs, fn, kh, ku, kv, r_,
                                o_, w_, (T*)nullptr, (T*)nullptr, ed);
   rain += r_;
   removed += o_;
@@ -1083,7 +1083,7 @@ __device__ __forceinline__ void finalize_warp(const FinalizeParams& F) {
 // warps copy an item's parameters to shared memory.
 template <typename T, int BANK> struct MemberBank { StageParams<T> m[BANK]; };
 
-template <typename T, int MINB, bool P2, bool EXTRA, int BANK>
+template <typename T, int MINB, int P2, bool EXTRA, int BANK>
 __global__ void __launch_bounds__(32 * kPersistWarps, MINB)
     persist_batch_kernel(const __grid_constant__ PersistParams<T> PP, const __grid_constant__ MemberBank<T, BANK> bank) {
   __shared__ __align__(16) StageParams<T> Psh[BANK > 1 ? 1 : kPersistWarps];
@@ -1162,7 +1162,7 @@ __global__ void __launch_bounds__(32 * kPersistWarps, MINB)
       const int pk = uniform(pick), st = uniform(s);
       if constexpr (BANK > 1) {
         const StageParams<T>& SP = bank.m[pk];
-        sweep_strip<T, P2, EXTRA, false, true>(SP, st, SP.strips[item], sm);
+        member_strip<T, P2, EXTRA, false, true>(SP, st, SP.strips[item], sm);
       } else {
         static_assert(sizeof(StageParams<T>) % 4 == 0, "parameter block copied as 32-bit words");
         const unsigned* src = reinterpret_cast<const unsigned*>(PP.Ps + pk);
@@ -1170,7 +1170,7 @@ __global__ void __launch_bounds__(32 * kPersistWarps, MINB)
         for (int i = lane; i < int(sizeof(StageParams<T>) / 4); i += 32) dst[i] = src[i];
         __syncwarp();
         const StageParams<T>& SP = Psh[wib];
-        sweep_strip<T, P2, EXTRA, false, true>(SP, st, SP.strips[item], sm);
+        member_strip<T, P2, EXTRA, false, true>(SP, st, SP.strips[item], sm);
       }
       __syncwarp();
     } else {

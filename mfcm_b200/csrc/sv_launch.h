@@ -4,6 +4,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 #include "sv_kernels.cuh"
 
 namespace svk {
@@ -19,23 +21,28 @@ template <typename T> cudaError_t launch_stage(const StageParams<T>& P, int st, 
 
 // Stage-kernel variants, in two schedules:
 //  fused (one pass per RK stage): 0..3 the tiled shared-memory kernel with kTiles[v]; 4..10 and
-//   12..17 the column sweep with the strip heights and register caps (resident 4-warp blocks per
-//   SM) of kSweeps; variant 5 takes both from the mesh size;
+//   12..15 the column sweep with the strip heights and register caps (resident 4-warp blocks per
+//   SM) of kSweeps (12..15 FP32 only); variant 5 takes both from the mesh size;
 //  split (two passes per RK stage): 11 the slopes pass (slopes_kernel) then the tiled 32 x 8
 //   kernel at 3 CTAs/SM reading those slopes.
-constexpr int kNumVariants = 18;
+constexpr int kNumVariants = 16;
 constexpr int kSplitVariant = 11;
 constexpr int kAutoVariant = 5;
 struct SweepShape { int rows, cap; };
 constexpr SweepShape kSweeps[kNumVariants] = {{0, 0},  {0, 0},  {0, 0},  {0, 0},  {16, 4}, {32, 4},
                                               {64, 4}, {32, 3}, {32, 4}, {32, 5}, {32, 6}, {0, 0},
-                                              {32, 3}, {32, 4}, {32, 7}, {32, 8}, {8, 4}, {4, 4}};
+                                              {32, 3}, {32, 4}, {32, 7}, {32, 8}};
 // the row-tile kernel (tile_rows_kernel): what variant 5 runs on small meshes
 constexpr int kTileRowsVariant = kNumVariants;
 // cell sizes within which the sweeps' FP64 quotients stay in the range of the exact division
 inline bool exact_mesh(double dx, double dy, bool fp64) {
   auto fits = [](double d) { return d >= 0x1p-30 && d <= 0x1p40; };
   return !fp64 || (fits(dx) && fits(dy));
+}
+// dx and dy both powers of two: the mesh divisions are exact multiplies
+inline bool pow2_mesh(double dx, double dy) {
+  int e;
+  return std::frexp(dx, &e) == 0.5 && std::frexp(dy, &e) == 0.5;
 }
 // resident blocks per SM of the batch kernels, and of the sweeps with every source term
 template <typename T> constexpr int kBatchCap = sizeof(T) == 8 ? 4 : 6;
@@ -122,13 +129,13 @@ template <typename T> cudaError_t launch_volume(const T* h, int nx, int ny, doub
 template <typename T> cudaError_t launch_debug(const StageParams<T>& P, const DebugParams<T>& D, T* nh, T* sf,
                                                cudaStream_t s);
 // stage `st` of every one of n solvers (host array Ps) in one launch per kBatchMembers of them;
-// p2 when every solver's dx and dy are powers of two, extra when any solver needs it
+// p2: kP2None, kP2All or kP2Some, extra when any solver needs it
 constexpr int kBatchVariant = 8;
-template <typename T> cudaError_t launch_sweep_batch(const StageParams<T>* Ps, int n, int st, bool p2, bool extra,
+template <typename T> cudaError_t launch_sweep_batch(const StageParams<T>* Ps, int n, int st, int p2, bool extra,
                                                      cudaStream_t s);
 // persistent batch kernel (persist_batch_kernel), cooperative launch filling the device; Ps: the
 // members' parameters on the host (PP.Ps: the same on the device)
-template <typename T> cudaError_t launch_persist(const PersistParams<T>& PP, const StageParams<T>* Ps, bool p2,
+template <typename T> cudaError_t launch_persist(const PersistParams<T>& PP, const StageParams<T>* Ps, int p2,
                                                  bool extra, cudaStream_t s);
 cudaError_t launch_persist_init(const FinalizeParams* Fs, PersistMember* mem, const long long* warp_start, int nact,
                                 cudaStream_t s);

@@ -178,6 +178,7 @@ extern "C" int sv_timestep_noalloc(const sv_mesh_desc* mesh, const sv_params* pa
   P.cell_area = dx * dy;
   P.mc.set(dx, dy);
   P.exact = svk::exact_mesh(dx, dy, true);
+  P.p2 = svk::pow2_mesh(dx, dy);
   // U_[0] is read from the inputs (cur = 0); the accumulator and U_[N] go to the outputs
   P.S[0][0] = const_cast<double*>(h); P.S[0][1] = const_cast<double*>(u); P.S[0][2] = const_cast<double*>(v);
   P.S[1][0] = h_out; P.S[1][1] = u_out; P.S[1][2] = v_out;

@@ -293,7 +293,7 @@ __device__ __noinline__ void sweep_rows_general(const StageParams<T>& P, int st,
       const FaceF<T> FE{dn1(FW.h), dn1(FW.u), dn1(FW.v), dn1(FW.z)};
       if (out_lane && r < ny) {
         const long long g = (long long)r * nx + gx;
-        finish_cell<T, CellCtx<T, DX>, EDDY, true, COH>(P, st, fc, c, g, gx, r, me.h, me.u, me.v, me.dhdx, me.dhdy,
+        finish_cell<T, CellCtx<T, DX>, EDDY, COH>(P, st, fc, c, g, gx, r, me.h, me.u, me.v, me.dhdx, me.dhdy,
                                                         me.dzdx, me.dzdy, FW, FE, FS, FN, cur, dt_d,
                                                         acc.rain, acc.removed, acc.walls, acc.xmax, acc.xmin, acc.vol,
                                                         &ed);
@@ -1064,6 +1064,11 @@ __device__ __forceinline__ void store_strip_sums(const StageParams<T>& P, int st
   }
 }
 
+// The members of a batch: none (0), all (1) or some (2) have cell sizes that are powers of two.
+// FP32 rounds differently in the two forms, so a member keeps the form of its solo run; in FP64
+// both give the same bits and 2 is not compiled.
+inline constexpr int kP2None = 0, kP2All = 1, kP2Some = 2;
+
 // One strip of one solver's stage: its class's sweep, then its partial sums. `entry` is the
 // strip's index (row-major over strips of kSweepOut columns x P.rows rows) times 4 plus its
 // class. SPLIT: interior strips run the form without edge tests.
@@ -1085,6 +1090,17 @@ __device__ __forceinline__ void sweep_strip(const StageParams<T>& P, int st, uns
     acc = rest;
   }
   store_strip_sums(P, st, gw, acc);
+}
+// sweep_strip of a batch member
+template <typename T, int P2, bool EXTRA, bool SPLIT, bool COH>
+__device__ __forceinline__ void member_strip(const StageParams<T>& P, int st, unsigned entry, SweepShared<T>& sm) {
+  if constexpr (P2 != kP2None) {
+    if (P2 == kP2All || P.p2) {
+      sweep_strip<T, true, EXTRA, SPLIT, COH>(P, st, entry, sm);
+      return;
+    }
+  }
+  if constexpr (P2 != kP2All) sweep_strip<T, false, EXTRA, SPLIT, COH>(P, st, entry, sm);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1305,7 +1321,7 @@ template <typename T> struct BatchParams {
 };
 static_assert(sizeof(BatchParams<double>) <= 32764 && sizeof(BatchParams<float>) <= 32764, "kernel parameters");
 
-template <typename T, int MINB, bool P2, bool EXTRA>
+template <typename T, int MINB, int P2, bool EXTRA>
 __global__ void __launch_bounds__(32 * kSweepWarps, MINB)
     sweep_batch_kernel(const __grid_constant__ BatchParams<T> B, const int st) {
   extern __shared__ __align__(16) unsigned char sweep_smem[];
@@ -1317,7 +1333,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, MINB)
   if (P.ctl->done) return;
   const int w = uniform(threadIdx.y), i = (int(blockIdx.x) - B.first_block[k]) * kSweepWarps + w;
   if (i >= P.n_strips) return;
-  sweep_strip<T, P2, EXTRA, !EXTRA, false>(P, st, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[w]);
+  member_strip<T, P2, EXTRA, !EXTRA, false>(P, st, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[w]);
 }
 
 }  // namespace svk
