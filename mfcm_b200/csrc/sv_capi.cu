@@ -198,10 +198,12 @@ struct Solver final : public sv_ctx {
   std::map<int, Strips> strips_;
   unsigned char* d_scls = nullptr;
   size_t scls_size = 0;
+  int mesh_rows[2] = {4, 4};  // variant 5's strip heights: lean sweep, every source term
   int batch_rows = 0;  // a batch member's strip height, chosen by its batch (0: none)
   int sweep_rows(int v) const {
-    return v == svk::kBatchVariant && batch_rows ? batch_rows
-                                                 : svk::variant_sweep_rows(v, (long long)mesh.nx, (long long)mesh.ny);
+    if (v == svk::kAutoVariant) return mesh_rows[extra()];
+    if (v == svk::kBatchVariant && batch_rows) return batch_rows;
+    return svk::variant_is_sweep(v) ? svk::kSweeps[v].rows : 0;
   }
   // the kernel that variant v launches: variant 5 is the row-tile kernel on small meshes without
   // further terms
@@ -214,7 +216,7 @@ struct Solver final : public sv_ctx {
   long long partials(int v) const {
     const int rows = kernel_of(v) == svk::kTileRowsVariant ? svk::kTileRows : sweep_rows(v);
     return rows ? svk::strip_count((long long)mesh.nx, (long long)mesh.ny, rows)
-                : svk::variant_partials(v, (long long)mesh.nx, (long long)mesh.ny);
+                : svk::tiled_partials(v, (long long)mesh.nx, (long long)mesh.ny);
   }
   void set_batch_rows(int rows) {
     if (rows == batch_rows) return;
@@ -316,7 +318,8 @@ struct Solver final : public sv_ctx {
     nfaces = (long long)(m->nx + 1) * (long long)m->ny + (long long)(m->ny + 1) * (long long)m->nx;
     tx = svk::kTiles[tile].tx;
     ty = svk::kTiles[tile].ty;
-    nblk = svk::variant_partials(variant, (long long)m->nx, (long long)m->ny);
+    for (int e = 0; e < 2; ++e) mesh_rows[e] = svk::auto_rows<T>((long long)m->nx, (long long)m->ny, e);
+    nblk = partials(variant);
     vol_nblk = (long long)((m->nx + tx - 1) / tx) * (long long)((m->ny + ty - 1) / ty);
     SV_CUDA(cudaSetDevice(dev));
     SV_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
@@ -347,10 +350,10 @@ struct Solver final : public sv_ctx {
     SV_CUDA(alloc(&ctl, 1));
     SV_CUDA(alloc(&dbg_ctl, 1));
     SV_CUDA(alloc(&fc, 1));
-    // the shortest strips (4 rows: variant 5 or a batch member on a small mesh) make the most slots
-    // of a sweep; kTileRows rows and more make fewer
-    long long maxp = std::max(vol_nblk, svk::strip_count((long long)m->nx, (long long)m->ny, 4));
-    for (int v = 0; v < svk::kNumVariants; ++v) maxp = std::max(maxp, svk::variant_partials(v, m->nx, m->ny));
+    // the shortest strips (4 rows: variant 5 or a batch member on a small mesh) and the smallest
+    // tile (variant 2) make the most slots
+    const long long maxp = std::max({vol_nblk, svk::strip_count((long long)m->nx, (long long)m->ny, 4),
+                                     svk::tiled_partials(2, (long long)m->nx, (long long)m->ny)});
     SV_CUDA(alloc(&part, size_t(svk::part_count(maxp))));
     SV_CUDA(alloc(&scalar, 4));
     Ctl c{};
@@ -1097,8 +1100,7 @@ struct Batch final : public sv_batch_base {
   svk::StepQueue* d_queue = nullptr;        // [nact] steps queued by the current advance
   int nact = 0, cap = 0;
   long long max_nblk = 0;  // partial slots of the largest member
-  int p2 = svk::kP2None;  // of the members' cell sizes
-  bool extra = false, dirty = true;
+  bool p2 = true, extra = false, dirty = true;
   std::vector<svk::StageParams<T>> params;  // [nact], as on the device
   std::vector<int> active;                  // slot ids in launch order
   std::vector<unsigned long long> versions; // members' pversion at the last rebuild
@@ -1230,7 +1232,7 @@ struct Batch final : public sv_batch_base {
     std::vector<svk::FinalizeParams> hf(std::max(nact, 1));
     std::vector<long long> ht(nact + 1, 0);
     std::vector<Ctl*> hc(std::max(nact, 1));
-    int n_p2 = 0;
+    p2 = true;
     extra = false;
     max_nblk = 0;
     // One strip height for all members: the tallest that gives the GPU two rounds of warps. Twice
@@ -1252,7 +1254,7 @@ struct Batch final : public sv_batch_base {
       if (rs) return fail(rs, "member " + std::to_string(active[k]) + ": " + m->err);
       ht[k + 1] = ht[k] + m->nblk;
       max_nblk = std::max(max_nblk, m->nblk);
-      n_p2 += svk::pow2_mesh(m->mesh.dx, m->mesh.dy);
+      p2 = p2 && svk::pow2_mesh(m->mesh.dx, m->mesh.dy);
       extra = extra || m->extra();
       params[k] = m->stage_params();
       hf[k] = m->finalize_params(true);
@@ -1260,7 +1262,6 @@ struct Batch final : public sv_batch_base {
       hf[k].fc = m->fc;
       hc[k] = m->ctl;
     }
-    p2 = n_p2 == nact ? svk::kP2All : (n_p2 > 0 && sizeof(T) == 4 ? svk::kP2Some : svk::kP2None);
     versions.assign(nact, 0);
     for (int k = 0; k < nact; ++k) versions[k] = members[active[k]]->pversion;
     if (nact > 0) {

@@ -102,17 +102,19 @@ constexpr int kRingBytes = kSweepWarps * int(sizeof(SweepShared<SV_T>));
 
 // The column sweep of a stage: the strips in P.strips, P.rows rows each. `cap`: resident blocks
 // per SM asked of the register allocator.
-template <int MINB, bool EXTRA> static cudaError_t launch_sweep_c(const StageParams<SV_T>& P, int st, cudaStream_t s) {
+template <int MINB, bool EXTRA, bool SPLIT = !EXTRA>
+static cudaError_t launch_sweep_c(const StageParams<SV_T>& P, int st, cudaStream_t s) {
   if (P.n_strips <= 0) return cudaSuccess;
   const dim3 grid(unsigned((P.n_strips + kSweepWarps - 1) / kSweepWarps)), block(32, kSweepWarps);
   if (pow2_mesh(P.dx, P.dy))
-    return launch_chained<sweep_kernel<SV_T, MINB, true, EXTRA>>(grid, block, kRingBytes, s, P, st);
-  return launch_chained<sweep_kernel<SV_T, MINB, false, EXTRA>>(grid, block, kRingBytes, s, P, st);
+    return launch_chained<sweep_kernel<SV_T, MINB, true, EXTRA, SPLIT>>(grid, block, kRingBytes, s, P, st);
+  return launch_chained<sweep_kernel<SV_T, MINB, false, EXTRA, SPLIT>>(grid, block, kRingBytes, s, P, st);
 }
 static cudaError_t launch_sweep(const StageParams<SV_T>& P, int st, int cap, bool extra, cudaStream_t s) {
   if (extra) return launch_sweep_c<kExtraCap<SV_T>, true>(P, st, s);
   if constexpr (sizeof(SV_T) == 8) {
-    return cap == 3 ? launch_sweep_c<3, false>(P, st, s) : launch_sweep_c<4, false>(P, st, s);
+    if (cap == 3) return launch_sweep_c<3, false>(P, st, s);
+    return splits_forms(P.n_strips) ? launch_sweep_c<4, false>(P, st, s) : launch_sweep_c<4, false, false>(P, st, s);
   } else {
     switch (cap) {
       case 4: return launch_sweep_c<4, false>(P, st, s);
@@ -171,18 +173,14 @@ template <> cudaError_t launch_to_f64<SV_T>(const SV_T* src, double* dst, long l
   return cudaGetLastError();
 }
 
-// kernels of a batch by the members' cell sizes (kP2Some: FP32 only)
-template <bool EXTRA> static cudaError_t launch_batch_chunk(const BatchParams<SV_T>& B, int st, int p2, cudaStream_t s) {
+template <bool EXTRA> static cudaError_t launch_batch_chunk(const BatchParams<SV_T>& B, int st, bool p2, cudaStream_t s) {
   constexpr int CAP = EXTRA ? kExtraCap<SV_T> : kBatchCap<SV_T>;
   const dim3 block(32, kSweepWarps), grid(unsigned(B.first_block[B.n]));
   if (grid.x == 0) return cudaSuccess;
-  if (p2 == kP2All) return launch_chained<sweep_batch_kernel<SV_T, CAP, kP2All, EXTRA>>(grid, block, kRingBytes, s, B, st);
-  if constexpr (sizeof(SV_T) == 4)
-    if (p2 == kP2Some)
-      return launch_chained<sweep_batch_kernel<SV_T, CAP, kP2Some, EXTRA>>(grid, block, kRingBytes, s, B, st);
-  return launch_chained<sweep_batch_kernel<SV_T, CAP, kP2None, EXTRA>>(grid, block, kRingBytes, s, B, st);
+  if (p2) return launch_chained<sweep_batch_kernel<SV_T, CAP, true, EXTRA>>(grid, block, kRingBytes, s, B, st);
+  return launch_chained<sweep_batch_kernel<SV_T, CAP, false, EXTRA>>(grid, block, kRingBytes, s, B, st);
 }
-template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, int n, int st, int p2, bool extra,
+template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, int n, int st, bool p2, bool extra,
                                                  cudaStream_t s) {
   for (int k0 = 0; k0 < n; k0 += kBatchMembers) {
     BatchParams<SV_T> B;
@@ -202,17 +200,12 @@ template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, in
 // device at once (every block resident, so warps that wait for another warp's work always
 // see it done).
 template <int BANK>
-static cudaError_t launch_persist_t(const PersistParams<SV_T>& PP, const StageParams<SV_T>* Ps, int p2, bool extra,
+static cudaError_t launch_persist_t(const PersistParams<SV_T>& PP, const StageParams<SV_T>* Ps, bool p2, bool extra,
                                     cudaStream_t s) {
   constexpr int CAP = kBatchCap<SV_T>, XCAP = kExtraCap<SV_T>;
   void (*kern)(const PersistParams<SV_T>, const MemberBank<SV_T, BANK>) =
-      extra ? persist_batch_kernel<SV_T, XCAP, kP2None, true, BANK> : persist_batch_kernel<SV_T, CAP, kP2None, false, BANK>;
-  if (p2 == kP2All)
-    kern = extra ? persist_batch_kernel<SV_T, XCAP, kP2All, true, BANK> : persist_batch_kernel<SV_T, CAP, kP2All, false, BANK>;
-  if constexpr (sizeof(SV_T) == 4)
-    if (p2 == kP2Some)
-      kern = extra ? persist_batch_kernel<SV_T, XCAP, kP2Some, true, BANK>
-                   : persist_batch_kernel<SV_T, CAP, kP2Some, false, BANK>;
+      extra ? (p2 ? persist_batch_kernel<SV_T, XCAP, true, true, BANK> : persist_batch_kernel<SV_T, XCAP, false, true, BANK>)
+            : (p2 ? persist_batch_kernel<SV_T, CAP, true, false, BANK> : persist_batch_kernel<SV_T, CAP, false, false, BANK>);
   int dev = 0, nsm = 0, per_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess && kRingBytes > 48 * 1024)
@@ -229,7 +222,7 @@ static cudaError_t launch_persist_t(const PersistParams<SV_T>& PP, const StagePa
   return cudaLaunchCooperativeKernel((const void*)kern, dim3(unsigned(per_sm * nsm)), dim3(32, kPersistWarps), args,
                                      kRingBytes, s);
 }
-template <> cudaError_t launch_persist<SV_T>(const PersistParams<SV_T>& PP, const StageParams<SV_T>* Ps, int p2,
+template <> cudaError_t launch_persist<SV_T>(const PersistParams<SV_T>& PP, const StageParams<SV_T>* Ps, bool p2,
                                              bool extra, cudaStream_t s) {
   if (PP.nact <= kBatchMembers) return launch_persist_t<kBatchMembers>(PP, Ps, p2, extra, s);
   return launch_persist_t<1>(PP, Ps, p2, extra, s);

@@ -133,7 +133,7 @@ template <typename T> struct StageParams {
   const unsigned* strips;
   int n_strips, rows;
   int exact;  // the cell sizes allow sweep_rows (exact_mesh)
-  int p2;     // dx and dy are powers of two (pow2_mesh)
+  int p2;     // dx and dy are powers of two (pow2_mesh): chooses the rounding in FP32 (MeshOps)
   // split schedule: the stage input's slopes dh/dx, du/dx, dv/dx, dh/dy, du/dy, dv/dy as
   // written by slopes_kernel (read by the stage kernel instead of computing them), or null
   T* pslp[6];
@@ -1083,7 +1083,7 @@ __device__ __forceinline__ void finalize_warp(const FinalizeParams& F) {
 // warps copy an item's parameters to shared memory.
 template <typename T, int BANK> struct MemberBank { StageParams<T> m[BANK]; };
 
-template <typename T, int MINB, int P2, bool EXTRA, int BANK>
+template <typename T, int MINB, bool P2, bool EXTRA, int BANK>
 __global__ void __launch_bounds__(32 * kPersistWarps, MINB)
     persist_batch_kernel(const __grid_constant__ PersistParams<T> PP, const __grid_constant__ MemberBank<T, BANK> bank) {
   __shared__ __align__(16) StageParams<T> Psh[BANK > 1 ? 1 : kPersistWarps];
@@ -1162,7 +1162,7 @@ __global__ void __launch_bounds__(32 * kPersistWarps, MINB)
       const int pk = uniform(pick), st = uniform(s);
       if constexpr (BANK > 1) {
         const StageParams<T>& SP = bank.m[pk];
-        member_strip<T, P2, EXTRA, false, true>(SP, st, SP.strips[item], sm);
+        sweep_strip<T, P2, EXTRA, false, true>(SP, st, SP.strips[item], sm);
       } else {
         static_assert(sizeof(StageParams<T>) % 4 == 0, "parameter block copied as 32-bit words");
         const unsigned* src = reinterpret_cast<const unsigned*>(PP.Ps + pk);
@@ -1170,7 +1170,7 @@ __global__ void __launch_bounds__(32 * kPersistWarps, MINB)
         for (int i = lane; i < int(sizeof(StageParams<T>) / 4); i += 32) dst[i] = src[i];
         __syncwarp();
         const StageParams<T>& SP = Psh[wib];
-        member_strip<T, P2, EXTRA, false, true>(SP, st, SP.strips[item], sm);
+        sweep_strip<T, P2, EXTRA, false, true>(SP, st, SP.strips[item], sm);
       }
       __syncwarp();
     } else {

@@ -55,17 +55,39 @@ inline bool variant_is_split(int v) { return v == kSplitVariant; }
 inline long long strip_count(long long nx, long long ny, int rows) {
   return ((nx + kSweepOut - 1) / kSweepOut) * ((ny + rows - 1) / rows);
 }
-// Strip height by mesh size: the tallest of 32, 16, 8 and 4 rows that still gives every SM its
-// 16 resident warps, else 4. A strip marches its rows one after another, so a mesh of few strips
-// waits for one warp's latency (2.0-3.3 us a row); a short strip repeats more of its neighbours'
-// rows. Per FP64 stage on B200, 32 / 16 / 8 / 4 rows: 117 / 64 / 38 / 27 us at 256 x 256,
-// 149 / 93 / 91 / 97 us at 1024 x 1024, 923 / 955 / 1059 / 1293 us at 4096 x 4096; FP32: 54 / 32 /
-// 22 / 17, 60 / 41 / 45 / 54, 445 / 485 / 581 / 793 us.
-constexpr long long kFillStrips = 148 * 16;
-inline int auto_rows(long long nx, long long ny) {
-  for (int rows = 32; rows > 4; rows /= 2)
-    if (strip_count(nx, ny, rows) >= kFillStrips) return rows;
-  return 4;
+// Strips that are resident at once with one warp per scheduler: 148 SMs, 4-warp blocks.
+constexpr long long kWaveStrips = 148 * 4;
+constexpr long long kFillStrips = 4 * kWaveStrips;
+// Strip height by mesh size, for variant 5. A strip marches its rows one after another, so a mesh
+// of few strips waits for single warps (FP64 3.7 us a row, FP32 1.6); a short strip repeats more
+// of its neighbours' rows; and a few strips more than are resident at once take a further wave.
+// The height with the smallest estimate is taken: rows + 3 times the waves `x` of strips, where
+// part of a wave is quicker a row than a full one, and a last wave that is nearly empty costs up
+// to 0.3 of one in the first waves and less the more there are (strips of unequal duration fill
+// in). Constants fitted to stage times of 4 to 64 rows on meshes of 0.3 to 17M cells; the choice
+// is within 7 % of the best height on each. Microseconds per stage on B200, the tallest of 32, 16,
+// 8 and 4 rows that fills the SMs / this choice: FP64 73 (8 rows) / 66 (10) at 900 x 700, 109 (16) /
+// 98 (9) at 1100 x 1001, 311 (32) / 288 (34) at 2048 x 2048, 974 (32) / 945 (44) at 4096 x 4096; FP32
+// 38 (8) / 31 (7) at 900 x 700, 130 (32) / 120 (43) at 2048 x 2048, 406 / 406 at 4096 x 4096; with
+// every source term FP32 88 (16) / 62 (17) at 1200 x 900, FP64 65 (4) / 58 (6) at 601 x 433.
+template <typename T> inline int auto_rows(long long nx, long long ny, bool extra) {
+  constexpr bool F64 = sizeof(T) == 8;
+  const double resident = double(kWaveStrips) * (extra ? kExtraCap<T> : F64 ? 4 : 6);
+  int best = 4;
+  double least = 0.0;
+  for (int rows = 4; rows <= 44; ++rows) {
+    const double x = double(strip_count(nx, ny, rows)) / resident;
+    double waves;
+    if (x <= 1.0) {
+      waves = extra ? 0.7 + 0.3 * x : F64 ? 0.88 + 0.3 * x : 0.6 + 0.4 * x;
+    } else {
+      const double y = 1.02 * x;
+      waves = x + 0.3 * (1.0 - (y - std::floor(y))) / std::floor(y);
+    }
+    const double cost = (rows + 3) * waves;
+    if (rows == 4 || cost < least) { best = rows; least = cost; }
+  }
+  return best;
 }
 // Whether variant 5 runs the row-tile kernel on a mesh: while its blocks (12 warps; one resident per
 // SM in FP64, two in FP32) take about two rounds. Per stage on B200, row tiles against 4-row
@@ -74,28 +96,28 @@ inline int auto_rows(long long nx, long long ny) {
 template <typename T> inline bool prefers_tile_rows(long long nx, long long ny) {
   return strip_count(nx, ny, kTileRows) <= (sizeof(T) == 8 ? 330 : 660);
 }
-// column-sweep variants: output rows per strip on a mesh (0 for the other variants)
-inline int variant_sweep_rows(int v, long long nx, long long ny) {
-  if (v == kAutoVariant) return auto_rows(nx, ny);
-  return variant_is_sweep(v) ? kSweeps[v].rows : 0;
-}
 // register caps compiled: FP64 3 and 4 blocks per SM, FP32 4 to 7 (tighter ones spill: FP64 stages at 4096 x 4096
 // 1.3 ms at 5 blocks against 0.92 at 4, FP32 455 us at 8 against 408 at 6)
 template <typename T> inline int clamp_cap(int cap) {
   const int lo = sizeof(T) == 8 ? 3 : 4, hi = sizeof(T) == 8 ? 4 : 7;
   return cap < lo ? lo : (cap > hi ? hi : cap);
 }
-// FP32, variant 5: 4 blocks per SM while all strips are resident at once (each warp then runs
-// fastest), else 6: 43 against 70 us a stage at 1024 x 1024, 445 against 408 at 4096 x 4096
+// FP32, variant 5: the fewest blocks per SM, from 4, with which all strips are resident at once
+// (each warp then runs fastest), else 6: at 900 x 700 and 8 rows (4.9 warps per scheduler) 38, 30 and 31
+// us at 4, 5 and 6 blocks per SM; at 10 rows (3.9) 32, 33 and 34; 445 against 408 at 4096 x 4096 at 4 and 6
 template <typename T> inline int variant_cap(int v, long long strips) {
-  if (v == kAutoVariant && sizeof(T) == 4) return strips <= kFillStrips + kFillStrips / 4 ? 4 : 6;
+  if (v == kAutoVariant && sizeof(T) == 4) return strips <= kFillStrips ? 4 : strips <= 5 * kWaveStrips ? 5 : 6;
   return clamp_cap<T>(kSweeps[v].cap);
 }
-// per-CTA (tiled) or per-warp (sweep) partial count
-inline long long variant_partials(int v, long long nx, long long ny) {
+// FP64: whether interior strips run the form without edge tests. It is the faster one (10 % at
+// 4096 x 4096), but while all strips are resident at once the SMs that hold both kinds evict one code
+// with the other from the instruction cache: 66 us with one form against 75 with two at 900 x 700 and 10 rows,
+// 40 against 45 at 600 x 500 and 5 rows; from 1.2 waves on two forms are as fast or faster.
+inline bool splits_forms(long long strips) { return strips > kFillStrips; }
+// per-CTA partial count of the tiled variants
+inline long long tiled_partials(int v, long long nx, long long ny) {
   if (v == kSplitVariant) v = 1;  // the split schedule's stage pass is the tiled 32 x 8 kernel
-  if (v < 4) return ((nx + kTiles[v].tx - 1) / kTiles[v].tx) * ((ny + kTiles[v].ty - 1) / kTiles[v].ty);
-  return strip_count(nx, ny, variant_sweep_rows(v, nx, ny));
+  return ((nx + kTiles[v].tx - 1) / kTiles[v].tx) * ((ny + kTiles[v].ty - 1) / kTiles[v].ty);
 }
 // a column-sweep variant with the shape of a lower one (the autotuner skips it)
 template <typename T> inline bool variant_repeats(int v) {
@@ -129,13 +151,13 @@ template <typename T> cudaError_t launch_volume(const T* h, int nx, int ny, doub
 template <typename T> cudaError_t launch_debug(const StageParams<T>& P, const DebugParams<T>& D, T* nh, T* sf,
                                                cudaStream_t s);
 // stage `st` of every one of n solvers (host array Ps) in one launch per kBatchMembers of them;
-// p2: kP2None, kP2All or kP2Some, extra when any solver needs it
+// p2 when every solver's dx and dy are powers of two, extra when any solver needs it
 constexpr int kBatchVariant = 8;
-template <typename T> cudaError_t launch_sweep_batch(const StageParams<T>* Ps, int n, int st, int p2, bool extra,
+template <typename T> cudaError_t launch_sweep_batch(const StageParams<T>* Ps, int n, int st, bool p2, bool extra,
                                                      cudaStream_t s);
 // persistent batch kernel (persist_batch_kernel), cooperative launch filling the device; Ps: the
 // members' parameters on the host (PP.Ps: the same on the device)
-template <typename T> cudaError_t launch_persist(const PersistParams<T>& PP, const StageParams<T>* Ps, int p2,
+template <typename T> cudaError_t launch_persist(const PersistParams<T>& PP, const StageParams<T>* Ps, bool p2,
                                                  bool extra, cudaStream_t s);
 cudaError_t launch_persist_init(const FinalizeParams* Fs, PersistMember* mem, const long long* warp_start, int nact,
                                 cudaStream_t s);

@@ -395,6 +395,11 @@ __device__ __forceinline__ double flip_sign(double x, double s) {
 // faster, but a velocity reconstructed across a full one-sided slope is then an exact zero where
 // the quotients leave a rounding error, and a face whose velocity is an exact zero has no
 // upwinding at all: results would move by 1e-4 of the velocity at a dam break's first timesteps.
+// For the same reason FP32 rounds the products of face_pair and friction by themselves there. With
+// power-of-two cells (StageParams::p2) the quotient form fuses them like the undivided one and, its
+// scalings being exact, gives the same bits: a batch of both kinds runs the quotient form for all,
+// and every member keeps its solo run's bits (both forms compiled into one kernel evicted each
+// other from the instruction cache: 62 against 51 ms for 16 catchments in the persistent kernel).
 template <typename T, bool P2> struct MeshOps {
   static constexpr bool SCALED = P2;
   const MeshConst<T>& mc;
@@ -423,9 +428,9 @@ template <typename T, bool P2> struct MeshOps {
 template <typename T> struct FaceG { T h, n, t, z; };
 
 // The doubled fluxes of a face from its two sides (FluxKernel.cpp:189-291); dv(x) is x / (2 d).
-// STRICT: products rounded by themselves (the same thing in FP64).
-template <typename T, bool STRICT, typename DV>
-__device__ __forceinline__ FaceG<T> face_pair(const Side<T>& m, const Side<T>& p, const DV& dv) {
+// strict: products rounded by themselves (the same thing in FP64).
+template <typename T, typename DV>
+__device__ __forceinline__ FaceG<T> face_pair(const Side<T>& m, const Side<T>& p, const DV& dv, bool strict) {
   const T g = T(kG);
   const bool rise = p.zb > m.zb;
   const T zf = rise ? p.zb : m.zb;
@@ -452,7 +457,7 @@ __device__ __forceinline__ FaceG<T> face_pair(const Side<T>& m, const Side<T>& p
   const T a = pick_max(a_p, a_m);
   const T nm = mad_(um, T(0.5) * um, gm);
   const T np = mad_(up, T(0.5) * up, am ? -gp : gp);
-  if constexpr (STRICT) {
+  if (sizeof(T) == 4 && strict) {
     G.h = (hp * up + hm * um) - a * (hp - hm);
     G.n = (np + nm) - a * (up - um);
     G.t = (tp * up + tm * um) - a * (tp - tm);
@@ -473,9 +478,8 @@ template <typename T> __device__ __forceinline__ T manning_n(T h, T ns, T nd, T 
   const T ss = t * t * (T(3) - T(2) * t);
   return ns + (nd - ns) * ss;
 }
-template <bool>
 __device__ __forceinline__ void friction(double h, double u, double v, double n, double dt, double, double& du,
-                                         double& dv) {
+                                         double& dv, bool) {
   const double sf = n * n * ssqrt(u * u + v * v) * pow43_(manning_inv_h(h));
   double fu = -kG * sf * u, fv = -kG * sf * v;
   if (fabs(fu * dt) > fabs(u)) fu = -div_slow(u, dt);
@@ -483,9 +487,9 @@ __device__ __forceinline__ void friction(double h, double u, double v, double n,
   du = du + fu;
   dv = dv + fv;
 }
-template <bool STRICT>
-__device__ __forceinline__ void friction(float h, float u, float v, float n, float dt, float rdt, float& du, float& dv) {
-  if constexpr (STRICT) {
+__device__ __forceinline__ void friction(float h, float u, float v, float n, float dt, float rdt, float& du, float& dv,
+                                         bool strict) {
+  if (strict) {
     const float sf = n * n * ssqrt(mad_(u, u, v * v)) * pow43_(manning_inv_h(h));
     float fu = -float(kG) * sf * u, fv = -float(kG) * sf * v;
     if (fabsf(fu * dt) > fabsf(u)) fu = -u * rdt;
@@ -569,7 +573,7 @@ __device__ __forceinline__ void lean_cell(const StageParams<T>& P, int st, int c
     if (ns != nd)
       n = manning_n<T>(h, ns, nd, P.man_p[2] ? ld(P.man_p[2], g) : P.man_s[2],
                        P.man_p[3] ? ld(P.man_p[3], g) : P.man_s[3]);
-    friction<!P2>(h, u, v, n, k.dt, k.rdt, du, dv);
+    friction(h, u, v, n, k.dt, k.rdt, du, dv, !P2 && !P.p2);
   };
   if constexpr (!EXTRA) {
     roughness();
@@ -915,7 +919,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
       const int row = k - 1;
       const bool yedge = EDGE && (row <= 0 || row >= ny - 1);
       auto yslope = [&](T a, T b, T lo, T hi, T& j, T& s) {
-        T hs = half_slope(a, b, F32 && SCALED ? a + b : mo.diff_y(hi - lo));
+        T hs = half_slope(a, b, F32 ? a + b : mo.diff_y(hi - lo));
         if (yedge) {  // one-sided: the slope is the present quotient
           if (row >= ny - 1) hs = T(0.5) * a;
           if (row <= 0) hs = ny > 1 ? T(0.5) * b : T(0);
@@ -931,7 +935,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
         const T e = dn1(x);
         const T b = mo.diff_x(e - x), a = up1(b);
         T cc;
-        if constexpr (F32 && SCALED) cc = a + b;
+        if constexpr (F32) cc = a + b;
         else cc = mo.diff_x(e - up1(x));
         T hs = half_slope(a, b, cc);
         if (xedge) {
@@ -963,7 +967,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
         if (fy == 0) m = {R0.z + R0.h * T(2), T(0), T(0), mo.side_y(R0.u, -J0.uy)};
         if (fy == ny) p = {Rm.z + Rm.h * T(2), T(0), T(0), mo.side_y(Rm.u, Jm.uy)};
       }
-      GN = face_pair<T, !P2>(m, p, [&](T x) { return mo.over_2dy(x); });
+      GN = face_pair<T>(m, p, [&](T x) { return mo.over_2dy(x); }, !P2 && !P.p2);
     }
     // output row k-2
     if (k >= y0 + 2) {
@@ -997,7 +1001,7 @@ __device__ __forceinline__ int sweep_rows(const StageParams<T>& P, int st, int t
         if (gx == 0) m = {wall, T(0), T(0), eut};
         if (gx == nx) p = {wl, T(0), T(0), utl};
       }
-      const FaceG<T> W = face_pair<T, !P2>(m, p, [&](T x) { return mo.over_2dx(x); });
+      const FaceG<T> W = face_pair<T>(m, p, [&](T x) { return mo.over_2dx(x); }, !P2 && !P.p2);
       const FaceG<T> E{dn1(W.h), dn1(W.n), dn1(W.t), dn1(W.z)};
       EddyIn<T> ed{};
       if constexpr (EXTRA) {
@@ -1064,11 +1068,6 @@ __device__ __forceinline__ void store_strip_sums(const StageParams<T>& P, int st
   }
 }
 
-// The members of a batch: none (0), all (1) or some (2) have cell sizes that are powers of two.
-// FP32 rounds differently in the two forms, so a member keeps the form of its solo run; in FP64
-// both give the same bits and 2 is not compiled.
-inline constexpr int kP2None = 0, kP2All = 1, kP2Some = 2;
-
 // One strip of one solver's stage: its class's sweep, then its partial sums. `entry` is the
 // strip's index (row-major over strips of kSweepOut columns x P.rows rows) times 4 plus its
 // class. SPLIT: interior strips run the form without edge tests.
@@ -1090,17 +1089,6 @@ __device__ __forceinline__ void sweep_strip(const StageParams<T>& P, int st, uns
     acc = rest;
   }
   store_strip_sums(P, st, gw, acc);
-}
-// sweep_strip of a batch member
-template <typename T, int P2, bool EXTRA, bool SPLIT, bool COH>
-__device__ __forceinline__ void member_strip(const StageParams<T>& P, int st, unsigned entry, SweepShared<T>& sm) {
-  if constexpr (P2 != kP2None) {
-    if (P2 == kP2All || P.p2) {
-      sweep_strip<T, true, EXTRA, SPLIT, COH>(P, st, entry, sm);
-      return;
-    }
-  }
-  if constexpr (P2 != kP2All) sweep_strip<T, false, EXTRA, SPLIT, COH>(P, st, entry, sm);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1186,7 +1174,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 8 ? 1 : 2)
     auto yslope = [&](int f, T x, T& j, T& s) {
       const T lo = val[f][w - 1][lane], hi = val[f][w + 1][lane];
       const T a = mo.diff_y(x - lo), b = mo.diff_y(hi - x);
-      T hs = half_slope(a, b, F32 && SCALED ? a + b : mo.diff_y(hi - lo));
+      T hs = half_slope(a, b, F32 ? a + b : mo.diff_y(hi - lo));
       if (row >= ny - 1) hs = T(0.5) * a;
       if (row <= 0) hs = ny > 1 ? T(0.5) * b : T(0);
       j = mo.jump_y(hs);
@@ -1198,7 +1186,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 8 ? 1 : 2)
     auto xslope = [&](T x, T& j, T& s) {
       const T e = dn1(x), b = mo.diff_x(e - x), a = up1(b);
       T cc;
-      if constexpr (F32 && SCALED) cc = a + b;
+      if constexpr (F32) cc = a + b;
       else cc = mo.diff_x(e - up1(x));
       T hs = half_slope(a, b, cc);
       if (gx >= nx - 1) hs = T(0.5) * a;
@@ -1231,7 +1219,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 8 ? 1 : 2)
     // walls at the mesh edge, FluxKernel.cpp:111-157 (rows past it hold the edge row's values)
     if (row == 0) m = {R.z + R.h * T(2), T(0), T(0), mo.side_y(R.u, -J.uy)};
     if (row == ny) p = {R.z + R.h * T(2), T(0), T(0), upper[4][w - 1][lane]};
-    GS = face_pair<T, !P2>(m, p, [&](T x) { return mo.over_2dy(x); });
+    GS = face_pair<T>(m, p, [&](T x) { return mo.over_2dy(x); }, !P2 && !P.p2);
     face[0][w][lane] = GS.h; face[1][w][lane] = GS.n; face[2][w][lane] = GS.t; face[3][w][lane] = GS.z;
   }
   FaceG<T> W{};
@@ -1250,7 +1238,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 8 ? 1 : 2)
     const T wl = up1(wall), utl = up1(p.ut);
     if (gx == 0) m = {wall, T(0), T(0), eut};
     if (gx == nx) p = {wl, T(0), T(0), utl};
-    W = face_pair<T, !P2>(m, p, [&](T x) { return mo.over_2dx(x); });
+    W = face_pair<T>(m, p, [&](T x) { return mo.over_2dx(x); }, !P2 && !P.p2);
   }
   __syncthreads();
   if (out_row) {
@@ -1298,7 +1286,7 @@ constexpr int kSweepWarps = 4;  // warps (strips) per block
 
 // The strips listed in P.strips (general and edge strips first: they take longer, so they do
 // not end up as the launch's tail).
-template <typename T, int MINB, bool P2, bool EXTRA>
+template <typename T, int MINB, bool P2, bool EXTRA, bool SPLIT>
 __global__ void __launch_bounds__(32 * kSweepWarps, MINB)
     sweep_kernel(const __grid_constant__ StageParams<T> P, const int st) {
   extern __shared__ __align__(16) unsigned char sweep_smem[];
@@ -1306,7 +1294,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, MINB)
   if (P.ctl->done) return;
   const int w = uniform(threadIdx.y), i = int(blockIdx.x) * kSweepWarps + w;
   if (i >= P.n_strips) return;  // whole warp: no block-level synchronisation below
-  sweep_strip<T, P2, EXTRA, !EXTRA, false>(P, st, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[w]);
+  sweep_strip<T, P2, EXTRA, SPLIT, false>(P, st, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[w]);
 }
 
 // Batched column sweep: the strips of up to kBatchMembers solvers in one launch. Their parameters
@@ -1321,7 +1309,7 @@ template <typename T> struct BatchParams {
 };
 static_assert(sizeof(BatchParams<double>) <= 32764 && sizeof(BatchParams<float>) <= 32764, "kernel parameters");
 
-template <typename T, int MINB, int P2, bool EXTRA>
+template <typename T, int MINB, bool P2, bool EXTRA>
 __global__ void __launch_bounds__(32 * kSweepWarps, MINB)
     sweep_batch_kernel(const __grid_constant__ BatchParams<T> B, const int st) {
   extern __shared__ __align__(16) unsigned char sweep_smem[];
@@ -1333,7 +1321,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps, MINB)
   if (P.ctl->done) return;
   const int w = uniform(threadIdx.y), i = (int(blockIdx.x) - B.first_block[k]) * kSweepWarps + w;
   if (i >= P.n_strips) return;
-  member_strip<T, P2, EXTRA, !EXTRA, false>(P, st, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[w]);
+  sweep_strip<T, P2, EXTRA, !EXTRA, false>(P, st, P.strips[i], reinterpret_cast<SweepShared<T>*>(sweep_smem)[w]);
 }
 
 }  // namespace svk

@@ -47,8 +47,9 @@ def test_row_tiles(shape, dx, nan_cells):
         assert out[0][0] == out[1][0]
 
 
-# rows chosen by the size rule in FP64: 4 just above the row tiles' sizes, then 8, 16 and 32; up to
-# 2048 strips are reduced by one block, more by a cluster
+# heights of the size rule in FP64: 4 just above the row tiles' sizes, then 9, 9 and 18; all strips
+# resident at once (one form of the sweep) and several waves of them (two forms); up to 2048 strips
+# reduced by one block, more by a cluster
 @pytest.mark.parametrize("shape", [(300, 280), (800, 701), (1100, 1001), (1500, 1450)])
 def test_strip_heights_of_the_size_rule(shape):
     nx, ny = shape
