@@ -247,15 +247,15 @@ int sv_run_timesteps(sv_ctx* ctx, uint64_t max_timesteps, int begin, sv_stats* o
                      sv_timing* timing);
 /* Stage-kernel variant (no reference counterpart: a launch-shape and schedule choice of this
  * library). Fused schedule, one pass per RK stage: 0-3 tiled shared-memory kernel (32x8, 32x8
- * at 3 CTAs/SM, 32x4 at 4 CTAs/SM, 64x4 at 3 CTAs/SM), 4-10 column-sweep kernel (16/32/64 rows
- * per warp, then 32 rows capped for 3, 4, 5 and 6 CTAs/SM; strips away from the mesh edge and
- * from coded-out cells run an interior form of it), 12-13 (FP32 solvers only) the 32-row
- * column sweep whose pairs of adjacent interior strips run two cells per lane with 8-byte
- * loads (capped for 3 and 4 CTAs/SM; meshes with an odd row length have no pairs), 14-15
- * (FP32 solvers only) the one-cell 32-row sweep capped for 7 and 8 CTAs/SM. Split
+ * at 3 CTAs/SM, 32x4 at 4 CTAs/SM, 64x4 at 3 CTAs/SM), 4-10 column-sweep kernel: 4 strips of 16
+ * rows, 6 of 64 rows, 7-10 of 32 rows capped for 3, 4, 5 and 6 CTAs/SM, and 5 (the default) chosen
+ * by the mesh's size: a kernel with one warp per row on small meshes, else the strip height and
+ * cap that fill the GPU. 12-15 (FP32 solvers only) 32-row sweeps capped for 3, 4, 7 and 8
+ * CTAs/SM. A cap outside the compiled ones (3-4 in FP64, 4-7 in FP32) runs the nearest. Split
  * schedule, two passes per RK stage: 11 a slopes pass, then the tiled 32x8 kernel reading
- * those slopes. Every variant computes bit-identical FP64 results; FP32 results are
- * reproducible per variant. SV_F32_DATUM64 solvers take the column-sweep variants only. */
+ * those slopes. Every variant computes bit-identical FP64 results; in FP32 the column-sweep
+ * variants give one another's bits, the tiled ones round in their own way. SV_F32_DATUM64
+ * solvers take the column-sweep variants only. */
 int sv_set_kernel_variant(sv_ctx* ctx, int variant);
 int sv_get_kernel_variant(sv_ctx* ctx, int* variant);
 /* Autotune: times every variant's stage kernel (both schedules) on the current state and keeps
@@ -267,7 +267,7 @@ int sv_get_autotune_ms(sv_ctx* ctx, float* ms, int n);
 
 /* ---- batches of independent catchments (no reference counterpart: the reference runs one
  *      catchment per process). Members are ordinary sv_ctx solvers; per timestep one batched
- *      launch per RK stage covers every member's tiles and one batched launch runs every
+ *      launch per RK stage covers every member's strips (one per 32 members) and one runs every
  *      member's reductions and dt controller, so each member keeps its own dt, step clock and
  *      tallies and its results are bit-identical to running it alone. All members share the
  *      batch's precision and a tableau whose stages use only the previous stage. ---------- */
@@ -318,17 +318,16 @@ int sv_batch_status(sv_batch* batch, int* status, int n);
 /* Persistent mode (no reference counterpart; the reference advances one catchment per
  * process, TemporalScheme.hpp:112-149): each sv_batch_advance / sv_batch_advance_steps runs as
  * ONE cooperative launch that fills the device. Every member advances through its queued
- * steps at its own dt; a member's timestep is its stage phases (column-sweep strips, 32 rows)
- * and a finalize phase (reductions, dt controller, step queue), and idle warps take work from
+ * steps at its own dt; a member's timestep is its stage phases (column-sweep strips) and a finalize phase (reductions, dt controller, step queue), and idle warps take work from
  * whichever member has some. on = 0 returns to one launch per stage. Two bounds end a launch
  * with SV_E_TIMEOUT: spin_limit polls of a waiting warp during which no warp completes a work
  * item (0: the default, 2^22 polls, about a second), and max_seconds of wall clock for the
  * whole launch (<= 0: the default, 120 s; queue fewer steps per call for longer runs). After a
- * timeout every member keeps the state of its last completed timestep. FP64 results are bit
- * for bit those of the other modes; FP32 results are reproducible for this mode. */
+ * timeout every member keeps the state of its last completed timestep. Results are bit for bit
+ * those of the other modes. */
 int sv_batch_set_persistent(sv_batch* batch, int on, uint64_t spin_limit, double max_seconds);
-/* the stage-kernel variant every member of the batch runs (FP32 results are reproducible
- * per variant: a solo run with this variant gives a member's bits) */
+/* the stage-kernel variant every member of the batch runs: a solo run with this variant gives a
+ * member's bits */
 int sv_batch_kernel_variant(sv_batch* batch, int* variant);
 /* number of members and their total device memory in bytes */
 int sv_batch_size(sv_batch* batch, int* n_members, uint64_t* device_bytes);
