@@ -102,7 +102,7 @@ constexpr int kRingBytes = kSweepWarps * int(sizeof(SweepShared<SV_T>));
 
 // The column sweep of a stage: the strips in P.strips, P.rows rows each. `cap`: resident blocks
 // per SM asked of the register allocator.
-template <int MINB, bool EXTRA, bool SPLIT = !EXTRA>
+template <int MINB, bool EXTRA, bool SPLIT>
 static cudaError_t launch_sweep_c(const StageParams<SV_T>& P, int st, cudaStream_t s) {
   if (P.n_strips <= 0) return cudaSuccess;
   const dim3 grid(unsigned((P.n_strips + kSweepWarps - 1) / kSweepWarps)), block(32, kSweepWarps);
@@ -111,16 +111,20 @@ static cudaError_t launch_sweep_c(const StageParams<SV_T>& P, int st, cudaStream
   return launch_chained<sweep_kernel<SV_T, MINB, false, EXTRA, SPLIT>>(grid, block, kRingBytes, s, P, st);
 }
 static cudaError_t launch_sweep(const StageParams<SV_T>& P, int st, int cap, bool extra, cudaStream_t s) {
-  if (extra) return launch_sweep_c<kExtraCap<SV_T>, true>(P, st, s);
+  const bool split = splits_forms<SV_T>(P.n_strips, extra);
   if constexpr (sizeof(SV_T) == 8) {
-    if (cap == 3) return launch_sweep_c<3, false>(P, st, s);
-    return splits_forms(P.n_strips) ? launch_sweep_c<4, false>(P, st, s) : launch_sweep_c<4, false, false>(P, st, s);
+    if (extra) return launch_sweep_c<kExtraCap<SV_T>, true, false>(P, st, s);
+    if (cap == 3) return launch_sweep_c<3, false, true>(P, st, s);
+    return split ? launch_sweep_c<4, false, true>(P, st, s) : launch_sweep_c<4, false, false>(P, st, s);
   } else {
+    if (extra)
+      return split ? launch_sweep_c<kExtraCap<SV_T>, true, true>(P, st, s)
+                   : launch_sweep_c<kExtraCap<SV_T>, true, false>(P, st, s);
     switch (cap) {
-      case 4: return launch_sweep_c<4, false>(P, st, s);
-      case 5: return launch_sweep_c<5, false>(P, st, s);
-      case 6: return launch_sweep_c<6, false>(P, st, s);
-      default: return launch_sweep_c<7, false>(P, st, s);
+      case 4: return launch_sweep_c<4, false, true>(P, st, s);
+      case 5: return launch_sweep_c<5, false, true>(P, st, s);
+      case 6: return launch_sweep_c<6, false, true>(P, st, s);
+      default: return launch_sweep_c<7, false, true>(P, st, s);
     }
   }
 }
@@ -174,7 +178,7 @@ template <> cudaError_t launch_to_f64<SV_T>(const SV_T* src, double* dst, long l
 }
 
 template <bool EXTRA> static cudaError_t launch_batch_chunk(const BatchParams<SV_T>& B, int st, bool p2, cudaStream_t s) {
-  constexpr int CAP = EXTRA ? kExtraCap<SV_T> : kBatchCap<SV_T>;
+  constexpr int CAP = EXTRA ? kBatchExtraCap<SV_T> : kBatchCap<SV_T>;
   const dim3 block(32, kSweepWarps), grid(unsigned(B.first_block[B.n]));
   if (grid.x == 0) return cudaSuccess;
   if (p2) return launch_chained<sweep_batch_kernel<SV_T, CAP, true, EXTRA>>(grid, block, kRingBytes, s, B, st);
@@ -202,7 +206,7 @@ template <> cudaError_t launch_sweep_batch<SV_T>(const StageParams<SV_T>* Ps, in
 template <int BANK>
 static cudaError_t launch_persist_t(const PersistParams<SV_T>& PP, const StageParams<SV_T>* Ps, bool p2, bool extra,
                                     cudaStream_t s) {
-  constexpr int CAP = kBatchCap<SV_T>, XCAP = kExtraCap<SV_T>;
+  constexpr int CAP = kBatchCap<SV_T>, XCAP = kBatchExtraCap<SV_T>;
   void (*kern)(const PersistParams<SV_T>, const MemberBank<SV_T, BANK>) =
       extra ? (p2 ? persist_batch_kernel<SV_T, XCAP, true, true, BANK> : persist_batch_kernel<SV_T, XCAP, false, true, BANK>)
             : (p2 ? persist_batch_kernel<SV_T, CAP, true, false, BANK> : persist_batch_kernel<SV_T, CAP, false, false, BANK>);

@@ -44,9 +44,12 @@ inline bool pow2_mesh(double dx, double dy) {
   int e;
   return std::frexp(dx, &e) == 0.5 && std::frexp(dy, &e) == 0.5;
 }
-// resident blocks per SM of the batch kernels, and of the sweeps with every source term
+// resident blocks per SM of the batch kernels, and of the sweeps with every source term: FP32 at 4 and 5 blocks
+// 526 and 457 us a stage at 3000 x 3000 with all terms (408 with two forms, splits_forms); FP64 at
+// 3 and 4, which spills, 571 and 816 at 2048 x 2048
 template <typename T> constexpr int kBatchCap = sizeof(T) == 8 ? 4 : 6;
-template <typename T> constexpr int kExtraCap = sizeof(T) == 8 ? 3 : 4;
+template <typename T> constexpr int kBatchExtraCap = sizeof(T) == 8 ? 3 : 4;
+template <typename T> constexpr int kExtraCap = sizeof(T) == 8 ? 3 : 5;
 // variants compiled for FP32 solvers only
 inline bool variant_is_fp32_only(int v) { return v >= 12 && v <= 15; }
 inline bool variant_is_sweep(int v) { return v >= 0 && v < kNumVariants && kSweeps[v].rows > 0; }
@@ -69,7 +72,7 @@ constexpr long long kFillStrips = 4 * kWaveStrips;
 // 8 and 4 rows that fills the SMs / this choice: FP64 73 (8 rows) / 66 (10) at 900 x 700, 109 (16) /
 // 98 (9) at 1100 x 1001, 311 (32) / 288 (34) at 2048 x 2048, 974 (32) / 945 (44) at 4096 x 4096; FP32
 // 38 (8) / 31 (7) at 900 x 700, 130 (32) / 120 (43) at 2048 x 2048, 406 / 406 at 4096 x 4096; with
-// every source term FP32 88 (16) / 62 (17) at 1200 x 900, FP64 65 (4) / 58 (6) at 601 x 433.
+// every source term FP32 64 (16) / 58 (14) at 1200 x 900, FP64 65 (4) / 58 (6) at 601 x 433.
 template <typename T> inline int auto_rows(long long nx, long long ny, bool extra) {
   constexpr bool F64 = sizeof(T) == 8;
   const double resident = double(kWaveStrips) * (extra ? kExtraCap<T> : F64 ? 4 : 6);
@@ -109,11 +112,16 @@ template <typename T> inline int variant_cap(int v, long long strips) {
   if (v == kAutoVariant && sizeof(T) == 4) return strips <= kFillStrips ? 4 : strips <= 5 * kWaveStrips ? 5 : 6;
   return clamp_cap<T>(kSweeps[v].cap);
 }
-// FP64: whether interior strips run the form without edge tests. It is the faster one (10 % at
-// 4096 x 4096), but while all strips are resident at once the SMs that hold both kinds evict one code
-// with the other from the instruction cache: 66 us with one form against 75 with two at 900 x 700 and 10 rows,
-// 40 against 45 at 600 x 500 and 5 rows; from 1.2 waves on two forms are as fast or faster.
-inline bool splits_forms(long long strips) { return strips > kFillStrips; }
+// Whether interior strips run the form without edge tests. It is the faster one (FP64 10 % at
+// 4096 x 4096, FP32 with every source term 11 % at 3000 x 3000), but while all strips are resident at
+// once the SMs that hold both kinds evict one code with the other from the instruction cache: FP64 66 us
+// with one form against 75 with two at 900 x 700 and 10 rows, 40 against 45 at 600 x 500 and 5 rows,
+// FP32 with eddy viscosity 58 against 64 at 1200 x 900 and 14 rows. The lean FP32 sweep is small
+// enough for two at any size; FP64 with every term is not at any (2 % either way).
+template <typename T> inline bool splits_forms(long long strips, bool extra) {
+  if (sizeof(T) == 8) return !extra && strips > kFillStrips;
+  return !extra || strips > kExtraCap<T> * kWaveStrips;
+}
 // per-CTA partial count of the tiled variants
 inline long long tiled_partials(int v, long long nx, long long ny) {
   if (v == kSplitVariant) v = 1;  // the split schedule's stage pass is the tiled 32 x 8 kernel
