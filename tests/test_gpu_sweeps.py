@@ -147,6 +147,32 @@ def test_fp32_kernels_round_alike(precision, dx, shape):
             assert_same(o[f], out[0][f], f"U_[N] field {f}")
 
 
+@pytest.mark.parametrize("dx", [2.0, 3.0])
+@pytest.mark.parametrize("shape", [(29, 9), (1500, 1100), (2100, 1800)])
+def test_fp32_sweeps_with_every_term_round_alike(dx, shape):
+    """Variant 5's height (all strips resident, then more than one wave: edge form only, then two
+    forms) against strips of 32 rows and of 64, which stay resident."""
+    nx, ny = shape
+    z, h, u, v = wet_dry_state(nx, ny, dx, seed=3)
+    rng = np.random.default_rng(2)
+    extra = {"ELOSS_FX": rng.uniform(0, 0.5, (ny, nx)), "ELOSS_FY": rng.uniform(0, 0.5, (ny, nx)),
+             "INFIL_RATE": rng.uniform(0, 2e-5, (ny, nx)), "INFIL_CAP": rng.uniform(0, 2e-4, (ny, nx))}
+    out = []
+    for variant in (5, 8, 6):
+        b = SaintVenantSolver(nx, ny, dx, precision="f32", rain_mode="physical")
+        b.set_kernel_variant(variant)
+        setup(b, z, h, u, v, n=(0.03, 0.06, 0.1, 0.3))
+        for name, a in extra.items():
+            b.set_field(name, a)
+        b.set_eddy_viscosity("smagorinsky")
+        b.set_forcing(forcing((2e-5, 1e-5), head=(0.01, 0.0), edges=EDGE_XMIN | EDGE_YMAX))
+        out.append(one_timestep(b)[1] + [b.get_field("INFIL_CAP")])
+        b.close()
+    for o in out[1:]:
+        for f in range(4):
+            assert_same(o[f], out[0][f], f"field {f}")
+
+
 @pytest.mark.parametrize("persistent", [False, True])
 @pytest.mark.parametrize("precision", ["f64", "f32", "f32_datum64"])
 @pytest.mark.parametrize("count", [3, 35])
